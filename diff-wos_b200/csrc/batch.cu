@@ -3,9 +3,8 @@
 // A plan holds many (scene, query set) items.  Items are grouped by
 // dimension, and within a group ordered by tree depth; each group runs its
 // phases (forward walks, per-point reduction, loss, adjoint) over the
-// concatenation of its items' walks: the walk phases as one persistent
-// work-queue launch per run of items of equal depth (each compiled for that
-// depth), the reductions as one launch per group.  The whole sequence is
+// concatenation of its items' walks, each as one launch per group, the walk
+// phases persistent over a work queue.  The whole sequence is
 // captured once into a CUDA graph that later runs replay with a single
 // launch.
 #include <algorithm>
@@ -20,9 +19,10 @@ namespace wosd {
 
 static size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Consecutive items of a group whose trees have the same depth.
+// Consecutive items of a group whose trees have the same depth (the slot tuner
+// times a sample of each).
 struct BatchRun {
-    int wl = 0;  // specialised_depth of the items' trees
+    int depth = 0;
     int first = 0, count = 0;
     long long base = 0, walks = 0;
 };
@@ -38,6 +38,7 @@ struct BatchGroup {
     std::vector<unsigned long long> gens;  // each scene's generation when `views` was read
     long long walks = 0;
     int points = 0;
+    int depth = 1;  // deepest tree
     bool has_src = false;
     long long acc_len = 0;  // doubles
     // device
@@ -134,21 +135,19 @@ static int enqueue(wos_batch_s *b, cudaStream_t st) {
         if (b->want_adjoint) BT(cudaMemsetAsync(g.acc, 0, sizeof(double) * g.acc_len, st));
         WalkOut o{g.vals, nullptr, b->want_adjoint ? g.wrec : nullptr, b->want_adjoint ? g.wds : nullptr,
                   nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        for (const BatchRun &r : g.runs)
-            if (int rc = launch_walk_batch(g.dim, r.wl, g.d_views + r.first, g.d_cfgs + r.first, g.d_items + r.first,
-                                           r.count, r.base, r.walks, b->slot[g.dim - 2][0], o, g.counters, st))
-                return rc;
+        if (int rc = launch_walk_batch(g.dim, g.depth, g.d_views, g.d_cfgs, g.d_items, n_items, 0, g.walks,
+                                       b->slot[g.dim - 2][0], o, g.counters, st))
+            return rc;
         if (int rc = launch_reduce_batch(g.vals, g.d_items, n_items, g.points, g.mean, g.var, st)) return rc;
         if (int rc = launch_loss_batch(g.mean, g.d_items, n_items, g.dLdu, g.loss, st)) return rc;
         if (b->want_adjoint) {
             if (int rc = launch_batch_order(g.dim, g.d_views, g.d_items, n_items, g.nkeys, g.wrec, g.walks,
                                             g.order_ws, g.order_bytes, &g.order, st))
                 return rc;
-            for (const BatchRun &r : g.runs)
-                if (int rc = launch_adjoint_batch(g.dim, r.wl, g.d_views + r.first, g.d_cfgs + r.first, a,
-                                                  g.d_items + r.first, r.count, r.base, r.walks, g.dLdu, g.wrec,
-                                                  g.wds, g.acc, b->slot[g.dim - 2][1], g.counters + 1, g.order, st))
-                    return rc;
+            if (int rc = launch_adjoint_batch(g.dim, g.depth, g.d_views, g.d_cfgs, a, g.d_items, n_items, 0, g.walks,
+                                              g.dLdu, g.wrec, g.wds, g.acc, b->slot[g.dim - 2][1], g.counters + 1,
+                                              g.order, st))
+                return rc;
             if (int rc = launch_acc_to_f32(g.acc, g.grad, g.acc_len, st)) return rc;
         }
     }
@@ -169,12 +168,12 @@ static int enqueue_slot(wos_batch_s *b, int dim, int phase, double frac, cudaStr
         for (const BatchRun &r : g.runs) {
             const long long w = std::max(1LL, std::min(r.walks, (long long)(frac * (double)r.walks)));
             if (phase == 0) {
-                if (int rc = launch_walk_batch(g.dim, r.wl, g.d_views + r.first, g.d_cfgs + r.first,
+                if (int rc = launch_walk_batch(g.dim, r.depth, g.d_views + r.first, g.d_cfgs + r.first,
                                                g.d_items + r.first, r.count, r.base, w, b->slot[dim - 2][0], o,
                                                g.counters, st))
                     return rc;
             } else if (b->want_adjoint) {
-                if (int rc = launch_adjoint_batch(g.dim, r.wl, g.d_views + r.first, g.d_cfgs + r.first, a,
+                if (int rc = launch_adjoint_batch(g.dim, r.depth, g.d_views + r.first, g.d_cfgs + r.first, a,
                                                   g.d_items + r.first, r.count, r.base, w, g.dLdu, g.wrec, g.wds,
                                                   g.acc, b->slot[dim - 2][1], g.counters + 1, g.order, st))
                     return rc;
@@ -227,10 +226,10 @@ int wos_batch_create(const wos_batch_item *items, int n_items, const wos_adjoint
             return fail(WOS_ERR_INVALID_ARGUMENT, "item " + std::to_string(i) + ": scene is NULL");
         }
     // within a dimension, items in order of tree depth (then caller order), so
-    // that each depth is one contiguous run of walks
+    // that each depth is one contiguous run of walks for the slot tuner's sample
     std::vector<int> order(n_items);
     for (int i = 0; i < n_items; ++i) order[i] = i;
-    auto depth = [&](int i) { return specialised_depth(items[i].scene->impl.wt_levels); };
+    auto depth = [&](int i) { return items[i].scene->impl.tree_depth; };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return depth(x) < depth(y); });
     for (int i : order) {
         const wos_batch_item &it = items[i];
@@ -260,10 +259,10 @@ int wos_batch_create(const wos_batch_item *items, int n_items, const wos_adjoint
         g.acc_len += 5;
         d.prim_off = g.nkeys;
         g.nkeys += (long long)S.nF + 1;
-        const int wl = specialised_depth(S.wt_levels);
-        if (g.runs.empty() || g.runs.back().wl != wl) {
+        g.depth = std::max(g.depth, S.tree_depth);
+        if (g.runs.empty() || g.runs.back().depth != S.tree_depth) {
             BatchRun r;
-            r.wl = wl;
+            r.depth = S.tree_depth;
             r.first = (int)g.items.size();
             r.base = g.walks;
             g.runs.push_back(r);

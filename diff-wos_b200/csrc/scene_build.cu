@@ -1,6 +1,6 @@
 // Scene construction on the GPU: vertex normals, scene AABB, primitive
 // precomputation and the LBVH (Morton codes, radix sort, Karras hierarchy,
-// bottom-up refit, breadth-first node order).
+// bottom-up refit, breadth-first node order) and the walk kernels' search tree.
 //
 // Replaces the reference's host Scene<N>::configure_normal / configure
 // (include/scene.cuh:368-453), which did the AABB on the host and the BVH in
@@ -406,59 +406,54 @@ __global__ void k_leaf_data(const unsigned long long *keys, int n, const float4 
     }
 }
 
-// Wide-tree leaf boxes.  Leaf i holds sorted positions [WT_LEAF i, WT_LEAF i
-// + WT_LEAF); its box is the union of its primitives' boxes and bounds it in
-// the level above.
+// Leaf blocks of the search tree (SceneView::prims) from the sorted primitives;
+// the last leaf repeats the last one (and its original index in lorig).
 template <int D>
-__global__ void k_wt_level1(const unsigned long long *keys, int nF, const float *pbox, float4 *out, int n1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n1) return;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    const int b0 = WT_LEAF * i, e = min(b0 + WT_LEAF, nF);
-    for (int s = b0; s < e; ++s) {
-        const float *b = pbox + (size_t)(unsigned)keys[s] * 2 * D;
-        for (int k = 0; k < D; ++k) {
-            lo[k] = fminf(lo[k], b[k]);
-            hi[k] = fmaxf(hi[k], b[D + k]);
-        }
-    }
+__global__ void k_tree_prims(int nF, int n_leaf, const float4 *lseg, const float *lseginv, const float4 *ltri,
+                             float4 *prims, int *lorig) {
+    constexpr int N = Tree<D>::LEAF, W = Tree<D>::LEAF_W;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n_leaf * N) return;
+    const int s = min(p, nF - 1), leaf = p / N, c = p % N;
+    if (p >= nF) lorig[p] = lorig[s];
+    float4 *b = prims + (size_t)leaf * W;
     if (D == 2) {
-        out[i] = make_float4(lo[0], lo[1], hi[0], hi[1]);
+        b[c] = lseg[s];
+        reinterpret_cast<float *>(b + 4)[c] = lseginv[s];
     } else {
-        out[2 * i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-        out[2 * i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        for (int k = 0; k < 3; ++k) b[3 * c + k] = ltri[3 * s + k];
     }
 }
 
-// Eigenvectors of a symmetric 3 x 3 matrix by cyclic Jacobi rotations in
-// double: on return the columns of v are orthonormal and a is (nearly)
+// Eigenvectors of a symmetric 3 x 3 matrix by cyclic Jacobi rotations: on
+// return the columns of v are orthonormal to float accuracy and a is (nearly)
 // diagonal, a[k][k] the eigenvalue of column k.
-__device__ void sym3_eigen(double a[3][3], double v[3][3]) {
+__device__ void sym3_eigen(float a[3][3], float v[3][3]) {
     for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 3; ++c) v[r][c] = r == c ? 1.0 : 0.0;
-    for (int sweep = 0; sweep < 32; ++sweep) {
-        const double off = a[0][1] * a[0][1] + a[0][2] * a[0][2] + a[1][2] * a[1][2];
-        const double dia = a[0][0] * a[0][0] + a[1][1] * a[1][1] + a[2][2] * a[2][2];
-        if (!(off > 1e-30 * dia)) break;
+        for (int c = 0; c < 3; ++c) v[r][c] = r == c ? 1.0f : 0.0f;
+    for (int sweep = 0; sweep < 8; ++sweep) {
+        const float off = a[0][1] * a[0][1] + a[0][2] * a[0][2] + a[1][2] * a[1][2];
+        const float dia = a[0][0] * a[0][0] + a[1][1] * a[1][1] + a[2][2] * a[2][2];
+        if (!(off > 1e-14f * dia)) break;
         for (int p = 0; p < 2; ++p) {
             for (int q = p + 1; q < 3; ++q) {
-                if (a[p][q] == 0.0) continue;
+                if (a[p][q] == 0.0f) continue;
                 // rotation in the (p, q) plane that zeroes a[p][q]: A <- J^T A J
-                const double th = (a[q][q] - a[p][p]) / (2.0 * a[p][q]);
-                const double t = (th >= 0.0 ? 1.0 : -1.0) / (fabs(th) + sqrt(th * th + 1.0));
-                const double c = 1.0 / sqrt(t * t + 1.0), s = t * c;
+                const float th = (a[q][q] - a[p][p]) / (2.0f * a[p][q]);
+                const float t = (th >= 0.0f ? 1.0f : -1.0f) / (fabsf(th) + sqrtf(th * th + 1.0f));
+                const float c = 1.0f / sqrtf(t * t + 1.0f), s = t * c;
                 for (int k = 0; k < 3; ++k) {
-                    const double akp = a[k][p], akq = a[k][q];
+                    const float akp = a[k][p], akq = a[k][q];
                     a[k][p] = c * akp - s * akq;
                     a[k][q] = s * akp + c * akq;
                 }
                 for (int k = 0; k < 3; ++k) {
-                    const double apk = a[p][k], aqk = a[q][k];
+                    const float apk = a[p][k], aqk = a[q][k];
                     a[p][k] = c * apk - s * aqk;
                     a[q][k] = s * apk + c * aqk;
                 }
                 for (int k = 0; k < 3; ++k) {
-                    const double vkp = v[k][p], vkq = v[k][q];
+                    const float vkp = v[k][p], vkq = v[k][q];
                     v[k][p] = c * vkp - s * vkq;
                     v[k][q] = s * vkp + c * vkq;
                 }
@@ -467,234 +462,256 @@ __device__ void sym3_eigen(double a[3][3], double v[3][3]) {
     }
 }
 
-// Oriented box of each wide-tree leaf, the bound the queries test leaves by.
-// Its axes are the principal axes of the leaf's vertices as the distance code
-// sees them (a and a + d for a segment; a, a + ab, a + ac for a triangle):
-// the eigenvectors of their covariance, rounded to float and shrunk by 2^-20
-// so that the float axes, with the third 3D axis u2 = u0 x u1 evaluated in
-// float exactly as the query does (cross3), form a matrix of norm below 1.
-// The centre c is rounded to float, and e_k bounds |u_k.(y - c)| over the
-// vertices y, evaluated in double with the float axes and centre and widened
-// by 1e-6 |y - c|max, which covers the query's float rounding of q - c and of
-// the dot products (relative 2^-22 of |q - c| <= |q - y| + |y - c|).  Layout:
-// 2D (u0.x, u0.y, c.x, c.y), (e0, e1, 0, 0) with u1 = (-u0.y, u0.x); 3D
-// (u0, e0), (u1, e1), (c, e2).
+// Sum / minimum / maximum of x over the TPN threads of one node (1, a warp or
+// the block); every thread gets the result.
+template <int TPN, class Op>
+__device__ __forceinline__ double node_reduce(double x, Op op, double *red) {
+    if constexpr (TPN > 1) {
+        for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
+    }
+    if constexpr (TPN > 32) {
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
+        __syncthreads();
+        x = red[threadIdx.x & 31];
+        for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
+    }
+    return x;
+}
+
+// Vertices of the primitive at sorted position s as the distance code sees them:
+// a and a + d of a segment; a, a + ab and a + ac of a triangle.
 template <int D>
-__global__ void k_wt_obb(const float4 *lseg, const float4 *ltri, int nF, float4 *obb, int n1) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n1) return;
-    const int b0 = WT_LEAF * i, e = min(b0 + WT_LEAF, nF);
-    constexpr int NV = D == 2 ? 2 : 3;
-    auto vertex = [&](int s, int j, double *y) {
-        if (D == 2) {
-            const float4 g = lseg[s];
-            y[0] = j == 0 ? (double)g.x : (double)g.x + g.z;
-            y[1] = j == 0 ? (double)g.y : (double)g.y + g.w;
-            y[2] = 0.0;
-        } else {
-            const float4 a = ltri[3 * s], ab = ltri[3 * s + 1], ac = ltri[3 * s + 2];
-            y[0] = j == 0 ? (double)a.x : (double)a.x + (j == 1 ? ab.x : ac.x);
-            y[1] = j == 0 ? (double)a.y : (double)a.y + (j == 1 ? ab.y : ac.y);
-            y[2] = j == 0 ? (double)a.z : (double)a.z + (j == 1 ? ab.z : ac.z);
-        }
-    };
-    double m[3] = {0.0, 0.0, 0.0}, y[3];
-    for (int s = b0; s < e; ++s)
-        for (int j = 0; j < NV; ++j) {
-            vertex(s, j, y);
-            for (int k = 0; k < D; ++k) m[k] += y[k];
-        }
-    const double nv = (double)((e - b0) * NV);
-    for (int k = 0; k < D; ++k) m[k] /= nv;
-    double cov[3][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
-    for (int s = b0; s < e; ++s)
-        for (int j = 0; j < NV; ++j) {
-            vertex(s, j, y);
-            for (int r = 0; r < D; ++r)
-                for (int c = 0; c < D; ++c) cov[r][c] += (y[r] - m[r]) * (y[c] - m[c]);
-        }
-    // float axes u[k][*]
-    float u[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
-    const double shrink = 1.0 - 0x1p-20;
+__device__ __forceinline__ void prim_vertices(const float4 *lseg, const float4 *ltri, int s, double y[3][3]) {
     if (D == 2) {
-        const double th = 0.5 * atan2(2.0 * cov[0][1], cov[0][0] - cov[1][1]);
+        const float4 g = lseg[s];
+        y[0][0] = g.x;
+        y[0][1] = g.y;
+        y[1][0] = (double)g.x + g.z;
+        y[1][1] = (double)g.y + g.w;
+    } else {
+        const float4 a = ltri[3 * (size_t)s], ab = ltri[3 * (size_t)s + 1], ac = ltri[3 * (size_t)s + 2];
+        const float o[3] = {a.x, a.y, a.z}, e[3] = {ab.x, ab.y, ab.z}, f[3] = {ac.x, ac.y, ac.z};
+        for (int k = 0; k < 3; ++k) {
+            y[0][k] = o[k];
+            y[1][k] = (double)o[k] + e[k];
+            y[2][k] = (double)o[k] + f[k];
+        }
+    }
+}
+
+// Bound of a node of `np` primitives from sorted position s0, by TPN threads, all
+// of which call.  The axes are the principal axes of the vertices, eigenvectors
+// of their covariance, made orthonormal, shrunk a little and rounded (2D: to
+// float, 3D: to multiples of 2^-15) so that the rounded axes -- with the third 3D
+// axis evaluated in float exactly as the query does (obb_axis2) -- form a matrix
+// of norm at most 1.  The centre -- the middle of the projections on the axes --
+// is rounded to float too, and the extents bound the vertices about the float
+// centre along the rounded axes, evaluated in double and widened by 1e-6 of the
+// largest |y - c|, which covers the query's float rounding of q - c and of the
+// products with it (relative 2^-22 of |q - c| <= |q - y| + |y - c|).
+//   2D: out = (u0, c, e0, e1).
+//   3D: out = (c, u0, u1, e) with the axes in units of 2^-15.
+template <int D, int TPN>
+__device__ __forceinline__ void node_bound(const float4 *lseg, const float4 *ltri, int s0, int np, int t, double *red,
+                                           float *out) {
+    constexpr int NV = D == 2 ? 2 : 3;
+    auto add = [](double a, double b) { return a + b; };
+    auto lower = [](double a, double b) { return fmin(a, b); };
+    auto upper = [](double a, double b) { return fmax(a, b); };
+    // moments about the first vertex
+    double y0[3], y[3][3], m[3] = {0.0, 0.0, 0.0}, cv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    prim_vertices<D>(lseg, ltri, s0, y);
+    for (int k = 0; k < D; ++k) y0[k] = y[0][k];
+    for (int i = t; i < np; i += TPN) {
+        prim_vertices<D>(lseg, ltri, s0 + i, y);
+        for (int j = 0; j < NV; ++j) {
+            double w[3];
+            for (int k = 0; k < D; ++k) {
+                w[k] = y[j][k] - y0[k];
+                m[k] += w[k];
+            }
+            cv[0] += w[0] * w[0];
+            cv[1] += w[0] * w[1];
+            cv[3] += w[1] * w[1];
+            if (D == 3) {
+                cv[2] += w[0] * w[2];
+                cv[4] += w[1] * w[2];
+                cv[5] += w[2] * w[2];
+            }
+        }
+    }
+    const double n = (double)np * NV;
+    for (int k = 0; k < D; ++k) m[k] = node_reduce<TPN>(m[k], add, red) / n;
+    for (int k = 0; k < 6; ++k)
+        if (D == 3 || k < 2 || k == 3) cv[k] = node_reduce<TPN>(cv[k], add, red) / n;
+    cv[0] -= m[0] * m[0];
+    cv[1] -= m[0] * m[1];
+    cv[3] -= m[1] * m[1];
+    // orthogonal axes u[0], u[1] (and u[2]: the normal)
+    // 3D: rounding moves an axis by up to 2.7e-5 and two axes' product by 5.3e-5
+    const double shrink = D == 2 ? 1.0 - 0x1p-20 : (1.0 - 6e-5) * 32768.0;
+    const double unit[3] = {D == 2 ? 1.0 : 0x1p-15, D == 2 ? 1.0 : 0x1p-15, 0x1p-30};  // of u[k]
+    float u[3][3];
+    if (D == 2) {
+        const double th = 0.5 * atan2(2.0 * cv[1], cv[0] - cv[3]);
         u[0][0] = (float)(cos(th) * shrink);
         u[0][1] = (float)(sin(th) * shrink);
         u[1][0] = -u[0][1];
         u[1][1] = u[0][0];
     } else {
-        double vec[3][3];
-        sym3_eigen(cov, vec);
-        // u0, u1: the two largest-variance axes; u2 = u0 x u1 (the normal)
-        int o[3] = {0, 1, 2};
+        cv[2] -= m[0] * m[2];
+        cv[4] -= m[1] * m[2];
+        cv[5] -= m[2] * m[2];
+        // scaled so that squares of tiny nodes' entries stay normal floats
+        const double tr = cv[0] + cv[3] + cv[5], sc = tr > 0.0 ? 1.0 / tr : 0.0;
+        float A[3][3] = {{(float)(cv[0] * sc), (float)(cv[1] * sc), (float)(cv[2] * sc)},
+                         {(float)(cv[1] * sc), (float)(cv[3] * sc), (float)(cv[4] * sc)},
+                         {(float)(cv[2] * sc), (float)(cv[4] * sc), (float)(cv[5] * sc)}};
+        float vec[3][3];
+        sym3_eigen(A, vec);
+        int o[3] = {0, 1, 2};  // by falling variance
         for (int a = 0; a < 2; ++a)
             for (int b = a + 1; b < 3; ++b)
-                if (cov[o[b]][o[b]] > cov[o[a]][o[a]]) {
-                    const int t = o[a];
+                if (A[o[b]][o[b]] > A[o[a]][o[a]]) {
+                    const int w = o[a];
                     o[a] = o[b];
-                    o[b] = t;
+                    o[b] = w;
                 }
+        double p[3], w[3], lp = 0.0, lw = 0.0, pw = 0.0;
+        for (int k = 0; k < 3; ++k) lp += (double)vec[k][o[0]] * vec[k][o[0]];
         for (int k = 0; k < 3; ++k) {
-            u[0][k] = (float)(vec[k][o[0]] * shrink);
-            u[1][k] = (float)(vec[k][o[1]] * shrink);
+            p[k] = vec[k][o[0]] / sqrt(lp);
+            pw += p[k] * vec[k][o[1]];
         }
-        cross3(u[0][0], u[0][1], u[0][2], u[1][0], u[1][1], u[1][2], u[2][0], u[2][1], u[2][2]);
+        for (int k = 0; k < 3; ++k) {
+            w[k] = vec[k][o[1]] - pw * p[k];
+            lw += w[k] * w[k];
+        }
+        for (int k = 0; k < 3; ++k) {
+            u[0][k] = (float)rint(p[k] * shrink);
+            u[1][k] = (float)rint(w[k] / sqrt(lw) * shrink);
+        }
+        obb_axis2(u[0], u[1], u[2]);
     }
-    // centre: the middle of the projection ranges about the mean
-    double pmin[3] = {INFINITY, INFINITY, INFINITY}, pmax[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (int s = b0; s < e; ++s)
-        for (int j = 0; j < NV; ++j) {
-            vertex(s, j, y);
+    // ranges of u_k.(y - y0), and the centre in the middle of them
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int i = t; i < np; i += TPN) {
+        prim_vertices<D>(lseg, ltri, s0 + i, y);
+        for (int j = 0; j < NV; ++j)
             for (int k = 0; k < D; ++k) {
                 double p = 0.0;
-                for (int c = 0; c < D; ++c) p += (double)u[k][c] * (y[c] - m[c]);
-                pmin[k] = fmin(pmin[k], p);
-                pmax[k] = fmax(pmax[k], p);
+                for (int c = 0; c < D; ++c) p += unit[k] * (double)u[k][c] * (y[j][c] - y0[c]);
+                lo[k] = fmin(lo[k], p);
+                hi[k] = fmax(hi[k], p);
             }
-        }
-    float cf[3] = {0.0f, 0.0f, 0.0f};
+    }
+    for (int k = 0; k < D; ++k) {
+        lo[k] = node_reduce<TPN>(lo[k], lower, red);
+        hi[k] = node_reduce<TPN>(hi[k], upper, red);
+    }
+    float cf[3];
     for (int c = 0; c < D; ++c) {
-        double x = m[c];
-        for (int k = 0; k < D; ++k) x += 0.5 * (pmin[k] + pmax[k]) * (double)u[k][c];
+        double x = y0[c];
+        for (int k = 0; k < D; ++k) x += 0.5 * (lo[k] + hi[k]) * (unit[k] * (double)u[k][c]);
         cf[c] = (float)x;
     }
-    double ext[3] = {0.0, 0.0, 0.0}, r2 = 0.0;
-    for (int s = b0; s < e; ++s)
-        for (int j = 0; j < NV; ++j) {
-            vertex(s, j, y);
-            double d2 = 0.0;
-            for (int c = 0; c < D; ++c) d2 += (y[c] - cf[c]) * (y[c] - cf[c]);
-            r2 = fmax(r2, d2);
-            for (int k = 0; k < D; ++k) {
-                double p = 0.0;
-                for (int c = 0; c < D; ++c) p += (double)u[k][c] * (y[c] - (double)cf[c]);
-                ext[k] = fmax(ext[k], fabs(p));
-            }
-        }
-    const double pad = 1e-6 * sqrt(r2);
+    double e[3] = {0.0, 0.0, 0.0};
+    for (int k = 0; k < D; ++k) {
+        double off = 0.0;
+        for (int c = 0; c < D; ++c) off += unit[k] * (double)u[k][c] * ((double)cf[c] - y0[c]);
+        e[k] = fmax(hi[k] - off, off - lo[k]);
+    }
+    // the axes are orthonormal to 3e-4, so |y - c| is at most this
+    const double pad = 1.001e-6 * sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
     float ef[3];
-    for (int k = 0; k < D; ++k) ef[k] = __double2float_ru(ext[k] + pad);
+    for (int k = 0; k < D; ++k) ef[k] = __double2float_ru(e[k] + pad);
     if (D == 2) {
-        obb[2 * i] = make_float4(u[0][0], u[0][1], cf[0], cf[1]);
-        obb[2 * i + 1] = make_float4(ef[0], ef[1], 0.0f, 0.0f);
+        out[0] = u[0][0];
+        out[1] = u[0][1];
+        out[2] = cf[0];
+        out[3] = cf[1];
+        out[4] = ef[0];
+        out[5] = ef[1];
     } else {
-        obb[3 * i] = make_float4(u[0][0], u[0][1], u[0][2], ef[0]);
-        obb[3 * i + 1] = make_float4(u[1][0], u[1][1], u[1][2], ef[1]);
-        obb[3 * i + 2] = make_float4(cf[0], cf[1], cf[2], ef[2]);
+        auto pair = [](float lo16, float hi16) {
+            return __uint_as_float((unsigned)((int)lo16 + 32768) | (unsigned)((int)hi16 + 32768) << 16);
+        };
+        // the upper half of a float not below x > 0
+        auto up = [](float x) { return (__float_as_uint(x) + 0xffffu) >> 16; };
+        for (int k = 0; k < 3; ++k) out[k] = cf[k];
+        out[3] = pair(u[0][0], u[0][1]);
+        out[4] = pair(u[0][2], u[1][0]);
+        out[5] = pair(u[1][1], u[1][2]);
+        out[6] = __uint_as_float(up(ef[0]) | up(ef[1]) << 16);
+        out[7] = ef[2];
     }
 }
 
+// Store the bound of node i of depth `depth` in its parent's block.
 template <int D>
-__global__ void k_wt_level(const float4 *in, int n_in, float4 *out, int n_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_out) return;
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    const int e = min(32 * i + 32, n_in);
-    for (int c = 32 * i; c < e; ++c) {
-        if (D == 2) {
-            const float4 b = in[c];
-            lo[0] = fminf(lo[0], b.x);
-            lo[1] = fminf(lo[1], b.y);
-            hi[0] = fmaxf(hi[0], b.z);
-            hi[1] = fmaxf(hi[1], b.w);
-        } else {
-            const float4 a = in[2 * c], b = in[2 * c + 1];
-            lo[0] = fminf(lo[0], a.x);
-            lo[1] = fminf(lo[1], a.y);
-            lo[2] = fminf(lo[2], a.z);
-            hi[0] = fmaxf(hi[0], b.x);
-            hi[1] = fmaxf(hi[1], b.y);
-            hi[2] = fmaxf(hi[2], b.z);
-        }
-    }
+__device__ __forceinline__ void write_bound(float4 *tree, int depth, int i, const float *o) {
+    float4 *b = tree + (size_t)tree_block(depth - 1, (unsigned)i >> 2) * Tree<D>::NODE_W;
+    const int c = i & 3;
     if (D == 2) {
-        out[i] = make_float4(lo[0], lo[1], hi[0], hi[1]);
+        b[c] = make_float4(o[0], o[1], o[2], o[3]);
+        reinterpret_cast<float2 *>(b + 4)[c] = make_float2(o[4], o[5]);
     } else {
-        out[2 * i] = make_float4(lo[0], lo[1], lo[2], 0.0f);
-        out[2 * i + 1] = make_float4(hi[0], hi[1], hi[2], 0.0f);
+        b[2 * c] = make_float4(o[0], o[1], o[2], o[3]);
+        b[2 * c + 1] = make_float4(o[4], o[5], o[6], o[7]);
     }
 }
 
-// Slab bounds of the level-2 nodes of a 3D wide tree (patches of up to 1024
-// triangles): n = the normalised sum of the unit face normals, and the
-// interval [oc - oh, oc + oh] of n.(v - c) over the vertices v as the distance
-// code sees them, c the node's box centre computed exactly as the query does,
-// evaluated in double and widened by the float roundings plus a relative
-// margin.  A node whose normals cancel gets n = 0 and oh = inf (no slab).  One block of
-// SLAB_THREADS per node; fixed-order reductions.  The half-thickness goes to
-// the box's first .w, the normal and the interval's centre to slab[node].
-constexpr int SLAB_THREADS = 256;
-__global__ void __launch_bounds__(SLAB_THREADS) k_wt_slab2(const float4 *ltri, int nF, float4 *box, float4 *slab,
-                                                            int n2) {
-    __shared__ double red[3][SLAB_THREADS];
-    const int i = blockIdx.x, t = threadIdx.x;
-    if (i >= n2) return;
-    const int b0 = WT_LEAF * 32 * i, e = min(b0 + WT_LEAF * 32, nF);
-    double ns[3] = {0.0, 0.0, 0.0};
-    for (int s = b0 + t; s < e; s += SLAB_THREADS) {
-        const float4 ab = ltri[3 * s + 1], ac = ltri[3 * s + 2];
-        double nn[3];
-        nn[0] = (double)ab.y * ac.z - (double)ab.z * ac.y;
-        nn[1] = (double)ab.z * ac.x - (double)ab.x * ac.z;
-        nn[2] = (double)ab.x * ac.y - (double)ab.y * ac.x;
-        const double l = sqrt(nn[0] * nn[0] + nn[1] * nn[1] + nn[2] * nn[2]);
-        if (l > 0.0)
-            for (int k = 0; k < 3; ++k) ns[k] += nn[k] / l;
+// Bounds of the tree's nodes.  A node of up to TREE_LANE_PRIMS primitives takes a
+// thread, of up to TREE_WARP_PRIMS a warp, a larger one a block; the large ones
+// (k_tree_bounds with LARGE) are few and each long, so their blocks are big.
+constexpr int TREE_THREADS = 256, TREE_LARGE_THREADS = 1024;
+constexpr int TREE_LANE_PRIMS = 16, TREE_WARP_PRIMS = 512;
+struct TreePlan {
+    int depth, nF;
+    int first[TREE_MAX_DEPTH + 2];  // first block of depth d's nodes, d = d0..d1; [d1 + 1]: blocks in all
+    int count[TREE_MAX_DEPTH + 1];  // nodes of depth d
+    int d0, d1;
+};
+__host__ __device__ inline long long node_prims(int leaf, int height) { return (long long)leaf << (2 * height); }
+__host__ __device__ inline int nodes_per_block(long long prims) {
+    return prims <= TREE_LANE_PRIMS ? TREE_THREADS : prims <= TREE_WARP_PRIMS ? TREE_THREADS / 32 : 1;
+}
+
+template <int D, bool LARGE>
+__global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_tree_bounds(
+    TreePlan P, const float4 *lseg, const float4 *ltri, float4 *tree) {
+    __shared__ double red[32];
+    int d = P.d0;
+    while (d < P.d1 && (int)blockIdx.x >= P.first[d + 1]) ++d;
+    const long long cap = node_prims(Tree<D>::LEAF, P.depth - d);
+    const int per = nodes_per_block(cap), base = ((int)blockIdx.x - P.first[d]) * per;
+    const int i = base + (LARGE ? 0 : per == TREE_THREADS ? (int)threadIdx.x : (int)threadIdx.x >> 5);
+    const bool there = i < P.count[d];
+    // a node beyond the last still takes part in its warp's reductions
+    const long long s0 = (there ? i : P.count[d] - 1) * cap;
+    const int np = (int)min(cap, (long long)P.nF - s0);
+    float o[8];
+    bool writer = there;
+    if (LARGE) {
+        node_bound<D, TREE_LARGE_THREADS>(lseg, ltri, (int)s0, np, threadIdx.x, red, o);
+        writer = writer && threadIdx.x == 0;
+    } else if (per == TREE_THREADS) {
+        node_bound<D, 1>(lseg, ltri, (int)s0, np, 0, red, o);
+    } else {
+        node_bound<D, 32>(lseg, ltri, (int)s0, np, threadIdx.x & 31, red, o);
+        writer = writer && (threadIdx.x & 31) == 0;
     }
-    for (int k = 0; k < 3; ++k) red[k][t] = ns[k];
-    __syncthreads();
-    for (int h = SLAB_THREADS / 2; h > 0; h >>= 1) {
-        if (t < h)
-            for (int k = 0; k < 3; ++k) red[k][t] += red[k][t + h];
-        __syncthreads();
-    }
-    for (int k = 0; k < 3; ++k) ns[k] = red[k][0];
-    __syncthreads();
-    const float4 ba = box[2 * i], bb = box[2 * i + 1];
-    const float lo[3] = {ba.x, ba.y, ba.z}, hi[3] = {bb.x, bb.y, bb.z};
-    float c[3];
-    for (int k = 0; k < 3; ++k) c[k] = (lo[k] + hi[k]) * 0.5f;
-    const double ln = sqrt(ns[0] * ns[0] + ns[1] * ns[1] + ns[2] * ns[2]);
-    float nf[3] = {0.0f, 0.0f, 0.0f};
-    float ocf = 0.0f, ohf = INFINITY;
-    if (ln > 1e-6) {
-        // unit normal, shrunk by 2^-20 so that |n| <= 1 after rounding
-        for (int k = 0; k < 3; ++k) nf[k] = (float)(ns[k] / ln * (1.0 - 0x1p-20));
-        double omin = INFINITY, omax = -INFINITY, diag2 = 0.0;
-        for (int k = 0; k < 3; ++k) diag2 += ((double)hi[k] - lo[k]) * ((double)hi[k] - lo[k]);
-        for (int s = b0 + t; s < e; s += SLAB_THREADS) {
-            const float4 a = ltri[3 * s], ab = ltri[3 * s + 1], ac = ltri[3 * s + 2];
-            const double av[3] = {a.x, a.y, a.z}, abv[3] = {ab.x, ab.y, ab.z}, acv[3] = {ac.x, ac.y, ac.z};
-            for (int j = 0; j < 3; ++j) {
-                double o = 0.0;
-                for (int k = 0; k < 3; ++k) {
-                    const double v = av[k] + (j == 1 ? abv[k] : j == 2 ? acv[k] : 0.0);
-                    o += (double)nf[k] * (v - (double)c[k]);
-                }
-                omin = fmin(omin, o);
-                omax = fmax(omax, o);
-            }
-        }
-        red[0][t] = omin;
-        red[1][t] = omax;
-        __syncthreads();
-        for (int h = SLAB_THREADS / 2; h > 0; h >>= 1) {
-            if (t < h) {
-                red[0][t] = fmin(red[0][t], red[0][t + h]);
-                red[1][t] = fmax(red[1][t], red[1][t + h]);
-            }
-            __syncthreads();
-        }
-        omin = red[0][0];
-        omax = red[1][0];
-        const double oc = 0.5 * (omin + omax);
-        ocf = (float)oc;
-        const double oh = 0.5 * (omax - omin) + fabs(oc - (double)ocf) + 1e-6 * sqrt(diag2);
-        ohf = __double2float_ru(oh);
-    }
-    if (t == 0) {
-        box[2 * i].w = ohf;
-        slab[i] = make_float4(nf[0], nf[1], nf[2], ocf);
+    if (!writer) return;
+    write_bound<D>(tree, d, i, o);
+    if (i == P.count[d] - 1) {
+        // the last node also fills its parent's block with infinitely far children
+        float far[8] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+        if (D == 2)
+            far[4] = -INFINITY;
+        else
+            far[6] = __uint_as_float(0xff800000u >> 16);  // e0 = -inf
+        for (int k = i + 1; (k & 3) != 0; ++k) write_bound<D>(tree, d, k, far);
     }
 }
 
@@ -708,7 +725,7 @@ static cudaError_t dalloc(T **p, size_t count, cudaStream_t st) {
 }
 
 void SceneImpl::release(cudaStream_t st) {
-    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, wt_box, wt_slab, wt_obb, guide};
+    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, tree, prims, guide};
     for (void *p : ptrs)
         if (p) cudaFreeAsync(p, st);
     V = nullptr;
@@ -724,10 +741,8 @@ void SceneImpl::release(cudaStream_t st) {
     ltri = nullptr;
     lorig = nullptr;
     cdf = nullptr;
-    wt_box = nullptr;
-    wt_slab = nullptr;
-    wt_obb = nullptr;
-    wt_n[0] = wt_n[1] = wt_n[2] = 0;
+    tree = nullptr;
+    prims = nullptr;
     guide = nullptr;
 }
 
@@ -860,49 +875,39 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
     }
     k_leaf_data<D><<<nblk(nF, TB), TB, 0, st>>>(skeys, nF, S.seg, S.seginv, S.tri, S.lseg, S.lseginv, S.ltri, S.lorig);
 
-    // ---- wide tree (levels 1..wt_levels, the top one with <= 32 nodes)
+    // ---- search tree, in the buffers of the first build (their sizes depend
+    // on nF alone): device views held elsewhere -- batch plans, captured
+    // graphs, launches on other streams -- keep pointing at live memory
     {
-        const int W = D == 2 ? 1 : 2;  // float4 per box
-        int count = (nF + WT_LEAF - 1) / WT_LEAF, level = 1, off = 0;
-        S.wt_count[0] = nF;
-        for (;;) {
-            if (level > WT_MAX_LEVELS) return fail(WOS_ERR_UNSUPPORTED, "scene too large for the wide tree");
-            S.wt_count[level] = count;
-            S.wt_off[level] = off;
-            off += count;
-            if (count <= 32) break;
-            count = (count + 31) / 32;
-            ++level;
+        constexpr int N = Tree<D>::LEAF;
+        const int n_leaf = (nF + N - 1) / N;
+        TreePlan P{};
+        P.depth = S.tree_depth;
+        P.nF = nF;
+        for (int d = 1; d <= P.depth; ++d) {
+            const long long cap = node_prims(N, P.depth - d);
+            P.count[d] = (int)((nF + cap - 1) / cap);
         }
-        S.wt_levels = level;
-        // The level sizes depend on nF alone, so a rebuild after the vertices
-        // move (wos_scene_update_vertices) refills the buffers of the first
-        // build in place: device views held elsewhere (batch plans, captured
-        // graphs, launches on other streams) keep pointing at live memory.
-        const bool slab2 = D == 3 && S.wt_levels >= 2;
-        const size_t n_box = (size_t)off * W, n_slab = slab2 ? (size_t)S.wt_count[2] : 0,
-                     n_obb = (size_t)S.wt_count[1] * (D == 2 ? 2 : 3);
-        if (S.wt_box == nullptr || S.wt_n[0] != n_box || S.wt_n[1] != n_slab || S.wt_n[2] != n_obb) {
-            if (S.wt_box) cudaFreeAsync(S.wt_box, st);
-            if (S.wt_slab) cudaFreeAsync(S.wt_slab, st);
-            if (S.wt_obb) cudaFreeAsync(S.wt_obb, st);
-            S.wt_box = S.wt_slab = S.wt_obb = nullptr;
-            WOS_TRY(dalloc(&S.wt_box, n_box, st));
-            WOS_TRY(dalloc(&S.wt_slab, n_slab, st));
-            WOS_TRY(dalloc(&S.wt_obb, n_obb, st));
-            S.wt_n[0] = n_box;
-            S.wt_n[1] = n_slab;
-            S.wt_n[2] = n_obb;
+        k_tree_prims<D><<<nblk((long long)n_leaf * N, TB), TB, 0, st>>>(nF, n_leaf, S.lseg, S.lseginv, S.ltri, S.prims,
+                                                                    S.lorig);
+        // the depths of large nodes, then the others
+        int split = 1;
+        while (split <= P.depth && node_prims(N, P.depth - split) > TREE_WARP_PRIMS) ++split;
+        for (int part = 0; part < 2; ++part) {
+            P.d0 = part == 0 ? 1 : split;
+            P.d1 = part == 0 ? split - 1 : P.depth;
+            int blocks = 0;
+            for (int d = P.d0; d <= P.d1; ++d) {
+                P.first[d] = blocks;
+                blocks += nblk(P.count[d], nodes_per_block(node_prims(N, P.depth - d)));
+            }
+            if (blocks == 0) continue;
+            P.first[P.d1 + 1] = blocks;
+            if (part == 0)
+                k_tree_bounds<D, true><<<blocks, TREE_LARGE_THREADS, 0, st>>>(P, S.lseg, S.ltri, S.tree);
+            else
+                k_tree_bounds<D, false><<<blocks, TREE_THREADS, 0, st>>>(P, S.lseg, S.ltri, S.tree);
         }
-        k_wt_level1<D><<<nblk(S.wt_count[1], TB), TB, 0, st>>>(skeys, nF, pbox, S.wt_box, S.wt_count[1]);
-        k_wt_obb<D><<<nblk(S.wt_count[1], 64), 64, 0, st>>>(S.lseg, S.ltri, nF, S.wt_obb, S.wt_count[1]);
-        for (int l = 2; l <= S.wt_levels; ++l)
-            k_wt_level<D><<<nblk(S.wt_count[l], TB), TB, 0, st>>>(S.wt_box + (size_t)S.wt_off[l - 1] * W,
-                                                                S.wt_count[l - 1], S.wt_box + (size_t)S.wt_off[l] * W,
-                                                                S.wt_count[l]);
-        if (slab2)
-            k_wt_slab2<<<S.wt_count[2], SLAB_THREADS, 0, st>>>(S.ltri, nF, S.wt_box + (size_t)S.wt_off[2] * W,
-                                                               S.wt_slab, S.wt_count[2]);
         WOS_TRY(cudaGetLastError());
     }
 
@@ -979,7 +984,16 @@ int SceneImpl::allocate(cudaStream_t st) {
         WOS_TRY(dalloc(&ltri, (size_t)nF * 3, st));
         WOS_TRY(dalloc(&node, (size_t)std::max(nF - 1, 1) * 4, st));
     }
-    WOS_TRY(dalloc(&lorig, nF, st));
+    const int N = D == 2 ? Tree<2>::LEAF : Tree<3>::LEAF;
+    const long long n_leaf = ((long long)nF + N - 1) / N;
+    WOS_TRY(dalloc(&lorig, (size_t)n_leaf * N, st));
+    tree_depth = 1;
+    while ((1LL << (2 * tree_depth)) < n_leaf) ++tree_depth;
+    if (tree_depth > TREE_MAX_DEPTH) return fail(WOS_ERR_UNSUPPORTED, "scene too large for the search tree");
+    // blocks: those of the depths above the leaves' parents, then the parents
+    const size_t blocks = (size_t)tree_block(tree_depth - 1, 0) + (size_t)((n_leaf + 3) / 4);
+    WOS_TRY(dalloc(&tree, blocks * (D == 2 ? Tree<2>::NODE_W : Tree<3>::NODE_W), st));
+    WOS_TRY(dalloc(&prims, (size_t)n_leaf * (D == 2 ? Tree<2>::LEAF_W : Tree<3>::LEAF_W), st));
     std::vector<float> c;
     build_g_cdf(c, 10000);
     n_cdf = (int)c.size();
@@ -1028,12 +1042,9 @@ SceneView SceneImpl::view() const {
     v.tri = tri;
     v.nNodes = nNodes;
     v.node = node;
-    // In input order the leaf-ordered copies equal the primitive arrays: point
-    // the kernels at one copy so the tree's leaf tests and the warm-start /
-    // record lookups share cache lines.
-    v.lseg = prim_order == 1 ? seg : lseg;
-    v.lseginv = prim_order == 1 ? seginv : lseginv;
-    v.ltri = prim_order == 1 ? tri : ltri;
+    v.lseg = lseg;
+    v.lseginv = lseginv;
+    v.ltri = ltri;
     v.lorig = lorig;
     for (int k = 0; k < 3; ++k) {
         v.lo[k] = lo[k];
@@ -1052,14 +1063,9 @@ SceneView SceneImpl::view() const {
     v.n_cdf = n_cdf;
     v.guide = guide;
     v.n_guide = n_guide;
-    v.wt_levels = wt_levels;
-    for (int k = 0; k < 8; ++k) {
-        v.wt_count[k] = wt_count[k];
-        v.wt_off[k] = wt_off[k];
-    }
-    v.wt_box = wt_box;
-    v.wt_slab = wt_slab;
-    v.wt_obb = wt_obb;
+    v.tree_depth = tree_depth;
+    v.tree = tree;
+    v.prims = prims;
     return v;
 }
 

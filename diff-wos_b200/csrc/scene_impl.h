@@ -50,13 +50,9 @@ struct SceneImpl {
     int n_cdf = 0;
     unsigned short *guide = nullptr;
     int n_guide = 0;
-    int wt_levels = 0;
-    int wt_count[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    int wt_off[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    float4 *wt_box = nullptr;
-    float4 *wt_slab = nullptr;
-    float4 *wt_obb = nullptr;
-    size_t wt_n[3] = {0, 0, 0};  // float4 counts allocated for wt_box, wt_slab, wt_obb
+    int tree_depth = 1;  // search tree (SceneView::tree)
+    float4 *tree = nullptr;
+    float4 *prims = nullptr;
     // Incremented by every build and source change: the by-value fields of
     // view() (bounding box, extents, source) may have changed since a view
     // was taken.

@@ -1,16 +1,17 @@
 // Walk-on-spheres kernels for sm_100a.
 //
-// Forward: a persistent kernel in which every warp keeps 32 walks in flight.
-// Each loop iteration runs exactly one nearest-primitive query per lane;
-// when a lane's walk ends, the warp refills idle lanes from a grabbed chunk
-// of the flattened (point, walk) index space (ballot + prefix rank), so
-// warps stay full while walk lengths differ.  Results depend only on the
-// Philox counters, never on which lane or block ran a walk.
+// Forward: a persistent kernel in which every lane runs its own walk.  A lane is
+// searching the tree for its walk's nearest primitive (search_run), ready to
+// take a step, or at an edge of its walk -- to be started, at its first query,
+// or ended.  The warp searches until enough lanes are ready; those step and
+// begin their next search.  Edges, whose code is long and whose lanes are few at
+// any time, wait until an eighth of the lanes are at one.  Results depend only
+// on the Philox counters, never on which lane or block ran a walk.
 //
 // Adjoint: the same persistent loop over (point, walk) samples, each sample a
 // small state machine -- primal walk, 10-step inscribed-ball bisection, two
 // antithetic walks on the ball -- in which every state transition is again one
-// nearest query, so lanes in different phases share the query code path.
+// search.
 //
 // Reference functions restated: WoSDevice<N>::walk (include/wos.cuh:97-145),
 // WoS<N>::solve / singleWalk launchers (:184-448), normal_derivative
@@ -62,76 +63,26 @@ __device__ __forceinline__ Hit query(const SceneView &S, const float *p, const f
 }
 
 // Add a warp's work counters to the global totals (counting launches only).
-// Cooperative queries count once per warp (every lane holds the same totals).
-template <bool COOP>
 __device__ __forceinline__ void flush_work(const Work &wk) {
     unsigned long long v[3] = {wk.nq, wk.nb, wk.np};
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        if (!COOP) {
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
-        }
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
         if ((threadIdx.x & 31) == 0) atomicAdd(&g_work[k], v[k]);
     }
 }
 
-// Nearest query of every active lane.  With the LBVH the lanes take turns:
-// the whole warp answers each lane's query cooperatively (wquery), starting
-// from the warm candidate `warm` (that lane's previous nearest primitive, or
-// -1).  A lane with ball_m > 0 asks instead for a primitive blocking the
-// ball of radius ball_m centred at x (wball): it gets that primitive, or
-// prim = -1 when none blocks.  Brute force runs per lane and always returns
-// the nearest primitive.  Must be called by all 32 lanes.
-template <int D, bool BVH, int WL = 0, class WK>
-__device__ __forceinline__ Hit warp_queries(const SceneView &S, bool active, const float *x, int warm, WK &work,
-                                            float ball_m = -1.0f) {
-    Hit mine{-1, INFINITY};
-    if (!BVH) {
-        if (active) mine = nearest_brute<D>(S, x, work);
-        return mine;
-    }
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    unsigned act = __ballot_sync(FULL, active);
-    // The per-point parts of each search -- the pruning tolerance (or the
-    // ball's bound) and the warm candidate's distance -- are computed by every
-    // lane for its own point at once, not by the whole warp once per query;
-    // the values are the same bits either way.
-    float lim = 0.0f, wd2 = INFINITY;
-    if (active) {
-        const float tol2 = prune_tol2<D>(S, x);
-        if (ball_m > 0.0f) {
-            lim = wball_bound(ball_m, tol2);
-        } else {
-            lim = tol2;
-            if (warm >= 0) wd2 = prim_d2<D>(S, warm, x);
-        }
-    }
-    while (act) {
-        const int j = __ffs(act) - 1;
-        act &= act - 1u;
-        float q[3];
-        q[0] = __shfl_sync(FULL, x[0], j);
-        q[1] = __shfl_sync(FULL, x[1], j);
-        q[2] = D == 3 ? __shfl_sync(FULL, x[2], j) : 0.0f;
-        const int wp = __shfl_sync(FULL, warm, j);
-        const float bm = __shfl_sync(FULL, ball_m, j);
-        const float lj = __shfl_sync(FULL, lim, j);
-        const float wj = __shfl_sync(FULL, wd2, j);
-        Hit h{-1, INFINITY};
-        if (bm > 0.0f) {
-            wball_b<D, WL>(S, q, lj, bm, h, work);
-        } else {
-            if (wp >= 0) {
-                h.prim = wp;
-                h.d2 = wj;
-            }
-            h = wquery_tol<D, WL>(S, q, h, lj, work);
-        }
-        if (lane == j) mine = h;
-    }
-    return mine;
+// Lanes of a warp that may still be searching when the others advance, of `n`
+// that were.  More left behind means that fewer lanes wait for the
+// slowest searches, but that each advance serves fewer lanes: a 3D search takes
+// several times the instructions of an advance and its length varies more.
+// (2D keeping 1/4, 3/8, 1/2, 5/8: the forward solve of 14,592 points x 64 walks
+// on 1,024 segments 0.747, 0.750, 0.758, 0.764 ms; 3D keeping 1/2, 5/8, 3/4:
+// 17.71, 17.77, 17.42 ms for 20,000 x 64 on 20,480 triangles.)
+template <int D>
+__device__ __forceinline__ int search_keep(int n) {
+    return D == 2 ? n / 4 : n * 5 / 8;
 }
 
 // ------------------------------------------------------------------ walker
@@ -143,7 +94,6 @@ struct Walker {
     float ds[5];
     int i;
     int last;  // nearest primitive of the previous query (warm start), -1 if none
-    bool fresh;
     __device__ __forceinline__ void start(const float *x, int D) {
         p[0] = x[0];
         p[1] = x[1];
@@ -153,7 +103,6 @@ struct Walker {
         for (int k = 0; k < 5; ++k) ds[k] = 0.0f;
         i = 0;
         last = -1;
-        fresh = true;
     }
 };
 
@@ -173,20 +122,23 @@ __device__ __forceinline__ void walk_origin(const WalkCfg &c, const float *P, ui
     }
 }
 
-// Process the query result at w.p: inside test on the first query, shell
-// test, truncation, then the source term and one step (include/wos.cuh:97-145).
+// First query of a walk: whether the walk goes on from w.p -- there is a
+// primitive at a finite distance (none: a NaN or overflowing point) and the
+// point is inside, unless the walk is double-sided (include/wos.cuh:97-105).
+template <int D>
+__device__ __forceinline__ bool walk_enters(const Walker &w, const SceneView &S, const Hit &hit, const WalkCfg &c) {
+    return hit.prim >= 0 && (c.double_sided || inside_test<D>(S, w.p, hit, nullptr));
+}
+
+// Process the query result at w.p: shell test, truncation, then the source term
+// and one step (include/wos.cuh:97-145).
 template <int D>
 __device__ __forceinline__ int walker_advance(Walker &w, const SceneView &S, const Hit &hit, const WalkCfg &c,
                                               float eps, bool project, bool prevent_fd, uint32_t pt, uint32_t wk,
                                               uint32_t role, bool want_ds, const unsigned short *guide) {
-    // no primitive at a finite distance (a NaN or overflowing point)
     if (hit.prim < 0) return W_INVALID;
     float d = sqrtf(hit.d2);
-    if (w.fresh) {
-        w.fresh = false;
-        if (!c.double_sided && !inside_test<D>(S, w.p, hit, nullptr)) return W_INVALID;
-        if (prevent_fd) d *= 0.5f;
-    }
+    if (prevent_fd && w.i == 0) d *= 0.5f;
     if (w.i < c.nsteps) {
         if (d < eps) return W_VALID;
         if (!project && w.i == c.nsteps - 1) return W_TRUNC;
@@ -222,22 +174,24 @@ __device__ __forceinline__ int walker_advance(Walker &w, const SceneView &S, con
     return project ? W_VALID : W_TRUNC;
 }
 
-// Dynamic shared memory: [G-CDF guide table][`thread_bytes` of scratch per
-// thread].  Sized to the byte: the carve-out the driver picks for the
-// kernel's resident blocks comes in steps, and every byte of it is L1 lost to
-// the tree.
-__host__ __device__ inline size_t smem_bytes(int n_guide, int nthreads, int thread_bytes) {
+// Dynamic shared memory: [G-CDF guide table][search stacks, `stack_entries` of
+// the block's threads][`thread_bytes` of scratch per thread].  Sized to the
+// byte: the carve-out the driver picks for the kernel's resident blocks comes
+// in steps, and every byte of it is L1 lost to the tree.
+__host__ __device__ inline size_t smem_bytes(int n_guide, int nthreads, int stack_entries, int thread_bytes) {
     size_t b = ((size_t)(n_guide + 1) * sizeof(unsigned short) + 15) & ~(size_t)15;
+    b += (size_t)nthreads * stack_entries * sizeof(unsigned);
     b += ((size_t)nthreads * thread_bytes + 15) & ~(size_t)15;
     return b;
 }
 
 struct Smem {
     const unsigned short *guide;
-    double *scratch;  // this thread's words
+    unsigned *stack;  // this thread's search stack, blockDim.x words between entries
+    double *scratch;  // the block's scratch
 };
 
-__device__ __forceinline__ Smem stage_smem(const SceneView &S, bool stage_guide, int thread_words, float4 *smem) {
+__device__ __forceinline__ Smem stage_smem(const SceneView &S, bool stage_guide, int stack_entries, float4 *smem) {
     Smem m;
     char *base = reinterpret_cast<char *>(smem);
     const int ng = stage_guide ? S.n_guide : -1;
@@ -248,7 +202,9 @@ __device__ __forceinline__ Smem stage_smem(const SceneView &S, bool stage_guide,
         m.guide = sg;
     }
     base += ((size_t)(ng + 1) * sizeof(unsigned short) + 15) & ~(size_t)15;
-    m.scratch = reinterpret_cast<double *>(base) + (size_t)threadIdx.x * thread_words;
+    m.stack = reinterpret_cast<unsigned *>(base) + threadIdx.x;
+    base += (size_t)blockDim.x * stack_entries * sizeof(unsigned);
+    m.scratch = reinterpret_cast<double *>(base);
     __syncthreads();
     return m;
 }
@@ -290,99 +246,224 @@ __device__ __forceinline__ bool refill(Queue &q, bool &active, long long &idx, u
     return __ballot_sync(FULL, active) != 0u;
 }
 
+// Walk (pt, walk) of index idx for nw walks per point.  Indices below 2^32 take
+// a 32-bit division.
+__device__ __forceinline__ void split_index(long long idx, int nw, uint32_t &pt, uint32_t &wk) {
+    if (idx <= 0xffffffffLL) {
+        pt = (uint32_t)idx / (uint32_t)nw;
+        wk = (uint32_t)idx - pt * (uint32_t)nw;
+    } else {
+        pt = (uint32_t)(idx / nw);
+        wk = (uint32_t)(idx - (long long)pt * nw);
+    }
+}
+
+// What a launch searches: one scene; and what one walks over: one scene and point
+// set, or many (batched).  A lane's `item` tells its scene.
+template <int D>
+struct PlainScene {
+    static constexpr bool MULTI = false;
+    const SceneView &S;
+    __device__ __forceinline__ const SceneView *scenes() const { return &S; }
+    __device__ __forceinline__ const SceneView &scene(int) const { return S; }
+};
+
+template <int D>
+struct OneScene {
+    static constexpr bool MULTI = false;
+    const SceneView &S;
+    const WalkCfg &c;
+    const float *P;
+    __device__ __forceinline__ const SceneView *scenes() const { return &S; }
+    __device__ __forceinline__ const SceneView &scene(int) const { return S; }
+    __device__ __forceinline__ const WalkCfg &cfg(int) const { return c; }
+    __device__ __forceinline__ const float *points(int) const { return P; }
+    // the walk of queue position idx
+    __device__ __forceinline__ void locate(long long &idx, int &, uint32_t &pt, uint32_t &wk) const {
+        split_index(idx, c.nwalks, pt, wk);
+        wk += c.walk_offset;
+    }
+};
+
+__device__ __forceinline__ int find_item(const BatchItemDev *__restrict__ items, int n_items, long long idx) {
+    int lo = 0, hi = n_items - 1;  // last item with walk_begin <= idx
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(&items[mid].walk_begin) <= idx)
+            lo = mid;
+        else
+            hi = mid - 1;
+    }
+    return lo;
+}
+
+template <int D>
+struct ManyScenes {
+    static constexpr bool MULTI = true;
+    const SceneView *views;
+    const WalkCfg *cfgs;
+    const BatchItemDev *items;
+    int n_items;
+    __device__ __forceinline__ const SceneView *scenes() const { return views; }
+    __device__ __forceinline__ const SceneView &scene(int i) const { return views[i]; }
+    __device__ __forceinline__ const WalkCfg &cfg(int i) const { return cfgs[i]; }
+    __device__ __forceinline__ const float *points(int i) const { return items[i].P; }
+    __device__ __forceinline__ void locate(long long &idx, int &item, uint32_t &pt, uint32_t &wk) const {
+        item = find_item(items, n_items, idx);
+        split_index(idx - items[item].walk_begin, items[item].nwalks, pt, wk);
+        wk += cfgs[item].walk_offset;
+    }
+};
+
+// The search of every lane with sr.dep == SEARCH_NEED begun, and the warp's
+// searches run on.  Brute force completes at once.
+template <int D, bool BVH, class CTX, class WK>
+__device__ __forceinline__ void lane_search(Search<D> &sr, const CTX &x, int item, const float *p, int warm,
+                                            float ball_m, unsigned *stack, WK &work) {
+    if (sr.dep == SEARCH_NEED) {
+        if (BVH) {
+            work.nq += 1;
+            search_begin<D>(sr, x.scene(item), p, warm, ball_m);
+        } else {
+            const Hit h = nearest_brute<D>(x.scene(item), p, work);
+            sr.pos = h.prim;
+            sr.d2 = h.d2;
+            sr.dep = SEARCH_DONE;
+        }
+    }
+    if (BVH) {
+        const int n = __popc(__ballot_sync(0xffffffffu, sr.dep >= 0));
+        search_run<D, CTX::MULTI>(sr, x.scenes(), item, p, stack, search_keep<D>(n), work);
+    }
+}
+
+// Its hit (ball_m as in search_hit).
+template <int D, bool BVH>
+__device__ __forceinline__ Hit lane_hit(const Search<D> &sr, const SceneView &S, float ball_m = -1.0f) {
+    if (BVH) return search_hit<D>(sr, S, ball_m);
+    return ball_m > 0.0f && !(sr.pos >= 0 && ball_blocks(sr.d2, ball_m)) ? Hit{-1, INFINITY} : Hit{sr.pos, sr.d2};
+}
+
 // ------------------------------------------------------------------ forward
-// COUNT: the instance that keeps work counters (launched while work
-// accounting is on); the others carry none.  The 3D instances are compiled
-// for 3 resident blocks of 512 (a 40-register cap): 1 % faster than 2 blocks
-// at 64 registers; the 2D ones stay at 64 registers.
-template <int D, bool BVH, bool RECORDS, int WL, bool COUNT>
-__global__ void __launch_bounds__(512, D == 3 ? 3 : 1) k_walk(SceneView S, WalkCfg c, const float *__restrict__ P, long long total,
-                                             unsigned long long *counter, int chunk, int n_top, int stage_cdf,
-                                             WalkOut out) {
-    extern __shared__ float4 smem[];
-    const Smem sm = stage_smem(S, stage_cdf != 0, 0, smem);
+// Walks of queue positions [0, total) (of idx0 onwards in index space).
+template <int D, bool BVH, bool RECORDS, class CTX, class WK>
+__device__ __forceinline__ void walk_lanes(const CTX &x, long long idx0, long long total,
+                                           unsigned long long *counter, int chunk, const WalkOut &out,
+                                           const unsigned short *guide, unsigned *stack, WK &work) {
+    const unsigned FULL = 0xffffffffu;
     Queue q{0, 0, false};
     bool active = false;
+    bool first = false;  // the outstanding or completed search is the walk's first
+    int ended = 0;       // the walk's end (W_VALID, ...), not yet written
     long long idx = 0;
+    int item = 0;
     uint32_t pt = 0, wk = 0;
     Walker w;
     w.last = -1;
-    typename std::conditional<COUNT, Work, NoWork>::type work{};
+    Search<D> sr;
+    sr.dep = SEARCH_DONE;
     for (;;) {
-        const bool was = active;
-        if (!refill(q, active, idx, counter, total, chunk)) break;
-        if (active && !was) {
-            if (RECORDS) {
-                pt = (uint32_t)idx;
-                wk = c.walk_offset;
-            } else {
-                pt = (uint32_t)(idx / c.nwalks);
-                wk = c.walk_offset + (uint32_t)(idx - (long long)pt * c.nwalks);
+        const bool done = active && sr.dep == SEARCH_DONE;
+        const bool edge = ended != 0 || (done && first) || (!active && !q.drained);
+        const int n_edge = __popc(__ballot_sync(FULL, edge)), n_other = __popc(__ballot_sync(FULL, active && !edge));
+        if (n_edge == 0 && n_other == 0) break;
+        if (n_edge != 0 && (7 * n_edge >= n_other || n_other == 0)) {
+            if (done && first && ended == 0) {
+                const Hit hit = lane_hit<D, BVH>(sr, x.scene(item));
+                first = false;
+                if (!walk_enters<D>(w, x.scene(item), hit, x.cfg(item))) ended = W_INVALID;
             }
-            float x0[3];
-            walk_origin<D>(c, P, pt, wk, x0);
-            w.start(x0, D);
-        }
-        const Hit hit = warp_queries<D, BVH, WL>(S, active, w.p, w.last, work);
-        if (!active) continue;
-        w.last = hit.prim;
-        const int r = walker_advance<D>(w, S, hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt, wk, ROLE_PRIMAL,
-                                        out.wds != nullptr, sm.guide);
-        if (r == W_CONTINUE) continue;
-        active = false;
-        if (RECORDS) {
-            const bool ok = r == W_VALID;
-            out.valid[pt] = ok ? 1 : 0;
-            Rec rec;
-            if (ok) rec = closest_record<D>(S, w.p, hit.prim);
+            if (ended != 0) {
+                const SceneView &S = x.scene(item);
+                const WalkCfg &c = x.cfg(item);
+                const bool ok = ended == W_VALID;
+                Rec rec;
+                if (ok) rec = closest_record<D>(S, w.p, w.last);
+                if (RECORDS) {
+                    out.valid[pt] = ok ? 1 : 0;
 #pragma unroll
-            for (int k = 0; k < D; ++k) {
-                if (out.pt) out.pt[(size_t)pt * D + k] = ok ? rec.p[k] : 0.0f;
-                if (out.nrm) out.nrm[(size_t)pt * D + k] = ok ? rec.n[k] : 0.0f;
-            }
-            if (out.tuv) {
-                out.tuv[2 * (size_t)pt] = ok ? rec.t0 : 0.0f;
-                out.tuv[2 * (size_t)pt + 1] = (ok && D == 3) ? rec.t1 : 0.0f;
-            }
-            if (out.prim) out.prim[pt] = ok ? hit.prim : -1;
-            if (out.contrib) out.contrib[pt] = ok ? w.contrib : 0.0f;
-        } else {
-            float v = 0.0f;
-            Rec rec;
-            if (r == W_VALID) {
-                rec = closest_record<D>(S, w.p, hit.prim);
-                v = dirichlet<D>(S, hit.prim, rec.t0, rec.t1, nullptr, nullptr);
-                if (c.include_source) v += w.contrib;
-                if (!isfinite(v)) atomicOr(&g_status, ST_NONFINITE);
-            }
-            out.values[idx] = v;
-            if (out.wrec) {
-                if (D == 2) {
-                    const int2 wr = r == W_VALID ? make_int2(hit.prim | (rec.flip ? 0x40000000 : 0),
-                                                             __float_as_int(rec.t0))
-                                                 : make_int2(-1, 0);
-                    reinterpret_cast<int2 *>(out.wrec)[idx] = wr;
+                    for (int k = 0; k < D; ++k) {
+                        if (out.pt) out.pt[(size_t)pt * D + k] = ok ? rec.p[k] : 0.0f;
+                        if (out.nrm) out.nrm[(size_t)pt * D + k] = ok ? rec.n[k] : 0.0f;
+                    }
+                    if (out.tuv) {
+                        out.tuv[2 * (size_t)pt] = ok ? rec.t0 : 0.0f;
+                        out.tuv[2 * (size_t)pt + 1] = (ok && D == 3) ? rec.t1 : 0.0f;
+                    }
+                    if (out.prim) out.prim[pt] = ok ? w.last : -1;
+                    if (out.contrib) out.contrib[pt] = ok ? w.contrib : 0.0f;
                 } else {
-                    const int4 wr = r == W_VALID ? make_int4(hit.prim | (rec.flip ? 0x40000000 : 0),
-                                                             __float_as_int(rec.t0), __float_as_int(rec.t1), 0)
-                                                 : make_int4(-1, 0, 0, 0);
-                    reinterpret_cast<int4 *>(out.wrec)[idx] = wr;
-                }
-            }
-            if (out.wds) {
+                    float v = 0.0f;
+                    if (ok) {
+                        v = dirichlet<D>(S, w.last, rec.t0, rec.t1, nullptr, nullptr);
+                        if (c.include_source) v += w.contrib;
+                        if (!isfinite(v)) atomicOr(&g_status, ST_NONFINITE);
+                    }
+                    out.values[idx] = v;
+                    if (out.wrec) {
+                        if (D == 2) {
+                            reinterpret_cast<int2 *>(out.wrec)[idx] =
+                                ok ? make_int2(w.last | (rec.flip ? 0x40000000 : 0), __float_as_int(rec.t0))
+                                   : make_int2(-1, 0);
+                        } else {
+                            reinterpret_cast<int4 *>(out.wrec)[idx] =
+                                ok ? make_int4(w.last | (rec.flip ? 0x40000000 : 0), __float_as_int(rec.t0),
+                                               __float_as_int(rec.t1), 0)
+                                   : make_int4(-1, 0, 0, 0);
+                        }
+                    }
+                    if (out.wds) {
 #pragma unroll
-                for (int k = 0; k < 5; ++k) out.wds[(size_t)idx * 5 + k] = r == W_VALID ? w.ds[k] : 0.0f;
+                        for (int k = 0; k < 5; ++k) out.wds[(size_t)idx * 5 + k] = ok ? w.ds[k] : 0.0f;
+                    }
+                    if (out.steps) out.steps[idx] = ended == W_TRUNC ? c.nsteps : w.i;
+                }
+                active = false;
+                ended = 0;
             }
-            if (out.steps) out.steps[idx] = r == W_TRUNC ? c.nsteps : w.i;
+            const bool was = active;
+            refill(q, active, idx, counter, total, chunk);
+            if (active && !was) {
+                idx += idx0;
+                if (RECORDS) {
+                    pt = (uint32_t)idx;
+                    wk = x.cfg(item).walk_offset;
+                } else {
+                    x.locate(idx, item, pt, wk);
+                }
+                float x0[3];
+                walk_origin<D>(x.cfg(item), x.points(item), pt, wk, x0);
+                w.start(x0, D);
+                first = true;
+                sr.dep = SEARCH_NEED;
+            }
         }
+        if (active && sr.dep == SEARCH_DONE && !first && ended == 0) {
+            const WalkCfg &c = x.cfg(item);
+            const Hit hit = lane_hit<D, BVH>(sr, x.scene(item));
+            w.last = hit.prim;
+            const int r = walker_advance<D>(w, x.scene(item), hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt,
+                                            wk, ROLE_PRIMAL, out.wds != nullptr, guide);
+            if (r == W_CONTINUE)
+                sr.dep = SEARCH_NEED;
+            else
+                ended = r;
+        }
+        lane_search<D, BVH>(sr, x, item, w.p, w.last, -1.0f, stack, work);
     }
-    if constexpr (COUNT) {
-        if (c.count) flush_work<BVH>(work);
-    } else {
-        // never taken (counting launches use the COUNT instance); with this
-        // epilogue in place the kernel measured 2-5 % faster than without it
-        if (c.count) flush_work<BVH>(Work{0, 0, 0});
-    }
+}
+
+// COUNT: the instance that keeps work counters (launched while work
+// accounting is on); the others carry none.
+template <int D, bool BVH, bool RECORDS, bool COUNT>
+__global__ void __launch_bounds__(512, 2) k_walk(SceneView S, WalkCfg c, const float *__restrict__ P, long long total,
+                                             unsigned long long *counter, int chunk, int stack_entries, int stage_cdf,
+                                             WalkOut out) {
+    extern __shared__ float4 smem[];
+    const Smem sm = stage_smem(S, stage_cdf != 0, stack_entries, smem);
+    typename std::conditional<COUNT, Work, NoWork>::type work{};
+    walk_lanes<D, BVH, RECORDS>(OneScene<D>{S, c, P}, 0, total, counter, chunk, out, sm.guide, sm.stack, work);
+    if constexpr (COUNT) flush_work(work);
 }
 
 // Reference-shaped kernel: one thread per (point, walk), no regeneration.
@@ -399,8 +480,9 @@ __global__ void __launch_bounds__(256) k_walk_plain(SceneView S, WalkCfg c, cons
     w.start(x0, D);
     Work work{0, 0, 0};
     float v = 0.0f;
-    for (;;) {
+    for (bool first = true;; first = false) {
         const Hit hit = query<D, BVH>(S, w.p, nullptr, 0, work);
+        if (first && !walk_enters<D>(w, S, hit, c)) break;
         const int r = walker_advance<D>(w, S, hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt, wk, ROLE_PRIMAL,
                                         false, S.guide);
         if (r == W_CONTINUE) continue;
@@ -454,72 +536,103 @@ __global__ void k_reduce(const float *__restrict__ vals, int n, int nw, double *
 }
 
 // ------------------------------------------------------------------ queries
+// Closest-point queries, a lane each at a time: a lane whose search is done
+// writes its record and goes on to its next point while the others search on.
+constexpr int QUERY_THREADS = 128;
 template <int D, bool BVH>
-__global__ void k_closest(SceneView S, const float *__restrict__ P, int n, QueryOut o) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float p[3] = {P[(size_t)i * D], P[(size_t)i * D + 1], D == 3 ? P[(size_t)i * D + 2] : 0.0f};
-    Work work{0, 0, 0};
-    const Hit hit = query<D, BVH>(S, p, nullptr, 0, work);
-    if (o.prim) o.prim[i] = hit.prim;
-    if (o.dist) o.dist[i] = sqrtf(hit.d2);
-    if (hit.prim < 0) {
-        atomicOr(&g_status, ST_BAD_PRIM);
-        return;
-    }
-    const Rec r = closest_record<D>(S, p, hit.prim);
+__global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const float *__restrict__ P, int n,
+                                                            QueryOut o) {
+    extern __shared__ float4 smem[];
+    unsigned *stack = reinterpret_cast<unsigned *>(smem) + threadIdx.x;
+    const PlainScene<D> x{S};
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    NoWork work;
+    Search<D> sr;
+    sr.dep = SEARCH_DONE;
+    float p[3] = {0.0f, 0.0f, 0.0f};
+    auto load = [&]() {
+        if (i >= n) return;
 #pragma unroll
-    for (int k = 0; k < D; ++k) {
-        if (o.pt) o.pt[(size_t)i * D + k] = r.p[k];
-        if (o.nrm) o.nrm[(size_t)i * D + k] = r.n[k];
-    }
-    if (o.tuv) {
-        o.tuv[2 * (size_t)i] = r.t0;
-        o.tuv[2 * (size_t)i + 1] = D == 3 ? r.t1 : 0.0f;
-    }
-    if (o.sdf || o.inside) {
-        float sd;
-        const bool in = inside_test<D>(S, p, hit, &sd);
-        if (o.sdf) o.sdf[i] = sd;
-        if (o.inside) o.inside[i] = in ? 1 : 0;
+        for (int k = 0; k < D; ++k) p[k] = P[(size_t)i * D + k];
+        sr.dep = SEARCH_NEED;
+    };
+    load();
+    while (__any_sync(0xffffffffu, i < n)) {
+        lane_search<D, BVH>(sr, x, 0, p, -1, -1.0f, stack, work);
+        if (i >= n || sr.dep >= 0) continue;
+        const Hit hit = lane_hit<D, BVH>(sr, S);
+        if (o.prim) o.prim[i] = hit.prim;
+        if (o.dist) o.dist[i] = sqrtf(hit.d2);
+        if (hit.prim < 0) {
+            atomicOr(&g_status, ST_BAD_PRIM);
+        } else {
+            const Rec r = closest_record<D>(S, p, hit.prim);
+#pragma unroll
+            for (int k = 0; k < D; ++k) {
+                if (o.pt) o.pt[(size_t)i * D + k] = r.p[k];
+                if (o.nrm) o.nrm[(size_t)i * D + k] = r.n[k];
+            }
+            if (o.tuv) {
+                o.tuv[2 * (size_t)i] = r.t0;
+                o.tuv[2 * (size_t)i + 1] = D == 3 ? r.t1 : 0.0f;
+            }
+            if (o.sdf || o.inside) {
+                float sd;
+                const bool in = inside_test<D>(S, p, hit, &sd);
+                if (o.sdf) o.sdf[i] = sd;
+                if (o.inside) o.inside[i] = in ? 1 : 0;
+            }
+        }
+        i += stride;
+        load();
     }
 }
 
-// Largest inscribed ball (include/scene.cuh:225-249).
+// Largest inscribed ball (include/scene.cuh:225-249), a lane each at a time.
 template <int D, bool BVH>
-__device__ __forceinline__ float inscribed_ball(const SceneView &S, const float *p, const float *n, float eps,
-                                                const float4 *top, int n_top) {
+__global__ void __launch_bounds__(QUERY_THREADS) k_ball(SceneView S, const uint8_t *valid, const float *pt,
+                                                         const float *nrm, int n, float eps, float *R) {
+    extern __shared__ float4 smem[];
+    unsigned *stack = reinterpret_cast<unsigned *>(smem) + threadIdx.x;
+    const PlainScene<D> x{S};
+    const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    float p[3] = {0.0f, 0.0f, 0.0f}, nn[3] = {0.0f, 0.0f, 0.0f}, q[3] = {0.0f, 0.0f, 0.0f};
+    const bool on = i < n && valid[i];
+    if (i < n && !on) R[i] = 0.0f;
+    if (on) {
+        for (int k = 0; k < D; ++k) {
+            p[k] = pt[(size_t)i * D + k];
+            nn[k] = nrm[(size_t)i * D + k];
+        }
+    }
     float b = S.half_min_extent, a = eps;
-    Work work{0, 0, 0};
-    for (int i = 0; i < 10; ++i) {
+    int step = on ? 0 : 10, last = -1;
+    NoWork work;
+    Search<D> sr;
+    sr.dep = SEARCH_DONE;
+    auto aim = [&]() {
         const float m = (a + b) * 0.5f;
-        float q[3] = {0.0f, 0.0f, 0.0f};
 #pragma unroll
-        for (int k = 0; k < D; ++k) q[k] = fmaf(n[k], m, p[k]);
-        const float d = sqrtf(query<D, BVH>(S, q, top, n_top, work).d2);
-        if (wosm::ball_accepts(d, m))
+        for (int k = 0; k < D; ++k) q[k] = fmaf(nn[k], m, p[k]);
+        sr.dep = SEARCH_NEED;
+    };
+    if (on) aim();
+    while (__any_sync(0xffffffffu, step < 10)) {
+        lane_search<D, BVH>(sr, x, 0, q, last, -1.0f, stack, work);
+        if (step >= 10 || sr.dep >= 0) continue;
+        const Hit hit = lane_hit<D, BVH>(sr, S);
+        last = hit.prim;
+        const float m = (a + b) * 0.5f;
+        if (wosm::ball_accepts(sqrtf(hit.d2), m))
             a = m;
         else
             b = m;
+        if (++step < 10)
+            aim();
+        else
+            R[i] = a;
     }
-    return a;
-}
-
-template <int D, bool BVH>
-__global__ void k_ball(SceneView S, const uint8_t *valid, const float *pt, const float *nrm, int n, float eps,
-                       float *R) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    if (!valid[i]) {
-        R[i] = 0.0f;
-        return;
-    }
-    float p[3] = {0, 0, 0}, nn[3] = {0, 0, 0};
-    for (int k = 0; k < D; ++k) {
-        p[k] = pt[(size_t)i * D + k];
-        nn[k] = nrm[(size_t)i * D + k];
-    }
-    R[i] = inscribed_ball<D, BVH>(S, p, nn, eps, nullptr, 0);
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -695,32 +808,30 @@ __device__ __forceinline__ void nd_finish(const NdState<D> &st, const SceneView 
     for (int k = 0; k < D; ++k) out[k] = grad * -st.rn[k];
 }
 
-// Lane-local part of one inscribed-ball bisection step at radius m, centre q:
-// the primitive that blocked the previous rejected radius decides a
-// rejection without a query (need = false, pre = that primitive); otherwise,
-// if the ball's own primitive rprim is within m + 1e-5f, the step is accepted
-// unless some primitive blocks, and the warp only searches for one
-// (ball_m = m; pre = rprim, the result when none blocks).  Else the step
-// takes the full nearest query (the reference's test on the nearest distance).
-template <int D>
-__device__ __forceinline__ void ball_precheck(const SceneView &S, const float *q, float m, int bwarm, int rprim,
-                                              bool &need, float &ball_m, Hit &pre) {
-    if (bwarm >= 0) {
-        const float d2 = prim_d2<D>(S, bwarm, q);
-        if (ball_blocks(d2, m)) {
-            pre = Hit{bwarm, d2};
-            need = false;
-            return;
-        }
-    }
-    const float d2 = prim_d2<D>(S, rprim, q);
-    if (sqrtf(d2) - m <= 1e-5f) {
-        pre = Hit{rprim, d2};
-        ball_m = m;
-    }
-}
-
-enum { PH_IDLE = 0, PH_PRIMAL = 1, PH_BALL = 2, PH_ANTI_START = 3, PH_ANTI_WALK = 4, PH_ND_START = 5 };
+// Phases of a sample.  With a search outstanding or completed:
+//   PH_PRIMAL      the primal walk
+//   PH_BALL        a bisection step decided by whether any primitive blocks
+//   PH_BALL_NEAR   a bisection step decided by the nearest distance
+//   PH_ANTI_START  the first query of a walk on the ball
+//   PH_ANTI_WALK   its later ones
+// and, at an edge:
+//   PH_PRIMAL_END  the primal walk has ended on the boundary
+//   PH_SETUP       the bisection is over
+//   PH_END_*       a ball walk has ended: in the shell at its start, on the
+//                  boundary, or invalid
+enum {
+    PH_IDLE,
+    PH_PRIMAL,
+    PH_BALL,
+    PH_BALL_NEAR,
+    PH_ANTI_START,
+    PH_ANTI_WALK,
+    PH_PRIMAL_END,
+    PH_SETUP,
+    PH_END_SHELL,
+    PH_END_WALK,
+    PH_END_NONE
+};
 
 // Per-thread adjoint state kept in shared memory: touched at phase changes,
 // not in the query loop, so it does not occupy registers.  Only 4-byte
@@ -752,6 +863,52 @@ __host__ __device__ constexpr int adj_thread_bytes(bool acc) {
 }
 
 template <int D>
+__device__ __forceinline__ void ball_begin(AdjSlot<D> &sl, const SceneView &S, const AdjCfg &a) {
+    sl.ba = a.ball_eps;
+    sl.bb = S.half_min_extent;
+    sl.bk = 0;
+    sl.bwarm = -1;
+}
+
+// The next search of a sample in its inscribed-ball bisection: sets the query
+// point q and the phase that takes its result, and returns the radius of a
+// blocking search (PH_BALL) or a negative number (PH_BALL_NEAR).  Steps that the
+// primitive which blocked the last rejected radius decides need no search and
+// are taken here.  Where the ball's own primitive is within m + 1e-5f the step
+// is accepted exactly unless some primitive blocks; else it takes the
+// reference's test on the nearest distance.  After the last step: PH_SETUP.
+template <int D>
+__device__ __forceinline__ float ball_next(AdjSlot<D> &sl, const SceneView &S, int rprim, int &phase, float *q) {
+    for (; sl.bk < 10; ++sl.bk) {
+        const float m = (sl.ba + sl.bb) * 0.5f;
+#pragma unroll
+        for (int k = 0; k < D; ++k) q[k] = fmaf(sl.st.rn[k], m, sl.st.p[k]);
+        if (sl.bwarm >= 0 && ball_blocks(prim_d2<D>(S, sl.bwarm, q), m)) {
+            sl.bb = m;
+            continue;
+        }
+        const bool own = m > 0.0f && sqrtf(prim_d2<D>(S, rprim, q)) - m <= 1e-5f;
+        phase = own ? PH_BALL : PH_BALL_NEAR;
+        return own ? m : -1.0f;
+    }
+    phase = PH_SETUP;
+    return -1.0f;
+}
+
+// Take the result of a bisection step's search.
+template <int D>
+__device__ __forceinline__ void ball_take(AdjSlot<D> &sl, const Hit &hit, int phase) {
+    const float m = (sl.ba + sl.bb) * 0.5f;
+    if (phase == PH_BALL ? hit.prim < 0 : wosm::ball_accepts(sqrtf(hit.d2), m)) {
+        sl.ba = m;
+    } else {
+        sl.bb = m;
+        sl.bwarm = hit.prim;
+    }
+    ++sl.bk;
+}
+
+template <int D>
 struct AdjSmem {
     double *acc;  // this thread's first accumulator; the k-th is acc[k * blockDim.x]
     AdjSlot<D> *slot;
@@ -766,346 +923,389 @@ __device__ __forceinline__ AdjSmem<D> adj_smem(double *base, bool acc) {
     return m;
 }
 
-// The adjoint kernel runs at most 256 threads per block and is compiled for
-// at least ADJ_MIN_BLOCKS resident blocks per SM: a 64-register cap.  The
-// single-scene 3D kernel, whose leaf loads wait on L2, is compiled for
-// ADJ_MIN_BLOCKS_3D (a 40-register cap): measured against 3, 4, 5, 7 and 8
-// blocks it is the fastest despite its spills (4 -> 6: C3 step -3 %; 7 and 8
-// spill far more and lose 10 %).  The 2D kernel is fastest at 4 and the
-// batched kernels, which carry more per-lane state, at 4 in both dimensions.
+// The adjoint kernels run at most 256 threads per block and are compiled for
+// ADJ_MIN_BLOCKS resident blocks per SM (a 64-register cap).
 #ifndef ADJ_MIN_BLOCKS
 #define ADJ_MIN_BLOCKS 4
 #endif
-#ifndef ADJ_MIN_BLOCKS_3D
-#define ADJ_MIN_BLOCKS_3D 6
-#endif
 
-// Persistent adjoint kernel.  ND_ONLY: the items are boundary records and the
-// kernel writes one normal-derivative estimate per record (the
-// wos_normal_derivative entry point); otherwise items are (point, walk)
-// samples and gradients are accumulated into dV / dg / dsrc.
-template <int D, bool BVH, int MODE, int WL, bool COUNT>
-__global__ void __launch_bounds__(256, D == 3 ? ADJ_MIN_BLOCKS_3D : ADJ_MIN_BLOCKS) k_adjoint(SceneView S, WalkCfg c, AdjCfg a, const float *__restrict__ P,
-                                                long long total, const float *__restrict__ dLdu,
-                                                unsigned long long *counter, int chunk, int n_top, int stage_cdf,
-                                                AdjOut out) {
-    extern __shared__ float4 smem[];
-    const Smem sm = stage_smem(S, stage_cdf != 0, 0, smem);
-    const unsigned short *cdf = sm.guide;
-    const bool src2 = D == 2 && S.src_type != 0;
-    constexpr bool ND_ONLY = MODE == ADJ_ND_ONLY;
-    const bool want_src = !ND_ONLY && a.want_dsrc && c.include_source && src2;
-    const AdjSmem<D> am = adj_smem<D>(sm.scratch, want_src);
-    AdjSlot<D> &slot = *am.slot;
-    double *acc_src = am.acc;  // k-th accumulator at acc_src[k * blockDim.x]
-    const int AS = blockDim.x;
-    if (want_src) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k) acc_src[k * AS] = 0.0;
-    }
+// Where the gradients of a launch go: FP64 accumulators of one scene, or of the
+// lane's item.
+template <class CTX>
+__device__ __forceinline__ double *grad_dV(const CTX &x, const AdjOut &out, int item) {
+    if constexpr (CTX::MULTI) return out.dV + x.items[item].dV_off;
+    return out.dV;
+}
+template <class CTX>
+__device__ __forceinline__ double *grad_dg(const CTX &x, const AdjOut &out, int item) {
+    if constexpr (CTX::MULTI) return out.dV + x.items[item].dg_off;
+    return out.dg;
+}
+// Weight of a sample: dL/du of its point over the point's walks.
+template <class CTX>
+__device__ __forceinline__ double sample_weight(const CTX &x, const float *dLdu, int item, uint32_t pt) {
+    if constexpr (CTX::MULTI)
+        return (double)__ldg(&dLdu[x.items[item].point_begin + pt]) / x.items[item].nwalks;
+    else
+        return (double)__ldg(&dLdu[pt]) / x.c.nwalks;
+}
+
+// Adjoint samples of queue positions [0, total) (of idx0 onwards in index
+// space).  MODE ADJ_ND_ONLY: the items are boundary records and the result is
+// one normal-derivative estimate per record; otherwise items are (point, walk)
+// samples and gradients are accumulated into dV / dg / dsrc (ADJ_TANGENT: the
+// directional derivative is gathered).  acc_src: this thread's source-gradient
+// accumulators, or null.
+//
+// Lanes wait for the code of their kind: a walk's step, run when a quarter of the
+// warp's lanes are at one, or a bisection step or an edge (start, end, set-up),
+// an eighth (a quarter: the 3D gradient of 50,000 points x 16 walks on 81,920
+// triangles 63.1 ms instead of 57.1; a sixteenth: no faster); or any when nothing
+// else is left to do.
+template <int D, bool BVH, int MODE, class CTX, class WK>
+__device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, long long idx0, long long total,
+                                              const float *__restrict__ dLdu, unsigned long long *counter, int chunk,
+                                              const AdjOut &out, const unsigned short *guide, unsigned *stack,
+                                              AdjSlot<D> &slot, double *acc_src, WK &work) {
+    constexpr bool ND_ONLY = MODE == ADJ_ND_ONLY, TAN = MODE == ADJ_TANGENT;
+    constexpr bool FROM_REC = MODE == ADJ_FROM_RECORDS || TAN, HAS_PRIMAL = MODE == ADJ_RECOMPUTE;
+    const unsigned FULL = 0xffffffffu;
+    const int AS = blockDim.x;  // k-th accumulator at acc_src[k * AS]
+    int acc_item = -1;          // item whose source gradient acc_src holds (batched)
     NdState<D> &st = slot.st;
-    float *rn = st.rn;
-    float &rt0 = slot.rt0, &rt1 = slot.rt1;
-    float &ba = slot.ba, &bb = slot.bb;
-    int &bk = slot.bk;
-    int &bwarm = slot.bwarm;
-    constexpr bool TAN = MODE == ADJ_TANGENT;
-    constexpr bool FROM_REC = MODE == ADJ_FROM_RECORDS || TAN;
-    float &tacc = slot.tacc;
-    const bool with_src = a.source_in_nd && src2;
     Queue q{0, 0, false};
     bool active = false;
+    bool first = false;  // PH_PRIMAL: at its first query
     long long idx = 0;
+    int item = 0;
     uint32_t pt = 0, wk = 0;
     int phase = PH_IDLE;
-    double W = 0.0;
-    Walker w;
     int rprim = 0;
-    float qpos[3] = {0, 0, 0};
-    typename std::conditional<COUNT, Work, NoWork>::type work{};
+    Walker w;
     w.last = -1;
-
-    // Every lane reaches warp_queries once per iteration: no `continue`
-    // between refill() and the query.
+    Search<D> sr;
+    sr.dep = SEARCH_DONE;
     for (;;) {
-        const bool was = active;
-        if (!refill(q, active, idx, counter, total, chunk)) break;
-        if (active && !was) {
-            if (ND_ONLY) {
-                pt = (uint32_t)idx;
-                wk = c.walk_offset;
-                const int rp = out.rprim[pt];
-                if (!out.rvalid[pt] || rp < 0 || rp >= S.nF) {
-                    if (out.rvalid[pt]) atomicOr(&g_status, ST_BAD_PRIM);
-#pragma unroll
-                    for (int k = 0; k < D; ++k) out.nd[(size_t)pt * D + k] = 0.0f;
+        const bool ready = active && sr.dep < 0;
+        const bool ball = ready && (phase == PH_BALL || phase == PH_BALL_NEAR);
+        const bool step = ready && (phase == PH_ANTI_WALK || (HAS_PRIMAL && phase == PH_PRIMAL && !first));
+        const bool edge = (ready && !ball && !step) || (!active && !q.drained);
+        const int n_ball = __popc(__ballot_sync(FULL, ball)), n_step = __popc(__ballot_sync(FULL, step));
+        const int n_edge = __popc(__ballot_sync(FULL, edge)), n_run = __popc(__ballot_sync(FULL, active && !ready));
+        const int n_all = n_ball + n_step + n_edge + n_run;
+        if (n_all == 0) break;
+        const bool any = 8 * n_ball >= n_all || 4 * n_step >= n_all || 8 * n_edge >= n_all || n_run == 0;
+        const bool all = n_run == 0 && 8 * n_ball < n_all && 4 * n_step < n_all && 8 * n_edge < n_all;
+        float ball_m = -1.0f;
+        if (any && n_edge != 0 && (all || 8 * n_edge >= n_all)) {
+            if (ready && phase == PH_ANTI_START) {
+                const Hit hit = lane_hit<D, BVH>(sr, x.scene(item));
+                if (sqrtf(hit.d2) < a.epsilon2) {
+                    phase = PH_END_SHELL;
+                    w.last = hit.prim;
+                } else {
+                    const float x0[3] = {w.p[0], w.p[1], w.p[2]};
+                    w.start(x0, D);
+                    phase = walk_enters<D>(w, x.scene(item), hit, x.cfg(item)) ? PH_ANTI_WALK : PH_END_NONE;
+                }
+            }
+            if (HAS_PRIMAL && ready && phase == PH_PRIMAL && first) {
+                first = false;
+                if (!walk_enters<D>(w, x.scene(item), lane_hit<D, BVH>(sr, x.scene(item)), x.cfg(item)))
                     active = false;
+            }
+            if (ready && (phase == PH_END_SHELL || phase == PH_END_WALK || phase == PH_END_NONE)) {
+                const SceneView &S = x.scene(item);
+                const WalkCfg &c = x.cfg(item);
+                const bool with_src = a.source_in_nd && D == 2 && S.src_type != 0;
+                float uq = 0.0f;
+                if (phase != PH_END_NONE) {
+                    const Rec r2 = closest_record<D>(S, w.p, w.last);
+                    uq = dirichlet<D>(S, w.last, r2.t0, r2.t1, nullptr, nullptr);
+                    if (with_src && phase == PH_END_WALK) uq += w.contrib;
                 }
-                rprim = active ? rp : 0;
-                rt0 = out.rtuv[2 * (size_t)pt];
-                rt1 = out.rtuv[2 * (size_t)pt + 1];
+                nd_accumulate<D>(st, a, uq);
+                st.which += 1;
+                if (st.which == 1) {
+                    nd_point<D>(st, w.p);
+                    phase = PH_ANTI_START;
+                    sr.dep = SEARCH_NEED;
+                } else {
+                    float gn[3];
+                    nd_finish<D>(st, S, c, a, pt, wk, with_src, gn);
+                    if (ND_ONLY) {
 #pragma unroll
-                for (int k = 0; k < D; ++k) {
-                    st.p[k] = out.rpt[(size_t)pt * D + k];
-                    rn[k] = out.rnrm[(size_t)pt * D + k];
-                }
-                phase = PH_ND_START;
-            } else {
-                if (FROM_REC && out.order != nullptr) idx = (long long)__ldg(&out.order[idx]);
-                pt = (uint32_t)(idx / c.nwalks);
-                wk = c.walk_offset + (uint32_t)(idx - (long long)pt * c.nwalks);
-                W = TAN ? 1.0 : (double)__ldg(&dLdu[pt]) / c.nwalks;
-                float x0[3];
-                walk_origin<D>(c, P, pt, wk, x0);
-                w.start(x0, D);
-                phase = PH_PRIMAL;
-                tacc = 0.0f;
-                if (W == 0.0) active = false;
-                if (FROM_REC && active) {
-                    // the primal walk ran in the forward pass: start from its record
-                    int code;
-                    if (D == 2) {
-                        const int2 wr = __ldg(reinterpret_cast<const int2 *>(out.wrec) + idx);
-                        code = wr.x;
-                        rt0 = __int_as_float(wr.y);
-                        rt1 = 0.0f;
+                        for (int k = 0; k < D; ++k) out.nd[(size_t)pt * D + k] = gn[k];
                     } else {
-                        const int4 wr = __ldg(reinterpret_cast<const int4 *>(out.wrec) + idx);
-                        code = wr.x;
-                        rt0 = __int_as_float(wr.y);
-                        rt1 = __int_as_float(wr.z);
-                    }
-                    if (code < 0) {
-                        active = false;
-                    } else {
-                        rprim = code & 0x3fffffff;
-                        const Rec rec = record_from<D>(S, rprim, rt0, rt1, (code & 0x40000000) != 0);
+                        float gt[3];
+                        tangent_derivative<D>(S, rprim, gt);
                         int vid[3];
                         float wts[3];
-                        st.uref = dirichlet<D>(S, rprim, rt0, rt1, vid, wts);
+                        dirichlet<D>(S, rprim, slot.rt0, slot.rt1, vid, wts);
                         if (TAN) {
-                            if (a.want_dg && out.tg != nullptr) {
+                            // d(sample) = -(grad_n + grad_t) . dx, dx = sum_s wts_s dV[vid_s]
+                            float tacc = slot.tacc;
 #pragma unroll
-                                for (int s2 = 0; s2 < D; ++s2) tacc = fmaf(wts[s2], __ldg(&out.tg[vid[s2]]), tacc);
-                            }
-                            if (want_src && out.ts != nullptr) {
+                            for (int s = 0; s < D; ++s)
 #pragma unroll
-                                for (int k = 0; k < 5; ++k)
-                                    tacc = fmaf(__ldg(&out.wds[(size_t)idx * 5 + k]), __ldg(&out.ts[k]), tacc);
-                            }
+                                for (int k = 0; k < D; ++k)
+                                    tacc = fmaf(-(wts[s] * (gn[k] + gt[k])), __ldg(&out.tV[(size_t)vid[s] * D + k]),
+                                                tacc);
+                            out.tan[idx] = tacc;
                         } else {
-                            if (a.want_dg) {
+                            const double W = sample_weight(x, dLdu, item, pt);
+                            double *dV = grad_dV(x, out, item);
 #pragma unroll
-                                for (int s2 = 0; s2 < D; ++s2) atomicAdd(&out.dg[vid[s2]], W * (double)wts[s2]);
-                            }
-                            if (want_src) {
+                            for (int s = 0; s < D; ++s)
 #pragma unroll
-                                for (int k = 0; k < 5; ++k)
-                                    acc_src[k * AS] += W * (double)__ldg(&out.wds[(size_t)idx * 5 + k]);
-                            }
+                                for (int k = 0; k < D; ++k)
+                                    atomicAdd(&dV[(size_t)vid[s] * D + k], W * (double)(-(wts[s] * (gn[k] + gt[k]))));
                         }
-                        if (!a.want_dV || (TAN && out.tV == nullptr)) {
-                            if (TAN) out.tan[idx] = tacc;
+                    }
+                    active = false;
+                }
+            }
+            if (HAS_PRIMAL && ready && phase == PH_PRIMAL_END) {
+                const SceneView &S = x.scene(item);
+                const Rec rec = closest_record<D>(S, w.p, w.last);
+                rprim = w.last;
+                slot.rt0 = rec.t0;
+                slot.rt1 = rec.t1;
+                int vid[3];
+                float wts[3];
+                st.uref = dirichlet<D>(S, rprim, rec.t0, rec.t1, vid, wts);
+                const double W = sample_weight(x, dLdu, item, pt);
+                if (a.want_dg) {
+                    double *dg = grad_dg(x, out, item);
+#pragma unroll
+                    for (int s = 0; s < D; ++s) atomicAdd(&dg[vid[s]], W * (double)wts[s]);
+                }
+                if (acc_src != nullptr) {
+#pragma unroll
+                    for (int k = 0; k < 5; ++k) acc_src[k * AS] += W * (double)w.ds[k];
+                }
+                if (!a.want_dV) {
+                    active = false;
+                } else {
+#pragma unroll
+                    for (int k = 0; k < D; ++k) {
+                        st.p[k] = rec.p[k];
+                        st.rn[k] = rec.n[k];
+                    }
+                    ball_begin<D>(slot, S, a);
+                    phase = PH_BALL;
+                    sr.dep = SEARCH_NEED;
+                }
+            }
+            if (ready && phase == PH_SETUP) {
+                st.R = slot.ba;
+                nd_setup<D>(st, x.scene(item), x.cfg(item), a, pt, wk);
+                nd_point<D>(st, w.p);
+                phase = PH_ANTI_START;
+                sr.dep = SEARCH_NEED;
+            }
+            const bool was = active;
+            refill(q, active, idx, counter, total, chunk);
+            if (active && !was) {
+                idx += idx0;
+                sr.dep = SEARCH_NEED;
+                phase = PH_BALL;
+                if (ND_ONLY) {
+                    const SceneView &S = x.scene(item);
+                    pt = (uint32_t)idx;
+                    wk = x.cfg(item).walk_offset;
+                    const int rp = out.rprim[pt];
+                    if (!out.rvalid[pt] || rp < 0 || rp >= S.nF) {
+                        if (out.rvalid[pt]) atomicOr(&g_status, ST_BAD_PRIM);
+#pragma unroll
+                        for (int k = 0; k < D; ++k) out.nd[(size_t)pt * D + k] = 0.0f;
+                        active = false;
+                    } else {
+                        rprim = rp;
+                        slot.rt0 = out.rtuv[2 * (size_t)pt];
+                        slot.rt1 = out.rtuv[2 * (size_t)pt + 1];
+#pragma unroll
+                        for (int k = 0; k < D; ++k) {
+                            st.p[k] = out.rpt[(size_t)pt * D + k];
+                            st.rn[k] = out.rnrm[(size_t)pt * D + k];
+                        }
+                        st.uref = dirichlet<D>(S, rprim, slot.rt0, slot.rt1, nullptr, nullptr);
+                        ball_begin<D>(slot, S, a);
+                        if (out.rR != nullptr) {
+                            // a given ball radius (override_R, wos/wos.py:71-74): no bisection
+                            slot.ba = out.rR[pt];
+                            phase = PH_SETUP;
+                        }
+                    }
+                } else {
+                    if (FROM_REC && out.order != nullptr) idx = (long long)__ldg(&out.order[idx]);
+                    x.locate(idx, item, pt, wk);
+                    slot.tacc = 0.0f;
+                    const double W = TAN ? 1.0 : sample_weight(x, dLdu, item, pt);
+                    if (W == 0.0) {
+                        active = false;
+                    } else if (!FROM_REC) {
+                        float x0[3];
+                        walk_origin<D>(x.cfg(item), x.points(item), pt, wk, x0);
+                        w.start(x0, D);
+                        phase = PH_PRIMAL;
+                        first = true;
+                    } else {
+                        // the primal walk ran in the forward pass: start from its record
+                        const SceneView &S = x.scene(item);
+                        int code;
+                        if (D == 2) {
+                            const int2 wr = __ldg(reinterpret_cast<const int2 *>(out.wrec) + idx);
+                            code = wr.x;
+                            slot.rt0 = __int_as_float(wr.y);
+                            slot.rt1 = 0.0f;
+                        } else {
+                            const int4 wr = __ldg(reinterpret_cast<const int4 *>(out.wrec) + idx);
+                            code = wr.x;
+                            slot.rt0 = __int_as_float(wr.y);
+                            slot.rt1 = __int_as_float(wr.z);
+                        }
+                        if (code < 0) {
                             active = false;
                         } else {
+                            rprim = code & 0x3fffffff;
+                            const Rec rec = record_from<D>(S, rprim, slot.rt0, slot.rt1, (code & 0x40000000) != 0);
+                            int vid[3];
+                            float wts[3];
+                            st.uref = dirichlet<D>(S, rprim, slot.rt0, slot.rt1, vid, wts);
+                            const bool src = acc_src != nullptr &&
+                                             (!CTX::MULTI || (a.want_dsrc && x.cfg(item).include_source &&
+                                                              S.src_type != 0));
+                            if (TAN) {
+                                if (a.want_dg && out.tg != nullptr) {
 #pragma unroll
-                            for (int k = 0; k < D; ++k) {
-                                st.p[k] = rec.p[k];
-                                rn[k] = rec.n[k];
+                                    for (int s = 0; s < D; ++s)
+                                        slot.tacc = fmaf(wts[s], __ldg(&out.tg[vid[s]]), slot.tacc);
+                                }
+                                if (src && out.ts != nullptr) {
+#pragma unroll
+                                    for (int k = 0; k < 5; ++k)
+                                        slot.tacc = fmaf(__ldg(&out.wds[(size_t)idx * 5 + k]), __ldg(&out.ts[k]),
+                                                         slot.tacc);
+                                }
+                            } else {
+                                if (a.want_dg) {
+                                    double *dg = grad_dg(x, out, item);
+#pragma unroll
+                                    for (int s = 0; s < D; ++s) atomicAdd(&dg[vid[s]], W * (double)wts[s]);
+                                }
+                                if (src) {
+                                    if constexpr (CTX::MULTI) {
+                                        if (acc_item != item) {
+#pragma unroll
+                                            for (int k = 0; k < 5; ++k) {
+                                                if (acc_item >= 0 && acc_src[k * AS] != 0.0)
+                                                    atomicAdd(&out.dV[x.items[acc_item].ds_off + k], acc_src[k * AS]);
+                                                acc_src[k * AS] = 0.0;
+                                            }
+                                            acc_item = item;
+                                        }
+                                    }
+#pragma unroll
+                                    for (int k = 0; k < 5; ++k)
+                                        acc_src[k * AS] += W * (double)__ldg(&out.wds[(size_t)idx * 5 + k]);
+                                }
                             }
-                            ba = a.ball_eps;
-                            bb = S.half_min_extent;
-                            bk = 0;
-                            bwarm = -1;
-                            const float m = (ba + bb) * 0.5f;
+                            if (!a.want_dV || (TAN && out.tV == nullptr)) {
+                                if (TAN) out.tan[idx] = slot.tacc;
+                                active = false;
+                            } else {
 #pragma unroll
-                            for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m, st.p[k]);
-                            phase = PH_BALL;
+                                for (int k = 0; k < D; ++k) {
+                                    st.p[k] = rec.p[k];
+                                    st.rn[k] = rec.n[k];
+                                }
+                                ball_begin<D>(slot, S, a);
+                            }
                         }
                     }
                 }
+                if (phase == PH_SETUP) sr.dep = SEARCH_DONE;
+            }
+            if (!active) {
+                sr.dep = SEARCH_DONE;
+                phase = PH_IDLE;
             }
         }
-        if (ND_ONLY && active && phase == PH_ND_START && out.rR != nullptr) {
-            // a given ball radius (override_R, wos/wos.py:71-74): no bisection
-            st.uref = dirichlet<D>(S, rprim, rt0, rt1, nullptr, nullptr);
-            st.R = out.rR[pt];
-            nd_setup<D>(st, S, c, a, pt, wk);
-            nd_point<D>(st, qpos);
-            phase = PH_ANTI_START;
+        if (any && n_ball != 0 && (all || 8 * n_ball >= n_all)) {
+            if (active && sr.dep < 0 && (phase == PH_BALL || phase == PH_BALL_NEAR)) {
+                if (sr.dep == SEARCH_DONE) {
+                    const float m = phase == PH_BALL ? (slot.ba + slot.bb) * 0.5f : -1.0f;
+                    ball_take<D>(slot, lane_hit<D, BVH>(sr, x.scene(item), m), phase);
+                }
+                ball_m = ball_next<D>(slot, x.scene(item), rprim, phase, w.p);
+                sr.dep = phase == PH_SETUP ? SEARCH_DONE : SEARCH_NEED;
+            }
         }
-        if (ND_ONLY && active && phase == PH_ND_START) {
-            // no query needed to start: set up the bisection
-            st.uref = dirichlet<D>(S, rprim, rt0, rt1, nullptr, nullptr);
-            ba = a.ball_eps;
-            bb = S.half_min_extent;
-            bk = 0;
-            bwarm = -1;
-            const float m = (ba + bb) * 0.5f;
-#pragma unroll
-            for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m, st.p[k]);
-            phase = PH_BALL;
-        }
-        // PH_PRIMAL and PH_ND_START occur only in their own modes: testing the
-        // mode too compiles the other phases' code out of each instance, which
-        // lowers register pressure (records mode: C2 adjoint 8 % faster)
-        constexpr bool HAS_PRIMAL = MODE == ADJ_RECOMPUTE;
-        const bool walking = (HAS_PRIMAL && phase == PH_PRIMAL) || phase == PH_ANTI_WALK;
-        float x[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) x[k] = walking ? w.p[k] : qpos[k];
-        bool need = active;
-        float ball_m = -1.0f;
-        Hit pre{-1, INFINITY};
-        if (active && phase == PH_BALL) ball_precheck<D>(S, qpos, (ba + bb) * 0.5f, bwarm, rprim, need, ball_m, pre);
-        Hit hit = warp_queries<D, BVH, WL>(S, need, x, walking ? w.last : rprim, work, ball_m);
-        if (!active) continue;
-        if (phase == PH_BALL && (!need || (ball_m > 0.0f && hit.prim < 0))) hit = pre;
-        if (walking) w.last = hit.prim;
-        bool finish_anti = false;
-        float uq = 0.0f;
-        if (HAS_PRIMAL && phase == PH_PRIMAL) {
-            const int r = walker_advance<D>(w, S, hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt, wk,
-                                            ROLE_PRIMAL, want_src, cdf);
-            if (r == W_CONTINUE) continue;
-            if (r != W_VALID) {
-                active = false;
-                continue;
-            }
-            const Rec rec = closest_record<D>(S, w.p, hit.prim);
-            rprim = hit.prim;
-            rt0 = rec.t0;
-            rt1 = rec.t1;
-            int vid[3];
-            float wts[3];
-            st.uref = dirichlet<D>(S, rprim, rt0, rt1, vid, wts);
-            if (a.want_dg) {
-#pragma unroll
-                for (int s = 0; s < D; ++s) atomicAdd(&out.dg[vid[s]], W * (double)wts[s]);
-            }
-            if (want_src) {
-#pragma unroll
-                for (int k = 0; k < 5; ++k) acc_src[k * AS] += W * (double)w.ds[k];
-            }
-            if (!a.want_dV) {
-                active = false;
-                continue;
-            }
-#pragma unroll
-            for (int k = 0; k < D; ++k) {
-                st.p[k] = rec.p[k];
-                rn[k] = rec.n[k];
-            }
-            ba = a.ball_eps;
-            bb = S.half_min_extent;
-            bk = 0;
-            bwarm = -1;
-            const float m = (ba + bb) * 0.5f;
-#pragma unroll
-            for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m, st.p[k]);
-            phase = PH_BALL;
-            continue;
-        }
-        if (phase == PH_BALL) {
-            const float d = sqrtf(hit.d2);
-            const float m = (ba + bb) * 0.5f;
-            if (wosm::ball_accepts(d, m)) {
-                ba = m;
-            } else {
-                bb = m;
-                bwarm = hit.prim;
-            }
-            ++bk;
-            if (bk < 10) {
-                const float m2 = (ba + bb) * 0.5f;
-#pragma unroll
-                for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m2, st.p[k]);
-                continue;
-            }
-            st.R = ba;
-            nd_setup<D>(st, S, c, a, pt, wk);
-            nd_point<D>(st, qpos);
-            phase = PH_ANTI_START;
-            continue;
-        }
-        const uint32_t role = st.which == 0 ? ROLE_ANTI_A : ROLE_ANTI_B;
-        // the ball walk's first query (PH_ANTI_START) either ends it inside the
-        // epsilon2 shell or starts the walk; both walk phases then share one
-        // walker_advance (one inlined copy keeps the kernel's code small)
-        bool advance = phase == PH_ANTI_WALK;
-        if (phase == PH_ANTI_START) {
-            const float d = sqrtf(hit.d2);
-            if (d < a.epsilon2) {
-                const Rec r2 = closest_record<D>(S, qpos, hit.prim);
-                uq = dirichlet<D>(S, hit.prim, r2.t0, r2.t1, nullptr, nullptr);
-                finish_anti = true;
-            } else {
-                w.start(qpos, D);
+        if (any && n_step != 0 && (all || 4 * n_step >= n_all)) {
+            const bool walking = phase == PH_ANTI_WALK || (HAS_PRIMAL && phase == PH_PRIMAL && !first);
+            if (active && sr.dep == SEARCH_DONE && walking) {
+                const SceneView &S = x.scene(item);
+                const WalkCfg &c = x.cfg(item);
+                const bool anti = !HAS_PRIMAL || phase == PH_ANTI_WALK;
+                const Hit hit = lane_hit<D, BVH>(sr, S);
                 w.last = hit.prim;
-                phase = PH_ANTI_WALK;
-                advance = true;
-            }
-        }
-        if (advance) {
-            const int r = walker_advance<D>(w, S, hit, c, a.epsilon2, c.project != 0, false, pt, wk, role, false, cdf);
-            if (r == W_CONTINUE) continue;
-            if (r == W_VALID) {
-                const Rec r2 = closest_record<D>(S, w.p, hit.prim);
-                uq = dirichlet<D>(S, hit.prim, r2.t0, r2.t1, nullptr, nullptr);
-                if (with_src) uq += w.contrib;
-            }
-            finish_anti = true;
-        }
-        if (finish_anti) {
-            nd_accumulate<D>(st, a, uq);
-            st.which += 1;
-            if (st.which == 1) {
-                nd_point<D>(st, qpos);
-                phase = PH_ANTI_START;
-                continue;
-            }
-            float gn[3];
-            nd_finish<D>(st, S, c, a, pt, wk, with_src, gn);
-            if (ND_ONLY) {
-#pragma unroll
-                for (int k = 0; k < D; ++k) out.nd[(size_t)pt * D + k] = gn[k];
-            } else {
-                float gt[3];
-                tangent_derivative<D>(S, rprim, gt);
-                int vid[3];
-                float wts[3];
-                dirichlet<D>(S, rprim, rt0, rt1, vid, wts);
-                if (TAN) {
-                    // d(sample) = -(grad_n + grad_t) . dx, dx = sum_s wts_s dV[vid_s]
-#pragma unroll
-                    for (int s = 0; s < D; ++s)
-#pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            tacc = fmaf(-(wts[s] * (gn[k] + gt[k])), __ldg(&out.tV[(size_t)vid[s] * D + k]), tacc);
-                    out.tan[idx] = tacc;
+                const uint32_t role = !anti ? ROLE_PRIMAL : st.which == 0 ? ROLE_ANTI_A : ROLE_ANTI_B;
+                const int r = walker_advance<D>(w, S, hit, c, anti ? a.epsilon2 : c.eps, c.project != 0,
+                                                !anti && c.prevent_fd != 0, pt, wk, role,
+                                                HAS_PRIMAL && !anti && acc_src != nullptr, guide);
+                if (r == W_CONTINUE) {
+                    sr.dep = SEARCH_NEED;
+                } else if (anti) {
+                    phase = r == W_VALID ? PH_END_WALK : PH_END_NONE;
+                } else if (r == W_VALID) {
+                    phase = PH_PRIMAL_END;
                 } else {
-#pragma unroll
-                    for (int s = 0; s < D; ++s)
-#pragma unroll
-                        for (int k = 0; k < D; ++k)
-                            atomicAdd(&out.dV[(size_t)vid[s] * D + k], W * (double)(-(wts[s] * (gn[k] + gt[k]))));
+                    active = false;
+                    phase = PH_IDLE;
                 }
             }
-            active = false;
-            phase = PH_IDLE;
+        }
+        // a bisection's search begins only with its radius, in the part above
+        const bool hold = sr.dep == SEARCH_NEED && phase == PH_BALL && ball_m < 0.0f;
+        const int dep = sr.dep;
+        if (hold) sr.dep = SEARCH_DONE;
+        const bool walking = phase == PH_ANTI_WALK || (HAS_PRIMAL && phase == PH_PRIMAL);
+        lane_search<D, BVH>(sr, x, item, w.p, walking ? w.last : rprim, ball_m, stack, work);
+        if (hold) sr.dep = dep;
+    }
+    if constexpr (CTX::MULTI) {
+        if (acc_item >= 0) {
+#pragma unroll
+            for (int k = 0; k < 5; ++k)
+                if (acc_src[k * AS] != 0.0) atomicAdd(&out.dV[x.items[acc_item].ds_off + k], acc_src[k * AS]);
         }
     }
-    if constexpr (COUNT) {
-        if (c.count) flush_work<BVH>(work);
-    } else {
-        // never taken (counting launches use the COUNT instance); with this
-        // epilogue in place the kernel measured 2-5 % faster than without it
-        if (c.count) flush_work<BVH>(Work{0, 0, 0});
+}
+
+template <int D, bool BVH, int MODE, bool COUNT>
+__global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint(SceneView S, WalkCfg c, AdjCfg a,
+                                                const float *__restrict__ P,
+                                                long long total, const float *__restrict__ dLdu,
+                                                unsigned long long *counter, int chunk, int stack_entries,
+                                                int stage_cdf, AdjOut out) {
+    extern __shared__ float4 smem[];
+    const Smem sm = stage_smem(S, stage_cdf != 0, stack_entries, smem);
+    const bool want_src =
+        MODE != ADJ_ND_ONLY && a.want_dsrc && c.include_source && D == 2 && S.src_type != 0;
+    const AdjSmem<D> am = adj_smem<D>(sm.scratch, want_src);
+    if (want_src) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) am.acc[k * blockDim.x] = 0.0;
     }
-    if (want_src && !TAN) {
+    typename std::conditional<COUNT, Work, NoWork>::type work{};
+    adjoint_lanes<D, BVH, MODE>(OneScene<D>{S, c, P}, a, 0, total, dLdu, counter, chunk, out, sm.guide, sm.stack,
+                                *am.slot, want_src ? am.acc : nullptr, work);
+    if constexpr (COUNT) flush_work(work);
+    if (want_src && MODE != ADJ_TANGENT) {
 #pragma unroll
         for (int k = 0; k < 5; ++k) {
-            double v = acc_src[k * AS];
+            double v = am.acc[k * blockDim.x];
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
             if ((threadIdx.x & 31) == 0 && v != 0.0) atomicAdd(&out.dsrc[k], v);
@@ -1218,7 +1418,7 @@ WalkCfg make_cfg(const wos_params &p) {
 }
 
 struct Shape {
-    int grid, block, n_top, stage_cdf;
+    int grid, block, stack, stage_cdf;
     size_t smem;
 };
 
@@ -1227,12 +1427,9 @@ static int shape_for(Kern kern, const SceneImpl &S, int D, bool bvh, bool want_c
                      int thread_bytes = 0, int max_block = 512) {
     const wos_launch_config &cfg = g_cfg[D - 2];
     sh.block = std::min(cfg.block_threads, max_block);
-    // the persistent kernels query the wide tree cooperatively; no binary-LBVH
-    // nodes are staged
-    sh.n_top = 0;
+    sh.stack = bvh ? tree_stack_entries(S.tree_depth) : 0;
     sh.stage_cdf = want_cdf ? 1 : 0;
-    sh.smem = smem_bytes(want_cdf ? S.n_guide : -1, sh.block, thread_bytes);
-    (void)bvh;
+    sh.smem = smem_bytes(want_cdf ? S.n_guide : -1, sh.block, sh.stack, thread_bytes);
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -1248,7 +1445,7 @@ static int shape_for(Kern kern, const SceneImpl &S, int D, bool bvh, bool want_c
 }
 
 
-template <int D, bool BVH, int WL, bool COUNT>
+template <int D, bool BVH, bool COUNT>
 static int launch_walk_t(const SceneImpl &S, const float *P, long long total, const wos_params &p, bool records,
                          const WalkOut &out, unsigned long long *counter, cudaStream_t st) {
     const SceneView v = S.view();
@@ -1257,19 +1454,19 @@ static int launch_walk_t(const SceneImpl &S, const float *P, long long total, co
     Shape sh;
     int rc;
     if (records)
-        rc = shape_for(k_walk<D, BVH, true, WL, COUNT>, S, D, BVH, want_cdf, sh);
+        rc = shape_for(k_walk<D, BVH, true, COUNT>, S, D, BVH, want_cdf, sh);
     else
-        rc = shape_for(k_walk<D, BVH, false, WL, COUNT>, S, D, BVH, want_cdf, sh);
+        rc = shape_for(k_walk<D, BVH, false, COUNT>, S, D, BVH, want_cdf, sh);
     if (rc) return rc;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
     const int chunk = g_cfg[D - 2].chunk;
     if (records)
-        k_walk<D, BVH, true, WL, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, P, total, counter, chunk,
-                                                                             sh.n_top, sh.stage_cdf, out);
+        k_walk<D, BVH, true, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, P, total, counter, chunk,
+                                                                             sh.stack, sh.stage_cdf, out);
     else
-        k_walk<D, BVH, false, WL, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, P, total, counter, chunk,
-                                                                              sh.n_top, sh.stage_cdf, out);
+        k_walk<D, BVH, false, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, P, total, counter, chunk,
+                                                                              sh.stack, sh.stage_cdf, out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_walk launch");
     return 0;
@@ -1279,21 +1476,14 @@ int launch_walk(const SceneImpl &S, const float *P, long long total, const wos_p
                 const WalkOut &out, unsigned long long *counter, cudaStream_t st) {
     if (total == 0) return 0;
     const bool bvh = p.use_bvh != 0;
-    const int wl = specialised_depth(S.wt_levels);
-    // work accounting runs the any-depth instance that keeps counters
+    // work accounting runs the instances that keep counters
     const bool count = work_counting_enabled() != 0;
-#define WOS_WALK(D_)                                                                                      \
-    if (count) {                                                                                          \
-        if (!bvh) return launch_walk_t<D_, false, 0, true>(S, P, total, p, records, out, counter, st);    \
-        return launch_walk_t<D_, true, 0, true>(S, P, total, p, records, out, counter, st);               \
-    }                                                                                                     \
-    if (!bvh) return launch_walk_t<D_, false, 0, false>(S, P, total, p, records, out, counter, st);       \
-    switch (wl) {                                                                                         \
-        case 1: return launch_walk_t<D_, true, 1, false>(S, P, total, p, records, out, counter, st);      \
-        case 2: return launch_walk_t<D_, true, 2, false>(S, P, total, p, records, out, counter, st);      \
-        case 3: return launch_walk_t<D_, true, 3, false>(S, P, total, p, records, out, counter, st);      \
-        default: return launch_walk_t<D_, true, 0, false>(S, P, total, p, records, out, counter, st);     \
-    }
+#define WOS_WALK(D_)                                                                                                 \
+    if (count)                                                                                                       \
+        return bvh ? launch_walk_t<D_, true, true>(S, P, total, p, records, out, counter, st)                        \
+                   : launch_walk_t<D_, false, true>(S, P, total, p, records, out, counter, st);                      \
+    return bvh ? launch_walk_t<D_, true, false>(S, P, total, p, records, out, counter, st)                           \
+               : launch_walk_t<D_, false, false>(S, P, total, p, records, out, counter, st);
     if (S.dim == 2) {
         WOS_WALK(2)
     }
@@ -1435,11 +1625,14 @@ __device__ void soft_tangents(const SceneView &S, const float *x, const float *x
     }
 }
 
-template <int D, bool BVH, int WL>
+template <int D, bool BVH>
 __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const float *__restrict__ P,
                                                    long long total, unsigned long long *counter, int chunk,
+                                                   int stack_entries,
                                                    const float *__restrict__ tV, const float *__restrict__ tg,
                                                    float *vals, float *tans) {
+    extern __shared__ float4 smem[];
+    const Smem sm = stage_smem(S, false, stack_entries, smem);
     Queue q{0, 0, false};
     bool active = false;
     long long idx = 0;
@@ -1451,6 +1644,8 @@ __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const
     const float eps = c.eps;
     const bool want_tan = tans != nullptr;
     Work work{0, 0, 0};
+    Search<D> sr;
+    sr.dep = SEARCH_DONE;
     for (;;) {
         const bool was = active;
         if (!refill(q, active, idx, counter, total, chunk)) break;
@@ -1464,9 +1659,23 @@ __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const
             i = 0;
             last = -1;
             fresh = true;
+            sr.dep = SEARCH_NEED;
         }
-        const Hit hit = warp_queries<D, BVH, WL>(S, active, p, last, work);
-        if (!active) continue;
+        Hit hit{-1, INFINITY};
+        if (BVH) {
+            if (active && sr.dep == SEARCH_NEED) {
+                work.nq += 1;
+                search_begin<D>(sr, S, p, last, -1.0f);
+            }
+            const int n = __popc(__ballot_sync(0xffffffffu, active));
+            search_run<D, false>(sr, &S, 0, p, sm.stack, search_keep<D>(n), work);
+            if (!active || sr.dep >= 0) continue;
+            hit = search_hit<D>(sr, S);
+        } else {
+            if (!active) continue;
+            hit = nearest_brute<D>(S, p, work);
+        }
+        sr.dep = SEARCH_NEED;
         last = hit.prim;
         bool done = hit.prim < 0;
         if (!done && fresh) {
@@ -1521,7 +1730,7 @@ __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const
         }
         ++i;
     }
-    if (c.count) flush_work<BVH>(work);
+    if (c.count) flush_work(work);
 }
 
 // ------------------------------------------------------------------ soft-edge walk, reverse mode
@@ -1634,30 +1843,45 @@ __global__ void __launch_bounds__(128) k_soft_adjoint(SceneView S, WalkCfg c, co
                                                       long long w0, long long nchunk,
                                                       const float *__restrict__ dLdu, float4 *state, float *sbeta,
                                                       double *dV, double *dg) {
+    extern __shared__ float4 smem[];
+    unsigned *stack = reinterpret_cast<unsigned *>(smem) + threadIdx.x;
+    const PlainScene<D> x0{S};
     const float eps = c.eps;
-    for (long long l = blockIdx.x * (long long)blockDim.x + threadIdx.x; l < nchunk;
-         l += (long long)gridDim.x * blockDim.x) {
-        const long long idx = w0 + l;
-        const uint32_t pt = (uint32_t)(idx / c.nwalks);
-        const uint32_t wk = c.walk_offset + (uint32_t)(idx - (long long)pt * c.nwalks);
-        const float W = dLdu[pt] / (float)c.nwalks;
-        if (W == 0.0f) continue;
-        float p[3];
-        walk_origin<D>(c, P, pt, wk, p);
-        Work work{0, 0, 0};
+    // whole warps stay in the loops: the searches are the warp's
+    const long long warp0 = blockIdx.x * (long long)blockDim.x + (threadIdx.x & ~31u);
+    for (long long l0 = warp0; l0 < nchunk; l0 += (long long)gridDim.x * blockDim.x) {
+        const long long l = l0 + (threadIdx.x & 31), idx = w0 + l;
+        bool ok = l < nchunk;
+        uint32_t pt = 0, wk = 0;
+        float p[3] = {0.0f, 0.0f, 0.0f}, W = 0.0f;
+        if (ok) {
+            split_index(idx, c.nwalks, pt, wk);
+            wk += c.walk_offset;
+            W = dLdu[pt] / (float)c.nwalks;
+            ok = W != 0.0f;
+            walk_origin<D>(c, P, pt, wk, p);
+        }
+        NoWork work;
+        Search<D> sr;
+        sr.dep = SEARCH_DONE;
         float beta = 1.0f;
-        bool ok = true;
-        for (int i = 0; i < c.nsteps; ++i) {
-            const Hit hit = query<D, BVH>(S, p, nullptr, 0, work);
+        int last = -1;
+        for (int i = 0; i < c.nsteps && __any_sync(0xffffffffu, ok); ++i) {
+            sr.dep = ok ? SEARCH_NEED : SEARCH_DONE;
+            while (__any_sync(0xffffffffu, sr.dep != SEARCH_DONE))
+                lane_search<D, BVH>(sr, x0, 0, p, last, -1.0f, stack, work);
+            if (!ok) continue;
+            const Hit hit = lane_hit<D, BVH>(sr, S);
+            last = hit.prim;
             if (hit.prim < 0 || (i == 0 && !c.double_sided && !inside_test<D>(S, p, hit, nullptr))) {
                 ok = false;  // the walk's value is 0 (k_walk_soft): no derivative
-                break;
+                continue;
             }
             state[(size_t)i * nchunk + l] = make_float4(p[0], p[1], D == 3 ? p[2] : 0.0f, __int_as_float(hit.prim));
             sbeta[(size_t)i * nchunk + l] = beta;
             const float d = sqrtf(hit.d2);
             beta = beta * (fminf(d, eps) / eps);
-            if (i == c.nsteps - 1) break;
+            if (i == c.nsteps - 1) continue;
             float dir[3];
             soft_dir<D>(c, pt, wk, i, dir);
             for (int k = 0; k < D; ++k) p[k] = fmaf(dir[k], d, p[k]);
@@ -1722,10 +1946,11 @@ static int launch_soft_adjoint_t(const SceneImpl &S, const float *P, long long t
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const size_t smem = smem_bytes(-1, 128, BVH ? tree_stack_entries(S.tree_depth) : 0, 0);
     for (long long w0 = 0; w0 < total && e == cudaSuccess; w0 += chunk) {
         const long long nc = std::min(chunk, total - w0);
         const int grid = (int)std::min<long long>((nc + 127) / 128, (long long)sms * 16);
-        k_soft_adjoint<D, BVH><<<grid, 128, 0, st>>>(v, c, P, w0, nc, dLdu, state, sbeta, dV, dg);
+        k_soft_adjoint<D, BVH><<<grid, 128, smem, st>>>(v, c, P, w0, nc, dLdu, state, sbeta, dV, dg);
         e = cudaGetLastError();
     }
     cudaFreeAsync(state, st);
@@ -1744,7 +1969,7 @@ int launch_soft_adjoint(const SceneImpl &S, const float *P, long long total, con
                : launch_soft_adjoint_t<3, false>(S, P, total, p, dLdu, dV, dg, st);
 }
 
-template <int D, bool BVH, int WL>
+template <int D, bool BVH>
 static int launch_soft_t(const SceneImpl &S, const float *P, long long total, const wos_params &p, const float *tV,
                          const float *tg, float *vals, float *tans, unsigned long long *counter, cudaStream_t st) {
     const SceneView v = S.view();
@@ -1753,12 +1978,16 @@ static int launch_soft_t(const SceneImpl &S, const float *P, long long total, co
     int dev = 0, sms = 148, per = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_walk_soft<D, BVH, WL>, 256, 0);
+    const int stack = BVH ? tree_stack_entries(S.tree_depth) : 0;
+    const size_t smem = smem_bytes(-1, 256, stack, 0);
+    cudaError_t e = cudaFuncSetAttribute(k_walk_soft<D, BVH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(k_walk_soft)");
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_walk_soft<D, BVH>, 256, smem);
     if (e != cudaSuccess) return fail_cuda(e, "occupancy(k_walk_soft)");
     grid = std::max(1, per) * sms;
     e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
-    k_walk_soft<D, BVH, WL><<<grid, 256, 0, st>>>(v, c, P, total, counter, 32, tV, tg, vals, tans);
+    k_walk_soft<D, BVH><<<grid, 256, smem, st>>>(v, c, P, total, counter, 32, stack, tV, tg, vals, tans);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_walk_soft launch");
     return 0;
@@ -1769,10 +1998,10 @@ int launch_walk_soft(const SceneImpl &S, const float *P, long long total, const 
     if (total == 0) return 0;
     const bool bvh = p.use_bvh != 0;
     if (S.dim == 2)
-        return bvh ? launch_soft_t<2, true, 0>(S, P, total, p, tV, tg, vals, tans, counter, st)
-                   : launch_soft_t<2, false, 0>(S, P, total, p, tV, tg, vals, tans, counter, st);
-    return bvh ? launch_soft_t<3, true, 0>(S, P, total, p, tV, tg, vals, tans, counter, st)
-               : launch_soft_t<3, false, 0>(S, P, total, p, tV, tg, vals, tans, counter, st);
+        return bvh ? launch_soft_t<2, true>(S, P, total, p, tV, tg, vals, tans, counter, st)
+                   : launch_soft_t<2, false>(S, P, total, p, tV, tg, vals, tans, counter, st);
+    return bvh ? launch_soft_t<3, true>(S, P, total, p, tV, tg, vals, tans, counter, st)
+               : launch_soft_t<3, false>(S, P, total, p, tV, tg, vals, tans, counter, st);
 }
 
 int launch_walk_plain(const SceneImpl &S, const float *P, long long total, const wos_params &p, float *values,
@@ -1809,21 +2038,33 @@ int launch_reduce(const float *vals, int n, int nw, double *mean, double *var, c
     return 0;
 }
 
+// Shared memory of the query kernels' search stacks.
+template <int D, bool BVH>
+static size_t query_smem(const SceneImpl &S) {
+    return BVH ? smem_bytes(-1, QUERY_THREADS, tree_stack_entries(S.tree_depth), 0) : 0;
+}
+
 int launch_closest(const SceneImpl &S, const float *P, int n, bool bvh, const QueryOut &o, cudaStream_t st) {
     if (n == 0) return 0;
     const SceneView v = S.view();
-    const int B = 128, G = (n + B - 1) / B;
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // a point per lane, up to about the resident lanes
+    const int G = (int)std::min<long long>(((long long)n + QUERY_THREADS - 1) / QUERY_THREADS, (long long)sms * 8);
+#define WOS_CLOSEST(D_, B_) k_closest<D_, B_><<<G, QUERY_THREADS, query_smem<D_, B_>(S), st>>>(v, P, n, o)
     if (S.dim == 2) {
         if (bvh)
-            k_closest<2, true><<<G, B, 0, st>>>(v, P, n, o);
+            WOS_CLOSEST(2, true);
         else
-            k_closest<2, false><<<G, B, 0, st>>>(v, P, n, o);
+            WOS_CLOSEST(2, false);
     } else {
         if (bvh)
-            k_closest<3, true><<<G, B, 0, st>>>(v, P, n, o);
+            WOS_CLOSEST(3, true);
         else
-            k_closest<3, false><<<G, B, 0, st>>>(v, P, n, o);
+            WOS_CLOSEST(3, false);
     }
+#undef WOS_CLOSEST
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_closest launch");
     return 0;
@@ -1833,24 +2074,26 @@ int launch_ball(const SceneImpl &S, const uint8_t *valid, const float *pt, const
                 bool bvh, float *R, cudaStream_t st) {
     if (n == 0) return 0;
     const SceneView v = S.view();
-    const int B = 128, G = (n + B - 1) / B;
+    const int G = (int)(((long long)n + QUERY_THREADS - 1) / QUERY_THREADS);
+#define WOS_BALL(D_, B_) k_ball<D_, B_><<<G, QUERY_THREADS, query_smem<D_, B_>(S), st>>>(v, valid, pt, nrm, n, eps, R)
     if (S.dim == 2) {
         if (bvh)
-            k_ball<2, true><<<G, B, 0, st>>>(v, valid, pt, nrm, n, eps, R);
+            WOS_BALL(2, true);
         else
-            k_ball<2, false><<<G, B, 0, st>>>(v, valid, pt, nrm, n, eps, R);
+            WOS_BALL(2, false);
     } else {
         if (bvh)
-            k_ball<3, true><<<G, B, 0, st>>>(v, valid, pt, nrm, n, eps, R);
+            WOS_BALL(3, true);
         else
-            k_ball<3, false><<<G, B, 0, st>>>(v, valid, pt, nrm, n, eps, R);
+            WOS_BALL(3, false);
     }
+#undef WOS_BALL
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_ball launch");
     return 0;
 }
 
-template <int D, bool BVH, int ND, int WL, bool COUNT>
+template <int D, bool BVH, int ND, bool COUNT>
 static int launch_adjoint_t(const SceneImpl &S, const float *P, long long total, const wos_params &p,
                             const AdjCfg &a, const float *dLdu, const AdjOut &out, unsigned long long *counter,
                             cudaStream_t st) {
@@ -1859,14 +2102,14 @@ static int launch_adjoint_t(const SceneImpl &S, const float *P, long long total,
     const bool want_cdf = D == 2 && S.src_type != 0 && p.use_IS_for_greens;
     Shape sh;
     const bool want_acc = ND != ADJ_ND_ONLY && a.want_dsrc && p.include_source && S.src_type != 0 && D == 2;
-    int rc = shape_for(k_adjoint<D, BVH, ND, WL, COUNT>, S, D, BVH, want_cdf, sh, adj_thread_bytes<D>(want_acc),
+    int rc = shape_for(k_adjoint<D, BVH, ND, COUNT>, S, D, BVH, want_cdf, sh, adj_thread_bytes<D>(want_acc),
                        256);
     if (rc) return rc;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
     const int chunk = std::max(1, g_cfg[D - 2].chunk / 2);
-    k_adjoint<D, BVH, ND, WL, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, a, P, total, dLdu, counter, chunk,
-                                                                         sh.n_top, sh.stage_cdf, out);
+    k_adjoint<D, BVH, ND, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, a, P, total, dLdu, counter, chunk,
+                                                                         sh.stack, sh.stage_cdf, out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_adjoint launch");
     return 0;
@@ -1876,35 +2119,29 @@ int launch_adjoint(const SceneImpl &S, const float *P, long long total, const wo
                    const float *dLdu, int mode, const AdjOut &out, unsigned long long *counter, cudaStream_t st) {
     if (total == 0) return 0;
     const bool bvh = p.use_bvh != 0;
-    const int wl = specialised_depth(S.wt_levels);
-    // work accounting runs the any-depth instance that keeps counters
+    // work accounting runs the instances that keep counters
     const bool count = work_counting_enabled() != 0;
-#define WOS_ADJ_M(D_, B_, W_, C_)                                                                                   \
-    switch (mode) {                                                                                                 \
-        case ADJ_ND_ONLY:                                                                                           \
-            return launch_adjoint_t<D_, B_, ADJ_ND_ONLY, W_, C_>(S, P, total, p, a, dLdu, out, counter, st);        \
-        case ADJ_FROM_RECORDS:                                                                                      \
-            return launch_adjoint_t<D_, B_, ADJ_FROM_RECORDS, W_, C_>(S, P, total, p, a, dLdu, out, counter, st);   \
-        case ADJ_TANGENT:                                                                                           \
-            return launch_adjoint_t<D_, B_, ADJ_TANGENT, W_, C_>(S, P, total, p, a, dLdu, out, counter, st);        \
-        default: return launch_adjoint_t<D_, B_, ADJ_RECOMPUTE, W_, C_>(S, P, total, p, a, dLdu, out, counter, st); \
+#define WOS_ADJ_M(D_, B_, C_)                                                                                    \
+    switch (mode) {                                                                                              \
+        case ADJ_ND_ONLY:                                                                                        \
+            return launch_adjoint_t<D_, B_, ADJ_ND_ONLY, C_>(S, P, total, p, a, dLdu, out, counter, st);         \
+        case ADJ_FROM_RECORDS:                                                                                   \
+            return launch_adjoint_t<D_, B_, ADJ_FROM_RECORDS, C_>(S, P, total, p, a, dLdu, out, counter, st);    \
+        case ADJ_TANGENT:                                                                                        \
+            return launch_adjoint_t<D_, B_, ADJ_TANGENT, C_>(S, P, total, p, a, dLdu, out, counter, st);         \
+        default: return launch_adjoint_t<D_, B_, ADJ_RECOMPUTE, C_>(S, P, total, p, a, dLdu, out, counter, st);  \
     }
-#define WOS_ADJ(D_)                          \
-    if (count) {                             \
-        if (!bvh) {                          \
-            WOS_ADJ_M(D_, false, 0, true)    \
-        }                                    \
-        WOS_ADJ_M(D_, true, 0, true)         \
-    }                                        \
-    if (!bvh) {                              \
-        WOS_ADJ_M(D_, false, 0, false)       \
-    }                                        \
-    switch (wl) {                            \
-        case 1: WOS_ADJ_M(D_, true, 1, false) \
-        case 2: WOS_ADJ_M(D_, true, 2, false) \
-        case 3: WOS_ADJ_M(D_, true, 3, false) \
-        default: WOS_ADJ_M(D_, true, 0, false) \
-    }
+#define WOS_ADJ(D_)                      \
+    if (count) {                         \
+        if (!bvh) {                      \
+            WOS_ADJ_M(D_, false, true)   \
+        }                                \
+        WOS_ADJ_M(D_, true, true)        \
+    }                                    \
+    if (!bvh) {                          \
+        WOS_ADJ_M(D_, false, false)      \
+    }                                    \
+    WOS_ADJ_M(D_, true, false)
     if (S.dim == 2) {
         WOS_ADJ(2)
     }
@@ -2014,19 +2251,7 @@ int launch_add_f64(const double *src, float *dst, long long n, cudaStream_t st) 
 // walk index space is the concatenation of every item's n x nwalks walks in
 // item order (scene-major), so warps move through the items together and each
 // scene's trees stay resident in L2 while its walks run.  Each lane carries
-// its item; the cooperative query serves one lane's item at a time.
-
-__device__ __forceinline__ int find_item(const BatchItemDev *__restrict__ items, int n_items, long long idx) {
-    int lo = 0, hi = n_items - 1;  // last item with walk_begin <= idx
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (__ldg(&items[mid].walk_begin) <= idx)
-            lo = mid;
-        else
-            hi = mid - 1;
-    }
-    return lo;
-}
+// its item.
 
 __device__ __forceinline__ int find_item_point(const BatchItemDev *__restrict__ items, int n_items, int p) {
     int lo = 0, hi = n_items - 1;
@@ -2040,125 +2265,19 @@ __device__ __forceinline__ int find_item_point(const BatchItemDev *__restrict__ 
     return lo;
 }
 
-template <int D, int WL = 0, class WK>
-__device__ __forceinline__ Hit warp_queries_batch(const SceneView *__restrict__ views, bool active, int item,
-                                                  const float *x, int warm, WK &work, float ball_m = -1.0f) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    Hit mine{-1, INFINITY};
-    unsigned act = __ballot_sync(FULL, active);
-    // per-point parts of each search, every lane for its own point at once
-    // (as in warp_queries)
-    float lim = 0.0f, wd2 = INFINITY;
-    if (active) {
-        const SceneView &Si = views[item];
-        const float tol2 = prune_tol2<D>(Si, x);
-        if (ball_m > 0.0f) {
-            lim = wball_bound(ball_m, tol2);
-        } else {
-            lim = tol2;
-            if (warm >= 0) wd2 = prim_d2<D>(Si, warm, x);
-        }
-    }
-    while (act) {
-        const int j = __ffs(act) - 1;
-        act &= act - 1u;
-        float q[3];
-        q[0] = __shfl_sync(FULL, x[0], j);
-        q[1] = __shfl_sync(FULL, x[1], j);
-        q[2] = D == 3 ? __shfl_sync(FULL, x[2], j) : 0.0f;
-        const int wp = __shfl_sync(FULL, warm, j);
-        const int it = __shfl_sync(FULL, item, j);
-        const float bm = __shfl_sync(FULL, ball_m, j);
-        const float lj = __shfl_sync(FULL, lim, j);
-        const float wj = __shfl_sync(FULL, wd2, j);
-        const SceneView &Sj = views[it];
-        Hit h{-1, INFINITY};
-        if (bm > 0.0f) {
-            wball_b<D, WL>(Sj, q, lj, bm, h, work);
-        } else {
-            if (wp >= 0) {
-                h.prim = wp;
-                h.d2 = wj;
-            }
-            h = wquery_tol<D, WL>(Sj, q, h, lj, work);
-        }
-        if (lane == j) mine = h;
-    }
-    return mine;
-}
-
 // One launch covers a run of items whose walks occupy [base, base + total)
-// of the group's walk index space; WL > 0: every item's tree has WL levels.
-template <int D, int WL, bool COUNT>
-__global__ void __launch_bounds__(512) k_walk_batch(const SceneView *__restrict__ views,
+// of the group's walk index space.
+template <int D, bool COUNT>
+__global__ void __launch_bounds__(512, 2) k_walk_batch(const SceneView *__restrict__ views,
                                                    const WalkCfg *__restrict__ cfgs,
                                                    const BatchItemDev *__restrict__ items, int n_items,
                                                    long long base, long long total, unsigned long long *counter,
-                                                   int chunk, WalkOut out, int count_work) {
-    Queue q{0, 0, false};
-    bool active = false;
-    long long idx = 0;
-    int item = 0;
-    uint32_t pt = 0, wk = 0;
-    Walker w;
-    w.last = -1;
+                                                   int chunk, WalkOut out) {
+    extern __shared__ float4 smem[];
     typename std::conditional<COUNT, Work, NoWork>::type work{};
-    for (;;) {
-        const bool was = active;
-        if (!refill(q, active, idx, counter, total, chunk)) break;
-        if (active && !was) {
-            idx += base;
-            item = find_item(items, n_items, idx);
-            const BatchItemDev &it = items[item];
-            const long long local = idx - it.walk_begin;
-            pt = (uint32_t)(local / it.nwalks);
-            wk = cfgs[item].walk_offset + (uint32_t)(local - (long long)pt * it.nwalks);
-            float x0[3];
-            walk_origin<D>(cfgs[item], it.P, pt, wk, x0);
-            w.start(x0, D);
-        }
-        const Hit hit = warp_queries_batch<D, WL>(views, active, item, w.p, w.last, work);
-        if (!active) continue;
-        const SceneView &S = views[item];
-        const WalkCfg &c = cfgs[item];
-        w.last = hit.prim;
-        const int r = walker_advance<D>(w, S, hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt, wk, ROLE_PRIMAL,
-                                        out.wds != nullptr, S.guide);
-        if (r == W_CONTINUE) continue;
-        active = false;
-        float v = 0.0f;
-        Rec rec;
-        if (r == W_VALID) {
-            rec = closest_record<D>(S, w.p, hit.prim);
-            v = dirichlet<D>(S, hit.prim, rec.t0, rec.t1, nullptr, nullptr);
-            if (c.include_source) v += w.contrib;
-            if (!isfinite(v)) atomicOr(&g_status, ST_NONFINITE);
-        }
-        out.values[idx] = v;
-        if (out.wrec) {
-            if (D == 2) {
-                reinterpret_cast<int2 *>(out.wrec)[idx] =
-                    r == W_VALID ? make_int2(hit.prim | (rec.flip ? 0x40000000 : 0), __float_as_int(rec.t0))
-                                 : make_int2(-1, 0);
-            } else {
-                reinterpret_cast<int4 *>(out.wrec)[idx] =
-                    r == W_VALID ? make_int4(hit.prim | (rec.flip ? 0x40000000 : 0), __float_as_int(rec.t0),
-                                             __float_as_int(rec.t1), 0)
-                                 : make_int4(-1, 0, 0, 0);
-            }
-        }
-        if (out.wds) {
-#pragma unroll
-            for (int k = 0; k < 5; ++k) out.wds[(size_t)idx * 5 + k] = r == W_VALID ? w.ds[k] : 0.0f;
-        }
-    }
-    if constexpr (COUNT) {
-        if (count_work) flush_work<true>(work);
-    } else {
-        // never taken; kept for the same reason as in k_walk
-        if (count_work) flush_work<true>(Work{0, 0, 0});
-    }
+    walk_lanes<D, true, false>(ManyScenes<D>{views, cfgs, items, n_items}, base, total, counter, chunk, out,
+                               views[0].guide, reinterpret_cast<unsigned *>(smem) + threadIdx.x, work);
+    if constexpr (COUNT) flush_work(work);
 }
 
 // Per-point FP64 mean / variance over the concatenated point space.
@@ -2213,221 +2332,28 @@ __global__ void k_loss_batch(const double *__restrict__ mean, const BatchItemDev
     if (threadIdx.x == 0) loss[blockIdx.x] = red[0];
 }
 
-// Adjoint of every item, starting from the forward records.  Gradients go to
-// per-item FP64 accumulators (acc + it.dV_off / dg_off / ds_off).
-template <int D, int WL, bool COUNT>
+// Adjoint of every item, starting from the forward records (out.wrec, out.wds).
+// Gradients go to per-item FP64 accumulators (out.dV + dV_off / dg_off / ds_off).
+template <int D, bool COUNT>
 __global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint_batch(
     const SceneView *__restrict__ views, const WalkCfg *__restrict__ cfgs, AdjCfg a,
     const BatchItemDev *__restrict__ items, int n_items, long long base, long long total,
-    const float *__restrict__ dLdu,
-    unsigned long long *counter, int chunk, const int *__restrict__ wrec, const float *__restrict__ wds, double *acc,
-    int count_work, const unsigned *__restrict__ order) {
+    const float *__restrict__ dLdu, unsigned long long *counter, int chunk, AdjOut out, int stack_entries) {
     extern __shared__ float4 smem[];
+    unsigned *stack = reinterpret_cast<unsigned *>(smem);
     // source-gradient accumulators only when the launch has source derivatives
     // (the launcher sizes shared memory the same way)
-    const bool acc_on = D == 2 && wds != nullptr;  // source derivatives exist in 2D only
-    const AdjSmem<D> am = adj_smem<D>(reinterpret_cast<double *>(smem), acc_on);
-    AdjSlot<D> &slot = *am.slot;
-    double *acc_src = am.acc;  // k-th accumulator at acc_src[k * blockDim.x]
-    const int AS = blockDim.x;
+    const bool acc_on = D == 2 && out.wds != nullptr;  // source derivatives exist in 2D only
+    const AdjSmem<D> am = adj_smem<D>(reinterpret_cast<double *>(stack + (size_t)blockDim.x * stack_entries), acc_on);
     if (acc_on) {
 #pragma unroll
-        for (int k = 0; k < 5; ++k) acc_src[k * AS] = 0.0;
+        for (int k = 0; k < 5; ++k) am.acc[k * blockDim.x] = 0.0;
     }
-    int acc_item = -1;  // item whose source gradient acc_src holds
-    NdState<D> &st = slot.st;
-    float *rn = st.rn;
-    float &rt0 = slot.rt0, &rt1 = slot.rt1;
-    float &ba = slot.ba, &bb = slot.bb;
-    int &bk = slot.bk;
-    int &bwarm = slot.bwarm;
-    Queue q{0, 0, false};
-    bool active = false;
-    long long idx = 0;
-    int item = 0;
-    uint32_t pt = 0, wk = 0;
-    int phase = PH_IDLE;
-    double W = 0.0;
-    Walker w;
-    int rprim = 0;
-    float qpos[3] = {0, 0, 0};
     typename std::conditional<COUNT, Work, NoWork>::type work{};
-    w.last = -1;
-    for (;;) {
-        const bool was = active;
-        if (!refill(q, active, idx, counter, total, chunk)) break;
-        if (active && !was) {
-            idx += base;
-            if (order != nullptr) idx = (long long)__ldg(&order[idx]);
-            item = find_item(items, n_items, idx);
-            const BatchItemDev &it = items[item];
-            const SceneView &S = views[item];
-            const WalkCfg &c = cfgs[item];
-            const long long local = idx - it.walk_begin;
-            pt = (uint32_t)(local / it.nwalks);
-            wk = c.walk_offset + (uint32_t)(local - (long long)pt * it.nwalks);
-            W = (double)__ldg(&dLdu[it.point_begin + pt]) / it.nwalks;
-            phase = PH_BALL;
-            int code = -1;
-            if (D == 2) {
-                const int2 wr = __ldg(reinterpret_cast<const int2 *>(wrec) + idx);
-                code = wr.x;
-                rt0 = __int_as_float(wr.y);
-                rt1 = 0.0f;
-            } else {
-                const int4 wr = __ldg(reinterpret_cast<const int4 *>(wrec) + idx);
-                code = wr.x;
-                rt0 = __int_as_float(wr.y);
-                rt1 = __int_as_float(wr.z);
-            }
-            if (W == 0.0 || code < 0) {
-                active = false;
-            } else {
-                rprim = code & 0x3fffffff;
-                const Rec rec = record_from<D>(S, rprim, rt0, rt1, (code & 0x40000000) != 0);
-                int vid[3];
-                float wts[3];
-                st.uref = dirichlet<D>(S, rprim, rt0, rt1, vid, wts);
-                if (a.want_dg) {
-#pragma unroll
-                    for (int s2 = 0; s2 < D; ++s2) atomicAdd(&acc[it.dg_off + vid[s2]], W * (double)wts[s2]);
-                }
-                if (acc_on && a.want_dsrc && c.include_source && S.src_type != 0) {
-                    if (acc_item != item) {
-                        if (acc_item >= 0) {
-#pragma unroll
-                            for (int k = 0; k < 5; ++k)
-                                if (acc_src[k * AS] != 0.0)
-                                    atomicAdd(&acc[items[acc_item].ds_off + k], acc_src[k * AS]);
-                        }
-#pragma unroll
-                        for (int k = 0; k < 5; ++k) acc_src[k * AS] = 0.0;
-                        acc_item = item;
-                    }
-#pragma unroll
-                    for (int k = 0; k < 5; ++k) acc_src[k * AS] += W * (double)__ldg(&wds[(size_t)idx * 5 + k]);
-                }
-                if (!a.want_dV) {
-                    active = false;
-                } else {
-#pragma unroll
-                    for (int k = 0; k < D; ++k) {
-                        st.p[k] = rec.p[k];
-                        rn[k] = rec.n[k];
-                    }
-                    ba = a.ball_eps;
-                    bb = S.half_min_extent;
-                    bk = 0;
-                    bwarm = -1;
-                    const float m = (ba + bb) * 0.5f;
-#pragma unroll
-                    for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m, st.p[k]);
-                }
-            }
-        }
-        const bool walking = phase == PH_ANTI_WALK;
-        float x[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) x[k] = walking ? w.p[k] : qpos[k];
-        bool need = active;
-        float ball_m = -1.0f;
-        Hit pre{-1, INFINITY};
-        if (active && phase == PH_BALL)
-            ball_precheck<D>(views[item], qpos, (ba + bb) * 0.5f, bwarm, rprim, need, ball_m, pre);
-        Hit hit = warp_queries_batch<D, WL>(views, need, item, x, walking ? w.last : rprim, work, ball_m);
-        if (!active) continue;
-        if (phase == PH_BALL && (!need || (ball_m > 0.0f && hit.prim < 0))) hit = pre;
-        const SceneView &S = views[item];
-        const WalkCfg &c = cfgs[item];
-        const bool with_src = a.source_in_nd && D == 2 && S.src_type != 0;
-        if (walking) w.last = hit.prim;
-        bool finish_anti = false;
-        float uq = 0.0f;
-        if (phase == PH_BALL) {
-            const float d = sqrtf(hit.d2);
-            const float m = (ba + bb) * 0.5f;
-            if (wosm::ball_accepts(d, m)) {
-                ba = m;
-            } else {
-                bb = m;
-                bwarm = hit.prim;
-            }
-            ++bk;
-            if (bk < 10) {
-                const float m2 = (ba + bb) * 0.5f;
-#pragma unroll
-                for (int k = 0; k < D; ++k) qpos[k] = fmaf(rn[k], m2, st.p[k]);
-                continue;
-            }
-            st.R = ba;
-            nd_setup<D>(st, S, c, a, pt, wk);
-            nd_point<D>(st, qpos);
-            phase = PH_ANTI_START;
-            continue;
-        }
-        const uint32_t role = st.which == 0 ? ROLE_ANTI_A : ROLE_ANTI_B;
-        // the ball walk's first query (PH_ANTI_START) either ends it inside the
-        // epsilon2 shell or starts the walk; both walk phases then share one
-        // walker_advance (one inlined copy keeps the kernel's code small)
-        bool advance = phase == PH_ANTI_WALK;
-        if (phase == PH_ANTI_START) {
-            const float d = sqrtf(hit.d2);
-            if (d < a.epsilon2) {
-                const Rec r2 = closest_record<D>(S, qpos, hit.prim);
-                uq = dirichlet<D>(S, hit.prim, r2.t0, r2.t1, nullptr, nullptr);
-                finish_anti = true;
-            } else {
-                w.start(qpos, D);
-                w.last = hit.prim;
-                phase = PH_ANTI_WALK;
-                advance = true;
-            }
-        }
-        if (advance) {
-            const int r = walker_advance<D>(w, S, hit, c, a.epsilon2, c.project != 0, false, pt, wk, role, false, S.guide);
-            if (r == W_CONTINUE) continue;
-            if (r == W_VALID) {
-                const Rec r2 = closest_record<D>(S, w.p, hit.prim);
-                uq = dirichlet<D>(S, hit.prim, r2.t0, r2.t1, nullptr, nullptr);
-                if (with_src) uq += w.contrib;
-            }
-            finish_anti = true;
-        }
-        if (finish_anti) {
-            nd_accumulate<D>(st, a, uq);
-            st.which += 1;
-            if (st.which == 1) {
-                nd_point<D>(st, qpos);
-                phase = PH_ANTI_START;
-                continue;
-            }
-            float gn[3], gt[3];
-            nd_finish<D>(st, S, c, a, pt, wk, with_src, gn);
-            tangent_derivative<D>(S, rprim, gt);
-            int vid[3];
-            float wts[3];
-            dirichlet<D>(S, rprim, rt0, rt1, vid, wts);
-            const long long off = items[item].dV_off;
-#pragma unroll
-            for (int s2 = 0; s2 < D; ++s2)
-#pragma unroll
-                for (int k = 0; k < D; ++k)
-                    atomicAdd(&acc[off + (long long)vid[s2] * D + k], W * (double)(-(wts[s2] * (gn[k] + gt[k]))));
-            active = false;
-            phase = PH_IDLE;
-        }
-    }
-    if constexpr (COUNT) {
-        if (count_work) flush_work<true>(work);
-    } else {
-        // never taken; kept for the same reason as in k_walk
-        if (count_work) flush_work<true>(Work{0, 0, 0});
-    }
-    if (acc_item >= 0) {
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            if (acc_src[k * AS] != 0.0) atomicAdd(&acc[items[acc_item].ds_off + k], acc_src[k * AS]);
-    }
+    adjoint_lanes<D, true, ADJ_FROM_RECORDS>(ManyScenes<D>{views, cfgs, items, n_items}, a, base, total, dLdu,
+                                             counter, chunk, out, views[0].guide, stack + threadIdx.x, *am.slot,
+                                             acc_on ? am.acc : nullptr, work);
+    if constexpr (COUNT) flush_work(work);
 }
 
 __global__ void k_acc_to_f32(const double *__restrict__ acc, float *out, long long n) {
@@ -2450,36 +2376,33 @@ static int persistent_grid(Kern kern, int block, size_t smem, int blocks_per_sm,
     return 0;
 }
 
-template <int D, int WL, bool COUNT>
-static int launch_walk_batch_t(const SceneView *views, const WalkCfg *cfgs, const BatchItemDev *items, int n_items,
-                               long long base, long long total, const BatchLaunch &L, const WalkOut &out,
-                               unsigned long long *counter, cudaStream_t st) {
+template <int D, bool COUNT>
+static int launch_walk_batch_t(int stack, const SceneView *views, const WalkCfg *cfgs, const BatchItemDev *items,
+                               int n_items, long long base, long long total, const BatchLaunch &L,
+                               const WalkOut &out, unsigned long long *counter, cudaStream_t st) {
     int grid = 0;
-    if (int rc = persistent_grid(k_walk_batch<D, WL, COUNT>, L.block, 0, L.blocks_per_sm, grid)) return rc;
-    k_walk_batch<D, WL, COUNT><<<grid, L.block, 0, st>>>(views, cfgs, items, n_items, base, total, counter, L.chunk,
-                                                         out, L.count_work);
+    const size_t smem = smem_bytes(-1, L.block, stack, 0);
+    if (int rc = persistent_grid(k_walk_batch<D, COUNT>, L.block, smem, L.blocks_per_sm, grid)) return rc;
+    k_walk_batch<D, COUNT><<<grid, L.block, smem, st>>>(views, cfgs, items, n_items, base, total, counter, L.chunk,
+                                                        out);
     return 0;
 }
 
-int launch_walk_batch(int D, int wl, const SceneView *views, const WalkCfg *cfgs, const BatchItemDev *items,
+int launch_walk_batch(int D, int depth, const SceneView *views, const WalkCfg *cfgs, const BatchItemDev *items,
                       int n_items, long long base, long long total, const BatchLaunch &L, const WalkOut &out,
                       unsigned long long *counter, cudaStream_t st) {
     if (total == 0 || n_items == 0) return 0;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
-    static_assert(WT_SPECIALISED_LEVELS == 3, "one instance per specialised depth");
     int rc = 0;
-#define WOS_WB(DD, WW, CC) \
-    rc = launch_walk_batch_t<DD, WW, CC>(views, cfgs, items, n_items, base, total, L, out, counter, st)
-    // work accounting runs the any-depth instance that keeps counters
+    const int stack = tree_stack_entries(depth);
+#define WOS_WB(DD, CC) \
+    rc = launch_walk_batch_t<DD, CC>(stack, views, cfgs, items, n_items, base, total, L, out, counter, st)
+    // work accounting runs the instances that keep counters
     if (L.count_work) {
-        if (D == 2) WOS_WB(2, 0, true); else WOS_WB(3, 0, true);
-    } else if (D == 2) {
-        if (wl == 1) WOS_WB(2, 1, false); else if (wl == 2) WOS_WB(2, 2, false);
-        else if (wl == 3) WOS_WB(2, 3, false); else WOS_WB(2, 0, false);
+        if (D == 2) WOS_WB(2, true); else WOS_WB(3, true);
     } else {
-        if (wl == 1) WOS_WB(3, 1, false); else if (wl == 2) WOS_WB(3, 2, false);
-        else if (wl == 3) WOS_WB(3, 3, false); else WOS_WB(3, 0, false);
+        if (D == 2) WOS_WB(2, false); else WOS_WB(3, false);
     }
 #undef WOS_WB
     if (rc) return rc;
@@ -2488,19 +2411,24 @@ int launch_walk_batch(int D, int wl, const SceneView *views, const WalkCfg *cfgs
     return 0;
 }
 
-template <int D, int WL, bool COUNT>
-static int launch_adjoint_batch_t(const SceneView *views, const WalkCfg *cfgs, const AdjCfg &a,
+template <int D, bool COUNT>
+static int launch_adjoint_batch_t(int stack, const SceneView *views, const WalkCfg *cfgs, const AdjCfg &a,
                                   const BatchItemDev *items, int n_items, long long base, long long total,
                                   const float *dLdu, const int *wrec, const float *wds, double *acc,
                                   const BatchLaunch &L, unsigned long long *counter, const unsigned *order,
                                   cudaStream_t st) {
     const int block = std::min(L.block, 256);
-    const size_t smem = (size_t)block * adj_thread_bytes<D>(wds != nullptr) + 16;
+    const size_t smem = smem_bytes(-1, block, stack, adj_thread_bytes<D>(wds != nullptr));
     const int chunk = std::max(1, L.chunk / 2);
     int grid = 0;
-    if (int rc = persistent_grid(k_adjoint_batch<D, WL, COUNT>, block, smem, L.blocks_per_sm, grid)) return rc;
-    k_adjoint_batch<D, WL, COUNT><<<grid, block, smem, st>>>(views, cfgs, a, items, n_items, base, total, dLdu,
-                                                             counter, chunk, wrec, wds, acc, L.count_work, order);
+    if (int rc = persistent_grid(k_adjoint_batch<D, COUNT>, block, smem, L.blocks_per_sm, grid)) return rc;
+    AdjOut out{};
+    out.dV = acc;
+    out.wrec = wrec;
+    out.wds = wds;
+    out.order = order;
+    k_adjoint_batch<D, COUNT><<<grid, block, smem, st>>>(views, cfgs, a, items, n_items, base, total, dLdu, counter,
+                                                         chunk, out, stack);
     return 0;
 }
 
@@ -2598,7 +2526,7 @@ int launch_batch_order(int D, const SceneView *views, const BatchItemDev *items,
     return 0;
 }
 
-int launch_adjoint_batch(int D, int wl, const SceneView *views, const WalkCfg *cfgs, const AdjCfg &a,
+int launch_adjoint_batch(int D, int depth, const SceneView *views, const WalkCfg *cfgs, const AdjCfg &a,
                          const BatchItemDev *items, int n_items, long long base, long long total,
                          const float *dLdu, const int *wrec, const float *wds, double *acc, const BatchLaunch &L,
                          unsigned long long *counter, const unsigned *order, cudaStream_t st) {
@@ -2606,18 +2534,15 @@ int launch_adjoint_batch(int D, int wl, const SceneView *views, const WalkCfg *c
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
     int rc = 0;
-#define WOS_AB(DD, WW, CC)                                                                                        \
-    rc = launch_adjoint_batch_t<DD, WW, CC>(views, cfgs, a, items, n_items, base, total, dLdu, wrec, wds, acc, L, \
-                                            counter, order, st)
-    // work accounting runs the any-depth instance that keeps counters
+    const int stack = tree_stack_entries(depth);
+#define WOS_AB(DD, CC)                                                                                             \
+    rc = launch_adjoint_batch_t<DD, CC>(stack, views, cfgs, a, items, n_items, base, total, dLdu, wrec, wds, acc, L, \
+                                        counter, order, st)
+    // work accounting runs the instances that keep counters
     if (L.count_work) {
-        if (D == 2) WOS_AB(2, 0, true); else WOS_AB(3, 0, true);
-    } else if (D == 2) {
-        if (wl == 1) WOS_AB(2, 1, false); else if (wl == 2) WOS_AB(2, 2, false);
-        else if (wl == 3) WOS_AB(2, 3, false); else WOS_AB(2, 0, false);
+        if (D == 2) WOS_AB(2, true); else WOS_AB(3, true);
     } else {
-        if (wl == 1) WOS_AB(3, 1, false); else if (wl == 2) WOS_AB(3, 2, false);
-        else if (wl == 3) WOS_AB(3, 3, false); else WOS_AB(3, 0, false);
+        if (D == 2) WOS_AB(2, false); else WOS_AB(3, false);
     }
 #undef WOS_AB
     if (rc) return rc;

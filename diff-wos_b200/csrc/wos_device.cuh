@@ -63,34 +63,47 @@ struct SceneView {
     // brackets the CDF search to a few entries
     const unsigned short *guide;
     int n_guide;
-    // Wide tree for the warp-cooperative query: an implicit tree over the
-    // Morton-ordered primitives.  Level 1 nodes are leaves, leaf i holding
-    // primitives [WT_LEAF i, WT_LEAF i + WT_LEAF) (in Morton order); level k
-    // node i bounds level k-1 nodes [32 i, 32 i + 32); level wt_levels has at
-    // most 32 nodes.  Boxes: 2D one float4 (lo.x, lo.y, hi.x, hi.y) per node,
-    // 3D two float4 (lo.xyz, w), (hi.xyz, 0); level k starts at
-    // wt_box[wt_off[k]] (in nodes).  The queries bound a leaf by its oriented
-    // box instead (wt_obb, built by k_wt_obb): principal axes u_k of its
-    // vertices, a centre c and half-extents e_k with |u_k.(y - c)| <= e_k;
-    // 2D two float4 (u0.xy, c.xy), (e0, e1, 0, 0) with u1 = (-u0.y, u0.x), 3D
-    // three (u0, e0), (u1, e1), (c, e2) with u2 = u0 x u1.  A 3D level-2 node
-    // also has a slab bound: unit normal n and [oc - oh, oc + oh] containing
-    // n.(v - c) for every vertex v, c its box centre; wt_slab[i] = (n.xyz, oc)
-    // with oh in the box's lo.w.  Any point y of the node is at least
-    // |n.(x - c) - oc| - oh from x.
-    int wt_levels;
-    int wt_count[8];
-    int wt_off[8];
-    const float4 *wt_box;
-    const float4 *wt_slab;
-    const float4 *wt_obb;
+    // Search tree of the walk kernels: an implicit 4-ary tree over the sorted
+    // primitives.  Leaf i holds the primitives at sorted positions [LEAF i,
+    // LEAF i + LEAF); the root is at depth 0, the leaves at depth tree_depth,
+    // and node i of depth d has the children [4 i, 4 i + 4) of depth d + 1.
+    // Every node is bounded by an oriented box (k_tree_bounds): orthonormal axes
+    // u_k, a centre c and half-extents e_k with |u_k.(y - c)| <= e_k for every
+    // point y of its primitives.  A node's four child boxes are one block of
+    // `tree`, block (4^d - 1) / 3 + i (tree_block):
+    //   2D, 6 float4: (u0.xy, c.xy) per child, then (e0, e1) of two children
+    //       each, with u1 = (-u0.y, u0.x);
+    //   3D, 8 float4, 32 bytes per child: c as 3 floats, u0 and u1 as six
+    //       16-bit integers in units of 2^-15 (offset by 32768), e0 and e1 as the
+    //       upper halves of floats, e2 as a float; u2 = u0 x u1.
+    // A child that does not exist is infinitely far (e0 = -inf).  A leaf's
+    // primitives are one block of `prims`: 2D 5 float4, the segments
+    // (a, b - a) and their 1/|b - a|^2; 3D 3 float4 per triangle, as in `tri`.
+    // The last leaf repeats the last primitive.
+    int tree_depth;
+    const float4 *tree;
+    const float4 *prims;
 };
 
-constexpr int WT_MAX_LEVELS = 5;
-// Primitives per leaf: one per lane.  (Leaves of 8 or 16 primitives, four or
-// two tested per warp step, were measured slower on both the 2D and the 3D
-// workloads: the extra pops cost more than the tighter leaves save.)
-constexpr int WT_LEAF = 32;
+// Shape of the search tree: primitives per leaf, float4 per node block and per
+// leaf block.
+template <int D>
+struct Tree;
+template <>
+struct Tree<2> {
+    static constexpr int LEAF = 4, NODE_W = 6, LEAF_W = 5;
+};
+template <>
+struct Tree<3> {
+    static constexpr int LEAF = 2, NODE_W = 8, LEAF_W = 3 * LEAF;
+};
+constexpr int TREE_MAX_DEPTH = 15;  // a stack entry holds the depth in 4 bits
+// Most entries on a search's stack: three siblings at each depth.
+__host__ __device__ constexpr int tree_stack_entries(int depth) { return 3 * depth; }
+// Block of the node i at depth d: the blocks of the depths above come first.
+__host__ __device__ __forceinline__ unsigned tree_block(int d, unsigned i) {
+    return i + (0x55555555u & ((1u << (2 * d)) - 1u));
+}
 
 template <int D>
 struct NodeWords;
@@ -312,11 +325,15 @@ struct NoWork {
 // squared distance exceeds (1 + 2^-10) best + 1025 (s 2^-20)^2, where s
 // bounds the coordinates' magnitude around the scene.
 template <int D>
-__device__ __forceinline__ float prune_tol2(const SceneView &S, const float *p) {
+__device__ __forceinline__ float prune_tol(const SceneView &S, const float *p) {
     float s = S.max_extent;
 #pragma unroll
     for (int k = 0; k < D; ++k) s += fabsf(p[k] - S.centre[k]);
-    const float e = s * 9.5367431640625e-07f;
+    return s * 9.5367431640625e-07f;
+}
+template <int D>
+__device__ __forceinline__ float prune_tol2(const SceneView &S, const float *p) {
+    const float e = prune_tol<D>(S, p);
     return 1025.0f * (e * e);
 }
 __device__ __forceinline__ float prune_bound(float best, float tol2) { return fmaf(best, 1.0009765625f, tol2); }
@@ -487,125 +504,6 @@ __device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, c
     return h;
 }
 
-// ------------------------------------------------------------------ wide tree
-// Warp minimum of a non-negative float (or +inf): for such values the IEEE
-// bit pattern orders like the value, so one redux.sync integer minimum does it.
-__device__ __forceinline__ float warp_min(float v) {
-    return __uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(v)));
-}
-__device__ __forceinline__ int warp_min_int(int v) { return __reduce_min_sync(0xffffffffu, v); }
-
-// Frontier key of a lane: its child's distance with the low 5 mantissa bits
-// replaced by the lane, so one redux.sync minimum gives both the nearest
-// child and its lane.  The distance read back from a key (low bits cleared)
-// is at most the true one, so pruning on it stays conservative; only the
-// order of near-equal children (within 32 ulps) changes.
-__device__ __forceinline__ unsigned frontier_key(float d, int lane) {
-    return (__float_as_uint(d) & ~31u) | (unsigned)lane;
-}
-__device__ __forceinline__ float key_dist(unsigned k) { return __uint_as_float(k & ~31u); }
-// A taken entry: the largest +inf key (a NaN pattern would never compare
-// above the bound, so the loop could not end).
-constexpr unsigned KEY_TAKEN = 0x7f80001fu;
-
-template <int D>
-__device__ __forceinline__ float wt_box_d2(const SceneView &S, int node, const float *q) {
-    float lo[3], hi[3];
-    if (D == 2) {
-        const float4 b = __ldg(&S.wt_box[node]);
-        lo[0] = b.x;
-        lo[1] = b.y;
-        hi[0] = b.z;
-        hi[1] = b.w;
-    } else {
-        const float4 a = __ldg(&S.wt_box[2 * node]), b = __ldg(&S.wt_box[2 * node + 1]);
-        lo[0] = a.x;
-        lo[1] = a.y;
-        lo[2] = a.z;
-        hi[0] = b.x;
-        hi[1] = b.y;
-        hi[2] = b.z;
-    }
-    return box_d2<D>(lo, hi, q);
-}
-
-// Lower bound on the squared distance from q to leaf `leaf`: the distance to
-// its oriented box, sum_k max(|u_k.(q - c)| - e_k, 0)^2, scaled by
-// (1 - 2^-18).  With |u_k.(y - c)| <= e_k for every point y of the leaf and
-// the axes' matrix of norm below 1, the exact value is at most |q - y|^2; the
-// float roundings of q - c and of the dot products (relative 2^-22 of
-// |q - c|) are covered by the 1e-6 |y - c| margin in e_k for the |y - c| part
-// and by the final scale for the rest, so the result stays below |q - y|^2 --
-// a bound as safe as the box distance, and tighter wherever a leaf's patch or
-// arc is tilted against the axes.
-template <int D>
-__device__ __forceinline__ float leaf_obb_d2(const SceneView &S, int leaf, const float *q) {
-    constexpr float SHRINK = 0.999996185302734375f;  // 1 - 2^-18
-    if (D == 2) {
-        const float4 a = __ldg(&S.wt_obb[2 * leaf]), e = __ldg(&S.wt_obb[2 * leaf + 1]);
-        const float vx = q[0] - a.z, vy = q[1] - a.w;
-        const float a0 = fmaxf(fabsf(dot2(a.x, a.y, vx, vy)) - e.x, 0.0f);
-        const float a1 = fmaxf(fabsf(dot2(-a.y, a.x, vx, vy)) - e.y, 0.0f);
-        return fmaf(a0, a0, a1 * a1) * SHRINK;
-    }
-    const float4 f0 = __ldg(&S.wt_obb[3 * leaf]), f1 = __ldg(&S.wt_obb[3 * leaf + 1]),
-                 f2 = __ldg(&S.wt_obb[3 * leaf + 2]);
-    float u2[3];
-    cross3(f0.x, f0.y, f0.z, f1.x, f1.y, f1.z, u2[0], u2[1], u2[2]);
-    const float vx = q[0] - f2.x, vy = q[1] - f2.y, vz = q[2] - f2.z;
-    const float a0 = fmaxf(fabsf(dot3(f0.x, f0.y, f0.z, vx, vy, vz)) - f0.w, 0.0f);
-    const float a1 = fmaxf(fabsf(dot3(f1.x, f1.y, f1.z, vx, vy, vz)) - f1.w, 0.0f);
-    const float a2 = fmaxf(fabsf(dot3(u2[0], u2[1], u2[2], vx, vy, vz)) - f2.w, 0.0f);
-    return fmaf(a0, a0, fmaf(a1, a1, a2 * a2)) * SHRINK;
-}
-
-// Lower bound on the squared distance from q to node `node` of level L: a
-// leaf's oriented-box distance; for a 3D level-2 node (a patch of 1024
-// triangles, whose box is loose wherever the surface is tilted against the
-// axes) the larger of its box distance and its slab distance; otherwise the
-// box distance.
-template <int D, int L>
-__device__ __forceinline__ float node_bound(const SceneView &S, int node, const float *q) {
-    float lo[3], hi[3], n[3], c[3], oc, oh;
-    if constexpr (L == 1) {
-        return leaf_obb_d2<D>(S, node, q);
-    } else if (D == 2 || L > 2) {
-        return wt_box_d2<D>(S, S.wt_off[L] + node, q);
-    } else {
-        const int bi = S.wt_off[L] + node;
-        const float4 a = __ldg(&S.wt_box[2 * bi]), b = __ldg(&S.wt_box[2 * bi + 1]);
-        const float4 sl = __ldg(&S.wt_slab[node]);
-        lo[0] = a.x;
-        lo[1] = a.y;
-        lo[2] = a.z;
-        hi[0] = b.x;
-        hi[1] = b.y;
-        hi[2] = b.z;
-        n[0] = sl.x;
-        n[1] = sl.y;
-        n[2] = sl.z;
-        oc = sl.w;
-        oh = a.w;
-    }
-    const float bd = box_d2<D>(lo, hi, q);
-#pragma unroll
-    for (int k = 0; k < D; ++k) c[k] = (lo[k] + hi[k]) * 0.5f;
-    const float t = dot3(n[0], n[1], n[2], q[0] - c[0], q[1] - c[1], q[2] - c[2]);
-    const float lb = fabsf(t - oc) - oh;
-    return lb > 0.0f ? fmaxf(bd, lb * lb) : bd;
-}
-
-// Squared distance to the primitive at Morton position s.
-template <int D>
-__device__ __forceinline__ float leaf_d2(const SceneView &S, int s, const float *q) {
-    if (D == 2) {
-        float t;
-        return seg_d2(__ldg(&S.lseg[s]), __ldg(&S.lseginv[s]), q[0], q[1], t);
-    }
-    return tri_d2_uniform(__ldg(&S.ltri[3 * s]), __ldg(&S.ltri[3 * s + 1]), __ldg(&S.ltri[3 * s + 2]), q[0], q[1],
-                          q[2]);
-}
-
 // Squared distance to primitive f in the original order.
 template <int D>
 __device__ __forceinline__ float prim_d2(const SceneView &S, int f, const float *q) {
@@ -616,87 +514,6 @@ __device__ __forceinline__ float prim_d2(const SceneView &S, int f, const float 
     return tri_d2(__ldg(&S.tri[3 * f]), __ldg(&S.tri[3 * f + 1]), __ldg(&S.tri[3 * f + 2]), q[0], q[1], q[2]);
 }
 
-// Pruning bound of the wide-tree descent, clamped to the largest float so
-// that +inf frontier entries (no child) are never taken, even before a first
-// candidate exists or when the query point is NaN or overflows.
-__device__ __forceinline__ float wt_bound(float best, float tol2) { return fminf(prune_bound(best, tol2), FLT_MAX); }
-
-// Warp-cooperative nearest primitive for one query point q (the same q in
-// every lane; every lane returns the same Hit).  Best-first descent of the
-// wide tree, one template instance per level: the level's frontier of up to
-// 32 child distances is one register per lane, the nearest unexpanded child
-// is a redux.sync minimum, and a node expansion is one coalesced load of 32
-// boxes (leaf bounds at level 1) or 32 primitives.  `best` may hold a
-// warm-start candidate (a real primitive with its distance); pruning is
-// conservative, so the result is the exact minimum of (d2, primitive index)
-// -- the same as the brute-force search.
-template <int D, int L, class WK>
-__device__ __forceinline__ void wdescend(const SceneView &S, const float *q, int first, float tol2, Hit &best,
-                                         WK &wk) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int child = first + lane;
-    float d = INFINITY;
-    if (child < S.wt_count[L]) d = node_bound<D, L>(S, child, q);
-    unsigned key = frontier_key(d, lane);
-    wk.nb += 1;
-    unsigned mk = __reduce_min_sync(FULL, key);
-    for (;;) {
-        if (key_dist(mk) > wt_bound(best.d2, tol2)) return;
-        const int j = (int)(mk & 31u);
-        if (lane == j) key = KEY_TAKEN;
-        const int node = first + j;
-        // the next frontier entry, reduced before this node's work (whose
-        // pruning cannot change the frontier) so that its latency overlaps it
-        mk = __reduce_min_sync(FULL, key);
-        if constexpr (L == 1) {
-            wk.np += 1;
-            const int s = node * WT_LEAF + lane;
-            float d2 = INFINITY;
-            if (s < S.nF) d2 = leaf_d2<D>(S, s, q);
-            const float m2 = warp_min(d2);
-            if (m2 <= best.d2 && m2 < INFINITY) {
-                const unsigned c2 = __ballot_sync(FULL, d2 == m2);
-                int o = 0x7fffffff;
-                if ((c2 >> lane) & 1u) o = __ldg(&S.lorig[s]);
-                const int omin = (__popc(c2) == 1) ? __shfl_sync(FULL, o, __ffs(c2) - 1) : warp_min_int(o);
-                if (m2 < best.d2 || omin < best.prim) {
-                    best.d2 = m2;
-                    best.prim = omin;
-                }
-            }
-        } else {
-            wdescend<D, L - 1>(S, q, node * 32, tol2, best, wk);
-        }
-    }
-}
-
-// WL > 0: the tree has exactly WL levels (a kernel compiled for one depth
-// holds one descent, which keeps its code small); WL = 0: any depth.  tol2
-// is prune_tol2<D>(S, q), passed in so that a warp can compute it for all its
-// lanes' points at once.
-template <int D, int WL = 0, class WK>
-__device__ __forceinline__ Hit wquery_tol(const SceneView &S, const float *q, Hit best, float tol2, WK &wk) {
-    wk.nq += 1;
-    if constexpr (WL > 0) {
-        wdescend<D, WL>(S, q, 0, tol2, best, wk);
-        return best;
-    }
-    switch (S.wt_levels) {
-        case 1: wdescend<D, 1>(S, q, 0, tol2, best, wk); break;
-        case 2: wdescend<D, 2>(S, q, 0, tol2, best, wk); break;
-        case 3: wdescend<D, 3>(S, q, 0, tol2, best, wk); break;
-        case 4: wdescend<D, 4>(S, q, 0, tol2, best, wk); break;
-        default: wdescend<D, 5>(S, q, 0, tol2, best, wk); break;
-    }
-    return best;
-}
-
-template <int D, int WL = 0, class WK>
-__device__ __forceinline__ Hit wquery(const SceneView &S, const float *q, Hit best, WK &wk) {
-    return wquery_tol<D, WL>(S, q, best, prune_tol2<D>(S, q), wk);
-}
-
 // ------------------------------------------------------------------ ball test
 // One bisection step of the inscribed-ball search accepts the radius m when
 // |d - m| <= 1e-5f for the nearest distance d from the candidate centre
@@ -704,72 +521,299 @@ __device__ __forceinline__ Hit wquery(const SceneView &S, const float *q, Hit be
 // step rejects exactly when some primitive "blocks" the ball,
 // sqrtf(d2) - m < -1e-5f, or when even the nearest distance is above
 // m + 1e-5f; the caller rules the second case out with the ball's own
-// primitive.  So a step needs no nearest search: it stops at the first
+// primitive.  So a step needs no nearest search: it may stop at the first
 // blocking primitive.
 __device__ __forceinline__ bool ball_blocks(float d2, float m) { return sqrtf(d2) - m < -1e-5f; }
 
-template <int D, int L, class WK>
-__device__ __forceinline__ bool wball_descend(const SceneView &S, const float *q, int first, float bound, float m,
-                                              Hit &hit, WK &wk) {
-    const unsigned FULL = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
-    const int child = first + lane;
-    float d = INFINITY;
-    if (child < S.wt_count[L]) d = node_bound<D, L>(S, child, q);
-    unsigned key = frontier_key(d, lane);
-    wk.nb += 1;
-    unsigned mk = __reduce_min_sync(FULL, key);
+// ------------------------------------------------------------------ tree search
+// Nearest-primitive search with one lane per query: a depth-first descent of
+// the 4-ary tree, nearest child first, that can be left after any step and
+// taken up again.  The 32 lanes of a warp are at different places of different
+// searches; per step the warp votes which kind runs, a node (four box bounds)
+// or a leaf (four exact distances), and the lanes at the other kind wait
+// (search_run).  A lane whose search ends waits only until enough others have
+// ended too, while the rest keep their state: no lane waits for the slowest
+// search of its warp.
+//
+// Why lanes and not the warp or a group per query: a query needs few boxes (24
+// in 2D at 4,096 segments, about 105 in 3D at 81,920 triangles) and the step
+// overhead -- reductions across lanes, loop control, the walk's own work -- is
+// paid per lane and not per warp.  Random 16-byte loads that hit L1 cost the SM
+// 11 cycles per warp load against 4.2 when consecutive, so 32 lanes at 32
+// places are affordable.  Measured against a warp per query on a 32-ary tree:
+// forward solve of 14,592 points x 64 walks on 1,024 segments 1.64 -> 0.74 ms, 2D
+// gradient of 80,222 x 256 on 4,096 segments 187 -> 106 ms, 3D solve of 20,000 x
+// 64 on 20,480 triangles 21.4 -> 16.2 ms, 3D gradient of 100,000 x 16 on 81,920
+// triangles 129 -> 97 ms.  (Groups of 8 lanes on a 16-ary tree: 1.60 and 154 ms
+// in 2D.)
+//
+// What bounds it: instruction issue (about 70 % of the slots), at 15 of 32 lanes
+// per instruction, since lanes wait at the other kind of step; L1 is 55-60 % busy.
+template <int D>
+struct Search {
+    float tol;     // pruning tolerance of the query point (search_bound)
+    float bound;   // nodes farther than this (squared) are pruned
+    float stop;    // a primitive this near (squared) ends the search (negative: none does)
+    float d2;      // best squared distance so far, and its sorted position (-1: none)
+    int pos;
+    unsigned idx;  // the node to visit next: index within its depth
+    int dep;       // its depth, or SEARCH_*
+    int sp;        // stack entries
+};
+enum { SEARCH_DONE = -1, SEARCH_NEED = -2 };  // no node left; no search begun
+
+// Pruning bound: a node farther than this (squared) holds no primitive whose
+// computed squared distance is below `best`.  Clamped to the largest float:
+// infinitely far boxes are never visited, even before a first candidate.
+// 3D: prune_bound, with tol = prune_tol2.  2D: (d (1 + 2^-18) + tol)^2 with d =
+// sqrt(best) and tol = prune_tol: a segment's computed distance is that of a point
+// on the segment up to 2^-23 of itself and 2^-24 of the segment's length, and a
+// box's computed bound exceeds the true one by at most 2^-20 of itself.  (The
+// squared form's 2^-10 costs a third more leaves: arcs a thousandth farther
+// than the nearest are many.  In 3D the barycentric coordinates of needle
+// triangles are far less exact, and it gains little there.)
+template <int D>
+__device__ __forceinline__ float search_bound(float best, float tol) {
+    if constexpr (D == 2) {
+        const float r = fmaf(sqrtf(best), 1.0f + 0x1p-18f, tol);
+        return fminf((r * r) * (1.0f + 0x1p-22f), FLT_MAX);
+    }
+    return fminf(prune_bound(best, tol), FLT_MAX);
+}
+
+// Begin a search at q.  warm: a primitive whose distance bounds the nearest
+// one's (that walk's previous nearest primitive), or -1; its own leaf lies
+// within that bound, so it is found again if nothing is nearer.  ball_m > 0: the
+// search is for a primitive blocking the ball of radius ball_m centred at q and
+// may stop at any; primitives that do not block are of no interest.
+template <int D>
+__device__ __forceinline__ void search_begin(Search<D> &s, const SceneView &S, const float *q, int warm,
+                                             float ball_m) {
+    s.tol = D == 2 ? prune_tol<D>(S, q) : prune_tol2<D>(S, q);
+    s.stop = -1.0f;
+    if (ball_m > 0.0f) {
+        s.bound = search_bound<D>((ball_m * ball_m) * (1.0f + 0x1p-20f), s.tol);
+        // blocking is monotone in the distance: if `stop` blocks, whatever is
+        // nearer does
+        const float t = ball_m - 1.1e-5f;
+        if (t > 0.0f && ball_blocks(t * t, ball_m)) s.stop = t * t;
+    } else {
+        s.bound = warm >= 0 ? search_bound<D>(prim_d2<D>(S, warm, q), s.tol) : FLT_MAX;
+    }
+    s.d2 = INFINITY;
+    s.pos = -1;
+    s.idx = 0;
+    s.sp = 0;
+    // a point that is not finite has no primitive at a finite distance
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < D; ++k) finite = finite && fabsf(q[k]) <= FLT_MAX;
+    s.dep = finite ? 0 : SEARCH_DONE;
+}
+
+// Next node from the stack: the last entry within the bound.  An entry is its
+// node's squared distance, the low 6 bits replaced by its depth and its place
+// among its siblings (rounded down, so pruning stays conservative); being on
+// the stack of a depth-first descent, it is a sibling of the current path's
+// node at that depth, which gives its index.
+constexpr unsigned ENTRY_LOW = 63u;
+template <int D>
+__device__ __forceinline__ void search_pop(Search<D> &s, const unsigned *stack) {
+    const unsigned b = __float_as_uint(s.bound) | ENTRY_LOW;
     for (;;) {
-        if (key_dist(mk) > bound) return false;
-        const int j = (int)(mk & 31u);
-        if (lane == j) key = KEY_TAKEN;
-        const int node = first + j;
-        mk = __reduce_min_sync(FULL, key);
-        if constexpr (L == 1) {
-            wk.np += 1;
-            const int s = node * WT_LEAF + lane;
-            float d2 = INFINITY;
-            if (s < S.nF) d2 = leaf_d2<D>(S, s, q);
-            const unsigned b = __ballot_sync(FULL, s < S.nF && ball_blocks(d2, m));
-            if (b) {
-                const int src = __ffs(b) - 1;
-                int o = 0;
-                if (lane == src) o = __ldg(&S.lorig[s]);
-                hit.prim = __shfl_sync(FULL, o, src);
-                hit.d2 = __shfl_sync(FULL, d2, src);
-                return true;
-            }
-        } else {
-            if (wball_descend<D, L - 1>(S, q, node * 32, bound, m, hit, wk)) return true;
+        if (s.sp == 0) {
+            s.dep = SEARCH_DONE;
+            return;
+        }
+        const unsigned e = stack[--s.sp * blockDim.x];
+        if (e <= b) {
+            const int dep = (int)((e >> 2) & 15u);
+            s.idx = ((s.idx >> (2 * (s.dep - dep))) & ~3u) | (e & 3u);
+            s.dep = dep;
+            return;
         }
     }
 }
 
-// Warp-cooperative blocking-primitive search for a ball of radius m centred
-// at q: returns true with a blocking primitive in `hit`, or false when no
-// primitive blocks.  Boxes are pruned against m^2 with the nearest search's
-// conservative tolerance, so no blocking primitive is missed.
-__device__ __forceinline__ float wball_bound(float m, float tol2) {
-    return wt_bound((m * m) * (1.0f + 0x1p-20f), tol2);
+// Squared distance to an oriented box, a lower bound for its primitives.  With
+// |u_k.(y - c)| <= e_k for every point y and axes whose matrix has norm below 1,
+// the exact value is at most |q - y|^2; the float roundings of q - c and of the
+// dot products (relative 2^-22 of |q - c|) are covered by the 1e-6 |y - c|
+// margin in e_k for the |y - c| part and by search_bound for the rest.
+__device__ __forceinline__ float obb_d2(float4 a, float e0, float e1, const float *q) {
+    const float vx = q[0] - a.z, vy = q[1] - a.w;
+    const float a0 = fmaxf(fabsf(dot2(a.x, a.y, vx, vy)) - e0, 0.0f);
+    const float a1 = fmaxf(fabsf(dot2(-a.y, a.x, vx, vy)) - e1, 0.0f);
+    return fmaf(a0, a0, a1 * a1);
+}
+// Third axis of a 3D box from the other two in units of 2^-15 (so itself in
+// units of 2^-30), evaluated alike here and where the box is built.
+__device__ __forceinline__ void obb_axis2(const float *a, const float *b, float *o) {
+    o[0] = fmaf(a[1], b[2], -(a[2] * b[1]));
+    o[1] = fmaf(a[2], b[0], -(a[0] * b[2]));
+    o[2] = fmaf(a[0], b[1], -(a[1] * b[0]));
+}
+// The float q of a 16-bit q + 32768, from a word's lower or upper half: as the
+// low bits of 2^23 + 32768 + q.
+__device__ __forceinline__ float obb_axis_lo(unsigned w) {
+    return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7610)) - 8421376.0f;
+}
+__device__ __forceinline__ float obb_axis_hi(unsigned w) {
+    return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7632)) - 8421376.0f;
+}
+struct Obb3 {
+    float c[3];
+    unsigned w[5];
+};
+__device__ __forceinline__ Obb3 load_obb3(const float4 *p) {
+    Obb3 o;
+    float w[5];
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(o.c[0]), "=f"(o.c[1]), "=f"(o.c[2]), "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]), "=f"(w[4])
+        : "l"(p));
+#pragma unroll
+    for (int k = 0; k < 5; ++k) o.w[k] = __float_as_uint(w[k]);
+    return o;
+}
+__device__ __forceinline__ float obb_d2(const Obb3 &o, const float *q) {
+    const float u0[3] = {obb_axis_lo(o.w[0]), obb_axis_hi(o.w[0]), obb_axis_lo(o.w[1])};
+    const float u1[3] = {obb_axis_hi(o.w[1]), obb_axis_lo(o.w[2]), obb_axis_hi(o.w[2])};
+    float u2[3];
+    obb_axis2(u0, u1, u2);
+    const float v[3] = {q[0] - o.c[0], q[1] - o.c[1], q[2] - o.c[2]};
+    const float e0 = __uint_as_float(o.w[3] << 16), e1 = __uint_as_float(o.w[3] & 0xffff0000u);
+    const float e2 = __uint_as_float(o.w[4]);
+    const float a0 = fmaxf(fmaf(fabsf(dot3(u0[0], u0[1], u0[2], v[0], v[1], v[2])), 0x1p-15f, -e0), 0.0f);
+    const float a1 = fmaxf(fmaf(fabsf(dot3(u1[0], u1[1], u1[2], v[0], v[1], v[2])), 0x1p-15f, -e1), 0.0f);
+    const float a2 = fmaxf(fmaf(fabsf(dot3(u2[0], u2[1], u2[2], v[0], v[1], v[2])), 0x1p-30f, -e2), 0.0f);
+    return fmaf(a0, a0, fmaf(a1, a1, a2 * a2));
 }
 
-// wball with its pruning bound wball_bound(m, prune_tol2<D>(S, q)) passed in.
-template <int D, int WL = 0, class WK>
-__device__ __forceinline__ bool wball_b(const SceneView &S, const float *q, float bound, float m, Hit &hit, WK &wk) {
-    wk.nq += 1;
-    if constexpr (WL > 0) return wball_descend<D, WL>(S, q, 0, bound, m, hit, wk);
-    switch (S.wt_levels) {
-        case 1: return wball_descend<D, 1>(S, q, 0, bound, m, hit, wk);
-        case 2: return wball_descend<D, 2>(S, q, 0, bound, m, hit, wk);
-        case 3: return wball_descend<D, 3>(S, q, 0, bound, m, hit, wk);
-        case 4: return wball_descend<D, 4>(S, q, 0, bound, m, hit, wk);
-        default: return wball_descend<D, 5>(S, q, 0, bound, m, hit, wk);
+// Visit an inner node: bound its four children, go to the nearest and leave the
+// others within the bound on the stack, the farthest first.
+template <int D>
+__device__ __forceinline__ void search_node(Search<D> &s, const SceneView &S, const float *q, unsigned *stack) {
+    const float4 *b = S.tree + (size_t)tree_block(s.dep, s.idx) * Tree<D>::NODE_W;
+    float d[4];
+    if constexpr (D == 2) {
+        const float4 e01 = __ldg(b + 4), e23 = __ldg(b + 5);
+        d[0] = obb_d2(__ldg(b), e01.x, e01.y, q);
+        d[1] = obb_d2(__ldg(b + 1), e01.z, e01.w, q);
+        d[2] = obb_d2(__ldg(b + 2), e23.x, e23.y, q);
+        d[3] = obb_d2(__ldg(b + 3), e23.z, e23.w, q);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d[c] = obb_d2(load_obb3(b + 2 * c), q);
+    }
+    const unsigned low = (unsigned)(s.dep + 1) << 2;
+    unsigned k[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) k[c] = (__float_as_uint(d[c]) & ~ENTRY_LOW) | (low + c);
+    // ascending
+    auto order = [&](int i, int j) {
+        const unsigned lo = min(k[i], k[j]), hi = max(k[i], k[j]);
+        k[i] = lo;
+        k[j] = hi;
+    };
+    order(0, 1);
+    order(2, 3);
+    order(0, 2);
+    order(1, 3);
+    order(1, 2);
+    const unsigned bound = __float_as_uint(s.bound) | ENTRY_LOW;
+#pragma unroll
+    for (int c = 3; c >= 1; --c)
+        if (k[c] <= bound) stack[s.sp++ * blockDim.x] = k[c];
+    if (k[0] <= bound) {
+        s.idx = 4u * s.idx + (k[0] & 3u);
+        s.dep += 1;
+    } else {
+        search_pop(s, stack);
     }
 }
 
-template <int D, int WL = 0, class WK>
-__device__ __forceinline__ bool wball(const SceneView &S, const float *q, float m, Hit &hit, WK &wk) {
-    return wball_b<D, WL>(S, q, wball_bound(m, prune_tol2<D>(S, q)), m, hit, wk);
+// Squared distances to the primitives of a leaf.
+template <int D>
+__device__ __forceinline__ void leaf_distances(const SceneView &S, unsigned leaf, const float *q, float *d2) {
+    const float4 *b = S.prims + (size_t)leaf * Tree<D>::LEAF_W;
+    if constexpr (D == 2) {
+        const float4 inv = __ldg(b + 4);
+        const float iv[4] = {inv.x, inv.y, inv.z, inv.w};
+        float t;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d2[c] = seg_d2(__ldg(b + c), iv[c], q[0], q[1], t);
+    } else {
+#pragma unroll
+        for (int c = 0; c < Tree<3>::LEAF; ++c)
+            d2[c] = tri_d2_uniform(__ldg(b + 3 * c), __ldg(b + 3 * c + 1), __ldg(b + 3 * c + 2), q[0], q[1], q[2]);
+    }
+}
+
+// Visit a leaf.  The search keeps the exact minimum of (d2, original index),
+// as nearest_brute does: indices are looked up only where distances are equal.
+template <int D>
+__device__ __forceinline__ void search_leaf(Search<D> &s, const SceneView &S, const float *q, unsigned *stack) {
+    constexpr int N = Tree<D>::LEAF;
+    float d2[N];
+    leaf_distances<D>(S, s.idx, q, d2);
+    float m = d2[0];
+#pragma unroll
+    for (int c = 1; c < N; ++c) m = fminf(m, d2[c]);
+    if (m <= s.d2 && m < INFINITY) {
+        const int p0 = (int)s.idx * N;
+        unsigned at = m == s.d2 ? 1u << N : 0u;  // who is at distance m: bit N the best so far
+#pragma unroll
+        for (int c = 0; c < N; ++c) at |= d2[c] == m ? 1u << c : 0u;
+        int pos = p0 + __ffs(at) - 1;
+        if ((at & (at - 1u)) != 0u) {
+            // equal distances: the lowest original index
+            int o = 0x7fffffff;
+            for (; at != 0u; at &= at - 1u) {
+                const int c = __ffs(at) - 1, p = c == N ? s.pos : p0 + c, op = __ldg(&S.lorig[p]);
+                if (op < o) {
+                    o = op;
+                    pos = p;
+                }
+            }
+        }
+        s.pos = pos;
+        s.d2 = m;
+        s.bound = fminf(s.bound, search_bound<D>(m, s.tol));
+        if (m <= s.stop) s.sp = 0;
+    }
+    search_pop(s, stack);
+}
+
+// Run the searches of a warp's lanes until at most `keep` of them still have a
+// node to visit.  scenes[MULTI ? item : 0] is the lane's scene.  Must be called
+// by all 32 lanes.
+template <int D, bool MULTI, class WK>
+__device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes, int item, const float *q,
+                                           unsigned *stack, int keep, WK &wk) {
+    const unsigned FULL = 0xffffffffu;
+    const SceneView &S = scenes[MULTI ? item : 0];
+    for (;;) {
+        const bool run = s.dep >= 0, leaf = run && s.dep == S.tree_depth;
+        const int nr = __popc(__ballot_sync(FULL, run)), nl = __popc(__ballot_sync(FULL, leaf));
+        if (nr <= keep) return;
+        if (2 * nl > nr) {
+            if (leaf) {
+                wk.np += 1;
+                search_leaf<D>(s, S, q, stack);
+            }
+        } else if (run && !leaf) {
+            wk.nb += 1;
+            search_node<D>(s, S, q, stack);
+        }
+    }
+}
+
+// The hit of a finished search: the original index of the nearest primitive
+// (ball searches: of one that blocks, else -1).
+template <int D>
+__device__ __forceinline__ Hit search_hit(const Search<D> &s, const SceneView &S, float ball_m = -1.0f) {
+    if (s.pos < 0 || (ball_m > 0.0f && !ball_blocks(s.d2, ball_m))) return Hit{-1, INFINITY};
+    return Hit{__ldg(&S.lorig[s.pos]), s.d2};
 }
 
 // ------------------------------------------------------------------ records
