@@ -209,41 +209,48 @@ __device__ __forceinline__ Smem stage_smem(const SceneView &S, bool stage_guide,
     return m;
 }
 
-// Warp-uniform refill of idle lanes from chunks of the global index space.
-// Returns false once the warp has no work left.
+// Warp-uniform refill of idle lanes from chunks of the global index space, at
+// most one chunk per call: with small chunks (queue_chunk) the warps that start
+// first do not fill up before the others have had theirs.
 struct Queue {
     long long cb, ce;
     bool drained;
 };
 
-__device__ __forceinline__ bool refill(Queue &q, bool &active, long long &idx, unsigned long long *counter,
+__device__ __forceinline__ void refill(Queue &q, bool &active, long long &idx, unsigned long long *counter,
                                        long long total, int chunk) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    unsigned idle = __ballot_sync(FULL, !active);
-    while (idle != 0u && !q.drained) {
-        if (q.cb >= q.ce) {
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(counter, (unsigned long long)chunk);
-            base = __shfl_sync(FULL, base, 0);
-            if ((long long)base >= total) {
-                q.drained = true;
-                break;
-            }
-            q.cb = (long long)base;
-            q.ce = min((long long)base + chunk, total);
+    const unsigned idle = __ballot_sync(FULL, !active);
+    if (idle == 0u || q.drained) return;
+    if (q.cb >= q.ce) {
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(counter, (unsigned long long)chunk);
+        base = __shfl_sync(FULL, base, 0);
+        if ((long long)base >= total) {
+            q.drained = true;
+            return;
         }
-        const int nidle = __popc(idle);
-        const long long avail = min((long long)nidle, q.ce - q.cb);
-        const int rank = __popc(idle & ((1u << lane) - 1u));
-        if (!active && rank < avail) {
-            idx = q.cb + rank;
-            active = true;
-        }
-        q.cb += avail;
-        idle = __ballot_sync(FULL, !active);
+        q.cb = (long long)base;
+        q.ce = min((long long)base + chunk, total);
     }
-    return __ballot_sync(FULL, active) != 0u;
+    const long long avail = min((long long)__popc(idle), q.ce - q.cb);
+    const int rank = __popc(idle & ((1u << lane) - 1u));
+    if (!active && rank < avail) {
+        idx = q.cb + rank;
+        active = true;
+    }
+    q.cb += avail;
+}
+
+// Walks per queue grab of a launch of `grid` blocks of `block` threads: at most
+// `chunk`, and few enough that every warp comes four times.  Small calls so
+// spread over all warps -- a lone walk per warp when there are no more --
+// instead of filling a few whose lanes wait for one another, and no warp is left
+// with a full chunk while others run dry.
+static int queue_chunk(int chunk, long long total, int grid, int block) {
+    const long long warps = (long long)grid * (block / 32);
+    return (int)std::min<long long>(chunk, std::max<long long>(1, total / (4 * warps)));
 }
 
 // Walk (pt, walk) of index idx for nw walks per point.  Indices below 2^32 take
@@ -1460,7 +1467,7 @@ static int launch_walk_t(const SceneImpl &S, const float *P, long long total, co
     if (rc) return rc;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
-    const int chunk = g_cfg[D - 2].chunk;
+    const int chunk = queue_chunk(g_cfg[D - 2].chunk, total, sh.grid, sh.block);
     if (records)
         k_walk<D, BVH, true, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, P, total, counter, chunk,
                                                                              sh.stack, sh.stage_cdf, out);
@@ -1648,7 +1655,11 @@ __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const
     sr.dep = SEARCH_DONE;
     for (;;) {
         const bool was = active;
-        if (!refill(q, active, idx, counter, total, chunk)) break;
+        refill(q, active, idx, counter, total, chunk);
+        if (!__any_sync(0xffffffffu, active)) {
+            if (q.drained) break;
+            continue;
+        }
         if (active && !was) {
             pt = (uint32_t)(idx / c.nwalks);
             wk = c.walk_offset + (uint32_t)(idx - (long long)pt * c.nwalks);
@@ -1987,7 +1998,8 @@ static int launch_soft_t(const SceneImpl &S, const float *P, long long total, co
     grid = std::max(1, per) * sms;
     e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
-    k_walk_soft<D, BVH><<<grid, 256, smem, st>>>(v, c, P, total, counter, 32, stack, tV, tg, vals, tans);
+    k_walk_soft<D, BVH><<<grid, 256, smem, st>>>(v, c, P, total, counter, queue_chunk(32, total, grid, 256),
+                                                       stack, tV, tg, vals, tans);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_walk_soft launch");
     return 0;
@@ -2107,7 +2119,7 @@ static int launch_adjoint_t(const SceneImpl &S, const float *P, long long total,
     if (rc) return rc;
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
-    const int chunk = std::max(1, g_cfg[D - 2].chunk / 2);
+    const int chunk = queue_chunk(std::max(1, g_cfg[D - 2].chunk / 2), total, sh.grid, sh.block);
     k_adjoint<D, BVH, ND, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, a, P, total, dLdu, counter, chunk,
                                                                          sh.stack, sh.stage_cdf, out);
     e = cudaGetLastError();
@@ -2383,8 +2395,8 @@ static int launch_walk_batch_t(int stack, const SceneView *views, const WalkCfg 
     int grid = 0;
     const size_t smem = smem_bytes(-1, L.block, stack, 0);
     if (int rc = persistent_grid(k_walk_batch<D, COUNT>, L.block, smem, L.blocks_per_sm, grid)) return rc;
-    k_walk_batch<D, COUNT><<<grid, L.block, smem, st>>>(views, cfgs, items, n_items, base, total, counter, L.chunk,
-                                                        out);
+    k_walk_batch<D, COUNT><<<grid, L.block, smem, st>>>(views, cfgs, items, n_items, base, total, counter,
+                                                        queue_chunk(L.chunk, total, grid, L.block), out);
     return 0;
 }
 
@@ -2419,9 +2431,9 @@ static int launch_adjoint_batch_t(int stack, const SceneView *views, const WalkC
                                   cudaStream_t st) {
     const int block = std::min(L.block, 256);
     const size_t smem = smem_bytes(-1, block, stack, adj_thread_bytes<D>(wds != nullptr));
-    const int chunk = std::max(1, L.chunk / 2);
     int grid = 0;
     if (int rc = persistent_grid(k_adjoint_batch<D, COUNT>, block, smem, L.blocks_per_sm, grid)) return rc;
+    const int chunk = queue_chunk(std::max(1, L.chunk / 2), total, grid, block);
     AdjOut out{};
     out.dV = acc;
     out.wrec = wrec;
