@@ -406,23 +406,163 @@ __global__ void k_leaf_data(const unsigned long long *keys, int n, const float4 
     }
 }
 
-// Leaf blocks of the search tree (SceneView::prims) from the sorted primitives;
-// the last leaf repeats the last one (and its original index in lorig).
+// Leaf blocks of the search tree (SceneView::prims) in the tree's order: torig,
+// or, where `keys` is given, the order of those sorted keys, stored to torig.  The
+// last leaf repeats the last primitive.
 template <int D>
-__global__ void k_tree_prims(int nF, int n_leaf, const float4 *lseg, const float *lseginv, const float4 *ltri,
-                             float4 *prims, int *lorig) {
+__global__ void k_tree_prims(int nF, int n_leaf, const unsigned long long *keys, const float4 *seg,
+                             const float *seginv, const float4 *tri, float4 *prims, int *torig) {
     constexpr int N = Tree<D>::LEAF, W = Tree<D>::LEAF_W;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n_leaf * N) return;
     const int s = min(p, nF - 1), leaf = p / N, c = p % N;
-    if (p >= nF) lorig[p] = lorig[s];
+    const int f = keys != nullptr ? (int)(unsigned)keys[s] : torig[s];
+    if (keys != nullptr || p >= nF) torig[p] = f;
     float4 *b = prims + (size_t)leaf * W;
     if (D == 2) {
-        b[c] = lseg[s];
-        reinterpret_cast<float *>(b + 4)[c] = lseginv[s];
+        b[c] = seg[f];
+        reinterpret_cast<float *>(b + 4)[c] = seginv[f];
     } else {
-        for (int k = 0; k < 3; ++k) b[3 * c + k] = ltri[3 * s + k];
+        for (int k = 0; k < 3; ++k) b[3 * c + k] = tri[3 * (size_t)f + k];
     }
+}
+
+// ------------------------------------------------------------------ tree order
+// Order of a mesh's triangles in its search tree: recursive median splits.  From
+// one segment of `cap` positions (a power of two times the leaf size, covering the
+// mesh) down to leaves, each segment is sorted along the longest axis of its
+// triangles' centres and cut in the middle, so that every node of the implicit
+// tree is a compact patch.  Runs of a Hilbert curve, whose cells cut a surface
+// anywhere, take 28 node and 5.7 leaf visits per query on 81,920 triangles where
+// these take 20 and 4.5.  Segments above SPLIT_SMALL positions are sorted by one
+// radix sort per level (keys: segment, then the quantised coordinate); one block
+// takes each smaller segment through all of its levels in shared memory.
+constexpr int SPLIT_SMALL = 1024;
+
+__device__ __forceinline__ float box_centre(const float *pbox, int f, int k) {
+    return (pbox[6 * (size_t)f + k] + pbox[6 * (size_t)f + 3 + k]) * 0.5f;
+}
+
+__global__ void k_split_init(int *bounds, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) bounds[i] = i % 6 < 3 ? 0x7fffffff : (int)0x80000000;
+}
+
+// Bounds of the segments' centres, ordered ints: 3 minima, 3 maxima each.
+// cap: a multiple of the block's size.
+__global__ void __launch_bounds__(256) k_split_bounds(const float *pbox, const int *ord, int nF, int cap, int *bounds) {
+    __shared__ int red[6];
+    if (threadIdx.x < 6) red[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : (int)0x80000000;
+    __syncthreads();
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int k = 0; k < 3; ++k) {
+        const bool on = p < nF;
+        const int c = on ? ordered_int(box_centre(pbox, ord[p], k)) : 0;
+        const int lo = __reduce_min_sync(0xffffffffu, on ? c : 0x7fffffff);
+        const int hi = __reduce_max_sync(0xffffffffu, on ? c : (int)0x80000000);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&red[k], lo);
+            atomicMax(&red[3 + k], hi);
+        }
+    }
+    __syncthreads();
+    int *b = bounds + 6 * ((blockIdx.x * blockDim.x) / cap);
+    if (threadIdx.x < 3) atomicMin(&b[threadIdx.x], red[threadIdx.x]);
+    else if (threadIdx.x < 6) atomicMax(&b[threadIdx.x], red[threadIdx.x]);
+}
+
+__device__ __forceinline__ int longest_axis(const int *b, float &lo, float &ext) {
+    int a = 0;
+    ext = -1.0f;
+    for (int k = 0; k < 3; ++k) {
+        const float l = from_ordered_int(b[k]), e = from_ordered_int(b[3 + k]) - l;
+        if (e > ext) {
+            a = k;
+            ext = e;
+            lo = l;
+        }
+    }
+    if (!(ext >= 0.0f)) lo = 0.0f;
+    return a;
+}
+
+__global__ void k_split_keys(const float *pbox, const int *ord, int nF, int cap, const int *bounds, unsigned *keys) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= nF) return;
+    const int seg = p / cap;
+    float lo, ext;
+    const int a = longest_axis(bounds + 6 * seg, lo, ext);
+    const float u = ext > 0.0f ? (box_centre(pbox, ord[p], a) - lo) / ext : 0.0f;
+    keys[p] = (unsigned)seg << 16 | (unsigned)fminf(fmaxf(u * 65536.0f, 0.0f), 65535.0f);
+}
+
+__global__ void __launch_bounds__(SPLIT_SMALL) k_split_small(const float *pbox, int nF, int leaf, int *ord) {
+    __shared__ float cen[3][SPLIT_SMALL];
+    __shared__ int ids[SPLIT_SMALL];
+    __shared__ unsigned long long buf[SPLIT_SMALL];
+    __shared__ int bounds[SPLIT_SMALL / 32][6];
+    const unsigned FULL = 0xffffffffu;
+    const int t = threadIdx.x, p = blockIdx.x * SPLIT_SMALL + t;
+    const bool on = p < nF;  // the last positions stay last: their keys are the largest
+    ids[t] = on ? ord[p] : -1;
+    for (int k = 0; k < 3; ++k) cen[k][t] = on ? box_centre(pbox, ids[t], k) : 0.0f;
+    __syncthreads();
+    for (int cap = SPLIT_SMALL; cap > leaf; cap >>= 1) {
+        // bounds of each segment's centres
+        const int seg = t / cap;
+        int b[6];
+        for (int k = 0; k < 3; ++k) {
+            const int c = ordered_int(cen[k][t]);
+            b[k] = on ? c : 0x7fffffff;
+            b[3 + k] = on ? c : (int)0x80000000;
+            for (int o = 1; o < min(cap, 32); o <<= 1) {
+                b[k] = min(b[k], __shfl_xor_sync(FULL, b[k], o));
+                b[3 + k] = max(b[3 + k], __shfl_xor_sync(FULL, b[3 + k], o));
+            }
+        }
+        if (cap > 32) {
+            if (t < SPLIT_SMALL / 32)
+                for (int k = 0; k < 6; ++k) bounds[t][k] = k < 3 ? 0x7fffffff : (int)0x80000000;
+            __syncthreads();
+            if ((t & 31) == 0)
+                for (int k = 0; k < 3; ++k) {
+                    atomicMin(&bounds[seg][k], b[k]);
+                    atomicMax(&bounds[seg][3 + k], b[3 + k]);
+                }
+            __syncthreads();
+            for (int k = 0; k < 6; ++k) b[k] = bounds[seg][k];
+            __syncthreads();
+        }
+        float lo, ext;
+        const int a = longest_axis(b, lo, ext);
+        // ascending bitonic sort of the segment: coordinate, then place
+        unsigned long long key =
+            (unsigned long long)(on ? (unsigned)ordered_int(cen[a][t]) ^ 0x80000000u : 0xffffffffu) << 32 | (unsigned)t;
+        for (int k = 2; k <= cap; k <<= 1)
+            for (int j = k >> 1; j > 0; j >>= 1) {
+                unsigned long long other;
+                if (j >= 32) {
+                    buf[t] = key;
+                    __syncthreads();
+                    other = buf[t ^ j];
+                    __syncthreads();
+                } else {
+                    other = __shfl_xor_sync(FULL, key, j);
+                }
+                const bool up = ((t & (cap - 1)) & k) == 0, first = (t & j) == 0;
+                if ((key > other) == (up == first)) key = other;
+            }
+        const int from = (int)(unsigned)key;
+        const float x = cen[0][from], y = cen[1][from], z = cen[2][from];
+        const int id = ids[from];
+        __syncthreads();
+        cen[0][t] = x;
+        cen[1][t] = y;
+        cen[2][t] = z;
+        ids[t] = id;
+        __syncthreads();
+    }
+    if (on) ord[p] = ids[t];
 }
 
 // Eigenvectors of a symmetric 3 x 3 matrix by cyclic Jacobi rotations: on
@@ -479,18 +619,20 @@ __device__ __forceinline__ double node_reduce(double x, Op op, double *red) {
     return x;
 }
 
-// Vertices of the primitive at sorted position s as the distance code sees them:
-// a and a + d of a segment; a, a + ab and a + ac of a triangle.
+// Vertices of the primitive at the tree's position s as the distance code sees
+// them: a and a + d of a segment; a, a + ab and a + ac of a triangle.
 template <int D>
-__device__ __forceinline__ void prim_vertices(const float4 *lseg, const float4 *ltri, int s, double y[3][3]) {
+__device__ __forceinline__ void prim_vertices(const float4 *prims, int s, double y[3][3]) {
+    const float4 *b = prims + (size_t)(s / Tree<D>::LEAF) * Tree<D>::LEAF_W;
+    const int i = s % Tree<D>::LEAF;
     if (D == 2) {
-        const float4 g = lseg[s];
+        const float4 g = b[i];
         y[0][0] = g.x;
         y[0][1] = g.y;
         y[1][0] = (double)g.x + g.z;
         y[1][1] = (double)g.y + g.w;
     } else {
-        const float4 a = ltri[3 * (size_t)s], ab = ltri[3 * (size_t)s + 1], ac = ltri[3 * (size_t)s + 2];
+        const float4 a = b[3 * i], ab = b[3 * i + 1], ac = b[3 * i + 2];
         const float o[3] = {a.x, a.y, a.z}, e[3] = {ab.x, ab.y, ab.z}, f[3] = {ac.x, ac.y, ac.z};
         for (int k = 0; k < 3; ++k) {
             y[0][k] = o[k];
@@ -500,7 +642,7 @@ __device__ __forceinline__ void prim_vertices(const float4 *lseg, const float4 *
     }
 }
 
-// Bound of a node of `np` primitives from sorted position s0, by TPN threads, all
+// Bound of a node of `np` primitives from position s0, by TPN threads, all
 // of which call.  The axes are the principal axes of the vertices, eigenvectors
 // of their covariance, made orthonormal, shrunk a little and rounded (2D: to
 // float, 3D: to multiples of 2^-15) so that the rounded axes -- with the third 3D
@@ -513,18 +655,17 @@ __device__ __forceinline__ void prim_vertices(const float4 *lseg, const float4 *
 //   2D: out = (u0, c, e0, e1).
 //   3D: out = (c, u0, u1, e) with the axes in units of 2^-15.
 template <int D, int TPN>
-__device__ __forceinline__ void node_bound(const float4 *lseg, const float4 *ltri, int s0, int np, int t, double *red,
-                                           float *out) {
+__device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, int t, double *red, float *out) {
     constexpr int NV = D == 2 ? 2 : 3;
     auto add = [](double a, double b) { return a + b; };
     auto lower = [](double a, double b) { return fmin(a, b); };
     auto upper = [](double a, double b) { return fmax(a, b); };
     // moments about the first vertex
     double y0[3], y[3][3], m[3] = {0.0, 0.0, 0.0}, cv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    prim_vertices<D>(lseg, ltri, s0, y);
+    prim_vertices<D>(prims, s0, y);
     for (int k = 0; k < D; ++k) y0[k] = y[0][k];
     for (int i = t; i < np; i += TPN) {
-        prim_vertices<D>(lseg, ltri, s0 + i, y);
+        prim_vertices<D>(prims, s0 + i, y);
         for (int j = 0; j < NV; ++j) {
             double w[3];
             for (int k = 0; k < D; ++k) {
@@ -597,7 +738,7 @@ __device__ __forceinline__ void node_bound(const float4 *lseg, const float4 *ltr
     // ranges of u_k.(y - y0), and the centre in the middle of them
     double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int i = t; i < np; i += TPN) {
-        prim_vertices<D>(lseg, ltri, s0 + i, y);
+        prim_vertices<D>(prims, s0 + i, y);
         for (int j = 0; j < NV; ++j)
             for (int k = 0; k < D; ++k) {
                 double p = 0.0;
@@ -680,7 +821,7 @@ __host__ __device__ inline int nodes_per_block(long long prims) {
 
 template <int D, bool LARGE>
 __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_tree_bounds(
-    TreePlan P, const float4 *lseg, const float4 *ltri, float4 *tree) {
+    TreePlan P, const float4 *prims, float4 *tree) {
     __shared__ double red[32];
     int d = P.d0;
     while (d < P.d1 && (int)blockIdx.x >= P.first[d + 1]) ++d;
@@ -694,12 +835,12 @@ __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_t
     float o[8];
     bool writer = there;
     if (LARGE) {
-        node_bound<D, TREE_LARGE_THREADS>(lseg, ltri, (int)s0, np, threadIdx.x, red, o);
+        node_bound<D, TREE_LARGE_THREADS>(prims, (int)s0, np, threadIdx.x, red, o);
         writer = writer && threadIdx.x == 0;
     } else if (per == TREE_THREADS) {
-        node_bound<D, 1>(lseg, ltri, (int)s0, np, 0, red, o);
+        node_bound<D, 1>(prims, (int)s0, np, 0, red, o);
     } else {
-        node_bound<D, 32>(lseg, ltri, (int)s0, np, threadIdx.x & 31, red, o);
+        node_bound<D, 32>(prims, (int)s0, np, threadIdx.x & 31, red, o);
         writer = writer && (threadIdx.x & 31) == 0;
     }
     if (!writer) return;
@@ -725,7 +866,7 @@ static cudaError_t dalloc(T **p, size_t count, cudaStream_t st) {
 }
 
 void SceneImpl::release(cudaStream_t st) {
-    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, tree, prims, guide};
+    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, tree, prims, torig, guide};
     for (void *p : ptrs)
         if (p) cudaFreeAsync(p, st);
     V = nullptr;
@@ -743,6 +884,8 @@ void SceneImpl::release(cudaStream_t st) {
     cdf = nullptr;
     tree = nullptr;
     prims = nullptr;
+    torig = nullptr;
+    tree_ordered = false;
     guide = nullptr;
 }
 
@@ -775,6 +918,58 @@ void build_g_guide(const std::vector<float> &cdf, int ng, std::vector<unsigned s
         while (l < n - 1 && !(u < cdf[l])) ++l;
         guide[k] = (unsigned short)l;
     }
+}
+
+__global__ void k_key_order(const unsigned long long *keys, int n, int *ord) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) ord[i] = (int)(unsigned)keys[i];
+}
+
+// S.torig: the median-split order of the triangles, from the boxes pbox; starts
+// from the sorted keys' order, which only settles ties.
+static int median_order(SceneImpl &S, const float *pbox, const unsigned long long *skeys, cudaStream_t st) {
+    const int nF = S.nF, TB = 256;
+    k_key_order<<<nblk(nF, TB), TB, 0, st>>>(skeys, nF, S.torig);
+    long long cap = SPLIT_SMALL;
+    while (cap < nF) cap *= 2;
+    if (cap > SPLIT_SMALL) {
+        const int max_seg = nblk(nF, 2 * SPLIT_SMALL);
+        int bits = 16;
+        while ((1LL << (bits - 16)) < max_seg) ++bits;
+        if (bits > 32) return fail(WOS_ERR_UNSUPPORTED, "scene too large for the search tree's order");
+        int *bounds = nullptr, *ord2 = nullptr;
+        unsigned *keys = nullptr, *keys2 = nullptr;
+        void *tmp = nullptr;
+        size_t tmp_bytes = 0;
+        WOS_TRY(dalloc(&bounds, (size_t)6 * max_seg, st));
+        WOS_TRY(dalloc(&ord2, nF, st));
+        WOS_TRY(dalloc(&keys, nF, st));
+        WOS_TRY(dalloc(&keys2, nF, st));
+        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, S.torig, ord2, nF, 0, bits, st);
+        WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
+        int *cur = S.torig, *alt = ord2;
+        for (; cap > SPLIT_SMALL; cap /= 2) {
+            const int n_seg = nblk(nF, (int)std::min<long long>(cap, 1LL << 30));
+            k_split_init<<<nblk(6 * n_seg, TB), TB, 0, st>>>(bounds, 6 * n_seg);
+            const int c = (int)std::min<long long>(cap, 1LL << 30);
+            k_split_bounds<<<nblk(nF, TB), TB, 0, st>>>(pbox, cur, nF, c, bounds);
+            k_split_keys<<<nblk(nF, TB), TB, 0, st>>>(pbox, cur, nF, c, bounds, keys);
+            int used = 16;
+            while ((1LL << (used - 16)) < n_seg) ++used;
+            WOS_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, cur, alt, nF, 0, used, st));
+            std::swap(cur, alt);
+        }
+        if (cur != S.torig)
+            WOS_TRY(cudaMemcpyAsync(S.torig, cur, sizeof(int) * nF, cudaMemcpyDeviceToDevice, st));
+        cudaFreeAsync(tmp, st);
+        cudaFreeAsync(bounds, st);
+        cudaFreeAsync(ord2, st);
+        cudaFreeAsync(keys, st);
+        cudaFreeAsync(keys2, st);
+    }
+    k_split_small<<<nblk(nF, SPLIT_SMALL), SPLIT_SMALL, 0, st>>>(pbox, nF, Tree<3>::LEAF, S.torig);
+    WOS_TRY(cudaGetLastError());
+    return 0;
 }
 
 template <int D>
@@ -888,8 +1083,11 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
             const long long cap = node_prims(N, P.depth - d);
             P.count[d] = (int)((nF + cap - 1) / cap);
         }
-        k_tree_prims<D><<<nblk((long long)n_leaf * N, TB), TB, 0, st>>>(nF, n_leaf, S.lseg, S.lseginv, S.ltri, S.prims,
-                                                                    S.lorig);
+        if (D == 3 && !S.tree_ordered)
+            if (int rc = median_order(S, pbox, skeys, st)) return rc;
+        S.tree_ordered = true;
+        k_tree_prims<D><<<nblk((long long)n_leaf * N, TB), TB, 0, st>>>(nF, n_leaf, D == 2 ? skeys : nullptr, S.seg,
+                                                                    S.seginv, S.tri, S.prims, S.torig);
         // the depths of large nodes, then the others
         int split = 1;
         while (split <= P.depth && node_prims(N, P.depth - split) > TREE_WARP_PRIMS) ++split;
@@ -904,9 +1102,9 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
             if (blocks == 0) continue;
             P.first[P.d1 + 1] = blocks;
             if (part == 0)
-                k_tree_bounds<D, true><<<blocks, TREE_LARGE_THREADS, 0, st>>>(P, S.lseg, S.ltri, S.tree);
+                k_tree_bounds<D, true><<<blocks, TREE_LARGE_THREADS, 0, st>>>(P, S.prims, S.tree);
             else
-                k_tree_bounds<D, false><<<blocks, TREE_THREADS, 0, st>>>(P, S.lseg, S.ltri, S.tree);
+                k_tree_bounds<D, false><<<blocks, TREE_THREADS, 0, st>>>(P, S.prims, S.tree);
         }
         WOS_TRY(cudaGetLastError());
     }
@@ -986,7 +1184,8 @@ int SceneImpl::allocate(cudaStream_t st) {
     }
     const int N = D == 2 ? Tree<2>::LEAF : Tree<3>::LEAF;
     const long long n_leaf = ((long long)nF + N - 1) / N;
-    WOS_TRY(dalloc(&lorig, (size_t)n_leaf * N, st));
+    WOS_TRY(dalloc(&lorig, nF, st));
+    WOS_TRY(dalloc(&torig, (size_t)n_leaf * N, st));
     tree_depth = 1;
     while ((1LL << (2 * tree_depth)) < n_leaf) ++tree_depth;
     if (tree_depth > TREE_MAX_DEPTH) return fail(WOS_ERR_UNSUPPORTED, "scene too large for the search tree");
@@ -1066,6 +1265,7 @@ SceneView SceneImpl::view() const {
     v.tree_depth = tree_depth;
     v.tree = tree;
     v.prims = prims;
+    v.torig = torig;
     return v;
 }
 

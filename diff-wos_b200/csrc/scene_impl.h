@@ -53,6 +53,8 @@ struct SceneImpl {
     int tree_depth = 1;  // search tree (SceneView::tree)
     float4 *tree = nullptr;
     float4 *prims = nullptr;
+    int *torig = nullptr;
+    bool tree_ordered = false;  // torig holds the order (3D: kept when vertices move)
     // Incremented by every build and source change: the by-value fields of
     // view() (bounding box, extents, source) may have changed since a view
     // was taken.

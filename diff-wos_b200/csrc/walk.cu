@@ -78,11 +78,11 @@ __device__ __forceinline__ void flush_work(const Work &wk) {
 // slowest searches, but that each advance serves fewer lanes: a 3D search takes
 // several times the instructions of an advance and its length varies more.
 // (2D keeping 1/4, 3/8, 1/2, 5/8: the forward solve of 14,592 points x 64 walks
-// on 1,024 segments 0.747, 0.750, 0.758, 0.764 ms; 3D keeping 1/2, 5/8, 3/4:
-// 17.71, 17.77, 17.42 ms for 20,000 x 64 on 20,480 triangles.)
+// on 1,024 segments 0.747, 0.750, 0.758, 0.764 ms; 3D keeping 1/2 or 5/8:
+// 10.36 or 10.57 ms for 20,000 x 64 on 20,480 triangles.)
 template <int D>
 __device__ __forceinline__ int search_keep(int n) {
-    return D == 2 ? n / 4 : n * 5 / 8;
+    return D == 2 ? n / 4 : n / 2;
 }
 
 // ------------------------------------------------------------------ walker
@@ -2182,9 +2182,9 @@ int set_sample_order(int mode) {
 
 int sample_order_mode() { return g_sample_order; }
 
-__global__ void k_prim_rank(const int *__restrict__ lorig, int nF, unsigned *rank) {
+__global__ void k_prim_rank(const int *__restrict__ torig, int nF, unsigned *rank) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s < nF) rank[__ldg(&lorig[s])] = (unsigned)s;
+    if (s < nF) rank[__ldg(&torig[s])] = (unsigned)s;
 }
 
 template <int D>
@@ -2232,7 +2232,7 @@ int launch_record_order(const SceneImpl &S, const int *wrec, long long total, vo
         b += al(sizeof(unsigned) * (size_t)total);
     }
     const size_t tmp_bytes = need - (size_t)(b - (char *)ws);
-    k_prim_rank<<<(S.nF + 255) / 256, 256, 0, st>>>(S.lorig, S.nF, rank);
+    k_prim_rank<<<(S.nF + 255) / 256, 256, 0, st>>>(S.torig, S.nF, rank);
     const int G = (int)std::min<long long>((total + 255) / 256, 148 * 16);
     if (S.dim == 2)
         k_record_keys<2><<<G, 256, 0, st>>>(wrec, total, rank, S.nF, buf[0], buf[2]);
@@ -2468,7 +2468,7 @@ __global__ void k_batch_prim_rank(const SceneView *__restrict__ views, const Bat
         const int i = find_item_prim(items, n_items, s);
         const long long off = __ldg(&items[i].prim_off);
         const long long local = s - off;
-        if (local < views[i].nF) rank[off + __ldg(&views[i].lorig[local])] = (unsigned)s;
+        if (local < views[i].nF) rank[off + __ldg(&views[i].torig[local])] = (unsigned)s;
     }
 }
 

@@ -63,9 +63,9 @@ struct SceneView {
     // brackets the CDF search to a few entries
     const unsigned short *guide;
     int n_guide;
-    // Search tree of the walk kernels: an implicit 4-ary tree over the sorted
-    // primitives.  Leaf i holds the primitives at sorted positions [LEAF i,
-    // LEAF i + LEAF); the root is at depth 0, the leaves at depth tree_depth,
+    // Search tree of the walk kernels: an implicit 4-ary tree over the
+    // primitives in an order of its own (torig: position -> original index).
+    // Leaf i holds the primitives at positions [LEAF i, LEAF i + LEAF); the root is at depth 0, the leaves at depth tree_depth,
     // and node i of depth d has the children [4 i, 4 i + 4) of depth d + 1.
     // Every node is bounded by an oriented box (k_tree_bounds): orthonormal axes
     // u_k, a centre c and half-extents e_k with |u_k.(y - c)| <= e_k for every
@@ -79,10 +79,11 @@ struct SceneView {
     // A child that does not exist is infinitely far (e0 = -inf).  A leaf's
     // primitives are one block of `prims`: 2D 5 float4, the segments
     // (a, b - a) and their 1/|b - a|^2; 3D 3 float4 per triangle, as in `tri`.
-    // The last leaf repeats the last primitive.
+    // The last leaf repeats the last primitive (and its original index).
     int tree_depth;
     const float4 *tree;
     const float4 *prims;
+    const int *torig;
 };
 
 // Shape of the search tree: primitives per leaf, float4 per node block and per
@@ -554,7 +555,7 @@ struct Search {
     float tol;     // pruning tolerance of the query point (search_bound)
     float bound;   // nodes farther than this (squared) are pruned
     float stop;    // a primitive this near (squared) ends the search (negative: none does)
-    float d2;      // best squared distance so far, and its sorted position (-1: none)
+    float d2;      // best squared distance so far, and its position (-1: none)
     int pos;
     unsigned idx;  // the node to visit next: index within its depth
     int dep;       // its depth, or SEARCH_*
@@ -769,7 +770,7 @@ __device__ __forceinline__ void search_leaf(Search<D> &s, const SceneView &S, co
             // equal distances: the lowest original index
             int o = 0x7fffffff;
             for (; at != 0u; at &= at - 1u) {
-                const int c = __ffs(at) - 1, p = c == N ? s.pos : p0 + c, op = __ldg(&S.lorig[p]);
+                const int c = __ffs(at) - 1, p = c == N ? s.pos : p0 + c, op = __ldg(&S.torig[p]);
                 if (op < o) {
                     o = op;
                     pos = p;
@@ -813,7 +814,7 @@ __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes
 template <int D>
 __device__ __forceinline__ Hit search_hit(const Search<D> &s, const SceneView &S, float ball_m = -1.0f) {
     if (s.pos < 0 || (ball_m > 0.0f && !ball_blocks(s.d2, ball_m))) return Hit{-1, INFINITY};
-    return Hit{__ldg(&S.lorig[s.pos]), s.d2};
+    return Hit{__ldg(&S.torig[s.pos]), s.d2};
 }
 
 // ------------------------------------------------------------------ records
