@@ -29,11 +29,22 @@ __device__ __forceinline__ int ordered_int(float f) {
 }
 __device__ __forceinline__ float from_ordered_int(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
 
-__global__ void k_check_indices(const int *F, long long n, int nV, int *bad) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int v = F[i];
-        if (v < 0 || v >= nV) atomicOr(bad, 1);
+// out[0]: whether an index is out of range; out[1] (2D): segments f whose end
+// vertex starts segment f + 1, cyclically.
+__global__ void k_check_indices(const int *F, int nF, int dim, int nV, int *out) {
+    int bad = 0, chain = 0;
+    for (long long f = blockIdx.x * (long long)blockDim.x + threadIdx.x; f < nF; f += (long long)gridDim.x * blockDim.x) {
+        for (int k = 0; k < dim; ++k) bad |= F[f * dim + k] < 0 || F[f * dim + k] >= nV;
+        if (dim == 2) chain += F[2 * f + 1] == F[2 * (f + 1 < nF ? f + 1 : 0)];
     }
+    if (bad) atomicOr(&out[0], 1);
+    if (chain) atomicAdd(&out[1], chain);
+}
+
+// Start of a build's counters: [0, 6) the bounding box's ordered ints, [6] the
+// deepest node.
+__global__ void k_build_init(int *c) {
+    if (threadIdx.x < 7) c[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : threadIdx.x < 6 ? (int)0x80000000 : 0;
 }
 
 __global__ void k_aabb(const float *V, int nV, int dim, int *lohi) {
@@ -62,9 +73,9 @@ __global__ void k_aabb(const float *V, int nV, int dim, int *lohi) {
     }
 }
 
-// Per (face, slot) normal contribution and its sort key (vertex << 32 | slot id).
+// Per (face, slot) normal contribution.
 template <int D>
-__global__ void k_face_normals(const float *V, const int *F, int nF, float *contrib, unsigned long long *keys) {
+__global__ void k_face_normals(const float *V, const int *F, int nF, float *contrib) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nF) return;
     if (D == 2) {
@@ -81,7 +92,6 @@ __global__ void k_face_normals(const float *V, const int *F, int nF, float *cont
         for (int s = 0; s < 2; ++s) {
             contrib[(size_t)(2 * f + s) * 2] = nx;
             contrib[(size_t)(2 * f + s) * 2 + 1] = ny;
-            keys[2 * f + s] = ((unsigned long long)(unsigned)F[2 * f + s] << 32) | (unsigned)(2 * f + s);
         }
     } else {
         const int i0 = F[3 * f], i1 = F[3 * f + 1], i2 = F[3 * f + 2];
@@ -111,27 +121,32 @@ __global__ void k_face_normals(const float *V, const int *F, int nF, float *cont
         const float ang[3] = {angle(e10, e20), angle(e21, e01), angle(e02, e12)};
         for (int s = 0; s < 3; ++s) {
             for (int k = 0; k < 3; ++k) contrib[(size_t)(3 * f + s) * 3 + k] = ang[s] * n[k];
-            keys[3 * f + s] = ((unsigned long long)(unsigned)F[3 * f + s] << 32) | (unsigned)(3 * f + s);
         }
     }
 }
 
-__global__ void k_segments(const unsigned long long *keys, int n, int *beg, int *end) {
+__global__ void k_iota(int *x, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const unsigned v = (unsigned)(keys[i] >> 32);
-    if (i == 0 || (unsigned)(keys[i - 1] >> 32) != v) beg[v] = i;
-    if (i == n - 1 || (unsigned)(keys[i + 1] >> 32) != v) end[v] = i + 1;
+    if (i < n) x[i] = i;
+}
+
+// First slot of each vertex in the sorted slots, first[nV] = n: vertices without
+// faces have an empty range.
+__global__ void k_vertex_ranges(const int *verts, int n, int nV, int *first) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > n) return;
+    const int lo = i == 0 ? 0 : verts[i - 1] + 1, hi = i == n ? nV : verts[i];
+    for (int v = lo; v <= hi; ++v) first[v] = i;
 }
 
 template <int D>
-__global__ void k_vertex_normals(const unsigned long long *keys, const float *contrib, const int *beg, const int *end,
-                                 int nV, float *N) {
+__global__ void k_vertex_normals(const int *slots, const int *first, const float *contrib, int nV, float *N) {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nV) return;
     float s[3] = {0.0f, 0.0f, 0.0f};
-    for (int i = beg[v]; i < end[v]; ++i) {
-        const unsigned slot = (unsigned)keys[i];
+    const int end = first[v + 1];
+    for (int i = first[v]; i < end; ++i) {
+        const int slot = slots[i];
         for (int k = 0; k < D; ++k) s[k] += contrib[(size_t)slot * D + k];
     }
     const float len = sqrtf(D == 2 ? dot2(s[0], s[1], s[0], s[1]) : dot3(s[0], s[1], s[2], s[0], s[1], s[2]));
@@ -185,23 +200,18 @@ __device__ __forceinline__ uint32_t hilbert3(uint32_t x0, uint32_t x1, uint32_t 
     return (spread3(X[0]) << 2) | (spread3(X[1]) << 1) | spread3(X[2]);
 }
 
-// Number of segments f whose end vertex starts segment f + 1 (cyclically).
-__global__ void k_chain_count(const int *F, int nF, int *count) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= nF) return;
-    const int next = f + 1 < nF ? f + 1 : 0;
-    if (F[2 * f + 1] == F[2 * next]) atomicAdd(count, 1);
-}
-
 // Primitive precomputation, primitive boxes and sort keys: Morton (order 0),
 // the input index (order 1) or Hilbert (order 2) of the box centre.
 template <int D>
-__global__ void k_prims(const float *V, const int *F, int nF, float lo0, float lo1, float lo2, float hi0, float hi1,
-                        float hi2, float4 *seg, float *seginv, float4 *tri, float *pbox, unsigned long long *keys,
-                        int order) {
+__global__ void k_prims(const float *V, const int *F, int nF, const int *lohi, float4 *seg, float *seginv,
+                        float4 *tri, float *pbox, unsigned long long *keys, int order) {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= nF) return;
-    const float slo[3] = {lo0, lo1, lo2}, shi[3] = {hi0, hi1, hi2};
+    float slo[3], shi[3];
+    for (int k = 0; k < D; ++k) {
+        slo[k] = from_ordered_int(lohi[k]);
+        shi[k] = from_ordered_int(lohi[3 + k]);
+    }
     float bl[3], bh[3];
     if (D == 2) {
         const int i0 = F[2 * f], i1 = F[2 * f + 1];
@@ -605,7 +615,7 @@ __device__ void sym3_eigen(float a[3][3], float v[3][3]) {
 // Sum / minimum / maximum of x over the TPN threads of one node (1, a warp or
 // the block); every thread gets the result.
 template <int TPN, class Op>
-__device__ __forceinline__ double node_reduce(double x, Op op, double *red) {
+__device__ __forceinline__ float node_reduce(float x, Op op, float *red) {
     if constexpr (TPN > 1) {
         for (int o = 16; o > 0; o >>= 1) x = op(x, __shfl_xor_sync(0xffffffffu, x, o));
     }
@@ -619,70 +629,72 @@ __device__ __forceinline__ double node_reduce(double x, Op op, double *red) {
     return x;
 }
 
-// Vertices of the primitive at the tree's position s as the distance code sees
-// them: a and a + d of a segment; a, a + ab and a + ac of a triangle.
+// Vertices, relative to o, of the primitive at the tree's position s as the
+// distance code sees them: a and a + d of a segment; a, a + ab and a + ac of a
+// triangle.
 template <int D>
-__device__ __forceinline__ void prim_vertices(const float4 *prims, int s, double y[3][3]) {
+__device__ __forceinline__ void prim_vertices(const float4 *prims, int s, const float *o, float y[3][3]) {
     const float4 *b = prims + (size_t)(s / Tree<D>::LEAF) * Tree<D>::LEAF_W;
     const int i = s % Tree<D>::LEAF;
     if (D == 2) {
         const float4 g = b[i];
-        y[0][0] = g.x;
-        y[0][1] = g.y;
-        y[1][0] = (double)g.x + g.z;
-        y[1][1] = (double)g.y + g.w;
+        y[0][0] = g.x - o[0];
+        y[0][1] = g.y - o[1];
+        y[1][0] = y[0][0] + g.z;
+        y[1][1] = y[0][1] + g.w;
     } else {
         const float4 a = b[3 * i], ab = b[3 * i + 1], ac = b[3 * i + 2];
-        const float o[3] = {a.x, a.y, a.z}, e[3] = {ab.x, ab.y, ab.z}, f[3] = {ac.x, ac.y, ac.z};
+        const float p[3] = {a.x, a.y, a.z}, e[3] = {ab.x, ab.y, ab.z}, f[3] = {ac.x, ac.y, ac.z};
         for (int k = 0; k < 3; ++k) {
-            y[0][k] = o[k];
-            y[1][k] = (double)o[k] + e[k];
-            y[2][k] = (double)o[k] + f[k];
+            y[0][k] = p[k] - o[k];
+            y[1][k] = y[0][k] + e[k];
+            y[2][k] = y[0][k] + f[k];
         }
     }
 }
 
-// Bound of a node of `np` primitives from position s0, by TPN threads, all
-// of which call.  The axes are the principal axes of the vertices, eigenvectors
-// of their covariance, made orthonormal, shrunk a little and rounded (2D: to
-// float, 3D: to multiples of 2^-15) so that the rounded axes -- with the third 3D
-// axis evaluated in float exactly as the query does (obb_axis2) -- form a matrix
-// of norm at most 1.  The centre -- the middle of the projections on the axes --
-// is rounded to float too, and the extents bound the vertices about the float
-// centre along the rounded axes, evaluated in double and widened by 1e-6 of the
-// largest |y - c|, which covers the query's float rounding of q - c and of the
-// products with it (relative 2^-22 of |q - c| <= |q - y| + |y - c|).
+// Bound of a node of `np` primitives from position s0, by TPN threads, all of
+// which call.  The axes are the principal axes of the vertices, eigenvectors of
+// their covariance, made orthonormal, shrunk a little and rounded (2D: to float,
+// 3D: to multiples of 2^-15) so that the rounded axes -- with the third 3D axis
+// evaluated in float exactly as the query does (obb_axis2) -- form a matrix of
+// norm at most 1.  The centre is the middle of the projections on the axes.  The
+// extents bound the vertices about the rounded centre along the rounded axes,
+// widened by 4e-6 of the node's diameter d.  That covers the query's float
+// rounding of q - c and of the products with it (relative 2^-22 of |q - c| <=
+// |q - y| + |y - c|: 1e-6 d for the latter) and the float evaluation here:
+// vertices relative to the node's first one (2 x 2^-24 of at most 2 d each),
+// their products with the axes (3.1e-7 d) and the centre's (3.7e-7 d), in all
+// 2.2e-6 d.
 //   2D: out = (u0, c, e0, e1).
 //   3D: out = (c, u0, u1, e) with the axes in units of 2^-15.
 template <int D, int TPN>
-__device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, int t, double *red, float *out) {
+__device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, int t, float *red, float *out) {
     constexpr int NV = D == 2 ? 2 : 3;
-    auto add = [](double a, double b) { return a + b; };
-    auto lower = [](double a, double b) { return fmin(a, b); };
-    auto upper = [](double a, double b) { return fmax(a, b); };
+    auto add = [](float a, float b) { return a + b; };
+    auto lower = [](float a, float b) { return fminf(a, b); };
+    auto upper = [](float a, float b) { return fmaxf(a, b); };
     // moments about the first vertex
-    double y0[3], y[3][3], m[3] = {0.0, 0.0, 0.0}, cv[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    prim_vertices<D>(prims, s0, y);
+    float y0[3] = {0.0f, 0.0f, 0.0f}, y[3][3], m[3] = {0.0f, 0.0f, 0.0f};
+    float cv[6] = {0.0f, 0.0f, 0.0f, 0.0f, 0.0f, 0.0f};
+    prim_vertices<D>(prims, s0, y0, y);
     for (int k = 0; k < D; ++k) y0[k] = y[0][k];
     for (int i = t; i < np; i += TPN) {
-        prim_vertices<D>(prims, s0 + i, y);
+        prim_vertices<D>(prims, s0 + i, y0, y);
         for (int j = 0; j < NV; ++j) {
-            double w[3];
-            for (int k = 0; k < D; ++k) {
-                w[k] = y[j][k] - y0[k];
-                m[k] += w[k];
-            }
-            cv[0] += w[0] * w[0];
-            cv[1] += w[0] * w[1];
-            cv[3] += w[1] * w[1];
+            const float *w = y[j];
+            for (int k = 0; k < D; ++k) m[k] += w[k];
+            cv[0] = fmaf(w[0], w[0], cv[0]);
+            cv[1] = fmaf(w[0], w[1], cv[1]);
+            cv[3] = fmaf(w[1], w[1], cv[3]);
             if (D == 3) {
-                cv[2] += w[0] * w[2];
-                cv[4] += w[1] * w[2];
-                cv[5] += w[2] * w[2];
+                cv[2] = fmaf(w[0], w[2], cv[2]);
+                cv[4] = fmaf(w[1], w[2], cv[4]);
+                cv[5] = fmaf(w[2], w[2], cv[5]);
             }
         }
     }
-    const double n = (double)np * NV;
+    const float n = (float)np * NV;
     for (int k = 0; k < D; ++k) m[k] = node_reduce<TPN>(m[k], add, red) / n;
     for (int k = 0; k < 6; ++k)
         if (D == 3 || k < 2 || k == 3) cv[k] = node_reduce<TPN>(cv[k], add, red) / n;
@@ -692,10 +704,11 @@ __device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, 
     // orthogonal axes u[0], u[1] (and u[2]: the normal)
     // 3D: rounding moves an axis by up to 2.7e-5 and two axes' product by 5.3e-5
     const double shrink = D == 2 ? 1.0 - 0x1p-20 : (1.0 - 6e-5) * 32768.0;
-    const double unit[3] = {D == 2 ? 1.0 : 0x1p-15, D == 2 ? 1.0 : 0x1p-15, 0x1p-30};  // of u[k]
+    const float unit[3] = {D == 2 ? 1.0f : 0x1p-15f, D == 2 ? 1.0f : 0x1p-15f, 0x1p-30f};  // of u[k]
     float u[3][3];
     if (D == 2) {
-        const double th = 0.5 * atan2(2.0 * cv[1], cv[0] - cv[3]);
+        double th = 0.5 * atan2(2.0 * (double)cv[1], (double)cv[0] - (double)cv[3]);
+        if (!(fabs(th) <= 2.0)) th = 0.0;  // overflow of the moments: any axes do
         u[0][0] = (float)(cos(th) * shrink);
         u[0][1] = (float)(sin(th) * shrink);
         u[1][0] = -u[0][1];
@@ -704,11 +717,20 @@ __device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, 
         cv[2] -= m[0] * m[2];
         cv[4] -= m[1] * m[2];
         cv[5] -= m[2] * m[2];
-        // scaled so that squares of tiny nodes' entries stay normal floats
-        const double tr = cv[0] + cv[3] + cv[5], sc = tr > 0.0 ? 1.0 / tr : 0.0;
-        float A[3][3] = {{(float)(cv[0] * sc), (float)(cv[1] * sc), (float)(cv[2] * sc)},
-                         {(float)(cv[1] * sc), (float)(cv[3] * sc), (float)(cv[4] * sc)},
-                         {(float)(cv[2] * sc), (float)(cv[4] * sc), (float)(cv[5] * sc)}};
+        // scaled so that squares of tiny nodes' entries stay normal floats; the
+        // coordinate axes where the moments leave the range of float
+        const float tr = cv[0] + cv[3] + cv[5];
+        const bool scaled = tr > 1e-36f && tr < INFINITY;
+        float A[3][3] = {{0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}, {0.0f, 0.0f, 0.0f}};
+        if (scaled) {
+            const float sc = 1.0f / tr;
+            A[0][0] = cv[0] * sc;
+            A[1][1] = cv[3] * sc;
+            A[2][2] = cv[5] * sc;
+            A[0][1] = A[1][0] = cv[1] * sc;
+            A[0][2] = A[2][0] = cv[2] * sc;
+            A[1][2] = A[2][1] = cv[4] * sc;
+        }
         float vec[3][3];
         sym3_eigen(A, vec);
         int o[3] = {0, 1, 2};  // by falling variance
@@ -721,52 +743,54 @@ __device__ __forceinline__ void node_bound(const float4 *prims, int s0, int np, 
                 }
         double p[3], w[3], lp = 0.0, lw = 0.0, pw = 0.0;
         for (int k = 0; k < 3; ++k) lp += (double)vec[k][o[0]] * vec[k][o[0]];
+        lp = 1.0 / sqrt(lp);
         for (int k = 0; k < 3; ++k) {
-            p[k] = vec[k][o[0]] / sqrt(lp);
+            p[k] = vec[k][o[0]] * lp;
             pw += p[k] * vec[k][o[1]];
         }
         for (int k = 0; k < 3; ++k) {
             w[k] = vec[k][o[1]] - pw * p[k];
             lw += w[k] * w[k];
         }
+        lw = shrink / sqrt(lw);
         for (int k = 0; k < 3; ++k) {
             u[0][k] = (float)rint(p[k] * shrink);
-            u[1][k] = (float)rint(w[k] / sqrt(lw) * shrink);
+            u[1][k] = (float)rint(w[k] * lw);
         }
         obb_axis2(u[0], u[1], u[2]);
     }
     // ranges of u_k.(y - y0), and the centre in the middle of them
-    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (int i = t; i < np; i += TPN) {
-        prim_vertices<D>(prims, s0 + i, y);
+        prim_vertices<D>(prims, s0 + i, y0, y);
         for (int j = 0; j < NV; ++j)
             for (int k = 0; k < D; ++k) {
-                double p = 0.0;
-                for (int c = 0; c < D; ++c) p += unit[k] * (double)u[k][c] * (y[j][c] - y0[c]);
-                lo[k] = fmin(lo[k], p);
-                hi[k] = fmax(hi[k], p);
+                const float p = D == 2 ? dot2(u[k][0], u[k][1], y[j][0], y[j][1])
+                                       : dot3(u[k][0], u[k][1], u[k][2], y[j][0], y[j][1], y[j][2]) * unit[k];
+                lo[k] = fminf(lo[k], p);
+                hi[k] = fmaxf(hi[k], p);
             }
     }
+    float d2 = 0.0f;
     for (int k = 0; k < D; ++k) {
         lo[k] = node_reduce<TPN>(lo[k], lower, red);
         hi[k] = node_reduce<TPN>(hi[k], upper, red);
+        d2 = fmaf(hi[k] - lo[k], hi[k] - lo[k], d2);
     }
-    float cf[3];
+    float cf[3], ef[3], w[3];
     for (int c = 0; c < D; ++c) {
-        double x = y0[c];
-        for (int k = 0; k < D; ++k) x += 0.5 * (lo[k] + hi[k]) * (unit[k] * (double)u[k][c]);
-        cf[c] = (float)x;
+        float x = 0.0f;
+        for (int k = 0; k < D; ++k) x = fmaf(0.5f * (lo[k] + hi[k]) * unit[k], u[k][c], x);
+        cf[c] = y0[c] + x;
+        w[c] = cf[c] - y0[c];
     }
-    double e[3] = {0.0, 0.0, 0.0};
+    // the axes are orthonormal to 3e-4, so the diameter is at most this
+    const float pad = 4.01e-6f * sqrtf(d2);
     for (int k = 0; k < D; ++k) {
-        double off = 0.0;
-        for (int c = 0; c < D; ++c) off += unit[k] * (double)u[k][c] * ((double)cf[c] - y0[c]);
-        e[k] = fmax(hi[k] - off, off - lo[k]);
+        const float off =
+            D == 2 ? dot2(u[k][0], u[k][1], w[0], w[1]) : dot3(u[k][0], u[k][1], u[k][2], w[0], w[1], w[2]) * unit[k];
+        ef[k] = __fadd_ru(fmaxf(hi[k] - off, off - lo[k]), pad);
     }
-    // the axes are orthonormal to 3e-4, so |y - c| is at most this
-    const double pad = 1.001e-6 * sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
-    float ef[3];
-    for (int k = 0; k < D; ++k) ef[k] = __double2float_ru(e[k] + pad);
     if (D == 2) {
         out[0] = u[0][0];
         out[1] = u[0][1];
@@ -822,7 +846,7 @@ __host__ __device__ inline int nodes_per_block(long long prims) {
 template <int D, bool LARGE>
 __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_tree_bounds(
     TreePlan P, const float4 *prims, float4 *tree) {
-    __shared__ double red[32];
+    __shared__ float red[32];
     int d = P.d0;
     while (d < P.d1 && (int)blockIdx.x >= P.first[d + 1]) ++d;
     const long long cap = node_prims(Tree<D>::LEAF, P.depth - d);
@@ -866,7 +890,7 @@ static cudaError_t dalloc(T **p, size_t count, cudaStream_t st) {
 }
 
 void SceneImpl::release(cudaStream_t st) {
-    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, tree, prims, torig, guide};
+    void *ptrs[] = {V, F, N, g, seg, seginv, tri, node, lseg, lseginv, ltri, lorig, cdf, tree, prims, torig, vslot, vfirst, guide};
     for (void *p : ptrs)
         if (p) cudaFreeAsync(p, st);
     V = nullptr;
@@ -885,6 +909,8 @@ void SceneImpl::release(cudaStream_t st) {
     tree = nullptr;
     prims = nullptr;
     torig = nullptr;
+    vslot = nullptr;
+    vfirst = nullptr;
     tree_ordered = false;
     guide = nullptr;
 }
@@ -972,102 +998,116 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
     return 0;
 }
 
+// The Green's function tables, the same for every scene, computed once.
+struct GTables {
+    std::vector<float> cdf;
+    std::vector<unsigned short> guide;
+};
+static const GTables &g_tables() {
+    static const GTables t = [] {
+        GTables x;
+        build_g_cdf(x.cdf, 10000);
+        build_g_guide(x.cdf, 2048, x.guide);
+        return x;
+    }();
+    return t;
+}
+
+// Temporaries of a build: one allocation, carved up.
+struct Arena {
+    char *base = nullptr;
+    size_t used = 0;
+    template <typename T>
+    T *take(size_t n) {
+        T *p = reinterpret_cast<T *>(base + used);
+        used += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
+static int index_bits(long long n) {
+    int b = 1;
+    while (b < 32 && (1LL << b) < n) ++b;
+    return b;
+}
+
+// Slots (face, corner) by vertex, in face order: vslot, and vfirst[v] the first
+// of vertex v.  They depend on the faces alone, so once per scene.
+static int build_vertex_slots(SceneImpl &S, cudaStream_t st) {
+    const int n = S.nF * S.dim, TB = 256, bits = index_bits(S.nV);
+    int *ids = nullptr, *verts = nullptr;
+    size_t tmp_bytes = 0;
+    WOS_TRY(dalloc(&S.vslot, n, st));
+    WOS_TRY(dalloc(&S.vfirst, (size_t)S.nV + 1, st));
+    cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, S.F, verts, ids, S.vslot, n, 0, bits, st);
+    Arena sizes, A;
+    sizes.take<int>(n);
+    sizes.take<int>(n);
+    sizes.take<char>(tmp_bytes);
+    WOS_TRY(cudaMallocAsync((void **)&A.base, sizes.used, st));
+    ids = A.take<int>(n);
+    verts = A.take<int>(n);
+    void *tmp = A.take<char>(tmp_bytes);
+    k_iota<<<nblk(n, TB), TB, 0, st>>>(ids, n);
+    WOS_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, S.F, verts, ids, S.vslot, n, 0, bits, st));
+    k_vertex_ranges<<<nblk((long long)n + 1, TB), TB, 0, st>>>(verts, n, S.nV, S.vfirst);
+    WOS_TRY(cudaGetLastError());
+    cudaFreeAsync(A.base, st);
+    return 0;
+}
+
 template <int D>
 static int build_geometry(SceneImpl &S, cudaStream_t st) {
-    const int nV = S.nV, nF = S.nF;
+    const int nV = S.nV, nF = S.nF, nInt = nF - 1;
     const int TB = 256;
-    // ---- AABB
-    int *lohi = nullptr;
-    WOS_TRY(dalloc(&lohi, 6, st));
-    {
-        int init[6] = {0x7fffffff, 0x7fffffff, 0x7fffffff, (int)0x80000000, (int)0x80000000, (int)0x80000000};
-        WOS_TRY(cudaMemcpyAsync(lohi, init, sizeof(init), cudaMemcpyHostToDevice, st));
-        WOS_TRY(cudaStreamSynchronize(st));
+    if (S.vslot == nullptr)
+        if (int rc = build_vertex_slots(S, st)) return rc;
+    // Sorts are stable and start in index order, so keys sort by their upper
+    // half alone: the Morton code or Hilbert index, and the node's depth.
+    const int key_bits = D == 2 ? 32 : 30, depth_bits = 12;
+    size_t tmp_bytes = 0, t2 = 0;
+    unsigned long long *none = nullptr;
+    if (S.prim_order != 1)
+        cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, none, none, nF, 32, 32 + key_bits, st);
+    if (nInt > 0) cub::DeviceRadixSort::SortKeys(nullptr, t2, none, none, nInt, 32, 32 + depth_bits, st);
+    tmp_bytes = std::max(tmp_bytes, t2);
+    Arena A;
+    int *counters = nullptr, *pint = nullptr, *pleaf = nullptr, *flags = nullptr, *new_of_old = nullptr;
+    float *contrib = nullptr, *pbox = nullptr, *nbox = nullptr;
+    unsigned long long *mkeys = nullptr, *skeys = nullptr, *dkeys = nullptr, *dkeys2 = nullptr;
+    int2 *child = nullptr;
+    void *tmp = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {  // sizes, then the buffers
+        A.used = 0;
+        counters = A.take<int>(8);
+        contrib = A.take<float>((size_t)nF * D * D);
+        pbox = A.take<float>((size_t)nF * 2 * D);
+        mkeys = A.take<unsigned long long>(nF);
+        skeys = S.prim_order == 1 ? mkeys : A.take<unsigned long long>(nF);
+        tmp = A.take<char>(tmp_bytes);
+        child = A.take<int2>(nInt);
+        pint = A.take<int>(nInt);
+        pleaf = A.take<int>(nF);
+        flags = A.take<int>(nInt);
+        new_of_old = A.take<int>(nInt);
+        nbox = A.take<float>((size_t)nInt * 2 * D);
+        dkeys = A.take<unsigned long long>(nInt);
+        dkeys2 = A.take<unsigned long long>(nInt);
+        if (pass == 0) WOS_TRY(cudaMallocAsync((void **)&A.base, A.used, st));
     }
-    k_aabb<<<std::min(nblk(nV, TB), 1024), TB, 0, st>>>(S.V, nV, D, lohi);
-    int lohi_h[6];
-    WOS_TRY(cudaMemcpyAsync(lohi_h, lohi, sizeof(lohi_h), cudaMemcpyDeviceToHost, st));
-    WOS_TRY(cudaStreamSynchronize(st));
-    cudaFreeAsync(lohi, st);
-    auto from_ord = [](int i) {
-        int b = i >= 0 ? i : i ^ 0x7fffffff;
-        float f;
-        memcpy(&f, &b, 4);
-        return f;
-    };
-    for (int k = 0; k < 3; ++k) {
-        S.lo[k] = k < D ? from_ord(lohi_h[k]) : 0.0f;
-        S.hi[k] = k < D ? from_ord(lohi_h[3 + k]) : 0.0f;
-    }
-    float ext = INFINITY;
-    for (int k = 0; k < D; ++k) ext = fminf(ext, fabsf(S.hi[k] - S.lo[k]));
-    S.half_min_extent = ext * 0.5f;
+    // ---- bounding box and vertex normals
+    k_build_init<<<1, 32, 0, st>>>(counters);
+    k_aabb<<<std::min(nblk(nV, TB), 1024), TB, 0, st>>>(S.V, nV, D, counters);
+    k_face_normals<D><<<nblk(nF, TB), TB, 0, st>>>(S.V, S.F, nF, contrib);
+    k_vertex_normals<D><<<nblk(nV, TB), TB, 0, st>>>(S.vslot, S.vfirst, contrib, nV, S.N);
 
-    // ---- vertex normals
-    {
-        const int ns = nF * D;
-        float *contrib = nullptr;
-        unsigned long long *keys = nullptr, *keys2 = nullptr;
-        int *beg = nullptr, *end = nullptr;
-        WOS_TRY(dalloc(&contrib, (size_t)ns * D, st));
-        WOS_TRY(dalloc(&keys, ns, st));
-        WOS_TRY(dalloc(&keys2, ns, st));
-        WOS_TRY(dalloc(&beg, nV, st));
-        WOS_TRY(dalloc(&end, nV, st));
-        WOS_TRY(cudaMemsetAsync(beg, 0, sizeof(int) * nV, st));
-        WOS_TRY(cudaMemsetAsync(end, 0, sizeof(int) * nV, st));
-        k_face_normals<D><<<nblk(nF, TB), TB, 0, st>>>(S.V, S.F, nF, contrib, keys);
-        size_t tmp_bytes = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, keys, keys2, ns, 0, 64, st);
-        void *tmp = nullptr;
-        WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
-        WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, keys, keys2, ns, 0, 64, st));
-        k_segments<<<nblk(ns, TB), TB, 0, st>>>(keys2, ns, beg, end);
-        k_vertex_normals<D><<<nblk(nV, TB), TB, 0, st>>>(keys2, contrib, beg, end, nV, S.N);
-        WOS_TRY(cudaGetLastError());
-        cudaFreeAsync(tmp, st);
-        cudaFreeAsync(contrib, st);
-        cudaFreeAsync(keys, st);
-        cudaFreeAsync(keys2, st);
-        cudaFreeAsync(beg, st);
-        cudaFreeAsync(end, st);
-    }
-
-    // ---- primitive order: a polyline whose segments follow each other keeps
-    // its input order (its leaves are then arcs of the curve, the most
-    // compact runs); other polylines sort by Morton code, meshes by Hilbert
-    // index.  Decided once: moving vertices keeps the order.
-    if (S.prim_order < 0) {
-        S.prim_order = D == 3 ? 2 : 0;
-        if (D == 2 && nF >= 2) {
-            int *cnt = nullptr;
-            WOS_TRY(dalloc(&cnt, 1, st));
-            WOS_TRY(cudaMemsetAsync(cnt, 0, sizeof(int), st));
-            k_chain_count<<<nblk(nF, TB), TB, 0, st>>>(S.F, nF, cnt);
-            int cnt_h = 0;
-            WOS_TRY(cudaMemcpyAsync(&cnt_h, cnt, sizeof(int), cudaMemcpyDeviceToHost, st));
-            WOS_TRY(cudaStreamSynchronize(st));
-            cudaFreeAsync(cnt, st);
-            if (cnt_h >= nF - nF / 10) S.prim_order = 1;
-        }
-    }
-
-    // ---- primitives + sort keys
-    float *pbox = nullptr;
-    unsigned long long *mkeys = nullptr, *skeys = nullptr;
-    WOS_TRY(dalloc(&pbox, (size_t)nF * 2 * D, st));
-    WOS_TRY(dalloc(&mkeys, nF, st));
-    WOS_TRY(dalloc(&skeys, nF, st));
-    k_prims<D><<<nblk(nF, TB), TB, 0, st>>>(S.V, S.F, nF, S.lo[0], S.lo[1], S.lo[2], S.hi[0], S.hi[1], S.hi[2], S.seg,
-                                           S.seginv, S.tri, pbox, mkeys, S.prim_order);
-    {
-        size_t tmp_bytes = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, mkeys, skeys, nF, 0, 64, st);
-        void *tmp = nullptr;
-        WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
-        WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, mkeys, skeys, nF, 0, 64, st));
-        cudaFreeAsync(tmp, st);
-    }
+    // ---- primitives and sort keys: a polyline whose segments follow each other
+    // keeps its input order (its leaves are then arcs of the curve, the most
+    // compact runs; the keys are sorted as they are); other polylines sort by
+    // Morton code, meshes by Hilbert index
+    k_prims<D><<<nblk(nF, TB), TB, 0, st>>>(S.V, S.F, nF, counters, S.seg, S.seginv, S.tri, pbox, mkeys, S.prim_order);
+    if (S.prim_order != 1)
+        WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, mkeys, skeys, nF, 32, 32 + key_bits, st));
     k_leaf_data<D><<<nblk(nF, TB), TB, 0, st>>>(skeys, nF, S.seg, S.seginv, S.tri, S.lseg, S.lseginv, S.ltri, S.lorig);
 
     // ---- search tree, in the buffers of the first build (their sizes depend
@@ -1110,58 +1150,37 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
     }
 
     // ---- hierarchy
-    const int nInt = nF - 1;
     S.nNodes = nInt;
-    S.depth = 0;
     if (nInt > 0) {
-        int2 *child = nullptr;
-        int *pint = nullptr, *pleaf = nullptr, *flags = nullptr, *maxd = nullptr, *new_of_old = nullptr;
-        float *nbox = nullptr;
-        unsigned long long *dkeys = nullptr, *dkeys2 = nullptr;
-        WOS_TRY(dalloc(&child, nInt, st));
-        WOS_TRY(dalloc(&pint, nInt, st));
-        WOS_TRY(dalloc(&pleaf, nF, st));
-        WOS_TRY(dalloc(&flags, nInt, st));
-        WOS_TRY(dalloc(&maxd, 1, st));
-        WOS_TRY(dalloc(&new_of_old, nInt, st));
-        WOS_TRY(dalloc(&nbox, (size_t)nInt * 2 * D, st));
-        WOS_TRY(dalloc(&dkeys, nInt, st));
-        WOS_TRY(dalloc(&dkeys2, nInt, st));
         WOS_TRY(cudaMemsetAsync(pint, 0xff, sizeof(int) * nInt, st));
         WOS_TRY(cudaMemsetAsync(pleaf, 0xff, sizeof(int) * nF, st));
         WOS_TRY(cudaMemsetAsync(flags, 0, sizeof(int) * nInt, st));
-        WOS_TRY(cudaMemsetAsync(maxd, 0, sizeof(int), st));
         k_karras<<<nblk(nInt, TB), TB, 0, st>>>(skeys, nF, child, pint, pleaf);
         k_refit<D><<<nblk(nF, TB), TB, 0, st>>>(skeys, nF, pbox, child, pint, pleaf, flags, nbox);
-        k_depth<<<nblk(nInt, TB), TB, 0, st>>>(pint, nInt, dkeys, maxd);
-        size_t tmp_bytes = 0;
-        cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, dkeys, dkeys2, nInt, 0, 64, st);
-        void *tmp = nullptr;
-        WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
-        WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, dkeys, dkeys2, nInt, 0, 64, st));
+        k_depth<<<nblk(nInt, TB), TB, 0, st>>>(pint, nInt, dkeys, counters + 6);
+        WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, dkeys, dkeys2, nInt, 32, 32 + depth_bits, st));
         k_bfs_rank<<<nblk(nInt, TB), TB, 0, st>>>(dkeys2, nInt, new_of_old);
         k_write_nodes<D><<<nblk(nInt, TB), TB, 0, st>>>(skeys, nInt, pbox, nbox, child, new_of_old, S.node);
-        WOS_TRY(cudaGetLastError());
-        int maxd_h = 0;
-        WOS_TRY(cudaMemcpyAsync(&maxd_h, maxd, sizeof(int), cudaMemcpyDeviceToHost, st));
-        WOS_TRY(cudaStreamSynchronize(st));
-        S.depth = maxd_h;
-        cudaFreeAsync(tmp, st);
-        cudaFreeAsync(child, st);
-        cudaFreeAsync(pint, st);
-        cudaFreeAsync(pleaf, st);
-        cudaFreeAsync(flags, st);
-        cudaFreeAsync(maxd, st);
-        cudaFreeAsync(new_of_old, st);
-        cudaFreeAsync(nbox, st);
-        cudaFreeAsync(dkeys, st);
-        cudaFreeAsync(dkeys2, st);
     }
-    cudaFreeAsync(pbox, st);
-    cudaFreeAsync(mkeys, st);
-    cudaFreeAsync(skeys, st);
     WOS_TRY(cudaGetLastError());
+    int host[7];
+    WOS_TRY(cudaMemcpyAsync(host, counters, sizeof(host), cudaMemcpyDeviceToHost, st));
+    cudaFreeAsync(A.base, st);
     WOS_TRY(cudaStreamSynchronize(st));
+    auto from_ord = [](int i) {
+        int b = i >= 0 ? i : i ^ 0x7fffffff;
+        float f;
+        memcpy(&f, &b, 4);
+        return f;
+    };
+    for (int k = 0; k < 3; ++k) {
+        S.lo[k] = k < D ? from_ord(host[k]) : 0.0f;
+        S.hi[k] = k < D ? from_ord(host[3 + k]) : 0.0f;
+    }
+    float ext = INFINITY;
+    for (int k = 0; k < D; ++k) ext = fminf(ext, fabsf(S.hi[k] - S.lo[k]));
+    S.half_min_extent = ext * 0.5f;
+    S.depth = host[6];
     return 0;
 }
 
@@ -1193,31 +1212,31 @@ int SceneImpl::allocate(cudaStream_t st) {
     const size_t blocks = (size_t)tree_block(tree_depth - 1, 0) + (size_t)((n_leaf + 3) / 4);
     WOS_TRY(dalloc(&tree, blocks * (D == 2 ? Tree<2>::NODE_W : Tree<3>::NODE_W), st));
     WOS_TRY(dalloc(&prims, (size_t)n_leaf * (D == 2 ? Tree<2>::LEAF_W : Tree<3>::LEAF_W), st));
-    std::vector<float> c;
-    build_g_cdf(c, 10000);
+    const GTables &tables = g_tables();
+    const std::vector<float> &c = tables.cdf;
+    const std::vector<unsigned short> &gd = tables.guide;
     n_cdf = (int)c.size();
-    std::vector<unsigned short> gd;
-    n_guide = 2048;
-    build_g_guide(c, n_guide, gd);
+    n_guide = (int)gd.size() - 1;
     WOS_TRY(dalloc(&cdf, c.size(), st));
     WOS_TRY(dalloc(&guide, gd.size(), st));
     WOS_TRY(cudaMemcpyAsync(cdf, c.data(), c.size() * sizeof(float), cudaMemcpyHostToDevice, st));
     WOS_TRY(cudaMemcpyAsync(guide, gd.data(), gd.size() * sizeof(unsigned short), cudaMemcpyHostToDevice, st));
-    WOS_TRY(cudaStreamSynchronize(st));
     return 0;
 }
 
+// Checks the faces and decides the primitives' order.
 int SceneImpl::check_indices(cudaStream_t st) {
-    int *bad = nullptr;
-    WOS_TRY(dalloc(&bad, 1, st));
-    WOS_TRY(cudaMemsetAsync(bad, 0, sizeof(int), st));
-    const long long n = (long long)nF * dim;
-    k_check_indices<<<std::min(nblk(n, 256), 4096), 256, 0, st>>>(F, n, nV, bad);
-    int bad_h = 0;
-    WOS_TRY(cudaMemcpyAsync(&bad_h, bad, sizeof(int), cudaMemcpyDeviceToHost, st));
+    int *out = nullptr;
+    WOS_TRY(dalloc(&out, 2, st));
+    WOS_TRY(cudaMemsetAsync(out, 0, 2 * sizeof(int), st));
+    k_check_indices<<<std::min(nblk(nF, 256), 4096), 256, 0, st>>>(F, nF, dim, nV, out);
+    int host[2] = {0, 0};
+    WOS_TRY(cudaMemcpyAsync(host, out, sizeof(host), cudaMemcpyDeviceToHost, st));
+    cudaFreeAsync(out, st);
     WOS_TRY(cudaStreamSynchronize(st));
-    cudaFreeAsync(bad, st);
-    if (bad_h) return fail(WOS_ERR_INVALID_ARGUMENT, "face index out of range [0, nV)");
+    if (host[0]) return fail(WOS_ERR_INVALID_ARGUMENT, "face index out of range [0, nV)");
+    // a polyline of which at least 90 % of the segments follow each other
+    prim_order = dim == 3 ? 2 : nF >= 2 && host[1] >= nF - nF / 10 ? 1 : 0;
     return 0;
 }
 

@@ -33,10 +33,9 @@ struct SceneImpl {
     float4 *tri = nullptr;
     int nNodes = 0;
     int depth = 0;
-    // Primitive order of the trees (decided at the first build, kept when
-    // vertices move): 0 Morton, 1 input order (a polyline whose segments
-    // follow each other), 2 Hilbert.
-    int prim_order = -1;
+    // Primitive order of the binary tree, and of the 2D search tree: 0 Morton,
+    // 1 input order (a polyline whose segments follow each other), 2 Hilbert.
+    int prim_order = 0;
     float4 *node = nullptr;
     float4 *lseg = nullptr;
     float *lseginv = nullptr;
@@ -54,6 +53,7 @@ struct SceneImpl {
     float4 *tree = nullptr;
     float4 *prims = nullptr;
     int *torig = nullptr;
+    int *vslot = nullptr, *vfirst = nullptr;  // (face, corner) slots by vertex, for the normals
     bool tree_ordered = false;  // torig holds the order (3D: kept when vertices move)
     // Incremented by every build and source change: the by-value fields of
     // view() (bounding box, extents, source) may have changed since a view
