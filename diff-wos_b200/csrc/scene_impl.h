@@ -53,6 +53,10 @@ struct SceneImpl {
     float4 *tree = nullptr;
     float4 *prims = nullptr;
     int *torig = nullptr;
+    int grid_bits = 0;  // its entry grid (SceneView::grid)
+    float4 *grid = nullptr;  // its place, the cells' nodes (from grid_node() on) and their boxes (from grid_box() on)
+    uint4 *grid_node() const { return reinterpret_cast<uint4 *>(grid) + 2; }
+    float4 *grid_box() const { return grid + 2 + ((size_t)1 << (dim * grid_bits)) + 2; }
     int *vslot = nullptr, *vfirst = nullptr;  // (face, corner) slots by vertex, for the normals
     bool tree_ordered = false;  // torig holds the order (3D: kept when vertices move)
     // Incremented by every build and source change: the by-value fields of

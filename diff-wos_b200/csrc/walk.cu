@@ -324,13 +324,13 @@ struct ManyScenes {
 
 // The search of every lane with sr.dep == SEARCH_NEED begun, and the warp's
 // searches run on.  Brute force completes at once.
-template <int D, bool BVH, class CTX, class WK>
+template <int D, bool BVH, bool GATHER, class CTX, class WK>
 __device__ __forceinline__ void lane_search(Search<D> &sr, const CTX &x, int item, const float *p, int warm,
                                             float ball_m, unsigned *stack, WK &work) {
     if (sr.dep == SEARCH_NEED) {
         if (BVH) {
             work.nq += 1;
-            search_begin<D>(sr, x.scene(item), p, warm, ball_m);
+            search_begin<D, GATHER>(sr, x.scene(item), p, warm, ball_m, stack, work);
         } else {
             const Hit h = nearest_brute<D>(x.scene(item), p, work);
             sr.pos = h.prim;
@@ -340,7 +340,7 @@ __device__ __forceinline__ void lane_search(Search<D> &sr, const CTX &x, int ite
     }
     if (BVH) {
         const int n = __popc(__ballot_sync(0xffffffffu, sr.dep >= 0));
-        search_run<D, CTX::MULTI>(sr, x.scenes(), item, p, stack, search_keep<D>(n), work);
+        search_run<D, GATHER, CTX::MULTI>(sr, x.scenes(), item, p, stack, search_keep<D>(n), work);
     }
 }
 
@@ -456,7 +456,7 @@ __device__ __forceinline__ void walk_lanes(const CTX &x, long long idx0, long lo
             else
                 ended = r;
         }
-        lane_search<D, BVH>(sr, x, item, w.p, w.last, -1.0f, stack, work);
+        lane_search<D, BVH, true>(sr, x, item, w.p, w.last, -1.0f, stack, work);
     }
 }
 
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const fl
     };
     load();
     while (__any_sync(0xffffffffu, i < n)) {
-        lane_search<D, BVH>(sr, x, 0, p, -1, -1.0f, stack, work);
+        lane_search<D, BVH, true>(sr, x, 0, p, -1, -1.0f, stack, work);
         if (i >= n || sr.dep >= 0) continue;
         const Hit hit = lane_hit<D, BVH>(sr, S);
         if (o.prim) o.prim[i] = hit.prim;
@@ -626,7 +626,7 @@ __global__ void __launch_bounds__(QUERY_THREADS) k_ball(SceneView S, const uint8
     };
     if (on) aim();
     while (__any_sync(0xffffffffu, step < 10)) {
-        lane_search<D, BVH>(sr, x, 0, q, last, -1.0f, stack, work);
+        lane_search<D, BVH, true>(sr, x, 0, q, last, -1.0f, stack, work);
         if (step >= 10 || sr.dep >= 0) continue;
         const Hit hit = lane_hit<D, BVH>(sr, S);
         last = hit.prim;
@@ -1278,7 +1278,7 @@ __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, lon
         const int dep = sr.dep;
         if (hold) sr.dep = SEARCH_DONE;
         const bool walking = phase == PH_ANTI_WALK || (HAS_PRIMAL && phase == PH_PRIMAL);
-        lane_search<D, BVH>(sr, x, item, w.p, walking ? w.last : rprim, ball_m, stack, work);
+        lane_search<D, BVH, false>(sr, x, item, w.p, walking ? w.last : rprim, ball_m, stack, work);
         if (hold) sr.dep = dep;
     }
     if constexpr (CTX::MULTI) {
@@ -1676,10 +1676,10 @@ __global__ void __launch_bounds__(256) k_walk_soft(SceneView S, WalkCfg c, const
         if (BVH) {
             if (active && sr.dep == SEARCH_NEED) {
                 work.nq += 1;
-                search_begin<D>(sr, S, p, last, -1.0f);
+                search_begin<D, true>(sr, S, p, last, -1.0f, sm.stack, work);
             }
             const int n = __popc(__ballot_sync(0xffffffffu, active));
-            search_run<D, false>(sr, &S, 0, p, sm.stack, search_keep<D>(n), work);
+            search_run<D, true, false>(sr, &S, 0, p, sm.stack, search_keep<D>(n), work);
             if (!active || sr.dep >= 0) continue;
             hit = search_hit<D>(sr, S);
         } else {
@@ -1880,7 +1880,7 @@ __global__ void __launch_bounds__(128) k_soft_adjoint(SceneView S, WalkCfg c, co
         for (int i = 0; i < c.nsteps && __any_sync(0xffffffffu, ok); ++i) {
             sr.dep = ok ? SEARCH_NEED : SEARCH_DONE;
             while (__any_sync(0xffffffffu, sr.dep != SEARCH_DONE))
-                lane_search<D, BVH>(sr, x0, 0, p, last, -1.0f, stack, work);
+                lane_search<D, BVH, true>(sr, x0, 0, p, last, -1.0f, stack, work);
             if (!ok) continue;
             const Hit hit = lane_hit<D, BVH>(sr, S);
             last = hit.prim;

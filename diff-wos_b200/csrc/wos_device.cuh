@@ -84,6 +84,15 @@ struct SceneView {
     const float4 *tree;
     const float4 *prims;
     const int *torig;
+    // Entry grid of the search tree over the bounding box, 2^grid_bits cells per
+    // axis and one more for all points outside.  A cell is a node block of its
+    // own, in `grid`: the boxes of up to four nodes whose subtrees hold, for
+    // every point of the cell, all its nearest primitives; their numbers
+    // (tree_node) are in grid_node.  Two float4 before those: the grid's corner
+    // and its cells per unit length.
+    int grid_bits;
+    const float4 *grid;
+    const uint4 *grid_node;
 };
 
 // Shape of the search tree: primitives per leaf, float4 per node block and per
@@ -105,6 +114,17 @@ __host__ __device__ constexpr int tree_stack_entries(int depth) { return 3 * dep
 __host__ __device__ __forceinline__ unsigned tree_block(int d, unsigned i) {
     return i + (0x55555555u & ((1u << (2 * d)) - 1u));
 }
+
+// Number of the node i at depth d >= 1: the child boxes of `tree` counted in
+// their order.  tree_place is the inverse.
+__host__ __device__ __forceinline__ unsigned tree_node(int d, unsigned i) {
+    return i + (0x55555554u & ((1u << (2 * d)) - 1u));
+}
+__device__ __forceinline__ void tree_place(unsigned node, int &d, unsigned &i) {
+    d = (31 - __clz(3u * node + 4u)) >> 1;
+    i = node - (0x55555554u & ((1u << (2 * d)) - 1u));
+}
+constexpr unsigned GRID_NONE = 0xffffffffu;
 
 template <int D>
 struct NodeWords;
@@ -548,7 +568,22 @@ __device__ __forceinline__ bool ball_blocks(float d2, float m) { return sqrtf(d2
 // triangles 129 -> 97 ms.  (Groups of 8 lanes on a 16-ary tree: 1.60 and 154 ms
 // in 2D.)
 //
-// What bounds it: instruction issue (about 70 % of the slots), at 15 of 32 lanes
+// A search starts at the nodes of its point's grid cell (SceneView::grid) instead
+// of the root: 2.9 instead of 6.1 node steps per query on 4,096 segments, 76 instead
+// of 95 warp instructions.  The forward solve above 0.755 -> 0.706 ms, the 3D one
+// (on the median-split order) 10.4 -> 8.9, the gradients 102.9 -> 100.8 and 60.8 ->
+// 57.5.  The cell's boxes are taken in one of two ways (GATHER):
+//   from the tree by their numbers, in a step of its own when the search begins:
+//     16 bytes per cell, so most of what it reads is in L1; the walks do this;
+//   from the cell's own block, as the first of the loop's node steps: 96 or 128
+//     bytes per cell, mostly from L2, but hardly any code; the adjoint does, whose
+//     loop is 40 KB of instructions and stalls on fetching them (gathering,
+//     no_instruction stalls went from 1.1 to 2.8 cycles per issue).
+// Each way in the other's place: the forward solves 0.773 and 9.2 ms, the gradients
+// 103.4 and 63.0.  (Lower bounds per cell instead of boxes: 2D solve 0.93 ms, as
+// leaves are visited that their boxes rule out.)
+//
+// What bounds it: instruction issue (about 70 % of the slots), at 14 of 32 lanes
 // per instruction, since lanes wait at the other kind of step; L1 is 55-60 % busy.
 template <int D>
 struct Search {
@@ -580,60 +615,6 @@ __device__ __forceinline__ float search_bound(float best, float tol) {
         return fminf((r * r) * (1.0f + 0x1p-22f), FLT_MAX);
     }
     return fminf(prune_bound(best, tol), FLT_MAX);
-}
-
-// Begin a search at q.  warm: a primitive whose distance bounds the nearest
-// one's (that walk's previous nearest primitive), or -1; its own leaf lies
-// within that bound, so it is found again if nothing is nearer.  ball_m > 0: the
-// search is for a primitive blocking the ball of radius ball_m centred at q and
-// may stop at any; primitives that do not block are of no interest.
-template <int D>
-__device__ __forceinline__ void search_begin(Search<D> &s, const SceneView &S, const float *q, int warm,
-                                             float ball_m) {
-    s.tol = D == 2 ? prune_tol<D>(S, q) : prune_tol2<D>(S, q);
-    s.stop = -1.0f;
-    if (ball_m > 0.0f) {
-        s.bound = search_bound<D>((ball_m * ball_m) * (1.0f + 0x1p-20f), s.tol);
-        // blocking is monotone in the distance: if `stop` blocks, whatever is
-        // nearer does
-        const float t = ball_m - 1.1e-5f;
-        if (t > 0.0f && ball_blocks(t * t, ball_m)) s.stop = t * t;
-    } else {
-        s.bound = warm >= 0 ? search_bound<D>(prim_d2<D>(S, warm, q), s.tol) : FLT_MAX;
-    }
-    s.d2 = INFINITY;
-    s.pos = -1;
-    s.idx = 0;
-    s.sp = 0;
-    // a point that is not finite has no primitive at a finite distance
-    bool finite = true;
-#pragma unroll
-    for (int k = 0; k < D; ++k) finite = finite && fabsf(q[k]) <= FLT_MAX;
-    s.dep = finite ? 0 : SEARCH_DONE;
-}
-
-// Next node from the stack: the last entry within the bound.  An entry is its
-// node's squared distance, the low 6 bits replaced by its depth and its place
-// among its siblings (rounded down, so pruning stays conservative); being on
-// the stack of a depth-first descent, it is a sibling of the current path's
-// node at that depth, which gives its index.
-constexpr unsigned ENTRY_LOW = 63u;
-template <int D>
-__device__ __forceinline__ void search_pop(Search<D> &s, const unsigned *stack) {
-    const unsigned b = __float_as_uint(s.bound) | ENTRY_LOW;
-    for (;;) {
-        if (s.sp == 0) {
-            s.dep = SEARCH_DONE;
-            return;
-        }
-        const unsigned e = stack[--s.sp * blockDim.x];
-        if (e <= b) {
-            const int dep = (int)((e >> 2) & 15u);
-            s.idx = ((s.idx >> (2 * (s.dep - dep))) & ~3u) | (e & 3u);
-            s.dep = dep;
-            return;
-        }
-    }
 }
 
 // Squared distance to an oriented box, a lower bound for its primitives.  With
@@ -690,27 +671,59 @@ __device__ __forceinline__ float obb_d2(const Obb3 &o, const float *q) {
     return fmaf(a0, a0, fmaf(a1, a1, a2 * a2));
 }
 
-// Visit an inner node: bound its four children, go to the nearest and leave the
-// others within the bound on the stack, the farthest first.
+// Cell of the entry grid that holds q.  The grid's place is read from memory: a
+// view taken before vertices moved finds the current one.
 template <int D>
-__device__ __forceinline__ void search_node(Search<D> &s, const SceneView &S, const float *q, unsigned *stack) {
-    const float4 *b = S.tree + (size_t)tree_block(s.dep, s.idx) * Tree<D>::NODE_W;
-    float d[4];
-    if constexpr (D == 2) {
-        const float4 e01 = __ldg(b + 4), e23 = __ldg(b + 5);
-        d[0] = obb_d2(__ldg(b), e01.x, e01.y, q);
-        d[1] = obb_d2(__ldg(b + 1), e01.z, e01.w, q);
-        d[2] = obb_d2(__ldg(b + 2), e23.x, e23.y, q);
-        d[3] = obb_d2(__ldg(b + 3), e23.z, e23.w, q);
-    } else {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) d[c] = obb_d2(load_obb3(b + 2 * c), q);
+__device__ __forceinline__ unsigned grid_cell(const SceneView &S, const float *q) {
+    const float4 *head = reinterpret_cast<const float4 *>(S.grid_node) - 2;
+    const float4 o = __ldg(head), inv = __ldg(head + 1);
+    const float g = (float)(1 << S.grid_bits);
+    const float x = (q[0] - o.x) * inv.x, y = (q[1] - o.y) * inv.y;
+    bool in = x >= 0.0f && x < g && y >= 0.0f && y < g;
+    unsigned cell = ((unsigned)y << S.grid_bits) + (unsigned)x;
+    if (D == 3) {
+        const float z = (q[2] - o.z) * inv.z;
+        in = in && z >= 0.0f && z < g;
+        cell += (unsigned)z << (2 * S.grid_bits);
     }
-    const unsigned low = (unsigned)(s.dep + 1) << 2;
-    unsigned k[4];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) k[c] = (__float_as_uint(d[c]) & ~ENTRY_LOW) | (low + c);
-    // ascending
+    return in ? cell : 1u << (D * S.grid_bits);
+}
+
+__device__ __forceinline__ unsigned grid_node(const SceneView &S, unsigned cell, unsigned c) {
+    return __ldg(reinterpret_cast<const unsigned *>(S.grid_node + cell) + c);
+}
+
+// Next node from the stack: the last entry within the bound.  An entry is its
+// node's squared distance, the low 6 bits replaced by its depth and its place
+// among its siblings (rounded down, so pruning stays conservative); being on
+// the stack of a depth-first descent, it is a sibling of the current path's
+// node at that depth, which gives its index.  Depth 0 stands for the nodes of
+// the query's grid cell.
+constexpr unsigned ENTRY_LOW = 63u;
+template <int D>
+__device__ __forceinline__ void search_pop(Search<D> &s, const SceneView &S, const float *q, const unsigned *stack) {
+    const unsigned b = __float_as_uint(s.bound) | ENTRY_LOW;
+    for (;;) {
+        if (s.sp == 0) {
+            s.dep = SEARCH_DONE;
+            return;
+        }
+        const unsigned e = stack[--s.sp * blockDim.x];
+        if (e <= b) {
+            const int dep = (int)((e >> 2) & 15u);
+            if (dep == 0) {
+                tree_place(grid_node(S, grid_cell<D>(S, q), e & 3u), s.dep, s.idx);
+                return;
+            }
+            s.idx = ((s.idx >> (2 * (s.dep - dep))) & ~3u) | (e & 3u);
+            s.dep = dep;
+            return;
+        }
+    }
+}
+
+// Ascending.
+__device__ __forceinline__ void sort4(unsigned *k) {
     auto order = [&](int i, int j) {
         const unsigned lo = min(k[i], k[j]), hi = max(k[i], k[j]);
         k[i] = lo;
@@ -721,15 +734,120 @@ __device__ __forceinline__ void search_node(Search<D> &s, const SceneView &S, co
     order(0, 2);
     order(1, 3);
     order(1, 2);
+}
+
+// Squared distances to the four boxes of a node block.
+template <int D>
+__device__ __forceinline__ void block_distances(const float4 *b, const float *q, float *d) {
+    if constexpr (D == 2) {
+        const float4 e01 = __ldg(b + 4), e23 = __ldg(b + 5);
+        d[0] = obb_d2(__ldg(b), e01.x, e01.y, q);
+        d[1] = obb_d2(__ldg(b + 1), e01.z, e01.w, q);
+        d[2] = obb_d2(__ldg(b + 2), e23.x, e23.y, q);
+        d[3] = obb_d2(__ldg(b + 3), e23.z, e23.w, q);
+    } else {
+#pragma unroll
+        for (int c = 0; c < 4; ++c) d[c] = obb_d2(load_obb3(b + 2 * c), q);
+    }
+}
+
+// Visit an inner node, or at depth 0 (not after search_cell) the nodes of the
+// query's grid cell: bound the four children, go to the nearest and leave the
+// others within the bound on the stack, the farthest first.
+template <int D, bool GATHER>
+__device__ __forceinline__ void search_node(Search<D> &s, const SceneView &S, const float *q, unsigned *stack) {
+    const bool top = !GATHER && s.dep == 0;
+    float d[4];
+    block_distances<D>((top ? S.grid : S.tree) + (size_t)tree_block(s.dep, s.idx) * Tree<D>::NODE_W, q, d);
+    const unsigned low = top ? 0u : (unsigned)(s.dep + 1) << 2;
+    unsigned k[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) k[c] = (__float_as_uint(d[c]) & ~ENTRY_LOW) | (low + c);
+    sort4(k);
     const unsigned bound = __float_as_uint(s.bound) | ENTRY_LOW;
 #pragma unroll
     for (int c = 3; c >= 1; --c)
         if (k[c] <= bound) stack[s.sp++ * blockDim.x] = k[c];
-    if (k[0] <= bound) {
+    if (k[0] > bound) {
+        search_pop(s, S, q, stack);
+    } else if (top) {
+        tree_place(grid_node(S, s.idx, k[0] & 3u), s.dep, s.idx);
+    } else {
         s.idx = 4u * s.idx + (k[0] & 3u);
         s.dep += 1;
+    }
+}
+
+// Squared distance to the box of one node (tree_node).
+template <int D>
+__device__ __forceinline__ float node_distance(const SceneView &S, unsigned node, const float *q) {
+    const float4 *b = S.tree + (size_t)(node >> 2) * Tree<D>::NODE_W;
+    const int c = (int)(node & 3u);
+    if constexpr (D == 2) {
+        const float2 e = __ldg(reinterpret_cast<const float2 *>(b + 4) + c);
+        return obb_d2(__ldg(b + c), e.x, e.y, q);
     } else {
-        search_pop(s, stack);
+        return obb_d2(load_obb3(b + 2 * c), q);
+    }
+}
+
+// The first step of a search: the nodes of its grid cell, their boxes gathered
+// from the tree.
+template <int D>
+__device__ __forceinline__ void search_cell(Search<D> &s, const SceneView &S, unsigned cell, const float *q,
+                                            unsigned *stack) {
+    const uint4 e = __ldg(S.grid_node + cell);
+    const unsigned n[4] = {e.x, e.y, e.z, e.w};
+    unsigned k[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const float d = node_distance<D>(S, n[c] == GRID_NONE ? 0u : n[c], q);
+        k[c] = n[c] == GRID_NONE ? GRID_NONE : (__float_as_uint(d) & ~ENTRY_LOW) | c;
+    }
+    sort4(k);
+    const unsigned bound = __float_as_uint(s.bound) | ENTRY_LOW;
+#pragma unroll
+    for (int c = 3; c >= 1; --c)
+        if (k[c] <= bound) stack[s.sp++ * blockDim.x] = k[c];
+    s.dep = SEARCH_DONE;
+    if (k[0] <= bound) {
+        const unsigned c = k[0] & 3u;
+        tree_place(c == 0 ? n[0] : c == 1 ? n[1] : c == 2 ? n[2] : n[3], s.dep, s.idx);
+    }
+}
+
+// Begin a search at q.  warm: a primitive whose distance bounds the nearest
+// one's (that walk's previous nearest primitive), or -1; its own leaf lies
+// within that bound, so it is found again if nothing is nearer.  ball_m > 0: the
+// search is for a primitive blocking the ball of radius ball_m centred at q and
+// may stop at any; primitives that do not block are of no interest.  GATHER: the
+// cell's nodes are visited at once (search_cell), else by the first search_node.
+template <int D, bool GATHER, class WK>
+__device__ __forceinline__ void search_begin(Search<D> &s, const SceneView &S, const float *q, int warm,
+                                             float ball_m, unsigned *stack, WK &wk) {
+    s.tol = D == 2 ? prune_tol<D>(S, q) : prune_tol2<D>(S, q);
+    s.stop = -1.0f;
+    if (ball_m > 0.0f) {
+        s.bound = search_bound<D>((ball_m * ball_m) * (1.0f + 0x1p-20f), s.tol);
+        // blocking is monotone in the distance: if `stop` blocks, whatever is
+        // nearer does
+        const float t = ball_m - 1.1e-5f;
+        if (t > 0.0f && ball_blocks(t * t, ball_m)) s.stop = t * t;
+    } else {
+        s.bound = warm >= 0 ? search_bound<D>(prim_d2<D>(S, warm, q), s.tol) : FLT_MAX;
+    }
+    s.d2 = INFINITY;
+    s.pos = -1;
+    s.idx = grid_cell<D>(S, q);
+    s.sp = 0;
+    // a point that is not finite has no primitive at a finite distance
+    bool finite = true;
+#pragma unroll
+    for (int k = 0; k < D; ++k) finite = finite && fabsf(q[k]) <= FLT_MAX;
+    s.dep = finite ? 0 : SEARCH_DONE;
+    if (GATHER && finite) {
+        wk.nb += 1;
+        search_cell<D>(s, S, s.idx, q, stack);
     }
 }
 
@@ -782,13 +900,13 @@ __device__ __forceinline__ void search_leaf(Search<D> &s, const SceneView &S, co
         s.bound = fminf(s.bound, search_bound<D>(m, s.tol));
         if (m <= s.stop) s.sp = 0;
     }
-    search_pop(s, stack);
+    search_pop(s, S, q, stack);
 }
 
 // Run the searches of a warp's lanes until at most `keep` of them still have a
 // node to visit.  scenes[MULTI ? item : 0] is the lane's scene.  Must be called
 // by all 32 lanes.
-template <int D, bool MULTI, class WK>
+template <int D, bool GATHER, bool MULTI, class WK>
 __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes, int item, const float *q,
                                            unsigned *stack, int keep, WK &wk) {
     const unsigned FULL = 0xffffffffu;
@@ -804,7 +922,7 @@ __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes
             }
         } else if (run && !leaf) {
             wk.nb += 1;
-            search_node<D>(s, S, q, stack);
+            search_node<D, GATHER>(s, S, q, stack);
         }
     }
 }
