@@ -522,8 +522,12 @@ int wos_solve_adjoint(wos_scene_t scene, const float *P, int n, const wos_params
     ao.dsrc = acc.ds;
     ao.wrec = wrec;
     ao.wds = wds;
-    if (int rc = launch_record_order(S, wrec, (long long)nw, b, need - (size_t)(b - s.base), &ao.order, st))
-        return rc;
+    // Ordered by boundary primitive only for the ball walks that start there: a
+    // gather of the values alone takes 50 us in any order (640,000 walks, 2D),
+    // as much as the keys and the sort.
+    if (a->want_dV)
+        if (int rc = launch_record_order(S, wrec, (long long)nw, b, need - (size_t)(b - s.base), &ao.order, st))
+            return rc;
     if (int rc = launch_adjoint(S, P, (long long)nw, *p, make_adj(*a), dLdu, ADJ_FROM_RECORDS, ao, counter, st))
         return rc;
     return finish_adjoint(S, a, acc, dV, dg, dsrc, st);
@@ -591,8 +595,9 @@ int wos_solve_tangent(wos_scene_t scene, const float *P, int n, const wos_params
     ao.tg = dg_dir;
     ao.ts = dsrc_dir;
     ao.tan = tan;
-    if (int rc = launch_record_order(S, wrec, (long long)nw, b, need - (size_t)(b - s.base), &ao.order, st))
-        return rc;
+    if (a->want_dV && dV_dir != nullptr)
+        if (int rc = launch_record_order(S, wrec, (long long)nw, b, need - (size_t)(b - s.base), &ao.order, st))
+            return rc;
     if (int rc = launch_adjoint(S, P, (long long)nw, *p, make_adj(*a), nullptr, ADJ_TANGENT, ao, counter, st))
         return rc;
     return launch_reduce(tan, n, p->nwalks, tangent, tangent_var, st);
@@ -768,7 +773,7 @@ int wos_adjoint_records(wos_scene_t scene, const float *P, int n, const wos_para
     ao.dsrc = acc.ds;
     ao.wrec = (const int *)records;
     ao.wds = dcontrib;
-    if (ordered && need_ordered > need)
+    if (a->want_dV && ordered && need_ordered > need)
         if (int rc = launch_record_order(S, ao.wrec, (long long)n * p->nwalks, s.base + need, need_ordered - need,
                                          &ao.order, st))
             return rc;

@@ -268,7 +268,8 @@ WOS_API int wos_solve_records(wos_scene_t scene, const float *P, int n, const wo
  * (wos/solver.py:109-114); the records make that recomputation unnecessary
  * and the result is the same.  Its workspace is wos_adjoint_workspace_size
  * bytes; given wos_adjoint_records_workspace_size bytes (or NULL) it also runs
- * the samples in boundary-primitive order (wos_set_sample_order). */
+ * the samples of a vertex gradient in boundary-primitive order
+ * (wos_set_sample_order). */
 WOS_API size_t wos_adjoint_records_workspace_size(wos_scene_t scene, int n, const wos_params *p);
 WOS_API int wos_adjoint_records(wos_scene_t scene, const float *P, int n, const wos_params *p,
                                 const wos_adjoint_params *a, const float *dLdu, const void *records,
