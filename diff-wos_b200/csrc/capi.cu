@@ -533,6 +533,34 @@ int wos_solve_adjoint(wos_scene_t scene, const float *P, int n, const wos_params
     return finish_adjoint(S, a, acc, dV, dg, dsrc, st);
 }
 
+// Derivative along a direction, from the walks' records: per-walk tangents and
+// their reduction.  Samples take the order of their boundary primitives only
+// where ball walks follow from it (a moving boundary).
+static size_t records_tangent_bytes(const SceneImpl &S, size_t nw) {
+    return align256(sizeof(float) * nw) + align256(record_order_bytes(S.nF, (long long)nw));
+}
+static int records_tangent(const SceneImpl &S, const float *P, int n, const wos_params &p, const wos_adjoint_params &a,
+                           const float *dV_dir, const float *dg_dir, const float *dsrc_dir, const int *wrec,
+                           const float *wds, double *tangent, double *tangent_var, unsigned long long *counter,
+                           char *ws, size_t ws_bytes, cudaStream_t st) {
+    const size_t nw = (size_t)n * (size_t)p.nwalks, tan_bytes = align256(sizeof(float) * nw);
+    float *tan = (float *)ws;
+    const cudaError_t e = cudaMemsetAsync(tan, 0, sizeof(float) * nw, st);
+    if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(tangents)");
+    AdjOut ao{};
+    ao.wrec = wrec;
+    ao.wds = wds;
+    ao.tV = dV_dir;
+    ao.tg = dg_dir;
+    ao.ts = dsrc_dir;
+    ao.tan = tan;
+    if (a.want_dV && dV_dir != nullptr)
+        if (int rc = launch_record_order(S, wrec, (long long)nw, ws + tan_bytes, ws_bytes - tan_bytes, &ao.order, st))
+            return rc;
+    if (int rc = launch_adjoint(S, P, (long long)nw, p, make_adj(a), nullptr, ADJ_TANGENT, ao, counter, st)) return rc;
+    return launch_reduce(tan, n, p.nwalks, tangent, tangent_var, st);
+}
+
 size_t wos_solve_tangent_workspace_size(wos_scene_t scene, int n, const wos_params *p, const wos_adjoint_params *a) {
     if (scene == nullptr || p == nullptr || a == nullptr || n < 0 || p->nwalks < 1) return 0;
     const SceneImpl &S = scene->impl;
@@ -541,8 +569,7 @@ size_t wos_solve_tangent_workspace_size(wos_scene_t scene, int n, const wos_para
     b += align256(sizeof(float) * nw);                                // per-walk values
     b += align256(wos_walk_record_bytes(S.dim) * nw);                 // per-walk records
     if (wants_wds(S, *p, *a)) b += align256(sizeof(float) * 5 * nw);  // per-walk source derivatives
-    b += align256(sizeof(float) * nw);                                // per-walk tangents
-    b += align256(record_order_bytes(S.nF, (long long)nw));           // sample order
+    b += records_tangent_bytes(S, nw);
     return b;
 }
 
@@ -581,26 +608,44 @@ int wos_solve_tangent(wos_scene_t scene, const float *P, int n, const wos_params
         wds = (float *)b;
         b += align256(sizeof(float) * 5 * nw);
     }
-    float *tan = (float *)b;
-    b += align256(sizeof(float) * nw);
-    cudaError_t e = cudaMemsetAsync(tan, 0, sizeof(float) * nw, st);
-    if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(tangents)");
     WalkOut o{vals, nullptr, wrec, wds, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
     if (int rc = launch_walk(S, P, (long long)nw, *p, false, o, counter, st)) return rc;
     if (int rc = launch_reduce(vals, n, p->nwalks, mean, var, st)) return rc;
-    AdjOut ao{};
-    ao.wrec = wrec;
-    ao.wds = wds;
-    ao.tV = dV_dir;
-    ao.tg = dg_dir;
-    ao.ts = dsrc_dir;
-    ao.tan = tan;
-    if (a->want_dV && dV_dir != nullptr)
-        if (int rc = launch_record_order(S, wrec, (long long)nw, b, need - (size_t)(b - s.base), &ao.order, st))
-            return rc;
-    if (int rc = launch_adjoint(S, P, (long long)nw, *p, make_adj(*a), nullptr, ADJ_TANGENT, ao, counter, st))
-        return rc;
-    return launch_reduce(tan, n, p->nwalks, tangent, tangent_var, st);
+    return records_tangent(S, P, n, *p, *a, dV_dir, dg_dir, dsrc_dir, wrec, wds, tangent, tangent_var, counter, b,
+                           need - (size_t)(b - s.base), st);
+}
+
+size_t wos_tangent_records_workspace_size(wos_scene_t scene, int n, const wos_params *p) {
+    if (scene == nullptr || p == nullptr || n < 0 || p->nwalks < 1) return 0;
+    return 256 + records_tangent_bytes(scene->impl, (size_t)n * (size_t)p->nwalks);
+}
+
+int wos_tangent_records(wos_scene_t scene, const float *P, int n, const wos_params *p, const wos_adjoint_params *a,
+                        const float *dV_dir, const float *dg_dir, const float *dsrc_dir, const void *records,
+                        const float *dcontrib, double *tangent, double *tangent_var, void *workspace,
+                        size_t workspace_bytes, wos_stream_t stream) {
+    if (scene == nullptr) return fail(WOS_ERR_INVALID_ARGUMENT, "scene is NULL");
+    if (int rc = check_params(p)) return rc;
+    if (int rc = check_adj(a)) return rc;
+    if (n < 0) return fail(WOS_ERR_INVALID_ARGUMENT, "n must be >= 0");
+    if (n == 0) return 0;
+    const SceneImpl &S = scene->impl;
+    if (wants_wds(S, *p, *a) && dcontrib == nullptr)
+        return fail(WOS_ERR_INVALID_ARGUMENT, "source derivative requested but dcontrib is NULL");
+    WOS_CHECK_DEV(P, "P");
+    WOS_CHECK_DEV(records, "records");
+    WOS_CHECK_DEV(tangent, "tangent");
+    WOS_CHECK_DEV_OPT(tangent_var, "tangent_var");
+    WOS_CHECK_DEV_OPT(dcontrib, "dcontrib");
+    WOS_CHECK_DEV_OPT(dV_dir, "dV_dir");
+    WOS_CHECK_DEV_OPT(dg_dir, "dg_dir");
+    WOS_CHECK_DEV_OPT(dsrc_dir, "dsrc_dir");
+    cudaStream_t st = (cudaStream_t)stream;
+    const size_t need = wos_tangent_records_workspace_size(scene, n, p);
+    Scratch s;
+    if (int rc = s.init(workspace, workspace_bytes, need, st)) return rc;
+    return records_tangent(S, P, n, *p, *a, dV_dir, dg_dir, dsrc_dir, (const int *)records, dcontrib, tangent,
+                           tangent_var, (unsigned long long *)s.base, s.base + 256, need - 256, st);
 }
 
 size_t wos_soft_walk_workspace_size(int n, const wos_params *p) {

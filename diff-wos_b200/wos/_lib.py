@@ -171,6 +171,12 @@ SIGNATURES = {
         [_P, _P, _I, ctypes.POINTER(WosParams), ctypes.POINTER(WosAdjointParams), _P, _P, _P, _P, _P, _P, _P, _P, _S,
          _P],
     ),
+    "wos_tangent_records_workspace_size": (_S, [_P, _I, ctypes.POINTER(WosParams)]),
+    "wos_tangent_records": (
+        _I,
+        [_P, _P, _I, ctypes.POINTER(WosParams), ctypes.POINTER(WosAdjointParams), _P, _P, _P, _P, _P, _P, _P, _P, _S,
+         _P],
+    ),
     "wos_solve_adjoint": (
         _I,
         [_P, _P, _I, ctypes.POINTER(WosParams), ctypes.POINTER(WosAdjointParams), _I, _P, _P, _P, _P, _P, _P, _P,

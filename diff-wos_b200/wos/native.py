@@ -296,6 +296,33 @@ class NativeScene:
                  workspace.data_ptr(), need, stream())
         return dict(mean=mean, var=var, loss=loss, dV=dV, dg=dg, dsrc=ds)
 
+    def _direction(self, dV, dg, dsrc):
+        tV = as_cuda(dV, torch.float32, self.dim) if dV is not None else None
+        if tV is not None and tV.shape[0] != self.nV:
+            raise ValueError("dV must be nV x dim")
+        tg = as_cuda(dg, torch.float32).reshape(-1) if dg is not None else None
+        if tg is not None and tg.numel() != self.nV:
+            raise ValueError("dg must have one entry per vertex")
+        ts = as_cuda(dsrc, torch.float32).reshape(-1) if dsrc is not None else None
+        if ts is not None and ts.numel() != 5:
+            raise ValueError("dsrc must have 5 entries")
+        return tV, tg, ts
+
+    def tangent_records(self, P, s: WalkSettings, a: AdjointSettings, rec, dc, dV=None, dg=None, dsrc=None):
+        """The tangent of solve_tangent() from the records of solve_records()
+        with the same points and settings."""
+        P = as_cuda(P, torch.float32, self.dim)
+        n = int(P.shape[0])
+        tan = torch.empty(n, dtype=torch.float64, device=self.device)
+        tV, tg, ts = self._direction(dV, dg, dsrc)
+        if n:
+            c, ca = s.c(), a.c()
+            need = _lib.lib().wos_tangent_records_workspace_size(self.h, n, ctypes.byref(c))
+            workspace = torch.empty(need, dtype=torch.uint8, device=self.device)
+            call("wos_tangent_records", self.h, P.data_ptr(), n, ctypes.byref(c), ctypes.byref(ca), _ptr(tV), _ptr(tg),
+                 _ptr(ts), rec.data_ptr(), _ptr(dc), tan.data_ptr(), None, workspace.data_ptr(), need, stream())
+        return tan
+
     def solve_tangent(self, P, s: WalkSettings, a: AdjointSettings, dV=None, dg=None, dsrc=None, want_var=False,
                       workspace: torch.Tensor | None = None):
         """Fused forward solve + forward-mode derivative of the per-point means
@@ -307,15 +334,7 @@ class NativeScene:
         tan = torch.empty(n, dtype=torch.float64, device=d)
         var = torch.empty(n, dtype=torch.float64, device=d) if want_var else None
         tvar = torch.empty(n, dtype=torch.float64, device=d) if want_var else None
-        tV = as_cuda(dV, torch.float32, self.dim) if dV is not None else None
-        if tV is not None and tV.shape[0] != self.nV:
-            raise ValueError("dV must be nV x dim")
-        tg = as_cuda(dg, torch.float32).reshape(-1) if dg is not None else None
-        if tg is not None and tg.numel() != self.nV:
-            raise ValueError("dg must have one entry per vertex")
-        ts = as_cuda(dsrc, torch.float32).reshape(-1) if dsrc is not None else None
-        if ts is not None and ts.numel() != 5:
-            raise ValueError("dsrc must have 5 entries")
+        tV, tg, ts = self._direction(dV, dg, dsrc)
         if n:
             c, ca = s.c(), a.c()
             need = _lib.lib().wos_solve_tangent_workspace_size(self.h, n, ctypes.byref(c), ctypes.byref(ca))

@@ -176,14 +176,23 @@ class _Job:
     def tangent(self, dV, dg, ds):
         """Forward mode: derivative of the per-point means along (dV, dg, ds)
         (any may be None), from the backward solver's estimator with the same
-        seed (wos_solve_tangent)."""
+        seed: from the forward's records where it kept what this takes
+        (wos_tangent_records), else by walking again (wos_solve_tangent)."""
         s = self.bwd.walk_settings(self.scene, self.seed, jitter=self.jitter)
         a = self.bwd.adjoint_settings(self.scene, dV is not None, dg is not None, ds is not None)
         if not (a.want_dV or a.want_dg or a.want_dsrc):
             return torch.zeros(self.P.shape[0], dtype=torch.float32, device=self.P.device)
-        out = self.scene._native.solve_tangent(self.P, s, a, dV=dV if a.want_dV else None,
-                                               dg=dg if a.want_dg else None, dsrc=ds if a.want_dsrc else None)
-        return out["tangent"].to(torch.float32)
+        d = dict(dV=dV if a.want_dV else None, dg=dg if a.want_dg else None, dsrc=ds if a.want_dsrc else None)
+        if self._recorded(s, a):
+            tan = self.scene._native.tangent_records(self.P, s, a, *self.records, **d)
+        else:
+            tan = self.scene._native.solve_tangent(self.P, s, a, **d)["tangent"]
+        return tan.to(torch.float32)
+
+    def _recorded(self, s, a):
+        """Whether the forward's records serve the derivatives that `a` asks for."""
+        return self.records is not None and (self.records[1] is not None or not a.want_dsrc or
+                                             not (s.include_source and self.scene.source_type != 0))
 
     def backward(self, grad, need_V, need_g, need_s):
         s = self.bwd.walk_settings(self.scene, self.seed, jitter=self.jitter)
@@ -191,8 +200,7 @@ class _Job:
         if not (a.want_dV or a.want_dg or a.want_dsrc):
             return None, None, None
         g = grad.to(torch.float32).contiguous()
-        if self.records is not None and (self.records[1] is not None or not a.want_dsrc or
-                                         not (s.include_source and self.scene.source_type != 0)):
+        if self._recorded(s, a):
             dV, dg, ds = self.scene._native.adjoint_records(self.P, s, a, g, *self.records)
         else:
             dV, dg, ds = self.scene._native.adjoint(self.P, s, a, g)

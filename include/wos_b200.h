@@ -311,6 +311,15 @@ WOS_API int wos_solve_tangent(wos_scene_t scene, const float *P, int n, const wo
                               const float *dsrc_dir, double *mean, double *var, double *tangent, double *tangent_var,
                               void *workspace, size_t workspace_bytes, wos_stream_t stream);
 
+/* The tangent of wos_solve_tangent from the records that wos_solve_records
+ * kept (same P, n and params) instead of walking again; the same result.
+ * dcontrib is needed where the source term's derivative is taken. */
+WOS_API size_t wos_tangent_records_workspace_size(wos_scene_t scene, int n, const wos_params *p);
+WOS_API int wos_tangent_records(wos_scene_t scene, const float *P, int n, const wos_params *p,
+                                const wos_adjoint_params *a, const float *dV_dir, const float *dg_dir,
+                                const float *dsrc_dir, const void *records, const float *dcontrib, double *tangent,
+                                double *tangent_var, void *workspace, size_t workspace_bytes, wos_stream_t stream);
+
 /* Workspace of wos_soft_walk. */
 WOS_API size_t wos_soft_walk_workspace_size(int n, const wos_params *p);
 
