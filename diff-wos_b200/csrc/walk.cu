@@ -546,6 +546,12 @@ __global__ void k_reduce(const float *__restrict__ vals, int n, int nw, double *
 // Closest-point queries, a lane each at a time: a lane whose search is done
 // writes its record and goes on to its next point while the others search on.
 constexpr int QUERY_THREADS = 128;
+// When a warp's lanes have no further points and this many are still searching,
+// after SHARE_STEPS more steps, its other lanes take part in their searches: most
+// searches are shorter and done sooner alone.  (200,003 points on 20,480 triangles,
+// closest points and signed distances: 0.70 ms without, 0.71 with 8 lanes and 32 steps,
+// 0.73 with 8 and 8, 0.74 with 16 and 16, 0.69 with 16 and 64.)
+constexpr int SHARE_LANES = 16, SHARE_STEPS = 64;
 template <int D, bool BVH>
 __global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const float *__restrict__ P, int n,
                                                             QueryOut o) {
@@ -567,6 +573,14 @@ __global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const fl
     load();
     while (__any_sync(0xffffffffu, i < n)) {
         lane_search<D, BVH, true>(sr, x, 0, p, -1, -1.0f, stack, work);
+        if (BVH) {
+            const unsigned run = __ballot_sync(0xffffffffu, sr.dep >= 0);
+            if (run != 0u && __popc(run) <= SHARE_LANES && !__any_sync(0xffffffffu, i + stride < n)) {
+                search_run<D, true, false, SHARE_STEPS>(sr, &S, 0, p, stack, 0, work);
+                for (unsigned left = __ballot_sync(0xffffffffu, sr.dep >= 0); left != 0u; left &= left - 1u)
+                    search_share<D>(sr, S, p, __ffs(left) - 1, stack);
+            }
+        }
         if (i >= n || sr.dep >= 0) continue;
         const Hit hit = lane_hit<D, BVH>(sr, S);
         if (o.prim) o.prim[i] = hit.prim;
@@ -2164,8 +2178,7 @@ int launch_adjoint(const SceneImpl &S, const float *P, long long total, const wo
 
 // ------------------------------------------------------------------ sample order
 // Adjoint samples that start from forward records run in the order of their
-// boundary primitive along the trees' primitive order (curve order in 2D,
-// Hilbert order in 3D).  Every sample begins with the inscribed-ball
+// boundary primitive along the search tree's order.  Every sample begins with the inscribed-ball
 // bisection around that primitive, so in this order the lanes of a warp --
 // and the warps the GPU runs at the same time -- start next to each other and
 // share cached tree nodes for those queries.  The gain is small (0.5-1 % of a
