@@ -1096,8 +1096,8 @@ def main():
         "plain_vs_persistent": plain,
         "walk_steps": steps_stats,
         "tree_work_per_launch": {"adjoint": adj_work, "forward": fwd_work,
-                                 "note": "this build's wide-tree counters: queries, node expansions and leaf "
-                                         "steps (one warp step each)"},
+                                 "note": "this build's search counters: queries, node steps and leaf steps of "
+                                         "single lanes"},
     }
     if clk is not None:
         line["clocks"] = clk
@@ -1114,7 +1114,7 @@ def main():
             "bound": "issue", "achieved": inst / adj_avg / 1e9, "peak": issue_peak / 1e9, "unit": "Ginst/s",
             "frac": inst / adj_avg / issue_peak, "traffic": traffic, "kernel": "k_adjoint",
             "peak_kind": f"148 SMs x 4 warp schedulers x {sm_mhz:.0f} MHz (median SM clock of the timed region)",
-            "per_unit": {"unit": "nearest query (one warp-cooperative wide-tree search)",
+            "per_unit": {"unit": "nearest query (one lane's tree search)",
                          "warp_instructions_per_query": ipq, "queries_per_launch": adj_work["queries"],
                          "source": tj.get("instructions_measured_on")},
             "note": "the scene and trees (~0.2 MB) stay in L1/L2 and DRAM traffic is the per-walk records "

@@ -407,8 +407,8 @@ typedef struct wos_batch_s *wos_batch_t;
 /* Plan a batched forward (+ adjoint if want_adjoint) over many items: items
  * of one dimension form a group whose walks are concatenated in order of the
  * scenes' tree depth, then item order (order the items scene-major); each
- * walk phase runs one persistent work-queue launch per run of equal depth
- * (compiled for that depth), the reductions one launch per group.
+ * walk phase runs one persistent work-queue launch per group, and so do the
+ * reductions.
  * wos_batch_info reports the number of groups (dimensions present).
  * Buffers for all outputs are owned by the plan (wos_batch_outputs).  The
  * plan reads the items' scenes, points and targets in place at every run:
@@ -519,8 +519,7 @@ typedef struct wos_launch_config {
  * their nearest-query totals to a device counter {queries, LBVH node visits,
  * primitive distance evaluations} (brute force: nF evaluations per query).
  * wos_work_counters reads it (synchronising the device); reset != 0 clears.
- * While enabled those kernels run an instance compiled with counters (one for
- * every tree depth); the default instances carry none, which saves 1-3 % of a
+ * While enabled those kernels run an instance compiled with counters; the default instances carry none, which saves 1-3 % of a
  * step.  Results are the same either way. */
 WOS_API int wos_set_work_counting(int enable);
 WOS_API int wos_work_counters(int reset, int64_t *out);
