@@ -586,7 +586,7 @@ def c3_line(args, compact=False):
         "forward_walks_per_s": walks / t_fwd,
         "plain_forward_walks_per_s": m * nw / t_plain,
         "tree_work": {"forward": fwd_work, "forward_and_adjoint": fused_work,
-                      "note": "queries, node expansions, leaf steps (one warp step each)"},
+                      "note": "queries, node steps and leaf steps of single lanes"},
         "accuracy": {"rmse_vs_exact": float(np.sqrt((err ** 2).mean())), "rms_standard_error":
                      float(np.sqrt((se ** 2).mean())),
                      "truncated_fraction": float((steps.cpu().numpy() >= 64).mean())},
