@@ -978,17 +978,25 @@ __device__ __forceinline__ double sample_weight(const CTX &x, const float *dLdu,
 // directional derivative is gathered).  acc_src: this thread's source-gradient
 // accumulators, or null.
 //
-// Lanes wait for the code of their kind: a walk's step, run when a quarter of the
-// warp's lanes are at one, or a bisection step or an edge (start, end, set-up),
-// an eighth (a quarter: the 3D gradient of 50,000 points x 16 walks on 81,920
-// triangles 63.1 ms instead of 57.1; a sixteenth: no faster); or any when nothing
-// else is left to do.
+// Lanes wait for the code of their kind: a walk's step or, in 2D and in batches, an
+// edge (start, end, set-up) is run when a quarter of the warp's lanes are at one, a
+// bisection step or, for one 3D scene, an edge when an eighth are; or any when nothing
+// else is left to do.  An edge is the largest part of the code, and each run of it
+// takes instruction cache from the searches (a batch's edges, which look up their
+// items, most of all); a 3D search is long, so that waiting costs more.  Edges at
+// 1/8, 1/5, 1/4, 1/3: the 2D gradient of 20,000 points x 256 walks on 4,096 segments
+// 26.1, 25.3, 25.1, 24.8 ms (80,222 points: 101.0 and 97.1 with 1/8 and 1/4) and 2D
+// and 3D scenes in a batch 49.2, 47.0, 46.8, 47.0; the 3D gradient of 50,000 x 16 on
+// 81,920 triangles 32.1, 32.4, 32.7, 34.0.
+// Bisection steps at 1/5: 32.6 there, at 1/12 31.8; walk steps at 1/6 or 1/3: within
+// 2 % everywhere.
 template <int D, bool BVH, int MODE, class CTX, class WK>
 __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, long long idx0, long long total,
                                               const float *__restrict__ dLdu, unsigned long long *counter, int chunk,
                                               const AdjOut &out, const unsigned short *guide, unsigned *stack,
                                               AdjSlot<D> &slot, double *acc_src, WK &work) {
     constexpr bool ND_ONLY = MODE == ADJ_ND_ONLY, TAN = MODE == ADJ_TANGENT;
+    constexpr int EDGE = D == 2 || CTX::MULTI ? 4 : 8;
     constexpr bool FROM_REC = MODE == ADJ_FROM_RECORDS || TAN, HAS_PRIMAL = MODE == ADJ_RECOMPUTE;
     const unsigned FULL = 0xffffffffu;
     const int AS = blockDim.x;  // k-th accumulator at acc_src[k * AS]
@@ -1015,10 +1023,10 @@ __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, lon
         const int n_edge = __popc(__ballot_sync(FULL, edge)), n_run = __popc(__ballot_sync(FULL, active && !ready));
         const int n_all = n_ball + n_step + n_edge + n_run;
         if (n_all == 0) break;
-        const bool any = 8 * n_ball >= n_all || 4 * n_step >= n_all || 8 * n_edge >= n_all || n_run == 0;
-        const bool all = n_run == 0 && 8 * n_ball < n_all && 4 * n_step < n_all && 8 * n_edge < n_all;
+        const bool any = 8 * n_ball >= n_all || 4 * n_step >= n_all || EDGE * n_edge >= n_all || n_run == 0;
+        const bool all = n_run == 0 && 8 * n_ball < n_all && 4 * n_step < n_all && EDGE * n_edge < n_all;
         float ball_m = -1.0f;
-        if (any && n_edge != 0 && (all || 8 * n_edge >= n_all)) {
+        if (any && n_edge != 0 && (all || EDGE * n_edge >= n_all)) {
             if (ready && phase == PH_ANTI_START) {
                 const Hit hit = lane_hit<D, BVH>(sr, x.scene(item));
                 if (sqrtf(hit.d2) < a.epsilon2) {
