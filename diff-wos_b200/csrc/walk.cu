@@ -1446,6 +1446,18 @@ WalkCfg make_cfg(const wos_params &p) {
     return c;
 }
 
+// Opens all of a block's shared memory to the launches of `kern`.  The limit belongs
+// to the kernel and not to a call: set to what one call needs (its scene's tree depth
+// decides that), a shallow scene's call on one thread would lower it between another
+// thread's setting it and launching on a deep scene, 50,176 bytes for a 3D adjoint of
+// depth 8.  How many blocks share an SM and its L1 follows from each launch's own size.
+template <typename Kern>
+static cudaError_t open_shared_memory(Kern kern, int dev) {
+    int most = 0;
+    const cudaError_t e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    return e != cudaSuccess ? e : cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+}
+
 struct Shape {
     int grid, block, stack, stage_cdf;
     size_t smem;
@@ -1462,7 +1474,7 @@ static int shape_for(Kern kern, const SceneImpl &S, int D, bool bvh, bool want_c
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh.smem);
+    cudaError_t e = open_shared_memory(kern, dev);
     if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, sh.block, sh.smem);
@@ -2013,7 +2025,7 @@ static int launch_soft_t(const SceneImpl &S, const float *P, long long total, co
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int stack = BVH ? tree_stack_entries(S.tree_depth) : 0;
     const size_t smem = smem_bytes(-1, 256, stack, 0);
-    cudaError_t e = cudaFuncSetAttribute(k_walk_soft<D, BVH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = open_shared_memory(k_walk_soft<D, BVH>, dev);
     if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(k_walk_soft)");
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_walk_soft<D, BVH>, 256, smem);
     if (e != cudaSuccess) return fail_cuda(e, "occupancy(k_walk_soft)");
@@ -2399,7 +2411,7 @@ static int persistent_grid(Kern kern, int block, size_t smem, int blocks_per_sm,
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = open_shared_memory(kern, dev);
     if (e != cudaSuccess) return fail_cuda(e, "cudaFuncSetAttribute(MaxDynamicSharedMemorySize)");
     int occ = 0;
     e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, block, smem);

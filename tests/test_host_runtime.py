@@ -1,0 +1,77 @@
+"""The library's host code on a stand-in for the CUDA runtime (fake_cudart.cpp), each
+test in a process of its own: what launches ask for and what failed calls leave
+behind.  No GPU."""
+from __future__ import annotations
+
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+
+PRELUDE = f"""
+import ctypes, importlib.util
+spec = importlib.util.spec_from_file_location("wos_lib", r"{ROOT}/diff-wos_b200/wos/_lib.py")
+_lib = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(_lib)
+fake = ctypes.CDLL("libcudart.so.12")
+fake.fake_live.restype = fake.fake_calls.restype = ctypes.c_longlong
+fake.fake_fail_at.argtypes = [ctypes.c_longlong]
+L = _lib.lib()
+D = ctypes.c_void_p(1 << 30)  # a device address; nothing reads it
+def create(dim, nV, nF):
+    h = ctypes.c_void_p()
+    rc = L.wos_scene_create(dim, D, nV, D, nF, D, 0, None, None, ctypes.byref(h))
+    return rc, h
+params = _lib.WosParams(4, 32, 1e-3, 0, 0, 0, 0, 0, 1, 0, 0)
+adjoint = _lib.WosAdjointParams(1e-3, 0.1, 1, 1, 1e-3, 1, 1, 0)
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    d = tmp_path_factory.mktemp("cudart")
+    (d / "map").write_text("libcudart.so.12 { global: *; };\n")
+    include = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", f"-I{include}", "-Wl,-soname,libcudart.so.12",
+                    f"-Wl,--version-script={d / 'map'}", "-o", str(d / "libcudart.so.12"),
+                    str(ROOT / "tests" / "fake_cudart.cpp")], check=True)
+
+    def run(code):
+        env = dict(os.environ, LD_LIBRARY_PATH=f"{d}:{os.environ.get('LD_LIBRARY_PATH', '')}")
+        r = subprocess.run([sys.executable, "-c", PRELUDE + code], env=env, capture_output=True, text=True,
+                           timeout=300)
+        assert r.returncode == 0, r.stdout + r.stderr
+    return run
+
+
+def test_shared_memory_limits_are_never_lowered(fake):
+    """A kernel's limit belongs to the process: a call for a shallow scene must not
+    take away what another thread's call for a deep one is about to launch with."""
+    fake("""
+rc, deep = create(3, 100000, 81920)
+assert rc == 0
+rc, shallow = create(3, 100, 80)
+assert rc == 0
+for scene in (deep, shallow, deep):
+    for call in (
+        lambda: L.wos_solve(scene, D, 10, ctypes.byref(params), D, D, None, 0, None),
+        lambda: L.wos_solve_adjoint(scene, D, 10, ctypes.byref(params), ctypes.byref(adjoint), 1, None, D, None, D,
+                                    D, D, None, None, 0, None),
+        lambda: L.wos_adjoint(scene, D, 10, ctypes.byref(params), ctypes.byref(adjoint), D, D, D, None, None, 0, None),
+        lambda: L.wos_soft_walk(scene, D, 10, ctypes.byref(params), None, None, D, D, None, None, None, 0, None),
+        lambda: L.wos_soft_walk_adjoint(scene, D, 10, ctypes.byref(params), D, D, D, None),
+    ):
+        rc = call()
+        assert rc == 0, L.wos_last_error_string()
+    item = (_lib.WosBatchItem * 1)(_lib.WosBatchItem(scene.value, D.value, 10, 1, None, params))
+    plan = ctypes.c_void_p()
+    assert L.wos_batch_create(item, 1, ctypes.byref(adjoint), 1, None, ctypes.byref(plan)) == 0
+    assert L.wos_batch_run(plan, 0, None) == 0
+    assert L.wos_batch_destroy(plan, None) == 0
+assert fake.fake_launches() > 0 and fake.fake_refused() == 0
+assert fake.fake_lowered() == 0, fake.fake_lowered()
+""")
