@@ -883,15 +883,57 @@ __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_t
 // ------------------------------------------------------------------ host
 static inline int nblk(long long n, int b) { return (int)((n + b - 1) / b); }
 
-// Entry grid of the search tree (SceneView::grid), a thread per cell.  U, the
-// distance from the cell's centre x to a primitive found by going to the nearest
-// child at each depth, bounds the distance from every point q of the cell to its
-// nearest primitive by U + h, h the cell's half diagonal, so all its nearest
-// primitives lie within U + 2 h of x: nodes farther than that are left out.
-// Distances take search_bound's slack wherever a computed one stands for a true
-// one or the reverse; h that of the rounding of a point's cell and of x.  The
-// cell's nodes are the root's children, replaced by their own children as long
-// as four are enough.  The cell of the points outside has the root's children.
+// How much farther than a triangle's closest point the one that tri_closest finds may
+// be, for query points up to R from the triangle's vertex a.  Its barycentric
+// coordinates are quotients of differences of products: with A = |ab|, B = |ac|, s the
+// sine between them and M = R + A + B, the products are below A B M^2 and carry up to
+// 16 x 2^-24 of that (and a few steps of the denormal floats), the quotients' denominator
+// is A^2 B^2 s^2, and the coordinates move the point along ab and ac.  A region taken
+// for its neighbour moves it by no more, and twice that is allowed for; the point always
+// lies on the triangle.  2e-6 of an edge for an even triangle near by, more than its
+// length for a needle of aspect 1e-4, whose coordinates are noise.
+__device__ __forceinline__ float closest_error(float4 t1, float4 t2, float ab2, float R) {
+    const double A = sqrtf(ab2), B = sqrtf(t2.w), M = (double)R + A + B, m = A * B * M * M;
+    const double det = (double)ab2 * t2.w - (double)t1.w * t1.w;
+    if (!(m < 1e37) || !(det > 0.0)) return INFINITY;  // the products overflow; no triangle
+    return (float)((32.0 * 0x1p-24 * m + 1e-44) / det * (A + B));
+}
+
+// Upper bound of the computed distance to the nearest of a leaf's primitives from any
+// point within h of x, less h.  2D: the computed distance at x, as distances to a segment
+// are exact to search_bound's slack.  3D: a triangle's is that at x and the error above,
+// or the distance to its farthest vertex.
+template <int D>
+__device__ __forceinline__ float leaf_reach(const SceneView &S, unsigned leaf, const float *x, float h) {
+    constexpr int N = Tree<D>::LEAF;
+    float d2[N], u = INFINITY;
+    leaf_distances<D>(S, leaf, x, d2);
+    if constexpr (D == 2) {
+        for (int c = 0; c < N; ++c) u = fminf(u, d2[c]);
+        return sqrtf(u);
+    } else {
+        const float4 *b = S.prims + (size_t)leaf * Tree<3>::LEAF_W;
+        for (int c = 0; c < N; ++c) {
+            const float4 t0 = b[3 * c], t1 = b[3 * c + 1], t2 = b[3 * c + 2];
+            const float v[3] = {x[0] - t0.x, x[1] - t0.y, x[2] - t0.z};
+            const float b0 = v[0] - t1.x, b1 = v[1] - t1.y, b2 = v[2] - t1.z;
+            const float c0 = v[0] - t2.x, c1 = v[1] - t2.y, c2 = v[2] - t2.z;
+            const float ra = dot3(v[0], v[1], v[2], v[0], v[1], v[2]);
+            const float far = fmaxf(ra, fmaxf(dot3(b0, b1, b2, b0, b1, b2), dot3(c0, c1, c2, c0, c1, c2)));
+            u = fminf(u, fminf(sqrtf(d2[c]) + closest_error(t1, t2, t0.w, sqrtf(ra) + h), sqrtf(far)));
+        }
+        return u;
+    }
+}
+
+// Entry grid of the search tree (SceneView::grid), a thread per cell.  U + h (leaf_reach),
+// for the leaf found by going to the nearest child at each depth from the cell's centre x
+// and h the cell's half diagonal, bounds the computed distance from every point q of the
+// cell to its nearest primitive, so all its nearest primitives lie within U + 2 h of x:
+// nodes farther than that are left out.  Distances take search_bound's slack wherever a
+// computed one stands for a true one or the reverse; h that of the rounding of a point's
+// cell and of x.  The cell's nodes are the root's children, replaced by their own children
+// as long as four are enough.  The cell of the points outside has the root's children.
 template <int D>
 __global__ void k_entry_grid(SceneView S, const int *lohi, uint4 *node, float4 *box) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x, bits = S.grid_bits, G = 1 << bits;
@@ -930,10 +972,7 @@ __global__ void k_entry_grid(SceneView S, const int *lohi, uint4 *node, float4 *
             if (d[c] < d[near]) near = c;
         idx = 4u * idx + near;
     }
-    float p[Tree<D>::LEAF], u = INFINITY;
-    leaf_distances<D>(S, idx, x, p);
-    for (int c = 0; c < Tree<D>::LEAF; ++c) u = fminf(u, p[c]);
-    const float r = h + widen(widen(widen(sqrtf(u)) + h)), r2 = (r * r) * (1.0f + 0x1p-20f);
+    const float r = h + widen(widen(widen(leaf_reach<D>(S, idx, x, h)) + h)), r2 = (r * r) * (1.0f + 0x1p-20f);
 
     unsigned n[4] = {0u, 1u, 2u, 3u};
     int count = 4;
