@@ -947,16 +947,17 @@ __global__ void k_entry_grid(SceneView S, const int *lohi, uint4 *node, float4 *
         ext_max = fmaxf(ext_max, ext[k]);
         abs_max = fmaxf(abs_max, fmaxf(fabsf(lo[k]), fabsf(hi)));
     }
+    const float unit = fmaxf(ext_max, FLT_MIN);
     float h2 = 0.0f, inv[3] = {0.0f, 0.0f, 0.0f};
     for (int k = 0; k < D; ++k) {
         ext[k] = fmaxf(ext[k], ext_max * 0x1p-20f);  // flat
         const float cell = ext[k] / (float)G;
         inv[k] = (float)G / ext[k];
         x[k] = lo[k] + ((float)(i >> (k * bits) & (G - 1)) + 0.5f) * cell;
-        h2 = fmaf(cell, cell, h2);
+        h2 = fmaf(cell / unit, cell / unit, h2);
     }
-    const float h = 0.5005f * sqrtf(h2) + 1e-6f * ext_max + 1e-6f * abs_max;
-    const float e = (1.0f + 0.5f * D) * 0x1.02p-20f * ext_max;  // prune_tol's largest in the box
+    const float h = 0.5005f * sqrtf(h2) * unit + 1e-6f * ext_max + 1e-6f * abs_max + TOL_MIN;
+    const float e = (1.0f + 0.5f * D) * 0x1.02p-20f * ext_max + TOL_MIN;  // prune_tol's largest in the box
     const float tol = D == 2 ? e : 1025.0f * (e * e);
     auto widen = [&](float d) { return sqrtf(search_bound<D>((d * d) * (1.0f + 0x1p-20f), tol)); };
 

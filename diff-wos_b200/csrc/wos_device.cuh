@@ -342,15 +342,17 @@ struct NoWork {
     NoCount nq, nb, np;
 };
 
-// Pruning slack (same rule as the oracle): a box is skipped only when its
-// squared distance exceeds (1 + 2^-10) best + 1025 (s 2^-20)^2, where s
-// bounds the coordinates' magnitude around the scene.
+// Pruning slack: a box is skipped only when its squared distance exceeds (1 + 2^-10)
+// best + 1025 (s 2^-20)^2 (2D searches: search_bound), where s bounds the coordinates'
+// magnitude around the scene.  s 2^-20 is at least 1e-22, whose square is 7 steps of the
+// denormal floats: squared distances that small are only exact to a few steps.
+constexpr float TOL_MIN = 1e-22f;
 template <int D>
 __device__ __forceinline__ float prune_tol(const SceneView &S, const float *p) {
     float s = S.max_extent;
 #pragma unroll
     for (int k = 0; k < D; ++k) s += fabsf(p[k] - S.centre[k]);
-    return s * 9.5367431640625e-07f;
+    return fmaf(s, 0x1p-20f, TOL_MIN);
 }
 template <int D>
 __device__ __forceinline__ float prune_tol2(const SceneView &S, const float *p) {
