@@ -1,5 +1,6 @@
-"""Scenes so small that squared distances are denormal floats, where rounding is a
-step and not a fraction: the tree against brute force, bit for bit."""
+"""Scenes so small that squared distances, or the products in a triangle's barycentric
+coordinates, are denormal floats, where rounding is a step and not a fraction: the tree
+against brute force, bit for bit."""
 from __future__ import annotations
 
 import numpy as np
@@ -8,7 +9,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("scale", [1e-16, 1e-17, 1e-18, 1e-19, 1e-20, 1e-21, 1e-22, 1e-23, 1e-25, 1e-30])
+@pytest.mark.parametrize("scale", [1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-13, 1e-16, 1e-17, 1e-18, 1e-19, 1e-20, 1e-21,
+                                   1e-22, 1e-23, 1e-25, 1e-30])
 @pytest.mark.parametrize("dim,size", [(2, 40), (2, 1024), (3, 2), (3, 4)])
 def test_small_scene_equals_brute_force(cuda, dim, size, scale):
     import wos
