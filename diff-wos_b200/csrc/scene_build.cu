@@ -969,6 +969,12 @@ __global__ void __launch_bounds__(128, 4) k_entry_grid(SceneView S, const int *l
     auto distances = [&](unsigned block, float *dd) {
         block_distances<D>(S.tree + (size_t)block * Tree<D>::NODE_W, x, dd);
     };
+    // A vertex that is not finite, or an extent that overflows, leaves no centre to
+    // descend from (children that do not exist are infinitely far from finite points
+    // only): such a cell has the root's children.
+    bool finite = true;
+    for (int k = 0; k < D; ++k) finite = finite && fabsf(x[k]) <= FLT_MAX;
+    for (int k = 0; k < D; ++k) x[k] = finite ? x[k] : 0.0f;
     float d[4];
     unsigned idx = 0;
     for (int dep = 0; dep < S.tree_depth; ++dep) {
@@ -979,7 +985,7 @@ __global__ void __launch_bounds__(128, 4) k_entry_grid(SceneView S, const int *l
         idx = 4u * idx + near;
     }
     const float r = h + widen(widen(widen(leaf_reach<D>(S, idx, x, h)) + h));
-    const float r2 = (r * r) * (1.0f + 0x1p-20f);
+    const float r2 = finite ? (r * r) * (1.0f + 0x1p-20f) : INFINITY;
 
     unsigned n[4] = {0u, 1u, 2u, 3u};
     int count = 4;
