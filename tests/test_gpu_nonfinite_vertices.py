@@ -9,6 +9,14 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def clean_status(cuda):
+    """Queries that find no primitive say so in the device's status word."""
+    import wos
+    yield
+    wos.device_status(reset=True)
+
+
 @pytest.mark.parametrize("what", ["inf", "-inf", "nan", "all_nan", "far", "huge"])
 @pytest.mark.parametrize("dim,n", [(2, 1), (2, 5), (2, 40), (2, 300), (3, 1), (3, 3), (3, 40), (3, 300)])
 def test_nonfinite_scene_equals_brute_force(cuda, dim, n, what):
