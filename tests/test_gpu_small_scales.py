@@ -9,6 +9,14 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+@pytest.fixture(autouse=True)
+def clean_status(cuda):
+    """Queries that find no primitive (every distance NaN) say so in the device's status."""
+    import wos
+    yield
+    wos.device_status(reset=True)
+
+
 @pytest.mark.parametrize("scale", [1e-7, 1e-8, 1e-9, 1e-10, 1e-11, 1e-13, 1e-16, 1e-17, 1e-18, 1e-19, 1e-20, 1e-21,
                                    1e-22, 1e-23, 1e-25, 1e-30])
 @pytest.mark.parametrize("dim,size", [(2, 40), (2, 1024), (3, 2), (3, 4)])
