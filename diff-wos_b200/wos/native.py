@@ -254,11 +254,22 @@ class NativeScene:
                  rec.data_ptr(), _ptr(dc), workspace.data_ptr(), need, stream())
         return mean, var, rec, dc
 
+    def _check_records(self, n, s: WalkSettings, a: AdjointSettings, rec, dc):
+        """The kernels read n x nwalks records (and source derivatives) in place."""
+        walks = n * int(s.nwalks)
+        if rec.numel() * rec.element_size() < walks * _lib.lib().wos_walk_record_bytes(self.dim) \
+                or not rec.is_contiguous():
+            raise ValueError("rec must hold the records of solve_records() for these points and settings")
+        if dc is not None and a.want_dsrc and s.include_source and (
+                dc.numel() < 5 * walks or dc.dtype != torch.float32 or not dc.is_contiguous()):
+            raise ValueError("dc must hold the source derivatives of solve_records() for these points and settings")
+
     def adjoint_records(self, P, s: WalkSettings, a: AdjointSettings, dLdu, rec, dc,
                         workspace: torch.Tensor | None = None):
         P = as_cuda(P, torch.float32, self.dim)
         dLdu = as_cuda(dLdu, torch.float32).reshape(-1)
         n = int(P.shape[0])
+        self._check_records(n, s, a, rec, dc)
         d = self.device
         dV = torch.zeros((self.nV, self.dim), dtype=torch.float32, device=d) if a.want_dV else None
         dg = torch.zeros(self.nV, dtype=torch.float32, device=d) if a.want_dg else None
@@ -313,6 +324,7 @@ class NativeScene:
         with the same points and settings."""
         P = as_cuda(P, torch.float32, self.dim)
         n = int(P.shape[0])
+        self._check_records(n, s, a, rec, dc)
         tan = torch.empty(n, dtype=torch.float64, device=self.device)
         tV, tg, ts = self._direction(dV, dg, dsrc)
         if n:

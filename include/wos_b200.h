@@ -312,8 +312,10 @@ WOS_API int wos_solve_tangent(wos_scene_t scene, const float *P, int n, const wo
                               void *workspace, size_t workspace_bytes, wos_stream_t stream);
 
 /* The tangent of wos_solve_tangent from the records that wos_solve_records
- * kept (same P, n and params) instead of walking again; the same result.
- * dcontrib is needed where the source term's derivative is taken. */
+ * kept (same scene, P, n and params) instead of walking again; the same result.
+ * dcontrib is needed where the source term's derivative is taken.  Here and in
+ * wos_adjoint_records, records of another scene give no meaningful result, but no
+ * read out of bounds; where they are sorted first they set WOS_STATUS_BAD_PRIM. */
 WOS_API size_t wos_tangent_records_workspace_size(wos_scene_t scene, int n, const wos_params *p);
 WOS_API int wos_tangent_records(wos_scene_t scene, const float *P, int n, const wos_params *p,
                                 const wos_adjoint_params *a, const float *dV_dir, const float *dg_dir,
