@@ -42,9 +42,11 @@ __global__ void k_check_indices(const int *F, int nF, int dim, int nV, int *out)
 }
 
 // Start of a build's counters: [0, 6) the bounding box's ordered ints, [6] the
-// deepest node.
+// deepest node, [7, 9) floats: the order's cost (k_tree_bounds).
+constexpr int BUILD_COUNTERS = 9;
 __global__ void k_build_init(int *c) {
-    if (threadIdx.x < 7) c[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : threadIdx.x < 6 ? (int)0x80000000 : 0;
+    if (threadIdx.x < BUILD_COUNTERS)
+        c[threadIdx.x] = threadIdx.x < 3 ? 0x7fffffff : threadIdx.x < 6 ? (int)0x80000000 : 0;
 }
 
 __global__ void k_aabb(const float *V, int nV, int dim, int *lohi) {
@@ -843,9 +845,30 @@ __host__ __device__ inline int nodes_per_block(long long prims) {
     return prims <= TREE_LANE_PRIMS ? TREE_THREADS : prims <= TREE_WARP_PRIMS ? TREE_THREADS / 32 : 1;
 }
 
+// Area of a node's box (an eighth of its surface) and of np triangles from position s0
+// (twice theirs), lengths times inv.
+__device__ __forceinline__ float box_area(const float *o, float inv) {
+    const unsigned e01 = __float_as_uint(o[6]);
+    const float e0 = __uint_as_float(e01 << 16) * inv, e1 = __uint_as_float(e01 & 0xffff0000u) * inv, e2 = o[7] * inv;
+    return fmaf(e0, e1, fmaf(e0, e2, e1 * e2));
+}
+__device__ __forceinline__ float triangle_area(const float4 *prims, int s0, int np, float inv) {
+    float a = 0.0f;
+    for (int s = s0; s < s0 + np; ++s) {
+        const float4 *b = prims + (size_t)(s / Tree<3>::LEAF) * Tree<3>::LEAF_W + 3 * (s % Tree<3>::LEAF);
+        const float4 ab = b[1], ac = b[2];
+        float n[3];
+        cross3(ab.x * inv, ab.y * inv, ab.z * inv, ac.x * inv, ac.y * inv, ac.z * inv, n[0], n[1], n[2]);
+        a += sqrtf(dot3(n[0], n[1], n[2], n[0], n[1], n[2]));
+    }
+    return a;
+}
+
+// cost (3D): adds the areas of all boxes to [0] and of all triangles to [1], in units of
+// the scene's largest extent (of its box, lohi).
 template <int D, bool LARGE>
 __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_tree_bounds(
-    TreePlan P, const float4 *prims, float4 *tree) {
+    TreePlan P, const float4 *prims, float4 *tree, const int *lohi, float *cost) {
     __shared__ float red[32];
     int d = P.d0;
     while (d < P.d1 && (int)blockIdx.x >= P.first[d + 1]) ++d;
@@ -866,6 +889,20 @@ __global__ void __launch_bounds__(LARGE ? TREE_LARGE_THREADS : TREE_THREADS) k_t
     } else {
         node_bound<D, 32>(prims, (int)s0, np, threadIdx.x & 31, red, o);
         writer = writer && (threadIdx.x & 31) == 0;
+    }
+    if (D == 3) {
+        float ext = 0.0f, area[2] = {0.0f, 0.0f};
+        for (int k = 0; k < 3; ++k) ext = fmaxf(ext, from_ordered_int(lohi[3 + k]) - from_ordered_int(lohi[k]));
+        const float inv = ext > 0.0f ? 1.0f / ext : 0.0f;
+        if (writer) {
+            area[0] = box_area(o, inv);
+            if (d == P.depth) area[1] = triangle_area(prims, (int)s0, np, inv);
+        }
+        for (int k = 0; k < 2; ++k) {
+            if (!(area[k] < INFINITY)) area[k] = 0.0f;  // vertices that are not finite
+            for (int x = 16; x > 0; x >>= 1) area[k] += __shfl_xor_sync(0xffffffffu, area[k], x);
+            if ((threadIdx.x & 31) == 0 && area[k] != 0.0f) atomicAdd(&cost[k], area[k]);
+        }
     }
     if (!writer) return;
     write_bound<D>(tree, d, i, o);
@@ -1171,6 +1208,20 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
     return 0;
 }
 
+// Whether a mesh has moved too far for the order of its triangles: the areas of the
+// tree's boxes have grown by a third since the order was made, in units of the scene's
+// extent or of the triangles' own area, or that area is another one altogether (the
+// scene was made from vertices that only held a place: flat, collapsed, shuffled).
+//   Search steps of the kept order over those of a new one, and the boxes' growth:
+// 20,480 loose triangles on a unit sphere displaced by up to 0.02, 0.05, 0.1, 0.5 take
+// 1.05, 1.26, 1.77, 16.4 times the steps at 1.11, 1.53, 2.5, 15.4; 20,000 in a box by
+// 0.1 2.15 at 1.6; a sphere twisted by 3 radians 2.5 at 1.75.  Spheres displaced by up
+// to 15 or 40 % in waves, rotated, squashed or stretched: 0.84 to 1.01 at up to 1.11.
+static bool order_worn(const float *then, const float *now) {
+    return now[0] > 1.3f * then[0] || now[0] * then[1] > 1.3f * then[0] * now[1] || now[1] > 4.0f * then[1] ||
+           now[1] < 0.25f * then[1];
+}
+
 // The Green's function tables, the same for every scene, computed once.
 struct GTables {
     std::vector<float> cdf;
@@ -1229,6 +1280,48 @@ static int build_vertex_slots(SceneImpl &S, cudaStream_t st) {
     return 0;
 }
 
+// The search tree of the primitives in the order torig (or that of `keys`), in the
+// buffers of the first build (their sizes depend on nF alone): device views held
+// elsewhere -- batch plans, captured graphs, launches on other streams -- keep pointing
+// at live memory.
+template <int D>
+static int build_tree(SceneImpl &S, const unsigned long long *keys, int *counters, cudaStream_t st) {
+    constexpr int N = Tree<D>::LEAF;
+    const int nF = S.nF, TB = 256, n_leaf = (nF + N - 1) / N;
+    TreePlan P{};
+    P.depth = S.tree_depth;
+    P.nF = nF;
+    for (int d = 1; d <= P.depth; ++d) {
+        const long long cap = node_prims(N, P.depth - d);
+        P.count[d] = (int)((nF + cap - 1) / cap);
+    }
+    k_tree_prims<D><<<nblk((long long)n_leaf * N, TB), TB, 0, st>>>(nF, n_leaf, keys, S.seg, S.seginv, S.tri, S.prims,
+                                                                S.torig);
+    // the depths of large nodes, then the others
+    int split = 1;
+    while (split <= P.depth && node_prims(N, P.depth - split) > TREE_WARP_PRIMS) ++split;
+    float *cost = reinterpret_cast<float *>(counters + 7);
+    for (int part = 0; part < 2; ++part) {
+        P.d0 = part == 0 ? 1 : split;
+        P.d1 = part == 0 ? split - 1 : P.depth;
+        int blocks = 0;
+        for (int d = P.d0; d <= P.d1; ++d) {
+            P.first[d] = blocks;
+            blocks += nblk(P.count[d], nodes_per_block(node_prims(N, P.depth - d)));
+        }
+        if (blocks == 0) continue;
+        P.first[P.d1 + 1] = blocks;
+        if (part == 0)
+            k_tree_bounds<D, true><<<blocks, TREE_LARGE_THREADS, 0, st>>>(P, S.prims, S.tree, counters, cost);
+        else
+            k_tree_bounds<D, false><<<blocks, TREE_THREADS, 0, st>>>(P, S.prims, S.tree, counters, cost);
+    }
+    const int cells = (1 << (D * S.grid_bits)) + 1;
+    k_entry_grid<D><<<nblk(cells, 128), 128, 0, st>>>(S.view(), counters, S.grid_node(), S.grid_box());
+    WOS_TRY(cudaGetLastError());
+    return 0;
+}
+
 template <int D>
 static int build_geometry(SceneImpl &S, cudaStream_t st) {
     const int nV = S.nV, nF = S.nF, nInt = nF - 1;
@@ -1252,7 +1345,7 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
     void *tmp = nullptr;
     for (int pass = 0; pass < 2; ++pass) {  // sizes, then the buffers
         A.used = 0;
-        counters = A.take<int>(8);
+        counters = A.take<int>(BUILD_COUNTERS);
         contrib = A.take<float>((size_t)nF * D * D);
         pbox = A.take<float>((size_t)nF * 2 * D);
         mkeys = A.take<unsigned long long>(nF);
@@ -1283,46 +1376,12 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
         WOS_TRY(cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, mkeys, skeys, nF, 32, 32 + key_bits, st));
     k_leaf_data<D><<<nblk(nF, TB), TB, 0, st>>>(skeys, nF, S.seg, S.seginv, S.tri, S.lseg, S.lseginv, S.ltri, S.lorig);
 
-    // ---- search tree, in the buffers of the first build (their sizes depend
-    // on nF alone): device views held elsewhere -- batch plans, captured
-    // graphs, launches on other streams -- keep pointing at live memory
-    {
-        constexpr int N = Tree<D>::LEAF;
-        const int n_leaf = (nF + N - 1) / N;
-        TreePlan P{};
-        P.depth = S.tree_depth;
-        P.nF = nF;
-        for (int d = 1; d <= P.depth; ++d) {
-            const long long cap = node_prims(N, P.depth - d);
-            P.count[d] = (int)((nF + cap - 1) / cap);
-        }
-        if (D == 3 && !S.tree_ordered)
-            if (int rc = median_order(S, pbox, skeys, st)) return rc;
-        S.tree_ordered = true;
-        k_tree_prims<D><<<nblk((long long)n_leaf * N, TB), TB, 0, st>>>(nF, n_leaf, D == 2 ? skeys : nullptr, S.seg,
-                                                                    S.seginv, S.tri, S.prims, S.torig);
-        // the depths of large nodes, then the others
-        int split = 1;
-        while (split <= P.depth && node_prims(N, P.depth - split) > TREE_WARP_PRIMS) ++split;
-        for (int part = 0; part < 2; ++part) {
-            P.d0 = part == 0 ? 1 : split;
-            P.d1 = part == 0 ? split - 1 : P.depth;
-            int blocks = 0;
-            for (int d = P.d0; d <= P.d1; ++d) {
-                P.first[d] = blocks;
-                blocks += nblk(P.count[d], nodes_per_block(node_prims(N, P.depth - d)));
-            }
-            if (blocks == 0) continue;
-            P.first[P.d1 + 1] = blocks;
-            if (part == 0)
-                k_tree_bounds<D, true><<<blocks, TREE_LARGE_THREADS, 0, st>>>(P, S.prims, S.tree);
-            else
-                k_tree_bounds<D, false><<<blocks, TREE_THREADS, 0, st>>>(P, S.prims, S.tree);
-        }
-        const int cells = (1 << (D * S.grid_bits)) + 1;
-        k_entry_grid<D><<<nblk(cells, 128), 128, 0, st>>>(S.view(), counters, S.grid_node(), S.grid_box());
-        WOS_TRY(cudaGetLastError());
-    }
+    // ---- search tree
+    const bool new_order = D == 3 && !S.tree_ordered;
+    if (new_order)
+        if (int rc = median_order(S, pbox, skeys, st)) return rc;
+    if (int rc = build_tree<D>(S, D == 2 ? skeys : nullptr, counters, st)) return rc;
+    S.tree_ordered = true;
 
     // ---- hierarchy
     S.nNodes = nInt;
@@ -1338,10 +1397,22 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
         k_write_nodes<D><<<nblk(nInt, TB), TB, 0, st>>>(skeys, nInt, pbox, nbox, child, new_of_old, S.node);
     }
     WOS_TRY(cudaGetLastError());
-    int host[7];
+    int host[BUILD_COUNTERS];
     WOS_TRY(cudaMemcpyAsync(host, counters, sizeof(host), cudaMemcpyDeviceToHost, st));
-    cudaFreeAsync(A.base, st);
     WOS_TRY(cudaStreamSynchronize(st));
+    float cost[2];
+    memcpy(cost, host + 7, sizeof(cost));
+    if (D == 3 && !new_order && order_worn(S.order_cost, cost)) {
+        WOS_TRY(cudaMemsetAsync(counters + 7, 0, sizeof(cost), st));
+        if (int rc = median_order(S, pbox, skeys, st)) return rc;
+        if (int rc = build_tree<D>(S, nullptr, counters, st)) return rc;
+        WOS_TRY(cudaMemcpyAsync(cost, counters + 7, sizeof(cost), cudaMemcpyDeviceToHost, st));
+        WOS_TRY(cudaStreamSynchronize(st));
+        memcpy(S.order_cost, cost, sizeof(cost));
+    } else if (new_order) {
+        memcpy(S.order_cost, cost, sizeof(cost));
+    }
+    cudaFreeAsync(A.base, st);
     auto from_ord = [](int i) {
         int b = i >= 0 ? i : i ^ 0x7fffffff;
         float f;

@@ -58,7 +58,8 @@ struct SceneImpl {
     uint4 *grid_node() const { return reinterpret_cast<uint4 *>(grid) + 2; }
     float4 *grid_box() const { return grid + 2 + ((size_t)1 << (dim * grid_bits)) + 2; }
     int *vslot = nullptr, *vfirst = nullptr;  // (face, corner) slots by vertex, for the normals
-    bool tree_ordered = false;  // torig holds the order (3D: kept when vertices move)
+    bool tree_ordered = false;  // torig holds the order (3D: kept when vertices move, while it serves: order_worn)
+    float order_cost[2] = {0.0f, 0.0f};  // 3D: areas of the boxes and of the triangles when the order was made
     // Incremented by every build and source change: the by-value fields of
     // view() (bounding box, extents, source) may have changed since a view
     // was taken.

@@ -152,7 +152,10 @@ WOS_API int wos_scene_update_values(wos_scene_t scene, const float *g, wos_strea
  * LBVH; returns after the rebuild.  The scene's device buffers stay where they
  * are (the trees are refilled in place), so batch plans and launches that hold
  * the scene keep reading live memory; kernels still running on another stream
- * race with the rebuild and must be ordered before it by the caller. */
+ * race with the rebuild and must be ordered before it by the caller.  A mesh's
+ * triangles keep their order in the search tree while it serves the new
+ * vertices, and are ordered anew when the tree's boxes have grown by 30 % since
+ * the order was made; searches then cost about what a new scene's do. */
 WOS_API int wos_scene_update_vertices(wos_scene_t scene, const float *V, wos_stream_t stream);
 
 /* Set the analytic source (include/scene.cuh:270-301): type 0 none,
