@@ -447,8 +447,9 @@ __global__ void k_tree_prims(int nF, int n_leaf, const unsigned long long *keys,
 // tree is a compact patch.  Runs of a Hilbert curve, whose cells cut a surface
 // anywhere, take 28 node and 5.7 leaf visits per query on 81,920 triangles where
 // these take 20 and 4.5.  Segments above SPLIT_SMALL positions are sorted by one
-// radix sort per level (keys: segment, then the quantised coordinate); one block
-// takes each smaller segment through all of its levels in shared memory.
+// radix sort per level (keys: segment, then the coordinate in 16 bits, or what is left
+// of 32 above 134 million triangles); one block takes each smaller segment through all of
+// its levels in shared memory.
 constexpr int SPLIT_SMALL = 1024;
 
 __device__ __forceinline__ float box_centre(const float *pbox, int f, int k) {
@@ -498,14 +499,16 @@ __device__ __forceinline__ int longest_axis(const int *b, float &lo, float &ext)
     return a;
 }
 
-__global__ void k_split_keys(const float *pbox, const int *ord, int nF, int cap, const int *bounds, unsigned *keys) {
+__global__ void k_split_keys(const float *pbox, const int *ord, int nF, int cap, int bits, const int *bounds,
+                             unsigned *keys) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= nF) return;
     const int seg = p / cap;
     float lo, ext;
     const int a = longest_axis(bounds + 6 * seg, lo, ext);
     const float u = ext > 0.0f ? (box_centre(pbox, ord[p], a) - lo) / ext : 0.0f;
-    keys[p] = (unsigned)seg << 16 | (unsigned)fminf(fmaxf(u * 65536.0f, 0.0f), 65535.0f);
+    const float n = (float)(1 << bits);
+    keys[p] = (unsigned)seg << bits | (unsigned)fminf(fmaxf(u * n, 0.0f), n - 1.0f);
 }
 
 __global__ void __launch_bounds__(SPLIT_SMALL) k_split_small(const float *pbox, int nF, int leaf, int *ord) {
@@ -1170,9 +1173,10 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
     while (cap < nF) cap *= 2;
     if (cap > SPLIT_SMALL) {
         const int max_seg = nblk(nF, 2 * SPLIT_SMALL);
-        int bits = 16;
-        while ((1LL << (bits - 16)) < max_seg) ++bits;
-        if (bits > 32) return fail(WOS_ERR_UNSUPPORTED, "scene too large for the search tree's order");
+        // at most 2^20 segments, as nF is an int
+        int seg_bits = 0;
+        while ((1LL << seg_bits) < max_seg) ++seg_bits;
+        const int bits = std::min(16, 32 - seg_bits);
         int *bounds = nullptr, *ord2 = nullptr;
         unsigned *keys = nullptr, *keys2 = nullptr;
         void *tmp = nullptr;
@@ -1181,7 +1185,7 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
         WOS_TRY(dalloc(&ord2, nF, st));
         WOS_TRY(dalloc(&keys, nF, st));
         WOS_TRY(dalloc(&keys2, nF, st));
-        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, S.torig, ord2, nF, 0, bits, st);
+        cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, S.torig, ord2, nF, 0, bits + seg_bits, st);
         WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
         int *cur = S.torig, *alt = ord2;
         for (; cap > SPLIT_SMALL; cap /= 2) {
@@ -1189,9 +1193,9 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
             k_split_init<<<nblk(6 * n_seg, TB), TB, 0, st>>>(bounds, 6 * n_seg);
             const int c = (int)std::min<long long>(cap, 1LL << 30);
             k_split_bounds<<<nblk(nF, TB), TB, 0, st>>>(pbox, cur, nF, c, bounds);
-            k_split_keys<<<nblk(nF, TB), TB, 0, st>>>(pbox, cur, nF, c, bounds, keys);
-            int used = 16;
-            while ((1LL << (used - 16)) < n_seg) ++used;
+            k_split_keys<<<nblk(nF, TB), TB, 0, st>>>(pbox, cur, nF, c, bits, bounds, keys);
+            int used = bits;
+            while ((1LL << (used - bits)) < n_seg) ++used;
             WOS_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, cur, alt, nF, 0, used, st));
             std::swap(cur, alt);
         }

@@ -75,3 +75,15 @@ for scene in (deep, shallow, deep):
 assert fake.fake_launches() > 0 and fake.fake_refused() == 0
 assert fake.fake_lowered() == 0, fake.fake_lowered()
 """)
+
+
+@pytest.mark.parametrize("nF", [134217728, 134217729, 300000000])
+def test_meshes_above_65536_split_segments_are_taken(fake, nF):
+    """Segments of 2,048 triangles and the coordinate within them share a sort key."""
+    fake(f"""
+rc, h = create(3, 1000000, {nF})
+assert rc == 0, L.wos_last_error_string()
+assert L.wos_scene_update_vertices(h, D, None) == 0
+L.wos_scene_destroy(h, None)
+assert fake.fake_live() == 0
+""")
