@@ -1159,6 +1159,24 @@ void build_g_guide(const std::vector<float> &cdf, int ng, std::vector<unsigned s
     }
 }
 
+// Temporaries: one allocation, carved up; freed on the stream when its scope is left.
+struct Arena {
+    cudaStream_t st = nullptr;
+    char *base = nullptr;
+    size_t used = 0;
+    explicit Arena(cudaStream_t s) : st(s) {}
+    Arena(const Arena &) = delete;
+    ~Arena() {
+        if (base) cudaFreeAsync(base, st);
+    }
+    template <typename T>
+    T *take(size_t n) {
+        T *p = reinterpret_cast<T *>(base + used);
+        used += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+};
+
 __global__ void k_key_order(const unsigned long long *keys, int n, int *ord) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) ord[i] = (int)(unsigned)keys[i];
@@ -1179,14 +1197,19 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
         const int bits = std::min(16, 32 - seg_bits);
         int *bounds = nullptr, *ord2 = nullptr;
         unsigned *keys = nullptr, *keys2 = nullptr;
-        void *tmp = nullptr;
         size_t tmp_bytes = 0;
-        WOS_TRY(dalloc(&bounds, (size_t)6 * max_seg, st));
-        WOS_TRY(dalloc(&ord2, nF, st));
-        WOS_TRY(dalloc(&keys, nF, st));
-        WOS_TRY(dalloc(&keys2, nF, st));
         cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, S.torig, ord2, nF, 0, bits + seg_bits, st);
-        WOS_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
+        void *tmp = nullptr;
+        Arena A(st);
+        for (int pass = 0; pass < 2; ++pass) {  // sizes, then the buffers
+            A.used = 0;
+            bounds = A.take<int>((size_t)6 * max_seg);
+            ord2 = A.take<int>(nF);
+            keys = A.take<unsigned>(nF);
+            keys2 = A.take<unsigned>(nF);
+            tmp = A.take<char>(tmp_bytes);
+            if (pass == 0) WOS_TRY(cudaMallocAsync((void **)&A.base, A.used, st));
+        }
         int *cur = S.torig, *alt = ord2;
         for (; cap > SPLIT_SMALL; cap /= 2) {
             const int n_seg = nblk(nF, (int)std::min<long long>(cap, 1LL << 30));
@@ -1201,11 +1224,6 @@ static int median_order(SceneImpl &S, const float *pbox, const unsigned long lon
         }
         if (cur != S.torig)
             WOS_TRY(cudaMemcpyAsync(S.torig, cur, sizeof(int) * nF, cudaMemcpyDeviceToDevice, st));
-        cudaFreeAsync(tmp, st);
-        cudaFreeAsync(bounds, st);
-        cudaFreeAsync(ord2, st);
-        cudaFreeAsync(keys, st);
-        cudaFreeAsync(keys2, st);
     }
     k_split_small<<<nblk(nF, SPLIT_SMALL), SPLIT_SMALL, 0, st>>>(pbox, nF, Tree<3>::LEAF, S.torig);
     WOS_TRY(cudaGetLastError());
@@ -1241,18 +1259,6 @@ static const GTables &g_tables() {
     return t;
 }
 
-// Temporaries of a build: one allocation, carved up.
-struct Arena {
-    char *base = nullptr;
-    size_t used = 0;
-    template <typename T>
-    T *take(size_t n) {
-        T *p = reinterpret_cast<T *>(base + used);
-        used += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
-        return p;
-    }
-};
-
 static int index_bits(long long n) {
     int b = 1;
     while (b < 32 && (1LL << b) < n) ++b;
@@ -1268,19 +1274,19 @@ static int build_vertex_slots(SceneImpl &S, cudaStream_t st) {
     WOS_TRY(dalloc(&S.vslot, n, st));
     WOS_TRY(dalloc(&S.vfirst, (size_t)S.nV + 1, st));
     cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, S.F, verts, ids, S.vslot, n, 0, bits, st);
-    Arena sizes, A;
-    sizes.take<int>(n);
-    sizes.take<int>(n);
-    sizes.take<char>(tmp_bytes);
-    WOS_TRY(cudaMallocAsync((void **)&A.base, sizes.used, st));
-    ids = A.take<int>(n);
-    verts = A.take<int>(n);
-    void *tmp = A.take<char>(tmp_bytes);
+    void *tmp = nullptr;
+    Arena A(st);
+    for (int pass = 0; pass < 2; ++pass) {
+        A.used = 0;
+        ids = A.take<int>(n);
+        verts = A.take<int>(n);
+        tmp = A.take<char>(tmp_bytes);
+        if (pass == 0) WOS_TRY(cudaMallocAsync((void **)&A.base, A.used, st));
+    }
     k_iota<<<nblk(n, TB), TB, 0, st>>>(ids, n);
     WOS_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, S.F, verts, ids, S.vslot, n, 0, bits, st));
     k_vertex_ranges<<<nblk((long long)n + 1, TB), TB, 0, st>>>(verts, n, S.nV, S.vfirst);
     WOS_TRY(cudaGetLastError());
-    cudaFreeAsync(A.base, st);
     return 0;
 }
 
@@ -1341,7 +1347,7 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
         cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, none, none, nF, 32, 32 + key_bits, st);
     if (nInt > 0) cub::DeviceRadixSort::SortKeys(nullptr, t2, none, none, nInt, 32, 32 + depth_bits, st);
     tmp_bytes = std::max(tmp_bytes, t2);
-    Arena A;
+    Arena A(st);
     int *counters = nullptr, *pint = nullptr, *pleaf = nullptr, *flags = nullptr, *new_of_old = nullptr;
     float *contrib = nullptr, *pbox = nullptr, *nbox = nullptr;
     unsigned long long *mkeys = nullptr, *skeys = nullptr, *dkeys = nullptr, *dkeys2 = nullptr;
@@ -1416,7 +1422,6 @@ static int build_geometry(SceneImpl &S, cudaStream_t st) {
     } else if (new_order) {
         memcpy(S.order_cost, cost, sizeof(cost));
     }
-    cudaFreeAsync(A.base, st);
     auto from_ord = [](int i) {
         int b = i >= 0 ? i : i ^ 0x7fffffff;
         float f;
@@ -1479,13 +1484,13 @@ int SceneImpl::allocate(cudaStream_t st) {
 
 // Checks the faces and decides the primitives' order.
 int SceneImpl::check_indices(cudaStream_t st) {
-    int *out = nullptr;
-    WOS_TRY(dalloc(&out, 2, st));
+    Arena A(st);
+    WOS_TRY(cudaMallocAsync((void **)&A.base, 2 * sizeof(int), st));
+    int *out = A.take<int>(2);
     WOS_TRY(cudaMemsetAsync(out, 0, 2 * sizeof(int), st));
     k_check_indices<<<std::min(nblk(nF, 256), 4096), 256, 0, st>>>(F, nF, dim, nV, out);
     int host[2] = {0, 0};
     WOS_TRY(cudaMemcpyAsync(host, out, sizeof(host), cudaMemcpyDeviceToHost, st));
-    cudaFreeAsync(out, st);
     WOS_TRY(cudaStreamSynchronize(st));
     if (host[0]) return fail(WOS_ERR_INVALID_ARGUMENT, "face index out of range [0, nV)");
     // a polyline of which at least 90 % of the segments follow each other

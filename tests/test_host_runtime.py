@@ -87,3 +87,27 @@ assert L.wos_scene_update_vertices(h, D, None) == 0
 L.wos_scene_destroy(h, None)
 assert fake.fake_live() == 0
 """)
+
+
+@pytest.mark.parametrize("dim,nV,nF", [(2, 500, 500), (3, 50, 1), (3, 3000, 5000)])
+def test_failed_builds_leave_nothing_allocated(fake, dim, nV, nF):
+    """Every call of a scene's making and of a rebuild fails once."""
+    fake(f"""
+fake.fake_fail_at(0)
+rc, scene = create({dim}, {nV}, {nF})
+assert rc == 0
+made, held = fake.fake_calls(), fake.fake_live()
+fake.fake_fail_at(0)
+assert L.wos_scene_update_vertices(scene, D, None) == 0
+moved = fake.fake_calls()
+assert fake.fake_live() == held
+for k in range(1, moved + 1):
+    fake.fake_fail_at(k)
+    assert L.wos_scene_update_vertices(scene, D, None) == _lib.WOS_ERR_CUDA, k
+    assert fake.fake_live() == held, k
+for k in range(1, made + 1):
+    fake.fake_fail_at(k)
+    rc, h = create({dim}, {nV}, {nF})
+    assert rc == _lib.WOS_ERR_CUDA and not h.value, k
+    assert fake.fake_live() == held, k
+""")
