@@ -311,7 +311,7 @@ def batched_line(args, compact=False):
     adj = AdjointSettings(epsilon2=1e-3, clamping=0.1, want_dV=True, want_dg=True, want_dsrc=False)
     plan = wos.BatchPlan(items, adj)
     info = plan.info()
-    # per (dimension, phase) slot; large plans time a prefix of each run
+    # per (dimension, phase) slot; large plans time a prefix of each item
     sample = min(1.0, (0.02 if compact else 0.1) / max(args.scale, 1e-9))
     slot_best, slot_ms = autotune.tune_batch_slots(plan, sample=sample)
     for _ in range(args.warmup):
@@ -399,7 +399,7 @@ def batched_line(args, compact=False):
         "config": {"workload": f"batched_{len(items)}_scenes_scale{args.scale:g}", "scenes": len(items),
                    "points": info["points"], "walks": info["walks"], "nsteps": 64, "epsilon": 1e-3,
                    "loss": "sum over scenes of mean((u - exact)^2); adjoint wrt vertices and values",
-                   "launch": "one persistent kernel per dimension, tree depth and phase, CUDA graph replay",
+                   "launch": "one persistent kernel per dimension and phase, CUDA graph replay",
                    "l2": "256 MiB buffer written between timed steps (L2 flush)"},
         "walks_per_s": info["walks"] / (ms * 1e-3),
         "autotuned_launch": {

@@ -8,6 +8,7 @@
 // captured once into a CUDA graph that later runs replay with a single
 // launch.
 #include <algorithm>
+#include <cmath>
 #include <string>
 #include <vector>
 
@@ -19,17 +20,8 @@ namespace wosd {
 
 static size_t al256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// Consecutive items of a group whose trees have the same depth (the slot tuner
-// times a sample of each).
-struct BatchRun {
-    int depth = 0;
-    int first = 0, count = 0;
-    long long base = 0, walks = 0;
-};
-
 struct BatchGroup {
     int dim = 0;
-    std::vector<BatchRun> runs;
     std::vector<int> user_index;  // item index in the caller's list
     std::vector<BatchItemDev> items;
     std::vector<SceneView> views;
@@ -154,33 +146,56 @@ static int enqueue(wos_batch_s *b, cudaStream_t st) {
     return 0;
 }
 
-// One phase (0 walks, 1 adjoint) of the dimension-dim group alone, over the
-// first `frac` of every run's walks (a prefix of the run's walk range), for
-// the slot tuner.  Needs a full step before it (the adjoint reads the walk
-// phase's records and dL/du); the accumulators it fills are overwritten by
-// the next full step.
-static int enqueue_slot(wos_batch_s *b, int dim, int phase, double frac, cudaStream_t st) {
-    const AdjCfg a = make_adj_cfg(b->adj);
-    for (BatchGroup &g : b->groups) {
-        if (g.dim != dim) continue;
+// What the slot tuner times of a group: the step's own launches over the first points of
+// every item, or over all of them.
+struct BatchPart {
+    BatchItemDev *items = nullptr;  // the items with fewer points; null: the group's own
+    unsigned *order = nullptr;      // their adjoint samples
+    long long walks = 0;
+    cudaStream_t st = nullptr;
+    ~BatchPart() {
+        if (items) cudaFreeAsync(items, st);
+        if (order) cudaFreeAsync(order, st);
+    }
+};
+
+// At least `frac` of the group's walks, and `least`: enough that a launch grabs the same
+// chunk from the queue as the step's.
+static int part_of(const BatchGroup &g, double frac, long long least, BatchPart &p, cudaStream_t st) {
+    p.st = st;
+    p.walks = g.walks;
+    if (g.walks == 0) return 0;
+    frac = std::max(frac, std::min(1.0, (double)least / (double)g.walks));
+    // an order holds 32-bit indices
+    if (!(frac < 1.0) || g.walks > 0xffffffffLL) return 0;
+    std::vector<BatchItemDev> items = g.items;
+    p.walks = 0;
+    for (BatchItemDev &it : items) {
+        it.walk_begin = p.walks;
+        it.n = std::min(it.n, (int)std::ceil(frac * (double)it.n));
+        p.walks += (long long)it.n * it.nwalks;
+    }
+    BT(cudaMallocAsync((void **)&p.items, sizeof(BatchItemDev) * items.size(), st));
+    BT(cudaMemcpyAsync(p.items, items.data(), sizeof(BatchItemDev) * items.size(), cudaMemcpyHostToDevice, st));
+    BT(cudaStreamSynchronize(st));
+    return 0;
+}
+
+// One phase (0 walks, 1 adjoint) of a group alone, over a part of it.  The adjoint reads
+// the records and dL/du of a full step before it, and adds to accumulators that the next
+// step clears; the walks of a part overwrite the records, so it comes first.
+static int enqueue_slot(wos_batch_s *b, BatchGroup &g, int phase, const BatchPart &p, cudaStream_t st) {
+    const int n_items = (int)g.items.size();
+    const BatchLaunch &L = b->slot[g.dim - 2][phase];
+    if (phase == 0) {
         WalkOut o{g.vals, nullptr, b->want_adjoint ? g.wrec : nullptr, b->want_adjoint ? g.wds : nullptr,
                   nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        for (const BatchRun &r : g.runs) {
-            const long long w = std::max(1LL, std::min(r.walks, (long long)(frac * (double)r.walks)));
-            if (phase == 0) {
-                if (int rc = launch_walk_batch(g.dim, r.depth, g.d_views + r.first, g.d_cfgs + r.first,
-                                               g.d_items + r.first, r.count, r.base, w, b->slot[dim - 2][0], o,
-                                               g.counters, st))
-                    return rc;
-            } else if (b->want_adjoint) {
-                if (int rc = launch_adjoint_batch(g.dim, r.depth, g.d_views + r.first, g.d_cfgs + r.first, a,
-                                                  g.d_items + r.first, r.count, r.base, w, g.dLdu, g.wrec, g.wds,
-                                                  g.acc, b->slot[dim - 2][1], g.counters + 1, g.order, st))
-                    return rc;
-            }
-        }
+        return launch_walk_batch(g.dim, g.depth, g.d_views, g.d_cfgs, p.items ? p.items : g.d_items, n_items, 0,
+                                 p.walks, L, o, g.counters, st);
     }
-    return 0;
+    return launch_adjoint_batch(g.dim, g.depth, g.d_views, g.d_cfgs, make_adj_cfg(b->adj), g.d_items, n_items, 0,
+                                p.walks, g.dLdu, g.wrec, g.wds, g.acc, L, g.counters + 1,
+                                p.items ? p.order : g.order, st);
 }
 
 static int capture(wos_batch_s *b) {
@@ -225,8 +240,8 @@ int wos_batch_create(const wos_batch_item *items, int n_items, const wos_adjoint
             delete b;
             return fail(WOS_ERR_INVALID_ARGUMENT, "item " + std::to_string(i) + ": scene is NULL");
         }
-    // within a dimension, items in order of tree depth (then caller order), so
-    // that each depth is one contiguous run of walks for the slot tuner's sample
+    // within a dimension, items in order of tree depth (then caller order): the
+    // lanes of a warp then search trees of like depth
     std::vector<int> order(n_items);
     for (int i = 0; i < n_items; ++i) order[i] = i;
     auto depth = [&](int i) { return items[i].scene->impl.tree_depth; };
@@ -260,15 +275,6 @@ int wos_batch_create(const wos_batch_item *items, int n_items, const wos_adjoint
         d.prim_off = g.nkeys;
         g.nkeys += (long long)S.nF + 1;
         g.depth = std::max(g.depth, S.tree_depth);
-        if (g.runs.empty() || g.runs.back().depth != S.tree_depth) {
-            BatchRun r;
-            r.depth = S.tree_depth;
-            r.first = (int)g.items.size();
-            r.base = g.walks;
-            g.runs.push_back(r);
-        }
-        g.runs.back().count += 1;
-        g.runs.back().walks += (long long)it.n * p.nwalks;
         g.items.push_back(d);
         g.scenes.push_back(it.scene);
         g.views.push_back(S.view());
@@ -442,23 +448,36 @@ int wos_batch_autotune_slots(wos_batch_t b, const int32_t *block_threads, const 
     }
     // one full step first: the adjoint slots read the walk phase's outputs
     int rc = enqueue(b, st);
-    for (int dim = 2; dim <= 3 && !rc; ++dim) {
-        bool present = false;
-        for (const BatchGroup &g : b->groups) present = present || g.dim == dim;
-        if (!present) continue;
-        for (int phase = 0; phase < (b->want_adjoint ? 2 : 1) && !rc; ++phase) {
-            BatchLaunch &L = b->slot[dim - 2][phase];
-            const int k = (dim - 2) * 2 + phase;
+    for (BatchGroup &g : b->groups) {
+        for (int phase = b->want_adjoint ? 1 : 0; phase >= 0 && !rc; --phase) {
+            BatchLaunch &L = b->slot[g.dim - 2][phase];
+            const int k = (g.dim - 2) * 2 + phase;
             int arg = -1;
             float best_ms = INFINITY;
-            for (int i = 0; i < n_candidates && !rc; ++i) {
+            auto shape = [&](int i) {
                 L.block = block_threads[i];
                 L.blocks_per_sm = blocks_per_sm[i];
                 L.chunk = chunk[i];
+            };
+            long long least = 0;
+            for (int i = 0; i < n_candidates; ++i) {
+                shape(i);
+                least = std::max(least, batch_chunk_walks(g.dim, phase, g.depth, g.wds != nullptr, L));
+            }
+            BatchPart part;
+            rc = part_of(g, sample, least, part, st);
+            if (!rc && phase == 1 && part.items != nullptr) {
+                e = cudaMallocAsync((void **)&part.order, sizeof(unsigned) * (size_t)part.walks, st);
+                rc = e != cudaSuccess ? fail_cuda(e, "cudaMallocAsync(part order)")
+                                      : launch_part_order(part.items, g.d_items, (int)g.items.size(), part.walks,
+                                                          g.order, part.order, st);
+            }
+            for (int i = 0; i < n_candidates && !rc; ++i) {
+                shape(i);
                 float t = INFINITY;
                 for (int r = 0; r < repeats && !rc; ++r) {
                     if ((e = cudaEventRecord(e0, st)) != cudaSuccess) rc = fail_cuda(e, "cudaEventRecord");
-                    if (!rc) rc = enqueue_slot(b, dim, phase, sample, st);
+                    if (!rc) rc = enqueue_slot(b, g, phase, part, st);
                     if (!rc && (e = cudaEventRecord(e1, st)) != cudaSuccess) rc = fail_cuda(e, "cudaEventRecord");
                     if (!rc && (e = cudaEventSynchronize(e1)) != cudaSuccess) rc = fail_cuda(e, "cudaEventSynchronize");
                     float x = 0.0f;
@@ -472,11 +491,7 @@ int wos_batch_autotune_slots(wos_batch_t b, const int32_t *block_threads, const 
                     arg = i;
                 }
             }
-            if (arg >= 0) {
-                L.block = block_threads[arg];
-                L.blocks_per_sm = blocks_per_sm[arg];
-                L.chunk = chunk[arg];
-            }
+            if (arg >= 0) shape(arg);
             if (best) best[k] = arg;
         }
     }

@@ -2313,8 +2313,8 @@ __device__ __forceinline__ int find_item_point(const BatchItemDev *__restrict__ 
     return lo;
 }
 
-// One launch covers a run of items whose walks occupy [base, base + total)
-// of the group's walk index space.
+// One launch covers items whose walks occupy [base, base + total) of the group's
+// walk index space.
 template <int D, bool COUNT>
 __global__ void __launch_bounds__(512, 2) k_walk_batch(const SceneView *__restrict__ views,
                                                    const WalkCfg *__restrict__ cfgs,
@@ -2522,6 +2522,40 @@ __global__ void k_batch_record_keys(const SceneView *__restrict__ views, const B
         keys[i] = (code < 0 || prim >= nF) ? (unsigned)(off + nF) : __ldg(&rank[off + prim]);
         ids[i] = (unsigned)i;
     }
+}
+
+__global__ void k_part_order(const BatchItemDev *__restrict__ part, const BatchItemDev *__restrict__ all, int n_items,
+                             long long total, const unsigned *__restrict__ all_order, unsigned *order) {
+    const long long stride = (long long)gridDim.x * blockDim.x;
+    for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < total; k += stride) {
+        const int it = find_item(part, n_items, k);
+        const long long at = __ldg(&all[it].walk_begin) + (k - __ldg(&part[it].walk_begin));
+        order[k] = all_order != nullptr ? __ldg(&all_order[at]) : (unsigned)at;
+    }
+}
+
+int launch_part_order(const BatchItemDev *part, const BatchItemDev *all, int n_items, long long total,
+                      const unsigned *all_order, unsigned *order, cudaStream_t st) {
+    k_part_order<<<(int)std::min<long long>((total + 255) / 256, 148 * 16), 256, 0, st>>>(part, all, n_items, total,
+                                                                                      all_order, order);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return fail_cuda(e, "k_part_order launch");
+    return 0;
+}
+
+template <int D>
+static long long batch_chunk_walks_t(int phase, int depth, bool src, const BatchLaunch &L) {
+    const int stack = tree_stack_entries(depth), block = phase == 0 ? L.block : std::min(L.block, 256);
+    const size_t smem = smem_bytes(-1, block, stack, phase == 0 ? 0 : adj_thread_bytes<D>(src));
+    int grid = 0;
+    const int rc = phase == 0 ? persistent_grid(k_walk_batch<D, false>, block, smem, L.blocks_per_sm, grid)
+                              : persistent_grid(k_adjoint_batch<D, false>, block, smem, L.blocks_per_sm, grid);
+    if (rc) return 0;
+    return 4LL * grid * (block / 32) * (phase == 0 ? L.chunk : std::max(1, L.chunk / 2));
+}
+
+long long batch_chunk_walks(int D, int phase, int depth, bool src, const BatchLaunch &L) {
+    return D == 2 ? batch_chunk_walks_t<2>(phase, depth, src, L) : batch_chunk_walks_t<3>(phase, depth, src, L);
 }
 
 static size_t batch_order_bytes_any_mode(long long nkeys, long long total) {

@@ -89,10 +89,9 @@ struct BatchLaunch {
 WalkCfg make_cfg(const wos_params &p);
 AdjCfg make_adj_cfg(const wos_adjoint_params &a);
 
-// A batch launch covers items [0, n_items) of `items` / `views` / `cfgs`
-// (callers pass pointers offset to a run of items) whose walks are
-// [base, base + total) of the group's walk index space; depth: at least every
-// item's tree depth.
+// A batch launch covers items [0, n_items) of `items` / `views` / `cfgs`, whose
+// walks are [base, base + total) of the group's walk index space; depth: at least
+// every item's tree depth.
 int launch_walk_batch(int D, int depth, const SceneView *views, const WalkCfg *cfgs, const BatchItemDev *items,
                       int n_items, long long base, long long total, const BatchLaunch &L, const WalkOut &out,
                       unsigned long long *counter, cudaStream_t st);
@@ -100,6 +99,14 @@ int launch_adjoint_batch(int D, int depth, const SceneView *views, const WalkCfg
                          const BatchItemDev *items, int n_items, long long base, long long total,
                          const float *dLdu, const int *wrec, const float *wds, double *acc, const BatchLaunch &L,
                          unsigned long long *counter, const unsigned *order, cudaStream_t st);
+// Walks (phase 0) or adjoint samples (1) from which on a launch of shape L grabs its
+// whole chunk from the queue (queue_chunk).  depth as above; src: the adjoint takes
+// source derivatives.  0: the shape does not fit.
+long long batch_chunk_walks(int D, int phase, int depth, bool src, const BatchLaunch &L);
+// For a launch over a part of a group: order[k], k in [0, total), the sample (or, all
+// null, the walk) at the place in its item of `all` that k has in that of `part`.
+int launch_part_order(const BatchItemDev *part, const BatchItemDev *all, int n_items, long long total,
+                      const unsigned *all_order, unsigned *order, cudaStream_t st);
 // Sample order of a batch group's adjoint (see launch_record_order): nkeys =
 // sum of nF + 1 over the group's items; 0 bytes: no order for this size.
 size_t batch_order_bytes(long long nkeys, long long total);

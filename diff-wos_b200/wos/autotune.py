@@ -97,7 +97,7 @@ def tune_batch(plan, candidates=None, repeats: int = 1):
 
 def tune_batch_slots(plan, candidates=None, repeats: int = 1, sample: float = 1.0):
     """Pick a launch shape per (dimension, phase) slot of a BatchPlan by
-    timing each slot's launches alone (wos_batch_autotune_slots): block size,
+    timing each slot's launch alone (wos_batch_autotune_slots): block size,
     resident blocks per SM and walks per queue grab.  `sample` < 1 times a
-    prefix of each run's walks, for large plans."""
+    prefix of each item's points, for large plans."""
     return plan.autotune_slots(candidates or SLOT_CANDIDATES, repeats, sample)

@@ -64,9 +64,10 @@ class BatchPlan:
         return cands[best.value], {c: float(ms[i]) for i, c in enumerate(cands)}
 
     def autotune_slots(self, candidates, repeats: int = 1, sample: float = 1.0):
-        """Per (dimension, phase) slot, time that slot's launches alone on the
-        first `sample` fraction of its walks for each (block_threads,
-        blocks_per_sm, chunk) candidate and keep the fastest
+        """Per (dimension, phase) slot, time that slot's launch alone on the
+        first `sample` fraction of every item's points (or more, where the
+        chunks need it) for each (block_threads, blocks_per_sm, chunk)
+        candidate and keep the fastest
         (wos_batch_autotune_slots).  Returns ({slot: best candidate},
         {slot: {candidate: ms}}) for the slots present, slot = (dim, phase)."""
         n = len(candidates)

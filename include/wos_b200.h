@@ -440,9 +440,10 @@ WOS_API int wos_batch_autotune(wos_batch_t b, const int32_t *block_threads, cons
 
 /* Slot-wise launch-shape tuner: the plan keeps one launch shape per slot
  * (dimension 2 or 3 x phase: walks, adjoint); after one full step it times,
- * for each slot present, that slot's launches alone over the first `sample`
- * fraction (0 < sample <= 1) of every run's walks for each candidate
- * (block_threads[i], blocks_per_sm[i] (0 = occupancy limit), chunk[i]) --
+ * for each slot present, that slot's launch alone over the first `sample`
+ * fraction (0 < sample <= 1) of every item's points, or as many more as the
+ * largest candidate needs for its chunk to be what the step would grab, for each
+ * candidate (block_threads[i], blocks_per_sm[i] (0 = occupancy limit), chunk[i]) --
  * the best of `repeats` -- and keeps the fastest for that slot.  ms
  * (4 x n_candidates floats, slot k = (dim - 2) * 2 + phase; NaN for absent
  * slots) and best (4 indices, -1 for absent slots) may be NULL.  Results do
@@ -510,8 +511,9 @@ WOS_API int wos_solve_noalloc(wos_scene_t scene, const float *P, int n, const wo
 /* ---------------------------------------------------------------- kernels */
 
 /* Launch shape of the persistent walk kernels: threads per block, blocks per
- * SM (0 = occupancy limit), walks taken per queue grab, LBVH nodes staged in
- * shared memory per block.  In wos_set_launch_config, block_threads = 0,
+ * SM (0 = occupancy limit), walks taken per queue grab (at most: a call with
+ * fewer than four grabs for each warp takes smaller ones; adjoint samples half of
+ * it), and smem_nodes, which is kept but has no effect.  In wos_set_launch_config, block_threads = 0,
  * chunk = 0, blocks_per_sm < 0 and smem_nodes < 0 keep the current value. */
 typedef struct wos_launch_config {
     int32_t block_threads;

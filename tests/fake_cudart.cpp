@@ -5,6 +5,8 @@
 // allocated, and at the shared-memory limits that the launches were given.
 #include <cstring>
 #include <map>
+#include <string>
+#include <vector>
 
 #include <cuda_runtime_api.h>
 
@@ -13,6 +15,10 @@ std::map<const void *, size_t> live;
 std::map<const void *, int> smem_limit;
 long long calls = 0, fail_at = 0;
 int lowered = 0, refused = 0, launches = 0;
+std::map<const void *, std::string> names;
+std::string watched;
+int watched_arg = 0;
+std::vector<int> seen;
 char *next_address = (char *)(1ull << 40);
 
 // The n-th call that can fail (fake_fail_at) does.
@@ -32,6 +38,13 @@ long long fake_calls() { return calls; }
 int fake_lowered() { return lowered; }
 int fake_refused() { return refused; }
 int fake_launches() { return launches; }
+// From here on, note the arg-th (an int) of every launch of a kernel named `name`.
+void fake_watch(const char *name, int arg) {
+    watched = name;
+    watched_arg = arg;
+    seen.clear();
+}
+int fake_seen(int i) { return i < (int)seen.size() ? seen[i] : -1; }
 void fake_fail_at(long long n) {
     calls = 0;
     fail_at = n;
@@ -60,7 +73,8 @@ cudaError_t cudaFuncSetAttribute(const void *f, cudaFuncAttribute a, int v) {
     limit = v;
     return cudaSuccess;
 }
-cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **, size_t smem, cudaStream_t) {
+cudaError_t cudaLaunchKernel(const void *f, dim3, dim3, void **args, size_t smem, cudaStream_t) {
+    if (!watched.empty() && names[f].find(watched) != std::string::npos) seen.push_back(*(int *)args[watched_arg]);
     const auto i = smem_limit.find(f);
     const size_t limit = i == smem_limit.end() || i->second < 48 * 1024 ? 48 * 1024 : (size_t)i->second;
     ++launches;
@@ -137,6 +151,8 @@ void **__cudaRegisterFatBinary(void *) {
 }
 void __cudaRegisterFatBinaryEnd(void **) {}
 void __cudaUnregisterFatBinary(void **) {}
-void __cudaRegisterFunction(void **, const char *, char *, const char *, int, void *, void *, void *, void *, int *) {}
+void __cudaRegisterFunction(void **, const char *f, char *, const char *name, int, void *, void *, void *, void *, int *) {
+    names[f] = name;
+}
 void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, int) {}
 }

@@ -111,3 +111,33 @@ for k in range(1, made + 1):
     assert rc == _lib.WOS_ERR_CUDA and not h.value, k
     assert fake.fake_live() == held, k
 """)
+
+
+@pytest.mark.parametrize("sample", [1.0, 0.001])
+def test_slot_tuner_times_the_launches_of_a_step(fake, sample):
+    """One launch per phase over the items of every depth, and the chunk that the step
+    would grab with the candidate."""
+    fake(f"""
+scenes = [create(3, 1000, nF)[1] for nF in (80, 5000, 80000)]
+big = _lib.WosParams(256, 32, 1e-3, 0, 0, 0, 0, 0, 1, 0, 0)
+item = (_lib.WosBatchItem * 3)(*[_lib.WosBatchItem(h.value, D.value, 100000, 1, None, big) for h in scenes])
+plan = ctypes.c_void_p()
+assert L.wos_batch_create(item, 3, ctypes.byref(adjoint), 1, None, ctypes.byref(plan)) == 0
+held = fake.fake_live()
+shapes = [(256, 0, 16), (256, 0, 64), (256, 0, 128), (512, 2, 128)]
+arr = [(ctypes.c_int32 * 4)(*v) for v in zip(*shapes)]
+for kernel, arg, slot in (("k_walk_batch", 7, (3, 0)), ("k_adjoint_batch", 9, (3, 1))):
+    step = []
+    for s in shapes:
+        assert L.wos_batch_set_launch_slot(plan, *slot, *s) == 0
+        fake.fake_watch(kernel.encode(), arg)
+        assert L.wos_batch_run(plan, 0, None) == 0
+        assert fake.fake_seen(1) == -1
+        step.append(fake.fake_seen(0))
+    assert len(set(step)) > 2
+    fake.fake_watch(kernel.encode(), arg)
+    assert L.wos_batch_autotune_slots(plan, *arr, 4, 1, {sample}, None, None, None) == 0
+    tuned = [fake.fake_seen(i) for i in range(1, 6)]  # after the full step's
+    assert tuned == step + [-1], (tuned, step)
+assert fake.fake_live() == held
+""")
