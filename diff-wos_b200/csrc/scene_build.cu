@@ -1013,8 +1013,7 @@ __global__ void __launch_bounds__(128, 4) k_entry_grid(SceneView S, const int *l
     }
     const float h = 0.5005f * sqrtf(h2) * unit + 1e-6f * ext_max + 1e-6f * abs_max + TOL_MIN;
     const float e = (1.0f + 0.5f * D) * 0x1.02p-20f * ext_max + TOL_MIN;  // prune_tol's largest in the box
-    const float tol = D == 2 ? e : 1025.0f * (e * e);
-    auto widen = [&](float d) { return sqrtf(search_bound<D>((d * d) * (1.0f + 0x1p-20f), tol)); };
+    auto widen = [&](float d) { return sqrtf(search_bound<D>((d * d) * (1.0f + 0x1p-20f), search_tol<D>(e))); };
 
     auto distances = [&](unsigned block, float *dd) {
         block_distances<D>(S.tree + (size_t)block * Tree<D>::NODE_W, x, dd);

@@ -323,10 +323,10 @@ struct ManyScenes {
 };
 
 // The search of every lane with sr.dep == SEARCH_NEED begun, and the warp's
-// searches run on.  Brute force completes at once.
-template <int D, bool BVH, bool GATHER, class CTX, class WK>
+// searches run on (few: by search_few).  Brute force completes at once.
+template <int D, bool BVH, bool GATHER, bool SHARE = false, class CTX, class WK>
 __device__ __forceinline__ void lane_search(Search<D> &sr, const CTX &x, int item, const float *p, int warm,
-                                            float ball_m, unsigned *stack, WK &work) {
+                                            float ball_m, unsigned *stack, WK &work, bool few = false) {
     if (sr.dep == SEARCH_NEED) {
         if (BVH) {
             work.nq += 1;
@@ -339,9 +339,17 @@ __device__ __forceinline__ void lane_search(Search<D> &sr, const CTX &x, int ite
         }
     }
     if (BVH) {
-        const int n = __popc(__ballot_sync(0xffffffffu, sr.dep >= 0));
-        search_run<D, GATHER, CTX::MULTI>(sr, x.scenes(), item, p, stack, search_keep<D>(n), work);
+        const int keep = search_keep<D>(__popc(__ballot_sync(0xffffffffu, sr.dep >= 0)));
+        if (SHARE)
+            search_few<D, GATHER, CTX::MULTI>(sr, x.scenes(), item, p, stack, keep, few, work);
+        else
+            search_run<D, GATHER, CTX::MULTI>(sr, x.scenes(), item, p, stack, keep, work);
     }
+}
+
+// Whether the queue is empty and most of the warp's lanes are done (search_few).
+__device__ __forceinline__ bool few_left(const Queue &q, bool active) {
+    return q.drained && __popc(__ballot_sync(0xffffffffu, active)) <= FEW_LANES;
 }
 
 // Its hit (ball_m as in search_hit).
@@ -576,9 +584,10 @@ __global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const fl
         if (BVH) {
             const unsigned run = __ballot_sync(0xffffffffu, sr.dep >= 0);
             if (run != 0u && __popc(run) <= SHARE_LANES && !__any_sync(0xffffffffu, i + stride < n)) {
-                search_run<D, true, false, SHARE_STEPS>(sr, &S, 0, p, stack, 0, work);
+                for (int it = 0; it < SHARE_STEPS && search_step<D, true>(sr, S, p, stack, 0, work); ++it) {
+                }
                 for (unsigned left = __ballot_sync(0xffffffffu, sr.dep >= 0); left != 0u; left &= left - 1u)
-                    search_share<D>(sr, S, p, __ffs(left) - 1, stack);
+                    search_share<D, true>(sr, S, p, __ffs(left) - 1, stack, work);
             }
         }
         if (i >= n || sr.dep >= 0) continue;
@@ -990,7 +999,7 @@ __device__ __forceinline__ double sample_weight(const CTX &x, const float *dLdu,
 // 81,920 triangles 32.1, 32.4, 32.7, 34.0.
 // Bisection steps at 1/5: 32.6 there, at 1/12 31.8; walk steps at 1/6 or 1/3: within
 // 2 % everywhere.
-template <int D, bool BVH, int MODE, class CTX, class WK>
+template <int D, bool BVH, int MODE, bool SHARE, class CTX, class WK>
 __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, long long idx0, long long total,
                                               const float *__restrict__ dLdu, unsigned long long *counter, int chunk,
                                               const AdjOut &out, const unsigned short *guide, unsigned *stack,
@@ -1302,7 +1311,8 @@ __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, lon
         const int dep = sr.dep;
         if (hold) sr.dep = SEARCH_DONE;
         const bool walking = phase == PH_ANTI_WALK || (HAS_PRIMAL && phase == PH_PRIMAL);
-        lane_search<D, BVH, false>(sr, x, item, w.p, walking ? w.last : rprim, ball_m, stack, work);
+        lane_search<D, BVH, false, SHARE>(sr, x, item, w.p, walking ? w.last : rprim, ball_m, stack, work,
+                                          SHARE && few_left(q, active));
         if (hold) sr.dep = dep;
     }
     if constexpr (CTX::MULTI) {
@@ -1314,7 +1324,7 @@ __device__ __forceinline__ void adjoint_lanes(const CTX &x, const AdjCfg &a, lon
     }
 }
 
-template <int D, bool BVH, int MODE, bool COUNT>
+template <int D, bool BVH, int MODE, bool COUNT, bool SHARE>
 __global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint(SceneView S, WalkCfg c, AdjCfg a,
                                                 const float *__restrict__ P,
                                                 long long total, const float *__restrict__ dLdu,
@@ -1330,7 +1340,7 @@ __global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint(SceneView S, Wa
         for (int k = 0; k < 5; ++k) am.acc[k * blockDim.x] = 0.0;
     }
     typename std::conditional<COUNT, Work, NoWork>::type work{};
-    adjoint_lanes<D, BVH, MODE>(OneScene<D>{S, c, P}, a, 0, total, dLdu, counter, chunk, out, sm.guide, sm.stack,
+    adjoint_lanes<D, BVH, MODE, SHARE>(OneScene<D>{S, c, P}, a, 0, total, dLdu, counter, chunk, out, sm.guide, sm.stack,
                                 *am.slot, want_src ? am.acc : nullptr, work);
     if constexpr (COUNT) flush_work(work);
     if (want_src && MODE != ADJ_TANGENT) {
@@ -2141,23 +2151,41 @@ int launch_ball(const SceneImpl &S, const uint8_t *valid, const float *pt, const
     return 0;
 }
 
-template <int D, bool BVH, int ND, bool COUNT>
+// Whether an adjoint launch of `total` samples over grid x block lanes runs the instance
+// whose warps share their last searches (search_few): in 3D, from trees of 6 levels (2,049
+// triangles) on, for up to one sample a lane there and one more with each level.  Below
+// 2,049 triangles no search is long enough; with more samples fewer warps run dry and
+// the instance's larger loop costs more than it gives.
+//   Samples on a sphere of 81,920 triangles, 1,000, 20,000, 150,000, 400,000, ms without
+// and with: 14.5 and 1.9, 17.2 and 4.5, 25.7 and 8.7, 33.1 and 17.0; on one displaced in
+// waves by 15 %: 1.47 and 1.37, 4.04 and 4.11, 6.93 and 7.02, 12.9 and 13.1.  On 5,120
+// triangles, 20,000 and 150,000: 4.55 and 2.41, 6.94 and 4.28; in waves 2.50 and 2.57,
+// 4.44 and 4.54 (400,000: 8.73 and 9.14).  On 1,280, 150,000 in waves: 3.70 and 3.80.
+template <int D, bool BVH, bool COUNT>
+constexpr bool can_share() {
+    return D == 3 && BVH && !COUNT;
+}
+static bool share_searches(long long total, int depth, int grid, int block) {
+    return total <= (long long)(depth - 5) * grid * block;
+}
+
+template <int D, bool BVH, int ND, bool COUNT, bool SHARE = false>
 static int launch_adjoint_t(const SceneImpl &S, const float *P, long long total, const wos_params &p,
                             const AdjCfg &a, const float *dLdu, const AdjOut &out, unsigned long long *counter,
                             cudaStream_t st) {
-    const SceneView v = S.view();
-    const WalkCfg c = make_cfg(p);
+    const auto kern = k_adjoint<D, BVH, ND, COUNT, SHARE>;
     const bool want_cdf = D == 2 && S.src_type != 0 && p.use_IS_for_greens;
-    Shape sh;
     const bool want_acc = ND != ADJ_ND_ONLY && a.want_dsrc && p.include_source && S.src_type != 0 && D == 2;
-    int rc = shape_for(k_adjoint<D, BVH, ND, COUNT>, S, D, BVH, want_cdf, sh, adj_thread_bytes<D>(want_acc),
-                       256);
-    if (rc) return rc;
+    Shape sh;
+    if (int rc = shape_for(kern, S, D, BVH, want_cdf, sh, adj_thread_bytes<D>(want_acc), 256)) return rc;
+    if constexpr (can_share<D, BVH, COUNT>() && !SHARE)
+        if (share_searches(total, S.tree_depth, sh.grid, sh.block))
+            return launch_adjoint_t<D, BVH, ND, COUNT, true>(S, P, total, p, a, dLdu, out, counter, st);
     cudaError_t e = cudaMemsetAsync(counter, 0, sizeof(unsigned long long), st);
     if (e != cudaSuccess) return fail_cuda(e, "cudaMemsetAsync(counter)");
     const int chunk = queue_chunk(std::max(1, g_cfg[D - 2].chunk / 2), total, sh.grid, sh.block);
-    k_adjoint<D, BVH, ND, COUNT><<<sh.grid, sh.block, sh.smem, st>>>(v, c, a, P, total, dLdu, counter, chunk,
-                                                                         sh.stack, sh.stage_cdf, out);
+    kern<<<sh.grid, sh.block, sh.smem, st>>>(S.view(), make_cfg(p), a, P, total, dLdu, counter, chunk, sh.stack,
+                                             sh.stage_cdf, out);
     e = cudaGetLastError();
     if (e != cudaSuccess) return fail_cuda(e, "k_adjoint launch");
     return 0;
@@ -2382,7 +2410,7 @@ __global__ void k_loss_batch(const double *__restrict__ mean, const BatchItemDev
 
 // Adjoint of every item, starting from the forward records (out.wrec, out.wds).
 // Gradients go to per-item FP64 accumulators (out.dV + dV_off / dg_off / ds_off).
-template <int D, bool COUNT>
+template <int D, bool COUNT, bool SHARE>
 __global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint_batch(
     const SceneView *__restrict__ views, const WalkCfg *__restrict__ cfgs, AdjCfg a,
     const BatchItemDev *__restrict__ items, int n_items, long long base, long long total,
@@ -2398,7 +2426,7 @@ __global__ void __launch_bounds__(256, ADJ_MIN_BLOCKS) k_adjoint_batch(
         for (int k = 0; k < 5; ++k) am.acc[k * blockDim.x] = 0.0;
     }
     typename std::conditional<COUNT, Work, NoWork>::type work{};
-    adjoint_lanes<D, true, ADJ_FROM_RECORDS>(ManyScenes<D>{views, cfgs, items, n_items}, a, base, total, dLdu,
+    adjoint_lanes<D, true, ADJ_FROM_RECORDS, SHARE>(ManyScenes<D>{views, cfgs, items, n_items}, a, base, total, dLdu,
                                              counter, chunk, out, views[0].guide, stack + threadIdx.x, *am.slot,
                                              acc_on ? am.acc : nullptr, work);
     if constexpr (COUNT) flush_work(work);
@@ -2459,7 +2487,7 @@ int launch_walk_batch(int D, int depth, const SceneView *views, const WalkCfg *c
     return 0;
 }
 
-template <int D, bool COUNT>
+template <int D, bool COUNT, bool SHARE = false>
 static int launch_adjoint_batch_t(int stack, const SceneView *views, const WalkCfg *cfgs, const AdjCfg &a,
                                   const BatchItemDev *items, int n_items, long long base, long long total,
                                   const float *dLdu, const int *wrec, const float *wds, double *acc,
@@ -2468,15 +2496,19 @@ static int launch_adjoint_batch_t(int stack, const SceneView *views, const WalkC
     const int block = std::min(L.block, 256);
     const size_t smem = smem_bytes(-1, block, stack, adj_thread_bytes<D>(wds != nullptr));
     int grid = 0;
-    if (int rc = persistent_grid(k_adjoint_batch<D, COUNT>, block, smem, L.blocks_per_sm, grid)) return rc;
+    const auto kern = k_adjoint_batch<D, COUNT, SHARE>;
+    if (int rc = persistent_grid(kern, block, smem, L.blocks_per_sm, grid)) return rc;
+    if constexpr (can_share<D, true, COUNT>() && !SHARE)
+        if (share_searches(total, stack / tree_stack_entries(1), grid, block))
+            return launch_adjoint_batch_t<D, COUNT, true>(stack, views, cfgs, a, items, n_items, base, total, dLdu,
+                                                          wrec, wds, acc, L, counter, order, st);
     const int chunk = queue_chunk(std::max(1, L.chunk / 2), total, grid, block);
     AdjOut out{};
     out.dV = acc;
     out.wrec = wrec;
     out.wds = wds;
     out.order = order;
-    k_adjoint_batch<D, COUNT><<<grid, block, smem, st>>>(views, cfgs, a, items, n_items, base, total, dLdu, counter,
-                                                         chunk, out, stack);
+    kern<<<grid, block, smem, st>>>(views, cfgs, a, items, n_items, base, total, dLdu, counter, chunk, out, stack);
     return 0;
 }
 
@@ -2549,7 +2581,7 @@ static long long batch_chunk_walks_t(int phase, int depth, bool src, const Batch
     const size_t smem = smem_bytes(-1, block, stack, phase == 0 ? 0 : adj_thread_bytes<D>(src));
     int grid = 0;
     const int rc = phase == 0 ? persistent_grid(k_walk_batch<D, false>, block, smem, L.blocks_per_sm, grid)
-                              : persistent_grid(k_adjoint_batch<D, false>, block, smem, L.blocks_per_sm, grid);
+                              : persistent_grid(k_adjoint_batch<D, false, false>, block, smem, L.blocks_per_sm, grid);
     if (rc) return 0;
     return 4LL * grid * (block / 32) * (phase == 0 ? L.chunk : std::max(1, L.chunk / 2));
 }

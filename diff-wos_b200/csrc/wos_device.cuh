@@ -8,6 +8,7 @@
 
 #include <cuda_runtime.h>
 #include <float.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include "wos_math.h"
@@ -342,9 +343,9 @@ struct NoWork {
     NoCount nq, nb, np;
 };
 
-// Pruning slack: a box is skipped only when its squared distance exceeds (1 + 2^-10)
-// best + 1025 (s 2^-20)^2 (2D searches: search_bound), where s bounds the coordinates'
-// magnitude around the scene.  s 2^-20 is at least 1e-22, whose square is 7 steps of the
+// Pruning slack of the LBVH: a box is skipped only when its squared distance exceeds
+// (1 + 2^-10) best + 1025 (s 2^-20)^2, where s bounds the coordinates' magnitude around
+// the scene (the search tree's: search_bound).  s 2^-20 is at least 1e-22, whose square is 7 steps of the
 // denormal floats: squared distances that small are only exact to a few steps.
 constexpr float TOL_MIN = 1e-22f;
 template <int D>
@@ -601,22 +602,30 @@ struct Search {
 enum { SEARCH_DONE = -1, SEARCH_NEED = -2 };  // no node left; no search begun
 
 // Pruning bound: a node farther than this (squared) holds no primitive whose
-// computed squared distance is below `best`.  Clamped to the largest float:
-// infinitely far boxes are never visited, even before a first candidate.
-// 3D: prune_bound, with tol = prune_tol2.  2D: (d (1 + 2^-18) + tol)^2 with d =
-// sqrt(best) and tol = prune_tol: a segment's computed distance is that of a point
-// on the segment up to 2^-23 of itself and 2^-24 of the segment's length, and a
-// box's computed bound exceeds the true one by at most 2^-20 of itself.  (The
-// squared form's 2^-10 costs a third more leaves: arcs a thousandth farther
-// than the nearest are many.  In 3D the barycentric coordinates of needle
-// triangles are far less exact, and it gains little there.)
+// computed squared distance is below `best`: at least (d (1 + 2^-18) + e)^2 with d =
+// sqrt(best) and e = prune_tol.  A computed distance is that of a point of the
+// primitive -- whichever: a needle triangle's is often not its closest -- up to 2^-24
+// of itself and of the primitive's length (at most 0.06 e: 96 million random triangles
+// as large as the scene, aspects 1 to 1e-7, points near to 30 lengths away), and a box's
+// computed bound exceeds the true one by at most 2^-20 of itself.
+//   2D: just that, tol = e.  (A slack of 2^-10 in the squared distance costs a third more
+// leaves: arcs a thousandth farther than the nearest are many.)  3D: without the root,
+// best (1 + 2^-12) + tol with tol = 4300 e^2 (2 d e <= t d^2 + e^2 / t).  (With 2^-10
+// a query near a sphere's centre visits a large part of the sphere.)
+// Clamped to the largest float: infinitely far boxes are never visited, even before a
+// first candidate.
+template <int D>
+__device__ __forceinline__ float search_tol(float e) {
+    return D == 2 ? e : 4300.0f * (e * e);
+}
+__device__ __forceinline__ float search_bound2(float d, float e) {
+    const float r = fmaf(d, 1.0f + 0x1p-18f, e);
+    return fminf((r * r) * (1.0f + 0x1p-22f), FLT_MAX);
+}
 template <int D>
 __device__ __forceinline__ float search_bound(float best, float tol) {
-    if constexpr (D == 2) {
-        const float r = fmaf(sqrtf(best), 1.0f + 0x1p-18f, tol);
-        return fminf((r * r) * (1.0f + 0x1p-22f), FLT_MAX);
-    }
-    return fminf(prune_bound(best, tol), FLT_MAX);
+    if constexpr (D == 2) return search_bound2(sqrtf(best), tol);
+    return fminf(fmaf(best, 1.0f + 0x1p-12f, tol), FLT_MAX);
 }
 
 // Squared distance to an oriented box, a lower bound for its primitives.  With
@@ -827,10 +836,12 @@ __device__ __forceinline__ void search_cell(Search<D> &s, const SceneView &S, un
 template <int D, bool GATHER, class WK>
 __device__ __forceinline__ void search_begin(Search<D> &s, const SceneView &S, const float *q, int warm,
                                              float ball_m, unsigned *stack, WK &wk) {
-    s.tol = D == 2 ? prune_tol<D>(S, q) : prune_tol2<D>(S, q);
+    const float e = prune_tol<D>(S, q);
+    s.tol = search_tol<D>(e);
     s.stop = -1.0f;
     if (ball_m > 0.0f) {
-        s.bound = search_bound<D>((ball_m * ball_m) * (1.0f + 0x1p-20f), s.tol);
+        // a blocking primitive is nearer than m - 1e-5 (ball_blocks)
+        s.bound = search_bound2(fmaxf(ball_m - 0.99e-5f, 0.0f) * (1.0f + 0x1p-20f), e);
         // blocking is monotone in the distance: if `stop` blocks, whatever is
         // nearer does
         const float t = ball_m - 1.1e-5f;
@@ -905,27 +916,34 @@ __device__ __forceinline__ void search_leaf(Search<D> &s, const SceneView &S, co
     search_pop(s, S, q, stack);
 }
 
+// One step of the searches of a warp's lanes, unless at most `keep` of them still have a
+// node to visit: then false.  S: the lane's scene.  Called by all 32 lanes.
+template <int D, bool GATHER, class WK>
+__device__ __forceinline__ bool search_step(Search<D> &s, const SceneView &S, const float *q, unsigned *stack,
+                                            int keep, WK &wk) {
+    const unsigned FULL = 0xffffffffu;
+    const bool run = s.dep >= 0, leaf = run && s.dep == S.tree_depth;
+    const int nr = __popc(__ballot_sync(FULL, run)), nl = __popc(__ballot_sync(FULL, leaf));
+    if (nr <= keep) return false;
+    if (2 * nl > nr) {
+        if (leaf) {
+            wk.np += 1;
+            search_leaf<D>(s, S, q, stack);
+        }
+    } else if (run && !leaf) {
+        wk.nb += 1;
+        search_node<D, GATHER>(s, S, q, stack);
+    }
+    return true;
+}
+
 // Run the searches of a warp's lanes until at most `keep` of them still have a
-// node to visit, or for STEPS steps (0: without end).  scenes[MULTI ? item : 0] is
-// the lane's scene.  Must be called by all 32 lanes.
-template <int D, bool GATHER, bool MULTI, int STEPS = 0, class WK>
+// node to visit.  scenes[MULTI ? item : 0] is the lane's scene.
+template <int D, bool GATHER, bool MULTI, class WK>
 __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes, int item, const float *q,
                                            unsigned *stack, int keep, WK &wk) {
-    const unsigned FULL = 0xffffffffu;
     const SceneView &S = scenes[MULTI ? item : 0];
-    for (int it = 0; STEPS == 0 || it < STEPS; it += STEPS != 0) {
-        const bool run = s.dep >= 0, leaf = run && s.dep == S.tree_depth;
-        const int nr = __popc(__ballot_sync(FULL, run)), nl = __popc(__ballot_sync(FULL, leaf));
-        if (nr <= keep) return;
-        if (2 * nl > nr) {
-            if (leaf) {
-                wk.np += 1;
-                search_leaf<D>(s, S, q, stack);
-            }
-        } else if (run && !leaf) {
-            wk.nb += 1;
-            search_node<D, GATHER>(s, S, q, stack);
-        }
+    while (search_step<D, GATHER>(s, S, q, stack, keep, wk)) {
     }
 }
 
@@ -933,16 +951,16 @@ __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes
 // each descends from a node of its own and they share the bound.  Per round, a lane
 // with nothing left takes over the lowest -- so nearest to the root -- stack entry
 // of the lane it is paired with, where that has one; the entry left behind is
-// GRID_NONE, which a pop passes over.  For nearest searches only (not ball_m), and
-// called by all 32 lanes.
+// GRID_NONE, which a pop passes over.  A ball search ends for all when one has found a
+// primitive at `stop` or nearer.  S: the owner's scene; called by all 32 lanes.
 //
 // What it is for: a query at about the same distance from much of a mesh visits
 // thousands of nodes one after the other, long after its warp's others are done.
 // 10,007 points on a mesh of 81,920 triangles, which it has just been moved to: 0.83
 // -> 0.69 ms with the rebuild.
-template <int D>
+template <int D, bool GATHER, class WK>
 __device__ __forceinline__ void search_share(Search<D> &s, const SceneView &S, const float *p, int owner,
-                                             unsigned *stack) {
+                                             unsigned *stack, WK &wk) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const bool helps = lane == owner || s.dep < 0;
@@ -952,7 +970,7 @@ __device__ __forceinline__ void search_share(Search<D> &s, const SceneView &S, c
     Search<D> t;
     t.tol = __shfl_sync(FULL, s.tol, owner);
     t.bound = __shfl_sync(FULL, s.bound, owner);
-    t.stop = -1.0f;
+    t.stop = __shfl_sync(FULL, s.stop, owner);
     t.d2 = lane == owner ? s.d2 : INFINITY;
     t.pos = lane == owner ? s.pos : -1;
     t.idx = lane == owner ? s.idx : 0u;
@@ -992,11 +1010,16 @@ __device__ __forceinline__ void search_share(Search<D> &s, const SceneView &S, c
         const bool on = t.dep >= 0, leaf = on && t.dep == S.tree_depth;
         const int nr = __popc(__ballot_sync(FULL, on)), nl = __popc(__ballot_sync(FULL, leaf));
         if (2 * nl > nr) {
-            if (leaf) search_leaf<D>(t, S, q, stack);
+            if (leaf) {
+                wk.np += 1;
+                search_leaf<D>(t, S, q, stack);
+            }
         } else if (on && !leaf) {
-            search_node<D, true>(t, S, q, stack);
+            wk.nb += 1;
+            search_node<D, GATHER>(t, S, q, stack);
         }
         t.bound = __uint_as_float(__reduce_min_sync(FULL, __float_as_uint(t.bound)));
+        if (__any_sync(FULL, t.d2 <= t.stop)) break;
     }
     // the lowest original index at the least distance
     const unsigned best = __reduce_min_sync(FULL, __float_as_uint(t.d2));
@@ -1010,6 +1033,34 @@ __device__ __forceinline__ void search_share(Search<D> &s, const SceneView &S, c
         s.pos = who != 0u ? pos : -1;
         s.dep = SEARCH_DONE;
         s.sp = 0;
+    }
+}
+
+// search_run for a warp most of whose lanes may have nothing left to do (few): then, a
+// few dozen steps on, the searches that are left, where they are more than `keep`, are
+// shared.
+//
+// What it is for: an adjoint with fewer samples than lanes, and the end of any, lasts as
+// long as its longest chain of searches, and balls that touch a mesh in much of it (the
+// last bisection steps in a sphere) visit thousands of nodes each.  1,000 samples on a
+// sphere of 81,920 triangles: 14.5 ms without sharing, 1.9 with it.  The lanes' limit and
+// pace (8 and 1) hardly matter: 4 or 8 lanes, half or a quarter of the pace within 3 %; 2
+// lanes take twice as long on a sphere with 30,000 samples, 16 lanes 10 % longer.
+constexpr int FEW_LANES = 8, FEW_MORE = 1;
+template <int D, bool GATHER, bool MULTI, class WK>
+__device__ __forceinline__ void search_few(Search<D> &s, const SceneView *scenes, int item, const float *p,
+                                           unsigned *stack, int keep, bool few, WK &wk) {
+    const unsigned FULL = 0xffffffffu;
+    // few: a lane more may be left every 32 / FEW_MORE steps
+    const int more = few ? FEW_MORE : 0;
+    for (int k = 32 * keep; search_step<D, GATHER>(s, scenes[MULTI ? item : 0], p, stack, k >> 5, wk); k += more) {
+    }
+    if (!few) return;
+    unsigned left = __ballot_sync(FULL, s.dep >= 0);
+    if (__popc(left) <= keep) return;
+    for (; left != 0u; left &= left - 1u) {
+        const int owner = __ffs(left) - 1;
+        search_share<D, GATHER>(s, scenes[MULTI ? __shfl_sync(FULL, item, owner) : 0], p, owner, stack, wk);
     }
 }
 
