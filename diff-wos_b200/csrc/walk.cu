@@ -469,9 +469,10 @@ __device__ __forceinline__ void walk_lanes(const CTX &x, long long idx0, long lo
 }
 
 // COUNT: the instance that keeps work counters (launched while work
-// accounting is on); the others carry none.
+// accounting is on); the others carry none.  Brute force has 128 registers for the loads
+// that it keeps in flight: one walk on 8,192 segments 2.36 ms, 3.14 with 64.
 template <int D, bool BVH, bool RECORDS, bool COUNT>
-__global__ void __launch_bounds__(512, 2) k_walk(SceneView S, WalkCfg c, const float *__restrict__ P, long long total,
+__global__ void __launch_bounds__(512, BVH ? 2 : 1) k_walk(SceneView S, WalkCfg c, const float *__restrict__ P, long long total,
                                              unsigned long long *counter, int chunk, int stack_entries, int stage_cdf,
                                              WalkOut out) {
     extern __shared__ float4 smem[];
