@@ -57,8 +57,8 @@ int read_work(int reset, unsigned long long *out) {
 }
 
 template <int D, bool BVH, class WK>
-__device__ __forceinline__ Hit query(const SceneView &S, const float *p, const float4 *top, int n_top, WK &wk) {
-    if (BVH) return nearest_bvh<D>(S, p, top, n_top, &g_status, wk);
+__device__ __forceinline__ Hit query(const SceneView &S, const float *p, WK &wk) {
+    if (BVH) return nearest_bvh<D>(S, p, &g_status, wk);
     return nearest_brute<D>(S, p, wk);
 }
 
@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(256) k_walk_plain(SceneView S, WalkCfg c, cons
     Work work{0, 0, 0};
     float v = 0.0f;
     for (bool first = true;; first = false) {
-        const Hit hit = query<D, BVH>(S, w.p, nullptr, 0, work);
+        const Hit hit = query<D, BVH>(S, w.p, work);
         if (first && !walk_enters<D>(w, S, hit, c)) break;
         const int r = walker_advance<D>(w, S, hit, c, c.eps, c.project != 0, c.prevent_fd != 0, pt, wk, ROLE_PRIMAL,
                                         false, S.guide);
@@ -558,8 +558,8 @@ constexpr int QUERY_THREADS = 128;
 // When a warp's lanes have no further points and this many are still searching,
 // after SHARE_STEPS more steps, its other lanes take part in their searches: most
 // searches are shorter and done sooner alone.  (200,003 points on 20,480 triangles,
-// closest points and signed distances: 0.70 ms without, 0.71 with 8 lanes and 32 steps,
-// 0.73 with 8 and 8, 0.74 with 16 and 16, 0.69 with 16 and 64.)
+// closest points and signed distances, take 0.69 ms with and without; with 8 lanes and 8
+// steps, or 16 and 16, 5 % more.)
 constexpr int SHARE_LANES = 16, SHARE_STEPS = 64;
 template <int D, bool BVH>
 __global__ void __launch_bounds__(QUERY_THREADS) k_closest(SceneView S, const float *__restrict__ P, int n,

@@ -34,8 +34,9 @@ enum StatusBits : int {
 //   2D: node[3k] = (L.lo, L.hi), node[3k+1] = (R.lo, R.hi), node[3k+2].xy = refs
 //   3D: node[4k..4k+2] = (L.lo.xyz, L.hi.xyz, R.lo.xyz, R.hi.xyz) packed,
 //       node[4k+3].xy = refs
-// A reference r >= 0 is an internal node, r < 0 is leaf ~r in Morton order;
-// leaf data is copied into Morton order (lseg/lseginv/ltri) with the original
+// A reference r >= 0 is an internal node, r < 0 is leaf ~r in the order of the
+// tree's sort keys (meshes: Hilbert, polylines: Morton or, where chained, the input's);
+// leaf data is copied into that order (lseg/lseginv/ltri) with the original
 // primitive index in lorig.
 struct SceneView {
     int dim, nV, nF;
@@ -66,8 +67,9 @@ struct SceneView {
     int n_guide;
     // Search tree of the walk kernels: an implicit 4-ary tree over the
     // primitives in an order of its own (torig: position -> original index).
-    // Leaf i holds the primitives at positions [LEAF i, LEAF i + LEAF); the root is at depth 0, the leaves at depth tree_depth,
-    // and node i of depth d has the children [4 i, 4 i + 4) of depth d + 1.
+    // Leaf i holds the primitives at positions [LEAF i, LEAF i + LEAF); the root is at
+    // depth 0, the leaves at depth tree_depth, and node i of depth d has the children
+    // [4 i, 4 i + 4) of depth d + 1.
     // Every node is bounded by an oriented box (k_tree_bounds): orthonormal axes
     // u_k, a centre c and half-extents e_k with |u_k.(y - c)| <= e_k for every
     // point y of its primitives.  A node's four child boxes are one block of
@@ -251,7 +253,7 @@ __device__ __forceinline__ float tri_closest(float4 t0, float4 t1, float4 t2, fl
     return dot3(dx, dy, dz, dx, dy, dz);
 }
 
-// Squared distance to a triangle for warp-wide leaf tests: a branch-free
+// Squared distance to a triangle for the search tree's leaves: a branch-free
 // form of tri_closest's region cascade.  Every region test is evaluated with
 // the cascade's own expressions, the first region that holds
 // picks the result, and the one division the edge and face regions need is
@@ -259,7 +261,7 @@ __device__ __forceinline__ float tri_closest(float4 t0, float4 t1, float4 t2, fl
 // same IEEE operation on the same operands as in the cascade, so the results
 // are identical to tri_closest's, but the lanes of a warp testing different
 // triangles do not diverge (and run one division instead of up to four in
-// turn).  Per-thread searches keep the cascade, which skips work per lane.
+// turn).  Brute force and the LBVH keep the cascade, which skips work per lane.
 __device__ __forceinline__ float tri_d2_uniform(float4 t0, float4 t1, float4 t2, float x, float y, float z) {
     const float axx = x - t0.x, axy = y - t0.y, axz = z - t0.z;
     const float ab2 = t0.w, abac = t1.w, ac2 = t2.w;
@@ -442,11 +444,9 @@ __device__ __forceinline__ void load_node(const float4 *base, int k, float (*lo)
 #endif
 
 // LBVH nearest: nearest-first descent with a per-thread stack, conservative
-// pruning, ties to the lowest original index.  The first n_top nodes (the
-// shallowest, breadth-first) are read from shared memory.
+// pruning, ties to the lowest original index.
 template <int D, class WK>
-__device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, const float4 *top, int n_top,
-                                           int *status, WK &wk) {
+__device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, int *status, WK &wk) {
     Hit h{-1, INFINITY};
     wk.nq += 1;
     if (S.nF == 1) {
@@ -466,7 +466,6 @@ __device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, c
     int sp = 1;
     stn[0] = 0;
     std2[0] = 0.0f;
-    int best_leaf = -1;
     while (sp > 0) {
         --sp;
         const int v = stn[sp];
@@ -474,10 +473,7 @@ __device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, c
         wk.nb += 1;
         float lo[2][3], hi[2][3];
         int ch[2];
-        if (v < n_top)
-            load_node<D>(top, v, lo, hi, ch[0], ch[1]);
-        else
-            load_node<D>(S.node, v, lo, hi, ch[0], ch[1]);
+        load_node<D>(S.node, v, lo, hi, ch[0], ch[1]);
         float bd[2];
         bd[0] = box_d2<D>(lo[0], hi[0], p);
         bd[1] = box_d2<D>(lo[1], hi[1], p);
@@ -504,7 +500,6 @@ __device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, c
                     if (d2 < h.d2 || orig < h.prim) {
                         h.d2 = d2;
                         h.prim = orig;
-                        best_leaf = leaf;
                     }
                 }
             }
@@ -528,7 +523,6 @@ __device__ __forceinline__ Hit nearest_bvh(const SceneView &S, const float *p, c
             }
         }
     }
-    (void)best_leaf;
     return h;
 }
 
@@ -960,8 +954,8 @@ __device__ __forceinline__ void search_run(Search<D> &s, const SceneView *scenes
 //
 // What it is for: a query at about the same distance from much of a mesh visits
 // thousands of nodes one after the other, long after its warp's others are done.
-// 10,007 points on a mesh of 81,920 triangles, which it has just been moved to: 0.83
-// -> 0.69 ms with the rebuild.
+// 10,007 points on a mesh of 81,920 triangles, which it has just been moved to: 0.76
+// -> 0.67 ms with the rebuild.
 template <int D, bool GATHER, class WK>
 __device__ __forceinline__ void search_share(Search<D> &s, const SceneView &S, const float *p, int owner,
                                              unsigned *stack, WK &wk) {

@@ -523,11 +523,13 @@ typedef struct wos_launch_config {
 } wos_launch_config;
 
 /* Work accounting: while enabled, the persistent walk and adjoint kernels add
- * their nearest-query totals to a device counter {queries, LBVH node visits,
- * primitive distance evaluations} (brute force: nF evaluations per query).
- * wos_work_counters reads it (synchronising the device); reset != 0 clears.
- * While enabled those kernels run an instance compiled with counters; the default instances carry none, which saves 1-3 % of a
- * step.  Results are the same either way. */
+ * their nearest-query totals to a device counter {queries, node steps, leaf
+ * steps}, steps of single lanes in the search tree (brute force: nF primitive
+ * distances per query instead of leaf steps).  wos_work_counters reads it
+ * (synchronising the device); reset != 0 clears.  While enabled those kernels run
+ * an instance compiled with counters, which does not share a warp's last searches;
+ * the default instances carry none, which saves 1-3 % of a step.  Results are the
+ * same either way. */
 WOS_API int wos_set_work_counting(int enable);
 WOS_API int wos_work_counters(int reset, int64_t *out);
 
